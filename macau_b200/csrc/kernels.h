@@ -35,6 +35,9 @@ void launch_pad(const long long* ptr, const long long* pptr, long long nrows, co
 // default shape).
 void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStream_t s,
                    int num_sms, int groups = 0);
+// Its FP64 form for KP <= 32, a warp per row with the Grams on the FP64 matrix instruction
+// (sample_mma.cu); groups = 2 or 4 (default) warps per CTA.
+void launch_sample_f64(const SampleParams& p, int KP, cudaStream_t s, int num_sms, int groups);
 // The default CTA shape of the CUDA-core sampler at KP, and the shapes the autotuner may pick
 // from (the default first).
 int sample_default_groups(int KP);

@@ -584,14 +584,8 @@ void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStre
   } else {
     switch (KP) {
       case 8:
-        if (groups == 2) return launch_t<8, 1, 2, false>(p, s, num_sms);
-        return launch_t<8, 1, 4, false>(p, s, num_sms);
       case 16:
-        if (groups == 2) return launch_t<16, 1, 2, false>(p, s, num_sms);
-        return launch_t<16, 1, 4, false>(p, s, num_sms);
-      case 32:
-        if (groups == 2) return launch_t<32, 1, 2, false>(p, s, num_sms);
-        return launch_t<32, 1, 4, false>(p, s, num_sms);
+      case 32: return launch_sample_f64(p, KP, s, num_sms, groups);
       case 64:
         if (groups == 1) return launch_t<64, 4, 1, false>(p, s, num_sms);
         return launch_t<64, 4, 2, false>(p, s, num_sms);
