@@ -345,7 +345,7 @@ int mg_blockcg(const int32_t* rows, const int32_t* cols, const double* vals, int
  *   seed, sweep, mode  key of the Wishart / mean draws (same keys as mg_update_prior)
  *   mu_out, Lambda_out device outputs (K and K x K); stream: cudaStream_t (NULL = default)
  *   err / errlen optional caller buffer for a message (NULL allowed)
- * Its scratch is one fixed 2.3 MB array in the library (every GPU that loads the library holds
+ * Its scratch is one fixed 2.1 MB array in the library (every GPU that loads the library holds
  * it until exit), so K is limited to 64; larger K, nu < K or kappa <= 0 return MG_ERR_ARG.  All
  * calls share that array and it keeps the last call's contents: calls whose kernels overlap on
  * the GPU race.  The first call in a device's CUDA context looks the array's address up.

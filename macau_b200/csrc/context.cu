@@ -459,12 +459,6 @@ class Context {
       stat_partials1_.alloc((size_t)stats_blocks(dims_[1]) * (K_ + K_ * K_));
       stat_final1_.alloc((size_t)(K_ + K_ * K_));
     }
-    nwbuf_.alloc(3 * (size_t)K_ + 4 * (size_t)K_ * K_);
-    nw_.vec = nwbuf_.p;
-    nw_.m0 = nwbuf_.p + 3 * K_;
-    nw_.m1 = nw_.m0 + K_ * K_;
-    nw_.m2 = nw_.m1 + K_ * K_;
-    nw_.m3 = nw_.m2 + K_ * K_;
     if (ntest_ > 0) {
       MG_CUDA(cudaMemsetAsync(pred_.p, 0, ntest_ * sizeof(double), s_));
       MG_CUDA(cudaMemsetAsync(pvar_.p, 0, ntest_ * sizeof(double), s_));
@@ -681,11 +675,11 @@ class Context {
     return mixed_ ? (const void*)lat32_[mode].p : (const void*)lat64_[mode].p;
   }
 
-  // Both modes have the plain BPMF prior at K <= 32: the sweep updates them together
+  // Both modes have the plain BPMF prior: the sweep updates them together
   // (launch_prior_pair: three launches instead of six, the same result bit for bit).  The
   // phase-timed sweeps keep one mode after the other, so each mode's prior is timed alone.
   bool pair_priors() const {
-    return K_ <= 32 && !prior_[0].macau && !prior_[0].one && !prior_[1].macau && !prior_[1].one;
+    return !prior_[0].macau && !prior_[0].one && !prior_[1].macau && !prior_[1].one;
   }
   void update_priors_pair() {
     PriorPair pp{};
@@ -722,7 +716,7 @@ class Context {
       // of U - Uhat with mu0 = 0, kappa = 2, W0 = I, nu = K, the BPMF defaults), sample_beta,
       // compute_uhat, sample_lambda_beta
       launch_normal_wishart(stat_final_.p, 1, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr, 0,
-                            nullptr, nw_, ctl_.p, cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
+                            nullptr, ctl_.p, cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
       launch_beta_one(p.Ft, p.colsq.p, p.lvl_ptr.p, p.lvl_feat.p, p.lvl_range.p, p.lvl_warp.p,
                       p.nlevels,
                       latents(mode),
@@ -736,7 +730,7 @@ class Context {
     }
     if (!p.macau) {  // BPMFPrior::update_prior (latentprior.cpp:79-81)
       launch_normal_wishart(stat_final_.p, 1, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr, 0,
-                            nullptr, nw_, ctl_.p, cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
+                            nullptr, ctl_.p, cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
       return;
     }
     // MacauPrior::update_prior (latentprior.cpp:255-264)
@@ -744,7 +738,7 @@ class Context {
     launch_stats(p.beta.p, false, nullptr, p.nfeat, K_, CP_, 0, p.bb_partials.p, nbb, s_);
     launch_reduce_parts(p.bb_partials.p, nbb, rec, p.bb_final.p, s_);
     launch_normal_wishart(stat_final_.p, 1, N, K_, p.mu0.p, p.b0, p.WI.p, p.df + (int)p.nfeat,
-                          p.bb_final.p, 1, p.lambda_beta.p, nw_, ctl_.p, cfg_.seed, mode, p.mu.p,
+                          p.bb_final.p, 1, p.lambda_beta.p, ctl_.p, cfg_.seed, mode, p.mu.p,
                           p.Lambda.p, s_);
     // sample_beta (latentprior.cpp:273-293)
     launch_small_chol(p.Lambda.p, K_, p.Lchol.p, ctl_.p, s_);
@@ -1463,10 +1457,9 @@ class Context {
   DBuf<double> lat64_[2];
   DBuf<float> lat32_[2];
   DBuf<__nv_bfloat16> lat16_[2];
-  DBuf<double> scratch_, stat_partials_, stat_final_, nwbuf_;
+  DBuf<double> scratch_, stat_partials_, stat_final_;
   DBuf<double> stat_partials1_, stat_final1_;  // mode 1's work of update_priors_pair
   DBuf<double> retry_work_;  // the fused tensor-core sampler's FP64-redo work areas
-  NwWork nw_{};
   DBuf<Ctl> ctl_;
   DBuf<int> trow_, tcol_;
   DBuf<double> tval_, pred_, pvar_, eval_partials_, rmse_;

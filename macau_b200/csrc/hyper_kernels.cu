@@ -1,15 +1,14 @@
 // Normal-Wishart hyperprior update and test-set evaluation.
 //
-//   k_stats           per-block partial sums of x and x x^T over the rows of a latent matrix
-//                     (optionally x = U - Uhat, the Macau residual of latentprior.cpp:257);
-//                     FP64 accumulation from FP64 or FP32 latents.
-//   k_stats32         the same for K <= 32 with 4 x 4 register tiles of the outer product (four
-//                     row groups per block, summed in group order at the end).
-//   k_nw32            k_normal_wishart for K <= 32: shared-memory matrices, warp-register
-//                     Cholesky factors (warp_finish.cuh) and a warp-parallel triangular inverse.
-//   k_normal_wishart  one CTA: reduces the partials in block order (deterministic), then
-//                     CondNormalWishart -> NormalWishart -> Wishart/WishartUnit -> MvNormal_prec
-//                     (mvnormal.cpp:169-184, 217-287, 314-336) in FP64 with keyed draws.
+//   k_stats32         per-block partial sums of x and x x^T over the rows of a latent matrix, K <=
+//                     32 (optionally x = U - Uhat, the Macau residual of latentprior.cpp:257);
+//                     FP64 accumulation from FP64 or FP32 latents, 4 x 4 register tiles of the
+//                     outer product (four row groups per block, summed in group order).
+//   k_nw32            one CTA, K <= 32: CondNormalWishart -> NormalWishart -> Wishart/WishartUnit
+//                     -> MvNormal_prec (mvnormal.cpp:169-184, 217-287, 314-336) in FP64 with keyed
+//                     draws; shared-memory matrices, warp-register Cholesky factors
+//                     (warp_finish.cuh) and a warp-parallel triangular inverse.
+//   (K > 32: hyper_wide.cu)
 //   k_lambda_beta     one CTA: posterior_lambda_beta + rgamma (latentprior.cpp:317-331).
 //   k_eval / k_eval_finish  eval_rmse (bpmfutils.h:86-114): online posterior mean / variance of
 //                     the test predictions and the two RMSEs.
@@ -23,211 +22,6 @@ namespace {
 
 constexpr int kStatThreads = 256;
 constexpr int kStatRows = 32;  // rows staged per step
-
-template <typename T, int PER>
-__global__ void __launch_bounds__(kStatThreads)
-    k_stats(const T* __restrict__ U, const double* __restrict__ Uhat, long long N, int K,
-            int stride, int uhat_stride, long long rows_per_block, double* __restrict__ partials) {
-  __shared__ double xs[kStatRows * 128];
-  const int KK = K * K;
-  const long long r0 = (long long)blockIdx.x * rows_per_block;
-  const long long r1 = min(N, r0 + rows_per_block);
-  double acc[PER];
-  int ii[PER], jj[PER];
-#pragma unroll
-  for (int q = 0; q < PER; q++) {
-    acc[q] = 0.0;
-    const int e = threadIdx.x + q * kStatThreads;
-    ii[q] = e < KK ? e % K : 0;
-    jj[q] = e < KK ? e / K : 0;
-  }
-  double su = 0.0;
-  for (long long b = r0; b < r1; b += kStatRows) {
-    const int cnt = (int)min((long long)kStatRows, r1 - b);
-    __syncthreads();
-    for (int e = threadIdx.x; e < cnt * K; e += kStatThreads) {
-      const int r = e / K, k = e % K;
-      double x = (double)U[(b + r) * stride + k];
-      if (Uhat) x -= Uhat[(b + r) * uhat_stride + k];
-      xs[r * K + k] = x;
-    }
-    __syncthreads();
-    if (threadIdx.x < K)
-      for (int r = 0; r < cnt; r++) su += xs[r * K + threadIdx.x];
-#pragma unroll
-    for (int q = 0; q < PER; q++) {
-      double s = acc[q];
-      for (int r = 0; r < cnt; r++) s += xs[r * K + ii[q]] * xs[r * K + jj[q]];
-      acc[q] = s;
-    }
-  }
-  double* out = partials + (size_t)blockIdx.x * (K + KK);
-  if (threadIdx.x < K) out[threadIdx.x] = su;
-#pragma unroll
-  for (int q = 0; q < PER; q++) {
-    const int e = threadIdx.x + q * kStatThreads;
-    if (e < KK) out[K + e] = acc[q];
-  }
-}
-
-// In-place left-looking lower Cholesky of the K x K column-major matrix A by one CTA (thread i
-// computes L(i, j)); the strict upper triangle is zeroed.  Returns false on a non-positive pivot
-// (same value in every thread).
-__device__ bool cta_chol(double* A, int K, bool* flag) {
-  (void)flag;
-  __syncthreads();
-  for (int j = 0; j < K; j++) {
-    double d = A[j + j * K];
-    for (int p = 0; p < j; p++) d -= A[j + p * K] * A[j + p * K];
-    if (!(d > 0.0)) {
-      __syncthreads();
-      return false;
-    }
-    const double ljj = sqrt(d);
-    for (int i = j + 1 + threadIdx.x; i < K; i += blockDim.x) {
-      double s = A[i + j * K];
-      for (int p = 0; p < j; p++) s -= A[i + p * K] * A[j + p * K];
-      A[i + j * K] = s / ljj;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) A[j + j * K] = ljj;
-    __syncthreads();
-  }
-  for (int q = threadIdx.x; q < K * K; q += blockDim.x) {
-    const int i = q % K, k = q / K;
-    if (i < k) A[i + k * K] = 0.0;
-  }
-  __syncthreads();
-  return true;
-}
-
-// x <- L^{-1} x then L^{-T} x for one column, sequential in the calling thread.
-__device__ void col_solve_llt(const double* L, double* x, int K, int xs) {
-  for (int i = 0; i < K; i++) {
-    double s = x[i * xs];
-    for (int p = 0; p < i; p++) s -= L[i + p * K] * x[p * xs];
-    x[i * xs] = s / L[i + i * K];
-  }
-  for (int i = K - 1; i >= 0; i--) {
-    double s = x[i * xs];
-    for (int p = i + 1; p < K; p++) s -= L[p + i * K] * x[p * xs];
-    x[i * xs] = s / L[i + i * K];
-  }
-}
-
-__global__ void __launch_bounds__(256)
-    k_normal_wishart(const double* __restrict__ partials, int nparts, long long N, int K,
-                     const double* __restrict__ mu0, double kappa, const double* __restrict__ T0,
-                     int nu, const double* __restrict__ bb_partials, int bb_nparts,
-                     const double* __restrict__ lambda_beta, NwWork w, Ctl* ctl,
-                     unsigned long long seed, int mode, double* __restrict__ mu_out,
-                     double* __restrict__ Lambda_out) {
-  const int KK = K * K;
-  const uint32_t sweep = ctl->sweep;
-  double* NU = w.vec;          // K
-  double* muc = w.vec + K;     // K
-  double* z = w.vec + 2 * K;   // K
-  double* X = w.m0;            // K x K
-  double* Tc = w.m1;
-  double* cB = w.m2;           // Bartlett factor (upper)
-  double* W = w.m3;
-  // 1. reduce partials in block order
-  for (int e = threadIdx.x; e < K + KK; e += blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < nparts; b++) s += partials[(size_t)b * (K + KK) + e];
-    if (e < K) NU[e] = s;
-    else X[e - K] = s;
-  }
-  if (bb_partials) {  // T = WI + lambda_beta * beta beta^T  (latentprior.cpp:258-260)
-    const double lb = *lambda_beta;
-    for (int e = threadIdx.x; e < KK; e += blockDim.x) {
-      double s = 0.0;
-      for (int b = 0; b < bb_nparts; b++) s += bb_partials[(size_t)b * (K + KK) + K + e];
-      W[e] = T0[e] + lb * s;
-    }
-  } else {
-    for (int e = threadIdx.x; e < KK; e += blockDim.x) W[e] = T0[e];
-  }
-  __syncthreads();
-  const double kappa_c = kappa + (double)N;
-  const int nu_c = nu + (int)N;
-  for (int i = threadIdx.x; i < K; i += blockDim.x) muc[i] = (kappa * mu0[i] + NU[i]) / kappa_c;
-  __syncthreads();
-  // 2. X = T + NS + kappa mu0 mu0^T - kappa_c mu_c mu_c^T
-  for (int e = threadIdx.x; e < KK; e += blockDim.x) {
-    const int i = e % K, j = e / K;
-    X[e] = W[e] + X[e] + kappa * mu0[i] * mu0[j] - kappa_c * muc[i] * muc[j];
-  }
-  // 3. T_c = X^{-1} through the Cholesky factor of X
-  bool ok = cta_chol(X, K, nullptr);
-  if (!ok) {
-    if (threadIdx.x == 0) atomicOr(&ctl->status, kStatHyperFail);
-    return;
-  }
-  for (int c = threadIdx.x; c < K; c += blockDim.x) {
-    for (int i = 0; i < K; i++) Tc[i + c * K] = (i == c) ? 1.0 : 0.0;
-    col_solve_llt(X, Tc + c * K, K, 1);
-  }
-  // 4. L = chol(T_c)
-  ok = cta_chol(Tc, K, nullptr);
-  if (!ok) {
-    if (threadIdx.x == 0) atomicOr(&ctl->status, kStatHyperFail);
-    return;
-  }
-  // 5. Bartlett factor c: c_ii = sqrt(2 Gamma((nu_c - i)/2)), c_ij ~ N(0,1) for j > i
-  for (int e = threadIdx.x; e < KK; e += blockDim.x) {
-    const int i = e % K, j = e / K;
-    double v = 0.0;
-    if (i == j)
-      v = sqrt(2.0 * gamma_draw(seed, sweep, stream_id(kWishartDiag, mode), (uint32_t)i,
-                                0.5 * (double)(nu_c - i)));
-    else if (j > i)
-      v = normal_draw(seed, sweep, stream_id(kWishartOff, mode), (uint32_t)i,
-                      (uint32_t)(j - i - 1));
-    cB[e] = v;
-  }
-  __syncthreads();
-  // 6. W = c^T c ; M = L W (into X) ; Lambda = M L^T
-  for (int e = threadIdx.x; e < KK; e += blockDim.x) {
-    const int i = e % K, j = e / K;
-    double s = 0.0;
-    for (int p = 0; p < K; p++) s += cB[p + i * K] * cB[p + j * K];
-    W[e] = s;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < KK; e += blockDim.x) {
-    const int i = e % K, j = e / K;
-    double s = 0.0;
-    for (int p = 0; p < K; p++) s += Tc[i + p * K] * W[p + j * K];
-    X[e] = s;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < KK; e += blockDim.x) {
-    const int i = e % K, j = e / K;
-    double s = 0.0;
-    for (int p = 0; p < K; p++) s += X[i + p * K] * Tc[j + p * K];
-    Lambda_out[e] = s;
-    cB[e] = s * kappa_c;
-  }
-  // 7. mu = mu_c + chol(kappa_c Lambda)^{-T} z
-  ok = cta_chol(cB, K, nullptr);
-  if (!ok) {
-    if (threadIdx.x == 0) atomicOr(&ctl->status, kStatHyperFail);
-    return;
-  }
-  for (int i = threadIdx.x; i < K; i += blockDim.x)
-    z[i] = normal_draw(seed, sweep, stream_id(kMuDraw, mode), 0u, (uint32_t)i);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = K - 1; i >= 0; i--) {
-      double s = z[i];
-      for (int p = i + 1; p < K; p++) s -= cB[p + i * K] * z[p];
-      z[i] = s / cB[i + i * K];
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < K; i += blockDim.x) mu_out[i] = z[i] + muc[i];
-}
 
 // lambda_beta ~ Gamma(nux/2, 2 mux/nux), nux = nu + K nfeat,
 // mux = mu nux / (nu + mu tr(B B^T Lambda))   (latentprior.cpp:317-331)
@@ -590,8 +384,7 @@ __global__ void __launch_bounds__(256)
 }
 
 // CondNormalWishart -> NormalWishart -> MvNormal_prec (mvnormal.cpp:169-184, 217-287, 314-336)
-// for K <= 32 in one CTA of 256 threads, matrices in shared memory (row-major, ld 33), same
-// draws as k_normal_wishart.  Two identities replace two of the reference's three Cholesky
+// for K <= 32 in one CTA of 256 threads, matrices in shared memory (row-major, ld 33).  Two identities replace two of the reference's three Cholesky
 // factorisations (results agree to FP64 rounding):
 //   * chol(X^{-1}) = J M^{-T} J with M = chol(J X J), J the index reversal: one Cholesky of the
 //     reversed X (warp 0's registers, warp_factor) and one triangular inverse Y = M^{-1}
@@ -758,7 +551,7 @@ __global__ void __launch_bounds__(256)
            seed, mode, mu_out, Lambda_out);
 }
 
-// ---- both modes' BPMF prior updates in one launch per step (K <= 32): blocks of mode 0, then
+// ---- both modes' BPMF prior updates in one launch per step: blocks of mode 0, then
 // of mode 1, each doing what the single-mode kernel's block does, so the results are the same
 // bit for bit; the two modes' steps only overlap ----
 template <typename T>
@@ -805,9 +598,10 @@ __global__ void __launch_bounds__(256) k_nw32_pair(PriorPair pp, int K, Ctl* ctl
 
 void launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl,
                        unsigned long long seed, cudaStream_t s) {
-  if (K > 32) throw MgError(MG_ERR_ARG, "the two-mode prior update needs K <= 32");
   const int nb = pp.nblocks[0] + pp.nblocks[1];
-  if (f32)
+  if (K > 32)
+    launch_stats_wide_pair(pp, f32, K, stride, s);
+  else if (f32)
     k_stats32_pair<float><<<nb, kStatThreads, 0, s>>>(pp, K, stride);
   else
     k_stats32_pair<double><<<nb, kStatThreads, 0, s>>>(pp, K, stride);
@@ -815,7 +609,8 @@ void launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ct
   const int len = K + K * K;
   k_reduce_parts_pair<<<2 * ((len + 31) / 32), 256, 0, s>>>(pp, len);
   MG_CUDA(cudaGetLastError());
-  k_nw32_pair<<<2, 256, 0, s>>>(pp, K, ctl, seed);
+  if (K > 32) launch_nw_wide_pair(pp, K, ctl, seed, s);
+  else k_nw32_pair<<<2, 256, 0, s>>>(pp, K, ctl, seed);
   MG_CUDA(cudaGetLastError());
 }
 
@@ -839,23 +634,7 @@ void launch_stats(const void* U, bool f32, const double* Uhat, long long N, int 
     MG_CUDA(cudaGetLastError());
     return;
   }
-  const int per = (K * K + kStatThreads - 1) / kStatThreads;
-#define MG_STATS(P)                                                                         \
-  if (per <= P) {                                                                           \
-    if (f32)                                                                                \
-      k_stats<float, P><<<nblocks, kStatThreads, 0, s>>>((const float*)U, Uhat, N, K, stride, \
-                                                         uhat_stride, rpb, partials);       \
-    else                                                                                    \
-      k_stats<double, P><<<nblocks, kStatThreads, 0, s>>>((const double*)U, Uhat, N, K,     \
-                                                          stride, uhat_stride, rpb, partials); \
-    MG_CUDA(cudaGetLastError());                                                            \
-    return;                                                                                 \
-  }
-  MG_STATS(1)
-  MG_STATS(4)
-  MG_STATS(16)
-  MG_STATS(64)
-#undef MG_STATS
+  launch_stats_wide(U, f32, Uhat, N, K, stride, uhat_stride, partials, nblocks, s);
 }
 
 // ---- batched problems (batch.cu): one statistics block and one Normal-Wishart block per
@@ -911,15 +690,17 @@ void launch_reduce_parts(const double* parts, int nparts, int len, double* out, 
 void launch_normal_wishart(const double* partials, int nparts, long long N, int K,
                            const double* mu0, double kappa, const double* T0, int nu,
                            const double* bb_partials, int bb_nparts, const double* lambda_beta,
-                           const NwWork& w, Ctl* ctl, unsigned long long seed, int mode,
-                           double* mu_out, double* Lambda_out, cudaStream_t s) {
-  if (K <= 32)
-    k_nw32<<<1, 256, 0, s>>>(partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials, bb_nparts,
-                             lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
-  else
-    k_normal_wishart<<<1, 256, 0, s>>>(partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials,
-                                       bb_nparts, lambda_beta, w, ctl, seed, mode, mu_out,
-                                       Lambda_out);
+                           Ctl* ctl, unsigned long long seed, int mode, double* mu_out,
+                           double* Lambda_out, cudaStream_t s) {
+  if (K > 32) {  // the wide kernel reads reduced statistics
+    if (nparts != 1 || (bb_partials && bb_nparts != 1))
+      throw MgError(MG_ERR_STATE, "Normal-Wishart update of unreduced statistics at K > 32");
+    launch_nw_wide(partials, N, K, mu0, kappa, T0, nu, bb_partials, lambda_beta, ctl, seed, mode,
+                   mu_out, Lambda_out, s);
+    return;
+  }
+  k_nw32<<<1, 256, 0, s>>>(partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials, bb_nparts,
+                           lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
   MG_CUDA(cudaGetLastError());
 }
 

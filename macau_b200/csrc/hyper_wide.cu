@@ -1,0 +1,412 @@
+// Normal-Wishart hyperprior update for 32 < K <= 128, FP64 on the matrix instruction m8n8k4.f64.
+//
+//   k_stats_wide  per-block partial sums of x and x x^T over the rows of a latent matrix (x = U, or
+//                 U - Uhat): the lower-triangle tiles spread over the block's warps as in the row
+//                 sampler, rows read straight into fragments.
+//   k_nw_wide     one block per update: CondNormalWishart -> NormalWishart -> Wishart ->
+//                 MvNormal_prec (mvnormal.cpp:169-184, 217-287, 314-336), all matrices in shared
+//                 memory as 8 x 8 tiles of their lower triangles.
+//
+// What bounds k_nw_wide: the chain of the panel factor, about 1,900 cycles per 8 columns; the
+// triangular inverse and the three products that follow are matrix instructions on 16 warps.  The
+// version this replaces kept the matrices in global memory and gave one thread a dot product (or a
+// whole substitution) at a time: 4.28 ms at K = 128 and 0.81 ms at K = 64.
+#include "common.cuh"
+#include "kernels.h"
+#include "rng.cuh"
+#include "wide_tiles.cuh"
+
+namespace mg {
+namespace {
+
+template <int KP>
+struct StatW {
+  static constexpr int W = KP == 64 ? 4 : 8, T = 32 * W;
+  static constexpr int RB = KP == 64 ? 2 : 4, ND = KP == 64 ? 1 : 2;
+};
+
+// What a launch updates: one mode, or both (block rows of mode 0, then of mode 1).
+struct StatsArgs {
+  const void* U[2];
+  const double* Uhat;  // one mode only
+  long long N[2], rows_per_block[2];
+  int nblocks[2];
+  double* partials[2];
+};
+
+// A warp's tiles over rows r0 .. r1 - 1.  DIAG: also the column sums of its blocks.
+template <typename V, int KP, bool DIAG>
+__device__ __forceinline__ void stats_warp(const V* __restrict__ U, const double* __restrict__ Uhat,
+                                           long long r0, long long r1, int K, int stride,
+                                           int uhat_stride, int br, int bc,
+                                           double* __restrict__ out) {
+  using C = StatW<KP>;
+  constexpr int NR = DIAG ? 4 * C::ND : C::RB, NC = DIAG ? 0 : 4;
+  constexpr int NT = DIAG ? 10 * C::ND : 4 * C::RB;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double acc[NT][2], racc[NR], f[2][NR + NC];
+#pragma unroll
+  for (int q = 0; q < NT; q++) acc[q][0] = acc[q][1] = 0.0;
+#pragma unroll
+  for (int b = 0; b < NR; b++) racc[b] = 0.0;
+  auto load = [&](int stage, long long row) {
+#pragma unroll
+    for (int b = 0; b < NR + NC; b++) {
+      const int k = 8 * (b < NR ? br + b : bc + b - NR) + g;
+      double x = 0.0;
+      if (row < r1 && k < K) {
+        x = (double)U[row * stride + k];
+        if (Uhat) x -= Uhat[row * uhat_stride + k];
+      }
+      f[stage][b] = x;
+    }
+  };
+  load(0, r0 + t);
+  for (long long r = r0; r < r1; r += 8) {
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      load(1 - u, r + 4 * (u + 1) + t);
+      int q = 0;
+      if constexpr (DIAG) {
+#pragma unroll
+        for (int s = 0; s < C::ND; s++)
+#pragma unroll
+          for (int a = 0; a < 4; a++) {
+            racc[4 * s + a] += f[u][4 * s + a];
+#pragma unroll
+            for (int b = 0; b <= a; b++) {
+              mma_f64(acc[q][0], acc[q][1], f[u][4 * s + a], f[u][4 * s + b]);
+              q++;
+            }
+          }
+      } else {
+#pragma unroll
+        for (int a = 0; a < NR; a++)
+#pragma unroll
+          for (int b = 0; b < NC; b++) {
+            mma_f64(acc[q][0], acc[q][1], f[u][a], f[u][NR + b]);
+            q++;
+          }
+      }
+    }
+  }
+  auto put = [&](int bi, int bj, const double (&v)[2]) {
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int i = 8 * bi + g, j = 8 * bj + 2 * t + e;
+      if (i < K && j < K) {
+        out[K + i + (size_t)j * K] = v[e];
+        if (bi != bj) out[K + j + (size_t)i * K] = v[e];
+      }
+    }
+  };
+  int q = 0;
+  if constexpr (DIAG) {
+#pragma unroll
+    for (int b = 0; b < NR; b++) {
+      double s = racc[b];
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      if (t == 0 && 8 * (br + b) + g < K) out[8 * (br + b) + g] = s;
+    }
+#pragma unroll
+    for (int s = 0; s < C::ND; s++)
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b <= a; b++) put(br + 4 * s + a, br + 4 * s + b, acc[q++]);
+  } else {
+#pragma unroll
+    for (int a = 0; a < NR; a++)
+#pragma unroll
+      for (int b = 0; b < NC; b++) put(br + a, bc + b, acc[q++]);
+  }
+}
+
+template <typename V, int KP>
+__global__ void __launch_bounds__(StatW<KP>::T)
+    k_stats_wide(const StatsArgs p, int K, int stride, int uhat_stride) {
+  const int m = (int)blockIdx.x < p.nblocks[0] ? 0 : 1;
+  const int b = (int)blockIdx.x - (m ? p.nblocks[0] : 0);
+  const long long r0 = b * p.rows_per_block[m], r1 = min(p.N[m], r0 + p.rows_per_block[m]);
+  const V* U = static_cast<const V*>(p.U[m]);
+  double* out = p.partials[m] + (size_t)b * (K + (size_t)K * K);
+  const Part64 part = part_of<KP>(threadIdx.x >> 5);
+  if (part.diag)
+    stats_warp<V, KP, true>(U, p.Uhat, r0, r1, K, stride, uhat_stride, part.r0, 0, out);
+  else
+    stats_warp<V, KP, false>(U, p.Uhat, r0, r1, K, stride, uhat_stride, part.r0, part.c0, out);
+}
+
+template <typename V>
+void stats_launch(const StatsArgs& a, int K, int stride, int uhat_stride, cudaStream_t s) {
+  const int nb = a.nblocks[0] + a.nblocks[1];
+  if (K <= 64)
+    k_stats_wide<V, 64><<<nb, StatW<64>::T, 0, s>>>(a, K, stride, uhat_stride);
+  else
+    k_stats_wide<V, 128><<<nb, StatW<128>::T, 0, s>>>(a, K, stride, uhat_stride);
+  MG_CUDA(cudaGetLastError());
+}
+
+// ---- the Normal-Wishart draw ----
+struct NwArgs {
+  const double* stats;  // sums (K), then x x^T (K x K)
+  const double* bb;     // beta beta^T statistics of a Macau prior (same layout), or null
+  const double* lambda_beta;
+  const double* mu0;
+  const double* T0;
+  double kappa;
+  long long N;
+  int nu, mode;
+  double *mu, *Lambda;
+};
+struct NwPair {
+  NwArgs m[2];
+};
+
+constexpr int kNwThreads = 512, kNwHalf = 256;  // warps 0-7: factor, solve; warps 8-15: draws, Lambda
+
+template <int KP>
+struct NwW {
+  static constexpr int NB = KP / 8, TRI = NB * (NB + 1) / 2;
+  // M, then B | Y = M^-1 | the Bartlett factor's transpose | mu_c, y, x, 1 / diagonal, zeros, z |
+  // flag | tile table
+  static constexpr size_t kDoubles = 3 * (size_t)TRI * 64 + 6 * KP + 2 + (TRI + 7) / 8;
+};
+
+// Draws of the Bartlett factor c (upper triangular: c_ii = sqrt(2 Gamma((nu_c - i) / 2)), c_ij ~
+// N(0, 1) for j > i), stored as its transpose's lower-triangle tiles, the identity beyond K, and
+// the mean draw's z, by threads tid < nt.
+__device__ __forceinline__ void bartlett(double* Ct, double* z, int K, int n, int nu_c,
+                                         unsigned long long seed, uint32_t sweep, uint32_t mode,
+                                         int tid, int nt) {
+  for (int i = tid; i < K; i += nt) {
+    Ct[elem_at(i, i)] = sqrt(2.0 * gamma_draw(seed, sweep, stream_id(kWishartDiag, mode),
+                                              (uint32_t)i, 0.5 * (double)(nu_c - i)));
+    z[i] = normal_draw(seed, sweep, stream_id(kMuDraw, mode), 0u, (uint32_t)i);
+  }
+  const int warp = tid >> 5, lane = tid & 31;
+  for (int i = warp; i < K; i += nt >> 5)
+    for (int q = lane; 2 * q < K - 1 - i; q += 32) {
+      double z0, z1;
+      normal_pair(seed, sweep, stream_id(kWishartOff, mode), (uint32_t)i, (uint32_t)q, &z0, &z1);
+      Ct[elem_at(i + 1 + 2 * q, i)] = z0;
+      if (2 * q + 1 < K - 1 - i) Ct[elem_at(i + 2 + 2 * q, i)] = z1;
+    }
+  for (int i = K + tid; i < n; i += nt) {
+    for (int j = 0; j < i; j++) Ct[elem_at(i, j)] = 0.0;
+    Ct[elem_at(i, i)] = 1.0;
+    z[i] = 0.0;
+  }
+  for (int i = tid; i < n; i += nt)  // the diagonal tiles' upper parts are read too
+    for (int j = i + 1; j < (i | 7) + 1; j++) Ct[tile_at(i >> 3, i >> 3) + tile_pos(i & 7, j & 7)] = 0.0;
+}
+
+// The update in two identities of the row-reversed matrix (n = K rounded up to 8, the identity
+// before the reversed rows, so that both are whole tiles):
+//   chol(X^{-1}) = J M^{-T} J with M = chol(J X J), J the index reversal: L(i, j) = Y(n-1-j, n-1-i),
+//   Y = M^{-1};
+//   Lambda = L c^T c L^T = B B^T with B = L c^T lower triangular, so chol(kappa_c Lambda) =
+//   sqrt(kappa_c) B and mu = mu_c + B^{-T} z / sqrt(kappa_c).
+template <int KP>
+__global__ void __launch_bounds__(kNwThreads, 1)
+    k_nw_wide(const NwPair args, int K, Ctl* ctl, unsigned long long seed) {
+  using C = NwW<KP>;
+  extern __shared__ __align__(16) double nsm[];
+  const NwArgs& p = args.m[blockIdx.x];
+  double* M = nsm;
+  double* Y = M + (size_t)C::TRI * 64;
+  double* Ct = Y + (size_t)C::TRI * 64;
+  double* muc = Ct + (size_t)C::TRI * 64;
+  double *y = muc + KP, *x = y + KP, *rinv = x + KP, *zero = rinv + KP, *z = zero + KP;
+  volatile int* bad = reinterpret_cast<volatile int*>(z + KP);
+  unsigned char* tri = reinterpret_cast<unsigned char*>(z + KP + 2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int nb = (K + 7) / 8, n = 8 * nb, pad = n - K;
+  const uint32_t sweep = ctl->sweep;
+  const double kappa_c = p.kappa + (double)p.N;
+  const int nu_c = p.nu + (int)p.N;
+  if (tid == 0) *bad = 0;
+  for (int q = tid; q < C::TRI; q += kNwThreads) {
+    int a = 0;
+    while (q >= (a + 1) * (a + 2) / 2) a++;
+    tri[q] = (unsigned char)((a << 4) | (q - a * (a + 1) / 2));
+  }
+  for (int i = tid; i < n; i += kNwThreads) {
+    muc[i] = i < K ? (p.kappa * p.mu0[i] + p.stats[i]) / kappa_c : 0.0;
+    y[i] = zero[i] = 0.0;
+  }
+  __syncthreads();
+  // M = J (T + N S + kappa mu0 mu0^T - kappa_c mu_c mu_c^T) J
+  const double lb = p.bb ? *p.lambda_beta : 0.0;
+#pragma unroll 4
+  for (int e = tid; e < K * K; e += kNwThreads) {
+    const int i = e % K, j = e / K;
+    if (i > j) continue;
+    double T = p.T0[e];
+    if (p.bb) T += lb * p.bb[K + e];
+    M[elem_at(n - 1 - i, n - 1 - j)] = T + p.stats[K + e] + p.kappa * p.mu0[i] * p.mu0[j] -
+                                       kappa_c * muc[i] * muc[j];
+  }
+  for (int e = tid; e < pad * n; e += kNwThreads) {  // identity rows and columns before them
+    const int b = e % pad, a = e / pad;
+    if (a >= b) M[elem_at(a, b)] = a == b ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  if (warp < 8) {
+    wide_factor<double, KP, kNwHalf>(M, y, rinv, zero, nb, tri, 0.0, tid, 0, bad);
+  } else {
+    bartlett(Ct, z, K, n, nu_c, seed, sweep, (uint32_t)p.mode, tid - kNwHalf, kNwHalf);
+  }
+  __syncthreads();
+  if (*bad) {
+    if (tid == 0) atomicOr(&ctl->status, kStatHyperFail);
+    return;
+  }
+  // Y = M^{-1}.  Diagonal tiles: thread (block, column) solves its 8 x 8 column.
+  if (tid < n) {
+    const int b = tid >> 3, c = tid & 7;
+    const double* D = M + tile_at(b, b);
+    double v[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+      double s = r == c ? 1.0 : 0.0;
+#pragma unroll
+      for (int k = 0; k < r; k++) s = fma(-D[tile_pos(r, k)], v[k], s);
+      v[r] = r < c ? 0.0 : s * rinv[8 * b + r];
+    }
+#pragma unroll
+    for (int r = 0; r < 8; r++) Y[tile_at(b, b) + tile_pos(r, c)] = v[r];
+  }
+  __syncthreads();
+  // Below them: a warp per block column, Y(i, j) = -Y(i, i) sum_k M(i, k) Y(k, j)
+  for (int bj = warp; bj < nb; bj += kNwThreads / 32)
+    for (int bi = bj + 1; bi < nb; bi++) {
+      double s[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+      for (int k = bj; k < bi; k++) {
+        const double* A = M + tile_at(bi, k);
+        const double* B = Y + tile_at(k, bj);
+        mma_f64(s[0][0], s[0][1], A[tile_pos(g, t)], B[tile_pos(t, g)]);
+        mma_f64(s[1][0], s[1][1], A[tile_pos(g, t + 4)], B[tile_pos(t + 4, g)]);
+      }
+      double* out = Y + tile_at(bi, bj);
+      *reinterpret_cast<double2*>(out + tile_pos(g, 2 * t)) =
+          make_double2(s[0][0] + s[1][0], s[0][1] + s[1][1]);
+      __syncwarp();
+      const double* A = Y + tile_at(bi, bi);
+      const double b0 = out[tile_pos(t, g)], b1 = out[tile_pos(t + 4, g)];
+      double2 v = make_double2(0.0, 0.0);
+      __syncwarp();
+      mma_f64(v.x, v.y, -A[tile_pos(g, t)], b0);
+      mma_f64(v.x, v.y, -A[tile_pos(g, t + 4)], b1);
+      *reinterpret_cast<double2*>(out + tile_pos(g, 2 * t)) = v;
+      __syncwarp();
+    }
+  __syncthreads();
+  // B = L c^T over M, L(i, j) = Y(n-1-j, n-1-i)
+  for (int q = warp; q < nb * (nb + 1) / 2; q += kNwThreads / 32) {
+    const int bi = tri[q] >> 4, bj = tri[q] & 15;
+    double s[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    for (int k = bj; k <= bi; k++) {
+      const double* A = Y + tile_at(nb - 1 - k, nb - 1 - bi);
+      const double* B = Ct + tile_at(k, bj);
+      mma_f64(s[0][0], s[0][1], A[tile_pos(7 - t, 7 - g)], B[tile_pos(t, g)]);
+      mma_f64(s[1][0], s[1][1], A[tile_pos(3 - t, 7 - g)], B[tile_pos(t + 4, g)]);
+    }
+    *reinterpret_cast<double2*>(M + tile_at(bi, bj) + tile_pos(g, 2 * t)) =
+        make_double2(s[0][0] + s[1][0], s[0][1] + s[1][1]);
+  }
+  __syncthreads();
+  if (warp < 8) {
+    // mu = mu_c + B^{-T} z / sqrt(kappa_c)
+    if (tid < n) {
+      rinv[tid] = 1.0 / M[elem_at(tid, tid)];
+      y[tid] = z[tid] / sqrt(kappa_c);
+    }
+    group_sync<kNwHalf>(0);
+    wide_back<double, KP, kNwHalf>(M, y, rinv, x, nb, tid, 0);
+    if (tid < K) p.mu[tid] = x[tid] + muc[tid];
+  } else {
+    // Lambda = B B^T
+    for (int q = warp - 8; q < nb * (nb + 1) / 2; q += 8) {
+      const int bi = tri[q] >> 4, bj = tri[q] & 15;
+      double s[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+      for (int k = 0; k <= bj; k++) {
+        const double* A = M + tile_at(bi, k);
+        const double* B = M + tile_at(bj, k);
+        mma_f64(s[0][0], s[0][1], A[tile_pos(g, t)], B[tile_pos(g, t)]);
+        mma_f64(s[1][0], s[1][1], A[tile_pos(g, t + 4)], B[tile_pos(g, t + 4)]);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int i = 8 * bi + g, j = 8 * bj + 2 * t + e;
+        const double v = s[0][e] + s[1][e];
+        if (i < K && j < K) {
+          p.Lambda[i + (size_t)j * K] = v;
+          if (bi != bj) p.Lambda[j + (size_t)i * K] = v;
+        }
+      }
+    }
+  }
+}
+
+template <int KP>
+void nw_launch(const NwPair& a, int count, int K, Ctl* ctl, unsigned long long seed,
+               cudaStream_t s) {
+  constexpr size_t smem = sizeof(double) * NwW<KP>::kDoubles;
+  static_assert(smem <= 227 * 1024, "Normal-Wishart matrices exceed the shared memory of one CTA");
+  static bool configured[64] = {false};
+  int dev = 0;
+  MG_CUDA(cudaGetDevice(&dev));
+  if (!configured[dev & 63]) {
+    MG_CUDA(cudaFuncSetAttribute(k_nw_wide<KP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem));
+    configured[dev & 63] = true;
+  }
+  k_nw_wide<KP><<<count, kNwThreads, smem, s>>>(a, K, ctl, seed);
+  MG_CUDA(cudaGetLastError());
+}
+
+void nw_dispatch(const NwPair& a, int count, int K, Ctl* ctl, unsigned long long seed,
+                 cudaStream_t s) {
+  if (K <= 64) nw_launch<64>(a, count, K, ctl, seed, s);
+  else nw_launch<128>(a, count, K, ctl, seed, s);
+}
+
+}  // namespace
+
+void launch_stats_wide(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
+                       int uhat_stride, double* partials, int nblocks, cudaStream_t s) {
+  const StatsArgs a{{U, nullptr}, Uhat, {N, 0}, {(N + nblocks - 1) / nblocks, 0}, {nblocks, 0},
+                    {partials, nullptr}};
+  if (f32) stats_launch<float>(a, K, stride, uhat_stride, s);
+  else stats_launch<double>(a, K, stride, uhat_stride, s);
+}
+
+void launch_stats_wide_pair(const PriorPair& pp, bool f32, int K, int stride, cudaStream_t s) {
+  const StatsArgs a{{pp.U[0], pp.U[1]}, nullptr, {pp.N[0], pp.N[1]},
+                    {pp.rows_per_block[0], pp.rows_per_block[1]},
+                    {pp.nblocks[0], pp.nblocks[1]}, {pp.partials[0], pp.partials[1]}};
+  if (f32) stats_launch<float>(a, K, stride, 0, s);
+  else stats_launch<double>(a, K, stride, 0, s);
+}
+
+void launch_nw_wide(const double* stats, long long N, int K, const double* mu0, double kappa,
+                    const double* T0, int nu, const double* bb, const double* lambda_beta, Ctl* ctl,
+                    unsigned long long seed, int mode, double* mu, double* Lambda,
+                    cudaStream_t s) {
+  NwPair a{};
+  a.m[0] = NwArgs{stats, bb, lambda_beta, mu0, T0, kappa, N, nu, mode, mu, Lambda};
+  nw_dispatch(a, 1, K, ctl, seed, s);
+}
+
+void launch_nw_wide_pair(const PriorPair& pp, int K, Ctl* ctl, unsigned long long seed,
+                         cudaStream_t s) {
+  NwPair a{};
+  for (int m = 0; m < 2; m++)
+    a.m[m] = NwArgs{pp.final_[m], nullptr, nullptr, pp.mu0[m], pp.T0[m], pp.kappa[m], pp.N[m],
+                    pp.nu[m], m, pp.mu[m], pp.Lambda[m]};
+  nw_dispatch(a, 2, K, ctl, seed, s);
+}
+
+}  // namespace mg

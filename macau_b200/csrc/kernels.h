@@ -78,13 +78,6 @@ bool launch_gram_tc(const SampleParams& p, float* gram, const int4* split_rows, 
                     int KP, cudaStream_t s, int num_sms, cudaEvent_t mid = nullptr);
 
 // ---- hyperprior / eval (hyper_kernels.cu) ----
-struct NwWork {
-  double* vec;  // 3*K
-  double* m0;   // K*K each
-  double* m1;
-  double* m2;
-  double* m3;
-};
 int stats_blocks(long long N);
 // Sums `nparts` records of `len` doubles (stats partials) into one record, in a fixed order.
 void launch_reduce_parts(const double* parts, int nparts, int len, double* out, cudaStream_t s);
@@ -93,10 +86,10 @@ void launch_stats(const void* U, bool f32, const double* Uhat, long long N, int 
 void launch_normal_wishart(const double* partials, int nparts, long long N, int K,
                            const double* mu0, double kappa, const double* T0, int nu,
                            const double* bb_partials, int bb_nparts, const double* lambda_beta,
-                           const NwWork& w, Ctl* ctl, unsigned long long seed, int mode,
-                           double* mu_out, double* Lambda_out, cudaStream_t s);
-// Both modes' BPMF prior updates (BPMFPrior::update_prior, latentprior.cpp:79-81) at once, for
-// K <= 32: statistics, reduction and Normal-Wishart draw of mode m from the latents U[m]
+                           Ctl* ctl, unsigned long long seed, int mode, double* mu_out,
+                           double* Lambda_out, cudaStream_t s);
+// Both modes' BPMF prior updates (BPMFPrior::update_prior, latentprior.cpp:79-81) at once:
+// statistics, reduction and Normal-Wishart draw of mode m from the latents U[m]
 // (N[m] rows, stride `stride`), partials[m] (nblocks[m] records, rows_per_block[m] rows each)
 // and final_[m] as work, into mu[m] / Lambda[m].  Three launches instead of six; each mode's
 // blocks compute what launch_stats / launch_reduce_parts / launch_normal_wishart compute, with
@@ -117,6 +110,17 @@ struct PriorPair {
 };
 void launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl,
                        unsigned long long seed, cudaStream_t s);
+// The K > 32 forms of the statistics and of the draw (hyper_wide.cu); the draw reads one record
+// of reduced statistics (and of beta beta^T, null without side information).
+void launch_stats_wide(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
+                       int uhat_stride, double* partials, int nblocks, cudaStream_t s);
+void launch_stats_wide_pair(const PriorPair& pp, bool f32, int K, int stride, cudaStream_t s);
+void launch_nw_wide(const double* stats, long long N, int K, const double* mu0, double kappa,
+                    const double* T0, int nu, const double* bb, const double* lambda_beta, Ctl* ctl,
+                    unsigned long long seed, int mode, double* mu, double* Lambda,
+                    cudaStream_t s);
+void launch_nw_wide_pair(const PriorPair& pp, int K, Ctl* ctl, unsigned long long seed,
+                         cudaStream_t s);
 void launch_lambda_beta(const double* bb_partials, int nparts, int K, long long nfeat,
                         const double* Lambda, double nu, double mu, const Ctl* ctl,
                         unsigned long long seed, int mode, double* lambda_beta, cudaStream_t s);

@@ -1,20 +1,20 @@
 // Hyperprior update that allocates no device memory: mg_normal_wishart_noalloc.
 //
-// The context API (mg_update_prior) keeps its reduction partials and Normal-Wishart workspace in
+// The context API (mg_update_prior) keeps its reduction partials in
 // buffers it cudaMalloc's at mg_init.  Some hosts cannot allocate at the point where they want
 // to resample the hyperparameters: a serving process whose memory pool already owns all of the
 // device memory (a further cudaMalloc would fail, or would have to evict the pool's blocks), or
 // a latency-sensitive loop that cannot afford cudaMalloc's implicit device synchronisation.  For
-// them this entry point runs the same kernels (k_stats + k_normal_wishart) with all of their
+// them this entry point runs the same kernels (statistics, reduction, draw) with all of their
 // scratch in one file-scope __device__ array of fixed size, so the only device memory it touches
 // besides that array is the caller's inputs and outputs.
 //
 // Limits and sharing rules:
 //   * K <= kNoAllocMaxK (64); the row reduction uses at most kNoAllocMaxParts (64) partial sums.
-//     The array is 2.3 MB and every GPU that loads the library keeps it until the process exits.
+//     The array is 2.1 MB and every GPU that loads the library keeps it until the process exits.
 //   * Every call on a device uses the same array; it holds whatever the last call left in it.
 //     The control block (status word, sweep index) is cleared by each call; the partials and
-//     workspace are fully overwritten before they are read.  Calls whose kernels overlap on the
+//     their sum are fully overwritten before they are read.  Calls whose kernels overlap on the
 //     GPU (different streams, or different host threads without ordering) race on the array.
 //   * The call is synchronous: it copies the status word back and waits for `stream`, so it
 //     cannot be recorded into a CUDA graph.
@@ -36,9 +36,8 @@ namespace {
 constexpr int kNoAllocMaxK = 64;
 constexpr int kNoAllocMaxParts = 64;
 constexpr size_t kPartDoubles = (size_t)kNoAllocMaxParts * (kNoAllocMaxK + kNoAllocMaxK * kNoAllocMaxK);
-constexpr size_t kWorkDoubles = 3 * (size_t)kNoAllocMaxK + 4 * (size_t)kNoAllocMaxK * kNoAllocMaxK;
 constexpr size_t kCtlDoubles = (sizeof(Ctl) + sizeof(double) - 1) / sizeof(double);
-constexpr size_t kScratchDoubles = kPartDoubles + kWorkDoubles + kCtlDoubles;
+constexpr size_t kScratchDoubles = kPartDoubles + kCtlDoubles;
 
 // The scratch array.  In host code `g_noalloc_scratch` names a host-side stand-in, not device
 // memory: only the address returned by cudaGetSymbolAddress may be handed to kernels.
@@ -131,22 +130,24 @@ extern "C" int mg_normal_wishart_noalloc(const double* U, int64_t N, int K, int 
     MG_CUDA(scratch_address(&base));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     double* partials = base;
-    double* work = base + kPartDoubles;
-    Ctl* ctl = reinterpret_cast<Ctl*>(base + kPartDoubles + kWorkDoubles);
-    NwWork w;
-    w.vec = work;
-    w.m0 = work + 3 * K;
-    w.m1 = w.m0 + K * K;
-    w.m2 = w.m1 + K * K;
-    w.m3 = w.m2 + K * K;
+    Ctl* ctl = reinterpret_cast<Ctl*>(base + kPartDoubles);
     int nb = stats_blocks(N);
     if (nb > kNoAllocMaxParts) nb = kNoAllocMaxParts;
+    // K > 32: the draw reads one reduced record, which takes the last partial's place
+    if (K > 32 && nb == kNoAllocMaxParts) nb--;
     // the control block starts every call cleared (status = 0), then gets the sweep index
     MG_CUDA(cudaMemsetAsync(ctl, 0, sizeof(Ctl), s));
     launch_set_sweep(ctl, sweep, 0, s);
     launch_stats(U, false, nullptr, N, K, stride, 0, partials, nb, s);
-    launch_normal_wishart(partials, nb, N, K, mu0, kappa, T, nu, nullptr, 0, nullptr, w, ctl,
-                          seed, mode, mu_out, Lambda_out, s);
+    const int len = K + K * K;
+    double* stats = partials;
+    if (K > 32) {
+      stats = partials + (size_t)(kNoAllocMaxParts - 1) * len;
+      launch_reduce_parts(partials, nb, len, stats, s);
+      nb = 1;
+    }
+    launch_normal_wishart(stats, nb, N, K, mu0, kappa, T, nu, nullptr, 0, nullptr, ctl, seed, mode,
+                          mu_out, Lambda_out, s);
     int32_t status = 0;
     MG_CUDA(cudaMemcpyAsync(&status, &ctl->status, sizeof(status), cudaMemcpyDeviceToHost, s));
     MG_CUDA(cudaStreamSynchronize(s));
