@@ -35,7 +35,7 @@ struct StatsArgs {
 };
 
 // A warp's tiles over rows r0 .. r1 - 1.  DIAG: also the column sums of its blocks.
-template <typename V, int KP, bool DIAG>
+template <typename V, int KP, bool DIAG, bool HAT>
 __device__ __forceinline__ void stats_warp(const V* __restrict__ U, const double* __restrict__ Uhat,
                                            long long r0, long long r1, int K, int stride,
                                            int uhat_stride, int br, int bc,
@@ -44,28 +44,34 @@ __device__ __forceinline__ void stats_warp(const V* __restrict__ U, const double
   constexpr int NR = DIAG ? 4 * C::ND : C::RB, NC = DIAG ? 0 : 4;
   constexpr int NT = DIAG ? 10 * C::ND : 4 * C::RB;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  double acc[NT][2], racc[NR], f[2][NR + NC];
+  constexpr int R = 4;  // steps of four rows in flight
+  double acc[NT][2], racc[NR], f[R][NR + NC];
 #pragma unroll
   for (int q = 0; q < NT; q++) acc[q][0] = acc[q][1] = 0.0;
 #pragma unroll
   for (int b = 0; b < NR; b++) racc[b] = 0.0;
+  // this lane's components of each block; the loads of a step are independent and unconditional
+  // but for the bounds
+  int col[NR + NC];
+#pragma unroll
+  for (int b = 0; b < NR + NC; b++) col[b] = 8 * (b < NR ? br + b : bc + b - NR) + g;
   auto load = [&](int stage, long long row) {
+    const V* u = U + row * stride;
+    const double* h = HAT ? Uhat + row * uhat_stride : nullptr;
 #pragma unroll
     for (int b = 0; b < NR + NC; b++) {
-      const int k = 8 * (b < NR ? br + b : bc + b - NR) + g;
-      double x = 0.0;
-      if (row < r1 && k < K) {
-        x = (double)U[row * stride + k];
-        if (Uhat) x -= Uhat[row * uhat_stride + k];
-      }
+      const bool ok = row < r1 && col[b] < K;
+      double x = ok ? (double)__ldg(u + col[b]) : 0.0;
+      if constexpr (HAT) x -= ok ? __ldg(h + col[b]) : 0.0;
       f[stage][b] = x;
     }
   };
-  load(0, r0 + t);
-  for (long long r = r0; r < r1; r += 8) {
 #pragma unroll
-    for (int u = 0; u < 2; u++) {
-      load(1 - u, r + 4 * (u + 1) + t);
+  for (int u = 0; u < R - 1; u++) load(u, r0 + 4 * u + t);
+  for (long long r = r0; r < r1; r += 4 * R) {
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      load((u + R - 1) % R, r + 4 * (u + R - 1) + t);
       int q = 0;
       if constexpr (DIAG) {
 #pragma unroll
@@ -123,7 +129,7 @@ __device__ __forceinline__ void stats_warp(const V* __restrict__ U, const double
   }
 }
 
-template <typename V, int KP>
+template <typename V, int KP, bool HAT>
 __global__ void __launch_bounds__(StatW<KP>::T)
     k_stats_wide(const StatsArgs p, int K, int stride, int uhat_stride) {
   const int m = (int)blockIdx.x < p.nblocks[0] ? 0 : 1;
@@ -133,18 +139,20 @@ __global__ void __launch_bounds__(StatW<KP>::T)
   double* out = p.partials[m] + (size_t)b * (K + (size_t)K * K);
   const Part64 part = part_of<KP>(threadIdx.x >> 5);
   if (part.diag)
-    stats_warp<V, KP, true>(U, p.Uhat, r0, r1, K, stride, uhat_stride, part.r0, 0, out);
+    stats_warp<V, KP, true, HAT>(U, p.Uhat, r0, r1, K, stride, uhat_stride, part.r0, 0, out);
   else
-    stats_warp<V, KP, false>(U, p.Uhat, r0, r1, K, stride, uhat_stride, part.r0, part.c0, out);
+    stats_warp<V, KP, false, HAT>(U, p.Uhat, r0, r1, K, stride, uhat_stride, part.r0, part.c0, out);
 }
 
 template <typename V>
 void stats_launch(const StatsArgs& a, int K, int stride, int uhat_stride, cudaStream_t s) {
   const int nb = a.nblocks[0] + a.nblocks[1];
-  if (K <= 64)
-    k_stats_wide<V, 64><<<nb, StatW<64>::T, 0, s>>>(a, K, stride, uhat_stride);
+  if (K > 64)  // side information needs K <= 64
+    k_stats_wide<V, 128, false><<<nb, StatW<128>::T, 0, s>>>(a, K, stride, uhat_stride);
+  else if (a.Uhat)
+    k_stats_wide<V, 64, true><<<nb, StatW<64>::T, 0, s>>>(a, K, stride, uhat_stride);
   else
-    k_stats_wide<V, 128><<<nb, StatW<128>::T, 0, s>>>(a, K, stride, uhat_stride);
+    k_stats_wide<V, 64, false><<<nb, StatW<64>::T, 0, s>>>(a, K, stride, uhat_stride);
   MG_CUDA(cudaGetLastError());
 }
 
@@ -169,9 +177,9 @@ constexpr int kNwThreads = 512, kNwHalf = 256;  // warps 0-7: factor, solve; war
 template <int KP>
 struct NwW {
   static constexpr int NB = KP / 8, TRI = NB * (NB + 1) / 2;
-  // M, then B | Y = M^-1 | the Bartlett factor's transpose | mu_c, y, x, 1 / diagonal, zeros, z |
-  // flag | tile table
-  static constexpr size_t kDoubles = 3 * (size_t)TRI * 64 + 6 * KP + 2 + (TRI + 7) / 8;
+  // M, then B | Y = M^-1 | the Bartlett factor's transpose | inverses of the diagonal tiles | mu_c,
+  // y, x, zeros, z | flag | tile table
+  static constexpr size_t kDoubles = (3 * (size_t)TRI + NB) * 64 + 5 * KP + 2 + (TRI + 7) / 8;
 };
 
 // Draws of the Bartlett factor c (upper triangular: c_ii = sqrt(2 Gamma((nu_c - i) / 2)), c_ij ~
@@ -185,14 +193,22 @@ __device__ __forceinline__ void bartlett(double* Ct, double* z, int K, int n, in
                                               (uint32_t)i, 0.5 * (double)(nu_c - i)));
     z[i] = normal_draw(seed, sweep, stream_id(kMuDraw, mode), 0u, (uint32_t)i);
   }
-  const int warp = tid >> 5, lane = tid & 31;
-  for (int i = warp; i < K; i += nt >> 5)
-    for (int q = lane; 2 * q < K - 1 - i; q += 32) {
-      double z0, z1;
-      normal_pair(seed, sweep, stream_id(kWishartOff, mode), (uint32_t)i, (uint32_t)q, &z0, &z1);
-      Ct[elem_at(i + 1 + 2 * q, i)] = z0;
-      if (2 * q + 1 < K - 1 - i) Ct[elem_at(i + 2 + 2 * q, i)] = z1;
+  // off-diagonal draws two to a block: rows i and K - 2 - i together have at most K / 2 + 1 pairs
+  const int slots = K / 2 + 1;
+  for (int e = tid; e < slots * (K / 2); e += nt) {
+    const int s = e / slots, first = (K - s) / 2;  // pairs of row s
+    int i = s, q = e % slots;
+    if (q >= first) {
+      i = K - 2 - s;
+      q -= first;
+      if (i <= s || q >= (s + 2) / 2) continue;  // row s alone in the middle, or past the last pair
     }
+    const int left = K - 1 - i - 2 * q;  // draws of this pair on: 1 or more
+    double z0, z1;
+    normal_pair(seed, sweep, stream_id(kWishartOff, mode), (uint32_t)i, (uint32_t)q, &z0, &z1);
+    Ct[elem_at(i + 1 + 2 * q, i)] = z0;
+    if (left > 1) Ct[elem_at(i + 2 + 2 * q, i)] = z1;
+  }
   for (int i = K + tid; i < n; i += nt) {
     for (int j = 0; j < i; j++) Ct[elem_at(i, j)] = 0.0;
     Ct[elem_at(i, i)] = 1.0;
@@ -217,8 +233,9 @@ __global__ void __launch_bounds__(kNwThreads, 1)
   double* M = nsm;
   double* Y = M + (size_t)C::TRI * 64;
   double* Ct = Y + (size_t)C::TRI * 64;
-  double* muc = Ct + (size_t)C::TRI * 64;
-  double *y = muc + KP, *x = y + KP, *rinv = x + KP, *zero = rinv + KP, *z = zero + KP;
+  double* Di = Ct + (size_t)C::TRI * 64;
+  double* muc = Di + (size_t)C::NB * 64;
+  double *y = muc + KP, *x = y + KP, *zero = x + KP, *z = zero + KP;
   volatile int* bad = reinterpret_cast<volatile int*>(z + KP);
   unsigned char* tri = reinterpret_cast<unsigned char*>(z + KP + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -237,24 +254,30 @@ __global__ void __launch_bounds__(kNwThreads, 1)
     y[i] = zero[i] = 0.0;
   }
   __syncthreads();
-  // M = J (T + N S + kappa mu0 mu0^T - kappa_c mu_c mu_c^T) J
+  // M = J (T + N S + kappa mu0 mu0^T - kappa_c mu_c mu_c^T) J, a warp per tile; the identity in
+  // the first `pad` rows and columns
   const double lb = p.bb ? *p.lambda_beta : 0.0;
-#pragma unroll 4
-  for (int e = tid; e < K * K; e += kNwThreads) {
-    const int i = e % K, j = e / K;
-    if (i > j) continue;
-    double T = p.T0[e];
-    if (p.bb) T += lb * p.bb[K + e];
-    M[elem_at(n - 1 - i, n - 1 - j)] = T + p.stats[K + e] + p.kappa * p.mu0[i] * p.mu0[j] -
-                                       kappa_c * muc[i] * muc[j];
-  }
-  for (int e = tid; e < pad * n; e += kNwThreads) {  // identity rows and columns before them
-    const int b = e % pad, a = e / pad;
-    if (a >= b) M[elem_at(a, b)] = a == b ? 1.0 : 0.0;
+#pragma unroll 3
+  for (int q = warp; q < nb * (nb + 1) / 2; q += kNwThreads / 32) {
+    const int a = 8 * (tri[q] >> 4) + g;
+    double v[2];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int b = 8 * (tri[q] & 15) + 2 * t + e, i = n - 1 - a, j = n - 1 - b;
+      v[e] = a == b ? 1.0 : 0.0;
+      if (a >= pad && b >= pad) {
+        const size_t at = j + (size_t)i * K;
+        double T = p.T0[at];
+        if (p.bb) T += lb * p.bb[K + at];
+        v[e] = T + p.stats[K + at] + p.kappa * p.mu0[i] * p.mu0[j] - kappa_c * muc[i] * muc[j];
+      }
+    }
+    *reinterpret_cast<double2*>(M + tile_at(tri[q] >> 4, tri[q] & 15) + tile_pos(g, 2 * t)) =
+        make_double2(v[0], v[1]);
   }
   __syncthreads();
   if (warp < 8) {
-    wide_factor<double, KP, kNwHalf>(M, y, rinv, zero, nb, tri, 0.0, tid, 0, bad);
+    wide_factor<double, KP, kNwHalf>(M, y, Di, zero, nb, 0.0, tid, 0, bad);
   } else {
     bartlett(Ct, z, K, n, nu_c, seed, sweep, (uint32_t)p.mode, tid - kNwHalf, kNwHalf);
   }
@@ -263,20 +286,10 @@ __global__ void __launch_bounds__(kNwThreads, 1)
     if (tid == 0) atomicOr(&ctl->status, kStatHyperFail);
     return;
   }
-  // Y = M^{-1}.  Diagonal tiles: thread (block, column) solves its 8 x 8 column.
-  if (tid < n) {
-    const int b = tid >> 3, c = tid & 7;
-    const double* D = M + tile_at(b, b);
-    double v[8];
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      double s = r == c ? 1.0 : 0.0;
-#pragma unroll
-      for (int k = 0; k < r; k++) s = fma(-D[tile_pos(r, k)], v[k], s);
-      v[r] = r < c ? 0.0 : s * rinv[8 * b + r];
-    }
-#pragma unroll
-    for (int r = 0; r < 8; r++) Y[tile_at(b, b) + tile_pos(r, c)] = v[r];
+  // Y = M^{-1}.  Its diagonal tiles are the factor's inverses, transposed back.
+  for (int e = tid; e < 64 * nb; e += kNwThreads) {
+    const int b = e >> 6, r = (e >> 3) & 7, c = e & 7;
+    Y[tile_at(b, b) + tile_pos(r, c)] = Di[64 * b + tile_pos(c, r)];
   }
   __syncthreads();
   // Below them: a warp per block column, Y(i, j) = -Y(i, i) sum_k M(i, k) Y(k, j)
@@ -320,11 +333,22 @@ __global__ void __launch_bounds__(kNwThreads, 1)
   if (warp < 8) {
     // mu = mu_c + B^{-T} z / sqrt(kappa_c)
     if (tid < n) {
-      rinv[tid] = 1.0 / M[elem_at(tid, tid)];
+      // column c of the inverse of diagonal tile b
+      const int b = tid >> 3, c = tid & 7;
+      const double* D = M + tile_at(b, b);
+      double v[8];
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        double s = r == c ? 1.0 : 0.0;
+#pragma unroll
+        for (int k = 0; k < r; k++) s = fma(-D[tile_pos(r, k)], v[k], s);
+        v[r] = r < c ? 0.0 : s / D[tile_pos(r, r)];
+      }
+      store_row8(Di + 64 * b, c, v);
       y[tid] = z[tid] / sqrt(kappa_c);
     }
     group_sync<kNwHalf>(0);
-    wide_back<double, KP, kNwHalf>(M, y, rinv, x, nb, tid, 0);
+    wide_back<double, KP, kNwHalf>(M, y, Di, x, nb, tid, 0);
     if (tid < K) p.mu[tid] = x[tid] + muc[tid];
   } else {
     // Lambda = B B^T
@@ -379,6 +403,7 @@ void launch_stats_wide(const void* U, bool f32, const double* Uhat, long long N,
                        int uhat_stride, double* partials, int nblocks, cudaStream_t s) {
   const StatsArgs a{{U, nullptr}, Uhat, {N, 0}, {(N + nblocks - 1) / nblocks, 0}, {nblocks, 0},
                     {partials, nullptr}};
+  if (Uhat && K > 64) throw MgError(MG_ERR_ARG, "side information supports num_latent <= 64");
   if (f32) stats_launch<float>(a, K, stride, uhat_stride, s);
   else stats_launch<double>(a, K, stride, uhat_stride, s);
 }

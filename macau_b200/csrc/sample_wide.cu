@@ -53,9 +53,10 @@ struct Wide {
   // FP64 gather stages (of 4 entries); at 128 the accumulators leave no registers for a second
   // one, and four warps a sub-partition cover the latency
   static constexpr int R = KP == 64 ? 4 : 1;
-  // group's shared memory in doubles: tiles | rhs, y | draws | x | 1 / L(j, j) | diagonal | flags
-  static constexpr size_t kGroupDoubles = (size_t)TRI * 64 + 5 * KP + 2;
-  static constexpr size_t kCtaDoubles = KP + 2 * ((TRI + 15) / 16);  // Lambda mu | tile table
+  // group's shared memory in doubles: tiles | inverses of the diagonal's | rhs, y | draws | x |
+  // diagonal | flags
+  static constexpr size_t kGroupDoubles = (size_t)(TRI + NB) * 64 + 4 * KP + 2;
+  static constexpr size_t kCtaDoubles = KP;  // Lambda mu
 };
 
 // ---- FP64 Gram ----
@@ -337,11 +338,10 @@ __device__ __forceinline__ void store16(F* M, const double* Lambda, int K, F alp
 
 // The FP64 redo of the mixed path, kept out of line for its registers.
 template <int KP, int T>
-__device__ __noinline__ bool wide_factor_redo(double* M, double* y, double* rinv,
-                                              const double* diag0, int nb,
-                                              const unsigned char* tri, int tid, int grp,
+__device__ __noinline__ bool wide_factor_redo(double* M, double* y, double* Di,
+                                              const double* diag0, int nb, int tid, int grp,
                                               volatile int* bad) {
-  return wide_factor<double, KP, T>(M, y, rinv, diag0, nb, tri, 0.0, tid, grp, bad);
+  return wide_factor<double, KP, T>(M, y, Di, diag0, nb, 0.0, tid, grp, bad);
 }
 
 template <int KP, int G, bool MIXED>
@@ -352,24 +352,18 @@ __global__ void __launch_bounds__(Wide<KP, MIXED>::T* G, (KP == 64 ? 4 : 2) / G)
   constexpr int T = C::T, NT = C::NT, AE = C::AE;
   extern __shared__ __align__(16) double smem_w[];
   double* lmu_s = smem_w;
-  unsigned char* tri = reinterpret_cast<unsigned char*>(smem_w + KP);
   const int grp = threadIdx.x / T, tid = threadIdx.x % T;
   const int warp = tid >> 5, lane = tid & 31;
   double* M = smem_w + C::kCtaDoubles + (size_t)grp * C::kGroupDoubles;
-  double* rhs_s = M + (size_t)C::TRI * 64;  // Gram rhs, then the factor's y
+  double* Di = M + (size_t)C::TRI * 64;
+  double* rhs_s = Di + (size_t)C::NB * 64;  // Gram rhs, then the factor's y
   double* z_s = rhs_s + KP;
   double* x_s = z_s + KP;
-  double* rinv_s = x_s + KP;
-  double* diag_s = rinv_s + KP;
+  double* diag_s = x_s + KP;
   volatile int* bad = reinterpret_cast<volatile int*>(diag_s + KP);
   volatile int* bcast = bad + 1;  // [0]: task, [1]: whether this part finishes the row
   const int K = p.K, nb = (K + 7) / 8, ntasks = p.ntasks;
   if (tid == 0) bcast[0] = (int)atomicAdd(&p.ctl->queue[p.qslot], 1u);
-  for (int q = threadIdx.x; q < C::TRI; q += blockDim.x) {
-    int a = 0;
-    while (q >= (a + 1) * (a + 2) / 2) a++;
-    tri[q] = (unsigned char)((a << 4) | (q - a * (a + 1) / 2));
-  }
   for (int i = threadIdx.x; i < KP; i += blockDim.x) {
     double s = 0.0;
     if (i < K)
@@ -484,21 +478,21 @@ __global__ void __launch_bounds__(Wide<KP, MIXED>::T* G, (KP == 64 ? 4 : 2) / G)
       bool done = false;
       if constexpr (MIXED) {
         float* Mf = reinterpret_cast<float*>(M);
-        float* yf = reinterpret_cast<float*>(x_s);  // x_s and rinv_s halves: y | x and rinv | diag
+        float* Dif = reinterpret_cast<float*>(Di);
+        float* yf = reinterpret_cast<float*>(x_s);  // x_s holds y and x
         float* xf = yf + KP;
-        float* rf = reinterpret_cast<float*>(rinv_s);
-        float* df = rf + KP;
+        float* df = reinterpret_cast<float*>(diag_s);
         group_sync<T>(grp);  // x_s was the prior mean
         store16<float, KP>(Mf, p.Lambda, K, (float)alpha, warp, acc);
         if (tid < KP) yf[tid] = (float)rr;
         group_sync<T>(grp);
         if (tid < KP) df[tid] = Mf[elem_at(tid, tid)];
         group_sync<T>(grp);
-        done = wide_factor<float, KP, T>(Mf, yf, rf, df, nb, tri, 0x1p-20f, tid, grp, bad);
+        done = wide_factor<float, KP, T>(Mf, yf, Dif, df, nb, 0x1p-20f, tid, grp, bad);
         if (done) {
           if (tid < 8 * nb) yf[tid] += (float)z_s[tid];
           group_sync<T>(grp);
-          wide_back<float, KP, T>(Mf, yf, rf, xf, nb, tid, grp);
+          wide_back<float, KP, T>(Mf, yf, Dif, xf, nb, tid, grp);
           if (tid < K) {
             p.out_f32[(size_t)row * KP + tid] = xf[tid];
             store_copy(p, (size_t)row * KP + tid, xf[tid]);
@@ -526,13 +520,13 @@ __global__ void __launch_bounds__(Wide<KP, MIXED>::T* G, (KP == 64 ? 4 : 2) / G)
         group_sync<T>(grp);
         bool ok;
         if constexpr (MIXED)
-          ok = wide_factor_redo<KP, T>(M, rhs_s, rinv_s, diag_s, nb, tri, tid, grp, bad);
+          ok = wide_factor_redo<KP, T>(M, rhs_s, Di, diag_s, nb, tid, grp, bad);
         else
-          ok = wide_factor<double, KP, T>(M, rhs_s, rinv_s, diag_s, nb, tri, 0.0, tid, grp, bad);
+          ok = wide_factor<double, KP, T>(M, rhs_s, Di, diag_s, nb, 0.0, tid, grp, bad);
         if (ok) {
           if (tid < 8 * nb) rhs_s[tid] += z_s[tid];
           group_sync<T>(grp);
-          wide_back<double, KP, T>(M, rhs_s, rinv_s, x_s, nb, tid, grp);
+          wide_back<double, KP, T>(M, rhs_s, Di, x_s, nb, tid, grp);
           if (tid < K) {
             if constexpr (MIXED) {
               p.out_f32[(size_t)row * KP + tid] = (float)x_s[tid];

@@ -67,88 +67,96 @@ __device__ __forceinline__ void gather64(double (&f)[N], const double* src, bool
 }
 
 // ---- factor and solves over the tiles ----
-// Trailing tiles (bi, bj) -= P_bi P_bj^T of panel pn, P the panel's tiles: the pairs b <= a of the n1
-// block rows below it, the q-th of them to warp q mod W.  The FP64 form takes U tiles at a time,
-// so that their loads and products overlap.
-template <int W, int U>
-__device__ __forceinline__ void trail_tiles(double* M, const unsigned char* tri, int pn, int q0,
-                                            int lane) {
+// Tile (bi, pn) -= sum_{k < pn} L(bi, k) L(pn, k)^T by one warp (FP64: two accumulators, so that
+// consecutive products overlap).
+__device__ __forceinline__ void update_tile(double* M, int bi, int pn, int lane) {
   const int g = lane >> 2, t = lane & 3;
-  const int p0 = tile_pos(g, t), p1 = tile_pos(g, t + 4), pc = tile_pos(g, 2 * t);
-  double2* c[U];
-  double2 v[U];
-  double a[U][2], b[U][2];
-#pragma unroll
-  for (int u = 0; u < U; u++) {
-    const int ab = tri[q0 + u * W];
-    const int bi = pn + 1 + (ab >> 4), bj = pn + 1 + (ab & 15);
-    const double* Pi = M + tile_at(bi, pn);
-    const double* Pj = M + tile_at(bj, pn);
-    c[u] = reinterpret_cast<double2*>(M + tile_at(bi, bj) + pc);
-    v[u] = *c[u];
-    a[u][0] = -Pi[p0];
-    a[u][1] = -Pi[p1];
-    b[u][0] = Pj[p0];
-    b[u][1] = Pj[p1];
+  const int p0 = tile_pos(g, t), p1 = tile_pos(g, t + 4);
+  const double* A = M + tile_at(bi, 0);
+  const double* B = M + tile_at(pn, 0);
+  double2* c = reinterpret_cast<double2*>(M + tile_at(bi, pn) + tile_pos(g, 2 * t));
+  double2 v = *c, w = make_double2(0.0, 0.0);
+  int k = 0;
+#pragma unroll 2
+  for (; k + 1 < pn; k += 2) {
+    const double a0 = -A[64 * k + p0], a1 = -A[64 * k + p1];
+    const double a2 = -A[64 * k + 64 + p0], a3 = -A[64 * k + 64 + p1];
+    const double b0 = B[64 * k + p0], b1 = B[64 * k + p1];
+    const double b2 = B[64 * k + 64 + p0], b3 = B[64 * k + 64 + p1];
+    mma_f64(v.x, v.y, a0, b0);
+    mma_f64(w.x, w.y, a2, b2);
+    mma_f64(v.x, v.y, a1, b1);
+    mma_f64(w.x, w.y, a3, b3);
   }
-#pragma unroll
-  for (int k = 0; k < 2; k++)
-#pragma unroll
-    for (int u = 0; u < U; u++) mma_f64(v[u].x, v[u].y, a[u][k], b[u][k]);
-#pragma unroll
-  for (int u = 0; u < U; u++) *c[u] = v[u];
+  if (k < pn) {
+    mma_f64(v.x, v.y, -A[64 * k + p0], B[64 * k + p0]);
+    mma_f64(w.x, w.y, -A[64 * k + p1], B[64 * k + p1]);
+  }
+  *c = make_double2(v.x + w.x, v.y + w.y);
 }
-template <int W>
-__device__ __forceinline__ void trail(double* M, const unsigned char* tri, int pn, int n1, int warp,
-                                      int lane) {
-  const int n = n1 * (n1 + 1) / 2;
-  int q = warp;
-  for (; q + 2 * W < n; q += 3 * W) trail_tiles<W, 3>(M, tri, pn, q, lane);
-  for (; q < n; q += W) trail_tiles<W, 1>(M, tri, pn, q, lane);
-}
-template <int W>
-__device__ __forceinline__ void trail(float* M, const unsigned char* tri, int pn, int n1, int warp,
-                                      int lane) {
-  const int g = lane >> 2, t = lane & 3, n = n1 * (n1 + 1) / 2;
-  for (int q = warp; q < n; q += W) {
-    const int bi = pn + 1 + (tri[q] >> 4), bj = pn + 1 + (tri[q] & 15);
+__device__ __forceinline__ void update_tile(float* M, int bi, int pn, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  const float* A = M + tile_at(bi, 0);
+  const float* B = M + tile_at(pn, 0);
+  float2* c = reinterpret_cast<float2*>(M + tile_at(bi, pn) + tile_pos(g, 2 * t));
+  float2 v = *c;
+#pragma unroll 2
+  for (int k = 0; k < pn; k++) {
     float a[8], b0[8], b1[8];
-    load_row8(M + tile_at(bi, pn), g, a);
-    load_row8(M + tile_at(bj, pn), 2 * t, b0);
-    load_row8(M + tile_at(bj, pn), 2 * t + 1, b1);
-    float2* c = reinterpret_cast<float2*>(M + tile_at(bi, bj) + tile_pos(g, 2 * t));
-    float2 v = *c;
+    load_row8(A + 64 * k, g, a);
+    load_row8(B + 64 * k, 2 * t, b0);
+    load_row8(B + 64 * k, 2 * t + 1, b1);
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      v.x = fmaf(-a[k], b0[k], v.x);
-      v.y = fmaf(-a[k], b1[k], v.y);
+    for (int q = 0; q < 8; q++) {
+      v.x = fmaf(-a[q], b0[q], v.x);
+      v.y = fmaf(-a[q], b1[q], v.y);
     }
-    *c = v;
   }
+  *c = v;
 }
 
-// Factorises MM (nb blocks) in place by panels, y (the right-hand side) along with it, and leaves
-// 1 / L(j, j) in rinv.  A pivot that is not positive, or not above rel_floor times its original
-// diagonal, fails the group (all threads return false).  tri[q] = (a << 4) | b, the q-th pair
-// b <= a.
+// Factorises MM (nb blocks) in place by panels of 8 columns, left-looking, y (the right-hand side)
+// along with it, and leaves the transposed inverse of each diagonal tile in Di (a tile per panel,
+// for the backward substitution: eight more rows, those of the identity, go through the panel's
+// solve).  A pivot that is not positive, or not above
+// rel_floor times its original diagonal, fails the group (all threads return false).
+//   Per panel: a warp per tile subtracts the products of the panels before it (a right-looking
+//   update of every trailing tile per panel took 1,400 cycles a panel at K = 128, three times
+//   this: each product loaded and stored its tile); barrier; every thread that owns a row of the
+//   panel factors the diagonal tile for itself and solves its row; barrier.
 template <typename F, int KP, int T>
-__device__ __forceinline__ bool wide_factor(F* M, F* y, F* rinv, const F* diag0, int nb,
-                                            const unsigned char* tri, F rel_floor, int tid,
-                                            int grp, volatile int* bad) {
+__device__ __forceinline__ bool wide_factor(F* M, F* y, F* Di, const F* diag0, int nb,
+                                            F rel_floor, int tid, int grp, volatile int* bad) {
   const int warp = tid >> 5, lane = tid & 31;
   for (int pn = 0; pn < nb; pn++) {
-    // rows 8 pn .. of the panel, then y: one thread each
+    if (pn > 0) {
+      for (int bi = pn + warp; bi < nb; bi += T / 32) update_tile(M, bi, pn, lane);
+      // y's components from the panel on, by the panel before
+      const int j = 8 * pn + tid;
+      if (j < 8 * nb) {
+        F v[8], s = y[j];
+        load_row8(M + tile_at(j >> 3, pn - 1), j & 7, v);
+#pragma unroll
+        for (int c = 0; c < 8; c++) s = mfma(-v[c], y[8 * pn - 8 + c], s);
+        y[j] = s;
+      }
+      group_sync<T>(grp);
+    }
+    // rows 8 pn .. of the panel, the identity's, then y: one thread each
     const int rows = 8 * (nb - pn);
-    F* own = M + tile_at(pn + (tid >> 3), pn);  // the thread's tile when tid < rows
+    F* own = tid < rows ? M + tile_at(pn + (tid >> 3), pn) : Di + 64 * pn;
     F x[8];
-    if (tid <= rows) {
+    if (tid <= rows + 8) {
       const F* D = M + tile_at(pn, pn);
       F l[8][8];
 #pragma unroll
       for (int i = 0; i < 8; i++) load_row8(D, i, l[i]);
-      if (tid == rows) {
+      if (tid == rows + 8) {
 #pragma unroll
         for (int c = 0; c < 8; c++) x[c] = y[8 * pn + c];
+      } else if (tid >= rows) {
+#pragma unroll
+        for (int c = 0; c < 8; c++) x[c] = tid - rows == c ? (F)1 : (F)0;
       } else {
         load_row8(own, tid & 7, x);
       }
@@ -158,7 +166,6 @@ __device__ __forceinline__ bool wide_factor(F* M, F* y, F* rinv, const F* diag0,
         const F d = l[c][c];
         ok = ok && d > (F)0 && d > rel_floor * diag0[8 * pn + c];
         const F r = mrsqrt(d);
-        if (tid == 0) rinv[8 * pn + c] = r;
 #pragma unroll
         for (int i = c + 1; i < 8; i++) l[i][c] *= r;
         x[c] *= r;
@@ -170,7 +177,7 @@ __device__ __forceinline__ bool wide_factor(F* M, F* y, F* rinv, const F* diag0,
         }
       }
       if (!ok && tid == 0) *bad = 1;
-      if (tid == rows) {
+      if (tid == rows + 8) {
 #pragma unroll
         for (int c = 0; c < 8; c++) y[8 * pn + c] = x[c];
       } else if (tid >= 8) {
@@ -181,51 +188,45 @@ __device__ __forceinline__ bool wide_factor(F* M, F* y, F* rinv, const F* diag0,
     if (*bad) return false;
     // the factored diagonal tile's rows only now: every owner has read the tile
     if (tid < 8) store_row8(own, tid, x);
-    // trailing tiles, and y's remaining components
-    const int n1 = nb - pn - 1;
-    trail<T / 32>(M, tri, pn, n1, warp, lane);
-    const int j = 8 * (pn + 1) + tid;
-    if (j < 8 * nb) {
-      F v[8], s = y[j];
-      load_row8(M + tile_at(j >> 3, pn), j & 7, v);
-#pragma unroll
-      for (int c = 0; c < 8; c++) s = mfma(-v[c], y[8 * pn + c], s);
-      y[j] = s;
-    }
-    group_sync<T>(grp);
   }
+  group_sync<T>(grp);
   return true;
 }
 
-// x = L^{-T} b over the panels from the last, b in y (overwritten), one barrier each.
+// x = L^{-T} b over the panels from the last, b in y (overwritten), Di the diagonal tiles'
+// transposed inverses; one barrier a panel.  Each warp forms the panel's eight x for itself.
 template <typename F, int KP, int T>
-__device__ __forceinline__ void wide_back(const F* M, F* y, const F* rinv, F* x, int nb, int tid,
+__device__ __forceinline__ void wide_back(const F* M, F* y, const F* Di, F* x, int nb, int tid,
                                           int grp) {
+  const int warp = tid >> 5, r = tid & 7;
   for (int pn = nb - 1; pn >= 0; pn--) {
-    if (tid < 8 * pn || tid == T - 1) {
-      // every thread solves the panel's 8 x 8 system for itself
-      F b[8];
+    if (warp == 0 || 32 * warp < 8 * pn) {
+      F d[8], b[8], p[8];
+      load_row8(Di + 64 * pn, r, d);
 #pragma unroll
-      for (int c = 0; c < 8; c++) b[c] = y[8 * pn + c];
-      const F* D = M + tile_at(pn, pn);
+      for (int h = 0; h < 2; h++) {
+        const Vec4<F> q = lds4(y + 8 * pn + 4 * h);
 #pragma unroll
-      for (int c = 7; c >= 0; c--) {
-        F l[8];
-        load_row8(D, c, l);
-        b[c] *= rinv[8 * pn + c];
-#pragma unroll
-        for (int d = 0; d < c; d++) b[d] = mfma(-l[d], b[c], b[d]);
+        for (int u = 0; u < 4; u++) b[4 * h + u] = q.v[u];
       }
-      if (tid < 8 * pn) {
-        const F* P = M + tile_at(pn, tid >> 3);
-        F s = y[tid];
+      const bool on = tid < 8 * pn;
+      const F* P = M + tile_at(pn, on ? tid >> 3 : 0);
 #pragma unroll
-        for (int c = 0; c < 8; c++) s = mfma(-P[tile_pos(c, tid & 7)], b[c], s);
-        y[tid] = s;
-      } else {
+      for (int c = 0; c < 8; c++) p[c] = P[tile_pos(c, r)];
+      F s = on ? y[tid] : (F)0, u0 = (F)0, u1 = (F)0, s1 = (F)0;
 #pragma unroll
-        for (int c = 0; c < 8; c++) x[8 * pn + c] = b[c];
+      for (int c = 0; c < 8; c += 2) {
+        u0 = mfma(d[c], b[c], u0);
+        u1 = mfma(d[c + 1], b[c + 1], u1);
       }
+      const F xr = u0 + u1;
+#pragma unroll
+      for (int c = 0; c < 8; c += 2) {
+        s = mfma(-p[c], wshfl(xr, c), s);
+        s1 = mfma(-p[c + 1], wshfl(xr, c + 1), s1);
+      }
+      if (on) y[tid] = s + s1;
+      if (tid < 8) x[8 * pn + tid] = xr;
     }
     group_sync<T>(grp);
   }
