@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kNwThreads, 1)
   // M = J (T + N S + kappa mu0 mu0^T - kappa_c mu_c mu_c^T) J, a warp per tile; the identity in
   // the first `pad` rows and columns
   const double lb = p.bb ? *p.lambda_beta : 0.0;
-#pragma unroll 3
+#pragma unroll 5
   for (int q = warp; q < nb * (nb + 1) / 2; q += kNwThreads / 32) {
     const int a = 8 * (tri[q] >> 4) + g;
     double v[2];

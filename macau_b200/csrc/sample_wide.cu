@@ -12,16 +12,14 @@
 //          becomes element g of block 8h + b.  The blocks are thus a permutation of the
 //          components, undone when the Gram is stored.
 // Finish.  MM = Lambda + alpha G in shared memory as 8 x 8 tiles (lower triangle), factorised by
-// panels of 8 columns with two barriers each: every thread that owns a row of the panel factors
-// the panel's 8 x 8 diagonal tile for itself in registers (a chain of 8 reciprocal square roots;
-// sharing one factor would add a barrier and a broadcast to it) and solves its own row; then
-// the warps update the trailing tiles (FP64: m8n8k4.f64; FP32: FMAs).  The right-hand side rides
-// along as one more row, which is the forward substitution.  The backward substitution takes one
-// barrier per panel the same way.
+// panels of 8 columns with two barriers each (wide_tiles.cuh): one warp factors the diagonal tile
+// while the others bring the tiles below up to date, which are then multiplied by its inverse
+// (FP64: m8n8k4.f64; FP32: FMAs).  The right-hand side rides along as one more row, which is the
+// forward substitution.  The backward substitution takes one barrier per panel.
 //
-// What bounds it: short rows, the latency of the panel chain (about 1,000 cycles a panel), with
-// 2 (K > 64) or 4 rows in flight per SM; long rows, the matrix instructions.  The column-by-column
-// factor this replaces took three barriers a column, 78 us a row at K = 64.
+// What bounds it: short rows, the latency of the panel chain, with 2 (K > 64) or 4 rows in flight
+// per SM; long rows, the matrix instructions.  The column-by-column factor this replaces took
+// three barriers a column, 78 us a row at K = 64.
 #include <cuda_bf16.h>
 
 #include <algorithm>

@@ -34,10 +34,19 @@ __device__ __forceinline__ void load_row8(const F* tile, int r, F (&v)[8]) {
     for (int u = 0; u < 4; u++) v[4 * h + u] = q.v[u];
   }
 }
-template <typename F>
-__device__ __forceinline__ void store_row8(F* tile, int r, const F (&v)[8]) {
+__device__ __forceinline__ void store_row8(double* tile, int r, const double (&v)[8]) {
 #pragma unroll
-  for (int c = 0; c < 8; c++) tile[tile_pos(r, c)] = v[c];
+  for (int h = 0; h < 2; h++) {
+    double2* d = reinterpret_cast<double2*>(tile + r * 8 + 4 * (h ^ ((r >> 1) & 1)));
+    d[0] = make_double2(v[4 * h], v[4 * h + 1]);
+    d[1] = make_double2(v[4 * h + 2], v[4 * h + 3]);
+  }
+}
+__device__ __forceinline__ void store_row8(float* tile, int r, const float (&v)[8]) {
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+    *reinterpret_cast<float4*>(tile + r * 8 + 4 * (h ^ ((r >> 1) & 1))) =
+        make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
 }
 
 // ---- FP64 Grams: lower-triangle tiles by warp (4 warps at 64 components, 8 at 128) ----
@@ -67,41 +76,48 @@ __device__ __forceinline__ void gather64(double (&f)[N], const double* src, bool
 }
 
 // ---- factor and solves over the tiles ----
-// Tile (bi, pn) -= sum_{k < pn} L(bi, k) L(pn, k)^T by one warp (FP64: two accumulators, so that
-// consecutive products overlap).
-__device__ __forceinline__ void update_tile(double* M, int bi, int pn, int lane) {
+// Tile (bi, bj) -= sum_{k0 <= k < k1} L(bi, k) L(bj, k)^T by one warp.  FP64: two accumulators and
+// the next pair's operands in flight, so that neither loads nor products wait for one another.
+__device__ __forceinline__ void update_tile(double* M, int bi, int bj, int k0, int k1, int lane) {
   const int g = lane >> 2, t = lane & 3;
   const int p0 = tile_pos(g, t), p1 = tile_pos(g, t + 4);
-  const double* A = M + tile_at(bi, 0);
-  const double* B = M + tile_at(pn, 0);
-  double2* c = reinterpret_cast<double2*>(M + tile_at(bi, pn) + tile_pos(g, 2 * t));
+  const double* A = M + tile_at(bi, k0);
+  const double* B = M + tile_at(bj, k0);
+  double2* c = reinterpret_cast<double2*>(M + tile_at(bi, bj) + tile_pos(g, 2 * t));
   double2 v = *c, w = make_double2(0.0, 0.0);
-  int k = 0;
-#pragma unroll 2
-  for (; k + 1 < pn; k += 2) {
-    const double a0 = -A[64 * k + p0], a1 = -A[64 * k + p1];
-    const double a2 = -A[64 * k + 64 + p0], a3 = -A[64 * k + 64 + p1];
-    const double b0 = B[64 * k + p0], b1 = B[64 * k + p1];
-    const double b2 = B[64 * k + 64 + p0], b3 = B[64 * k + 64 + p1];
+  const int n = k1 - k0;
+  double a[4] = {}, b[4] = {};
+  auto fetch = [&](int k) {  // products k and k + 1 (the last one twice when n is odd)
+    const int k2 = k + 1 < n ? 64 * (k + 1) : 64 * k;
+    a[0] = A[64 * k + p0];
+    a[1] = A[64 * k + p1];
+    a[2] = A[k2 + p0];
+    a[3] = A[k2 + p1];
+    b[0] = -B[64 * k + p0];
+    b[1] = -B[64 * k + p1];
+    b[2] = -B[k2 + p0];
+    b[3] = -B[k2 + p1];
+  };
+  if (n > 0) fetch(0);
+  for (int k = 0; k < n; k += 2) {
+    const double a0 = a[0], a1 = a[1], a2 = a[2], a3 = a[3];
+    const double b0 = b[0], b1 = b[1], b2 = b[2], b3 = b[3];
+    if (k + 2 < n) fetch(k + 2);
     mma_f64(v.x, v.y, a0, b0);
-    mma_f64(w.x, w.y, a2, b2);
+    if (k + 1 < n) mma_f64(w.x, w.y, a2, b2);
     mma_f64(v.x, v.y, a1, b1);
-    mma_f64(w.x, w.y, a3, b3);
-  }
-  if (k < pn) {
-    mma_f64(v.x, v.y, -A[64 * k + p0], B[64 * k + p0]);
-    mma_f64(w.x, w.y, -A[64 * k + p1], B[64 * k + p1]);
+    if (k + 1 < n) mma_f64(w.x, w.y, a3, b3);
   }
   *c = make_double2(v.x + w.x, v.y + w.y);
 }
-__device__ __forceinline__ void update_tile(float* M, int bi, int pn, int lane) {
+__device__ __forceinline__ void update_tile(float* M, int bi, int bj, int k0, int k1, int lane) {
   const int g = lane >> 2, t = lane & 3;
   const float* A = M + tile_at(bi, 0);
-  const float* B = M + tile_at(pn, 0);
-  float2* c = reinterpret_cast<float2*>(M + tile_at(bi, pn) + tile_pos(g, 2 * t));
+  const float* B = M + tile_at(bj, 0);
+  float2* c = reinterpret_cast<float2*>(M + tile_at(bi, bj) + tile_pos(g, 2 * t));
   float2 v = *c;
 #pragma unroll 2
-  for (int k = 0; k < pn; k++) {
+  for (int k = k0; k < k1; k++) {
     float a[8], b0[8], b1[8];
     load_row8(A + 64 * k, g, a);
     load_row8(B + 64 * k, 2 * t, b0);
@@ -115,81 +131,129 @@ __device__ __forceinline__ void update_tile(float* M, int bi, int pn, int lane) 
   *c = v;
 }
 
+// Factor of a diagonal tile by one warp: lanes 0-7 hold its rows (x[j], j <= lane, in; the factor's
+// rows out), any other lane a row v that becomes v L^{-T}.  What a column needs of the other rows
+// is shuffled before its pivot is known (unscaled), so the chain from pivot to pivot is one
+// reciprocal square root, one product and one fma.  False when a pivot is not positive, or
+// not above rel_floor times its original diagonal.
+template <typename F>
+__device__ __forceinline__ bool diag_factor(F (&x)[8], const F* diag0, F rel_floor) {
+  bool ok = true;
+  F low[8];
+#pragma unroll
+  for (int c = 0; c < 8; c++) low[c] = rel_floor * diag0[c];
+  F d = wshfl(x[0], 0);
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    F w[8], v = (F)0;
+#pragma unroll
+    for (int j = c + 1; j < 8; j++) w[j] = wshfl(x[c], j);
+    if (c < 7) v = wshfl(x[c + 1], c + 1);
+    ok = ok & (d > (F)0) & (d > low[c]);
+    const F r = mrsqrt(d);
+    if (c < 7) {
+      const F l = w[c + 1] * r;
+      d = mfma(-l, l, v);
+    }
+    const F s = x[c] * (r * r);
+    x[c] *= r;
+#pragma unroll
+    for (int j = c + 1; j < 8; j++) x[j] = mfma(-s, w[j], x[j]);
+  }
+  return ok;
+}
+
+// Tile T <- T L^{-T}, Di the transposed inverse of L, by one warp.
+__device__ __forceinline__ void solve_tile(double* T, const double* Di, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  const double a0 = T[tile_pos(g, t)], a1 = T[tile_pos(g, t + 4)];
+  double2 v = make_double2(0.0, 0.0);
+  __syncwarp();
+  mma_f64(v.x, v.y, a0, Di[tile_pos(t, g)]);
+  mma_f64(v.x, v.y, a1, Di[tile_pos(t + 4, g)]);
+  *reinterpret_cast<double2*>(T + tile_pos(g, 2 * t)) = v;
+}
+__device__ __forceinline__ void solve_tile(float* T, const float* Di, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  float a[8];
+  load_row8(T, g, a);
+  float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const float2 b = *reinterpret_cast<const float2*>(Di + tile_pos(k, 2 * t));
+    v.x = fmaf(a[k], b.x, v.x);
+    v.y = fmaf(a[k], b.y, v.y);
+  }
+  __syncwarp();
+  *reinterpret_cast<float2*>(T + tile_pos(g, 2 * t)) = v;
+}
+
 // Factorises MM (nb blocks) in place by panels of 8 columns, left-looking, y (the right-hand side)
-// along with it, and leaves the transposed inverse of each diagonal tile in Di (a tile per panel,
-// for the backward substitution: eight more rows, those of the identity, go through the panel's
-// solve).  A pivot that is not positive, or not above
-// rel_floor times its original diagonal, fails the group (all threads return false).
-//   Per panel: a warp per tile subtracts the products of the panels before it (a right-looking
-//   update of every trailing tile per panel took 1,400 cycles a panel at K = 128, three times
-//   this: each product loaded and stored its tile); barrier; every thread that owns a row of the
-//   panel factors the diagonal tile for itself and solves its row; barrier.
+// along with it, and leaves the transposed inverse of each diagonal tile in Di (a tile per panel).
+// A pivot that is not positive, or not above rel_floor times its original diagonal, fails the
+// group (all threads return false).
+//   Per panel: warp 0 subtracts the last panel's product from the diagonal tile and factors it, with
+//   the identity's rows and y's among its lanes, while the other warps subtract all earlier
+//   panels' from the tiles below and from the next diagonal tile; barrier; the tiles below times the
+//   transposed inverse; barrier.  (Every row's owner factoring the diagonal tile for itself,
+//   without the second step, took 2,800 cycles a panel at K = 64 in FP64: 244 FP64 instructions
+//   a thread, in every warp.)
 template <typename F, int KP, int T>
 __device__ __forceinline__ bool wide_factor(F* M, F* y, F* Di, const F* diag0, int nb,
                                             F rel_floor, int tid, int grp, volatile int* bad) {
+  constexpr int W = T / 32;
   const int warp = tid >> 5, lane = tid & 31;
   for (int pn = 0; pn < nb; pn++) {
-    if (pn > 0) {
-      for (int bi = pn + warp; bi < nb; bi += T / 32) update_tile(M, bi, pn, lane);
-      // y's components from the panel on, by the panel before
-      const int j = 8 * pn + tid;
-      if (j < 8 * nb) {
-        F v[8], s = y[j];
-        load_row8(M + tile_at(j >> 3, pn - 1), j & 7, v);
+    // y's components by the panel before: the panel's own by warp 0, the others by warps 1 ..
+    const int j = warp == 0 ? 8 * pn + (lane & 7) : 8 * pn + 8 + tid - 32;
+    F s = (F)0;
+    if (pn > 0 && j < 8 * nb) {
+      F v[8];
+      load_row8(M + tile_at(j >> 3, pn - 1), j & 7, v);
+      s = y[j];
+      F s1 = (F)0;
 #pragma unroll
-        for (int c = 0; c < 8; c++) s = mfma(-v[c], y[8 * pn - 8 + c], s);
-        y[j] = s;
+      for (int c = 0; c < 8; c += 2) {
+        s = mfma(-v[c], y[8 * pn - 8 + c], s);
+        s1 = mfma(-v[c + 1], y[8 * pn - 7 + c], s1);
       }
-      group_sync<T>(grp);
+      s += s1;
     }
-    // rows 8 pn .. of the panel, the identity's, then y: one thread each
-    const int rows = 8 * (nb - pn);
-    F* own = tid < rows ? M + tile_at(pn + (tid >> 3), pn) : Di + 64 * pn;
-    F x[8];
-    if (tid <= rows + 8) {
-      const F* D = M + tile_at(pn, pn);
-      F l[8][8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) load_row8(D, i, l[i]);
-      if (tid == rows + 8) {
-#pragma unroll
-        for (int c = 0; c < 8; c++) x[c] = y[8 * pn + c];
-      } else if (tid >= rows) {
-#pragma unroll
-        for (int c = 0; c < 8; c++) x[c] = tid - rows == c ? (F)1 : (F)0;
+    if (warp == 0) {
+      if (pn > 0) {
+        update_tile(M, pn, pn, pn - 1, pn, lane);
+        if (lane < 8) y[j] = s;
+      }
+      __syncwarp();
+      // lanes 0-7: the tile's rows, 8-15: the identity's, 16: y
+      F* row = lane < 8 ? M + tile_at(pn, pn) : (lane < 16 ? Di + 64 * pn : y + 8 * pn);
+      const int r = lane < 16 ? lane & 7 : 0;
+      F x[8];
+      if (lane < 8 || lane == 16) {
+        load_row8(row, r, x);
       } else {
-        load_row8(own, tid & 7, x);
+#pragma unroll
+        for (int c = 0; c < 8; c++) x[c] = lane - 8 == c ? (F)1 : (F)0;
       }
-      bool ok = true;
-#pragma unroll
-      for (int c = 0; c < 8; c++) {
-        const F d = l[c][c];
-        ok = ok && d > (F)0 && d > rel_floor * diag0[8 * pn + c];
-        const F r = mrsqrt(d);
-#pragma unroll
-        for (int i = c + 1; i < 8; i++) l[i][c] *= r;
-        x[c] *= r;
-#pragma unroll
-        for (int j = c + 1; j < 8; j++) {
-#pragma unroll
-          for (int i = j; i < 8; i++) l[i][j] = mfma(-l[i][c], l[j][c], l[i][j]);
-          x[j] = mfma(-x[c], l[j][c], x[j]);
-        }
-      }
-      if (!ok && tid == 0) *bad = 1;
-      if (tid == rows + 8) {
-#pragma unroll
-        for (int c = 0; c < 8; c++) y[8 * pn + c] = x[c];
-      } else if (tid >= 8) {
-        store_row8(own, tid & 7, x);
+      __syncwarp();
+      const bool ok = diag_factor(x, diag0 + 8 * pn, rel_floor);
+      if (lane <= 16) store_row8(row, r, x);
+      if (!ok && lane == 0) *bad = 1;
+    } else {
+      if (pn > 0) {
+        if (j < 8 * nb) y[j] = s;
+        for (int bi = pn + warp; bi < nb; bi += W - 1) update_tile(M, bi, pn, 0, pn, lane);
+        // the next diagonal tile, by the warp whose turn is next
+        if (pn + 1 < nb && warp == 1 + (nb - pn - 1) % (W - 1))
+          update_tile(M, pn + 1, pn + 1, 0, pn, lane);
       }
     }
     group_sync<T>(grp);
     if (*bad) return false;
-    // the factored diagonal tile's rows only now: every owner has read the tile
-    if (tid < 8) store_row8(own, tid, x);
+    for (int bi = pn + 1 + warp; bi < nb; bi += W)
+      solve_tile(M + tile_at(bi, pn), Di + 64 * pn, lane);
+    group_sync<T>(grp);
   }
-  group_sync<T>(grp);
   return true;
 }
 
