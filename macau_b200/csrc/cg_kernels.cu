@@ -75,91 +75,111 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------- SpMM over a work split (DevCsr::tasks) ----------------
-// One warp per task (a whole row, or one part of a long row).  Entries are read four at a time
-// (independent gathers in flight) and added in CSR order.  A part stores its FP64 partial row in
-// A.parts; the last part of a row to finish (arrival counter) adds the parts in part order and
-// writes the row.  Whole rows give the same sums as k_spmm.
-template <typename V, int NRP>
+// One warp per task (a whole row, or one part of a long row).  LPE lanes share an entry, each with
+// two components (one 16-byte load in FP64), so 32 / LPE entries are read per load instruction and
+// eight such loads are in flight; the indices come 32 at a time by one coalesced load, the next 32
+// ahead.  A part stores its FP64 partial row in A.parts; the last part of a row to finish (arrival
+// counter) adds the parts in a fixed order and writes the row.
+//   What bounds it: for short tasks the latency of index and gather, for the others the gathers
+//   from L2 (256 bytes per entry at 32 components).  One 8-byte load per lane and entry, four in
+//   flight behind scalar index loads, took 52 us for the 4,099 columns (150,000 entries, parts
+//   of 256) of a 5,003-row feature matrix.
+template <typename V>
+struct Vec2;
+template <>
+struct Vec2<double> {
+  using T = double2;
+};
+template <>
+struct Vec2<float> {
+  using T = float2;
+};
+
+template <typename V, int LPE>
 __global__ void __launch_bounds__(256)
     k_spmm_split(const DevCsr A, const V* __restrict__ src, int sstride, V* __restrict__ dst,
                  int dstride, int ncomp, const V* __restrict__ add, int astride, double reg,
                  const double* __restrict__ reg_dev, const uint32_t* __restrict__ done) {
   if (done && *done) return;
-  constexpr int C = NRP / 32;
-  const int lane = threadIdx.x & 31;
+  using T2 = typename Vec2<V>::T;
+  constexpr int EPS = 32 / LPE, U = 8;  // entries per load, loads in flight
+  static_assert(EPS * U <= 32, "a step stays inside its chunk of 32 entries");
+  const int lane = threadIdx.x & 31, grp = lane / LPE, k0 = 2 * (lane % LPE);
   const int nw = gridDim.x * (blockDim.x >> 5);
   const bool weighted = sizeof(V) == 8 ? A.val != nullptr : A.valf != nullptr;
+  const V* base = src + k0;
+  auto combine = [](T2& v) {  // the groups' sums, by a fixed tree
+#pragma unroll
+    for (int o = LPE; o < 32; o <<= 1) {
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+      v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+    }
+  };
   for (int ti = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); ti < A.ntasks; ti += nw) {
     const RowTask tk = A.tasks[ti];
-    V acc[C];
-#pragma unroll
-    for (int c = 0; c < C; c++) acc[c] = (V)0;
-    const long long b = tk.begin, e = tk.begin + tk.len;
-    long long q = b;
-    for (; q + 4 <= e; q += 4) {
-      const V* s0 = src + (size_t)A.idx[q] * sstride;
-      const V* s1 = src + (size_t)A.idx[q + 1] * sstride;
-      const V* s2 = src + (size_t)A.idx[q + 2] * sstride;
-      const V* s3 = src + (size_t)A.idx[q + 3] * sstride;
-      V w0 = (V)1, w1 = (V)1, w2 = (V)1, w3 = (V)1;
-      if (weighted) {
-        if constexpr (sizeof(V) == 8) {
-          w0 = (V)A.val[q]; w1 = (V)A.val[q + 1]; w2 = (V)A.val[q + 2]; w3 = (V)A.val[q + 3];
-        } else {
-          w0 = (V)A.valf[q]; w1 = (V)A.valf[q + 1]; w2 = (V)A.valf[q + 2]; w3 = (V)A.valf[q + 3];
-        }
+    T2 acc{};
+    auto load_chunk = [&](int off, int& c, V& w) {
+      const bool in = off + lane < tk.len;
+      c = in ? A.idx[tk.begin + off + lane] : 0;
+      w = (V)1;
+      if (weighted && in) {
+        if constexpr (sizeof(V) == 8) w = (V)A.val[tk.begin + off + lane];
+        else w = (V)A.valf[tk.begin + off + lane];
       }
+    };
+    int c_cur, c_nxt = 0;
+    V w_cur, w_nxt = (V)1;
+    load_chunk(0, c_cur, w_cur);
+    for (int off = 0; off < tk.len; off += 32) {
+      load_chunk(off + 32, c_nxt, w_nxt);
 #pragma unroll
-      for (int c = 0; c < C; c++) {
-        const int k = lane + 32 * c;
-        if (k < ncomp) {
-          const V x0 = s0[k], x1 = s1[k], x2 = s2[k], x3 = s3[k];
-          if (weighted) {
-            acc[c] += x0 * w0;
-            acc[c] += x1 * w1;
-            acc[c] += x2 * w2;
-            acc[c] += x3 * w3;
-          } else {
-            acc[c] += x0;
-            acc[c] += x1;
-            acc[c] += x2;
-            acc[c] += x3;
+      for (int u = 0; u < 32; u += EPS * U) {
+        if (off + u < tk.len) {
+          T2 x[U];
+#pragma unroll
+          for (int i = 0; i < U; i++) {
+            const int en = u + i * EPS + grp;
+            const int col = __shfl_sync(0xffffffffu, c_cur, en);
+            x[i] = T2{};
+            if (off + en < tk.len)
+              x[i] = *reinterpret_cast<const T2*>(base + (size_t)col * sstride);
+          }
+#pragma unroll
+          for (int i = 0; i < U; i++) {
+            if (weighted) {
+              const V w = __shfl_sync(0xffffffffu, w_cur, u + i * EPS + grp);
+              acc.x += x[i].x * w;
+              acc.y += x[i].y * w;
+            } else {
+              acc.x += x[i].x;
+              acc.y += x[i].y;
+            }
           }
         }
       }
+      c_cur = c_nxt;
+      w_cur = w_nxt;
     }
-    for (; q < e; q++) {
-      const V* s0 = src + (size_t)A.idx[q] * sstride;
-      V w0 = (V)1;
-      if (weighted) {
-        if constexpr (sizeof(V) == 8) w0 = (V)A.val[q];
-        else w0 = (V)A.valf[q];
-      }
-#pragma unroll
-      for (int c = 0; c < C; c++) {
-        const int k = lane + 32 * c;
-        if (k < ncomp) acc[c] += weighted ? s0[k] * w0 : s0[k];
-      }
-    }
+    combine(acc);
     const V r = (V)(reg_dev ? *reg_dev : reg);
-    if (tk.nparts == 1) {
+    auto write = [&](V x, V y) {
+      if (grp != 0) return;
+      const V o[2] = {x, y};
 #pragma unroll
-      for (int c = 0; c < C; c++) {
-        const int k = lane + 32 * c;
-        if (k < ncomp) {
-          V o = acc[c];
-          if (add) o += r * add[(size_t)tk.row * astride + k];
-          dst[(size_t)tk.row * dstride + k] = o;
+      for (int c = 0; c < 2; c++)
+        if (k0 + c < ncomp) {
+          V v = o[c];
+          if (add) v += r * add[(size_t)tk.row * astride + k0 + c];
+          dst[(size_t)tk.row * dstride + k0 + c] = v;
         }
-      }
+    };
+    if (tk.nparts == 1) {
+      write(acc.x, acc.y);
       continue;
     }
-    double* pp = A.parts + (size_t)(tk.slot + tk.part) * 64;
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-      const int k = lane + 32 * c;
-      if (k < ncomp) pp[k] = (double)acc[c];
-    }
+    if (grp == 0)
+      *reinterpret_cast<double2*>(A.parts + (size_t)(tk.slot + tk.part) * 64 + k0) =
+          make_double2((double)acc.x, (double)acc.y);
     __threadfence();
     __syncwarp();
     unsigned last = 0;
@@ -167,18 +187,20 @@ __global__ void __launch_bounds__(256)
     last = __shfl_sync(0xffffffffu, last, 0);
     if (!last) continue;
     __threadfence();
-    const double* p0 = A.parts + (size_t)tk.slot * 64;
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-      const int k = lane + 32 * c;
-      if (k < ncomp) {
-        double t = 0.0;
-        for (int pt = 0; pt < tk.nparts; pt++) t += __ldcg(p0 + (size_t)pt * 64 + k);
-        V o = (V)t;
-        if (add) o += r * add[(size_t)tk.row * astride + k];
-        dst[(size_t)tk.row * dstride + k] = o;
-      }
+    const double* p0 = A.parts + (size_t)tk.slot * 64 + k0;
+    double2 t = make_double2(0.0, 0.0);
+#pragma unroll 8
+    for (int pt = grp; pt < tk.nparts; pt += EPS) {
+      const double2 v = __ldcg(reinterpret_cast<const double2*>(p0 + (size_t)pt * 64));
+      t.x += v.x;
+      t.y += v.y;
     }
+#pragma unroll
+    for (int o = LPE; o < 32; o <<= 1) {
+      t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+      t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+    }
+    write((V)t.x, (V)t.y);
     if (lane == 0) A.split_cnt[tk.split] = 0u;
   }
 }
@@ -742,8 +764,13 @@ void spmm_t(const DevCsr& A, const V* src, int sstride, V* dst, int dstride, int
             const V* add, int astride, double reg, const double* reg_dev, cudaStream_t s,
             const uint32_t* done = nullptr) {
   if (A.tasks) {
-    k_spmm_split<V, NRP><<<grid_for(A.ntasks, 8), 256, 0, s>>>(
-        A, src, sstride, dst, dstride, ncomp, add, astride, reg, reg_dev, done);
+    // lanes per entry: two components each, rounded up to a power of two (the rows are padded to
+    // 32 or 64 components, so the lanes past ncomp read padding and write nothing)
+    const auto kern = ncomp <= 16   ? k_spmm_split<V, 8>
+                      : ncomp <= 32 ? k_spmm_split<V, 16>
+                                    : k_spmm_split<V, 32>;
+    kern<<<grid_for(A.ntasks, 8), 256, 0, s>>>(A, src, sstride, dst, dstride, ncomp, add, astride,
+                                               reg, reg_dev, done);
     MG_CUDA(cudaGetLastError());
     return;
   }

@@ -132,15 +132,16 @@ struct ModeData {
 };
 
 // Work split of a CSR for the side-information SpMMs (k_spmm_split): rows longer than
-// max(256, nnz / (64 warps per SM)) entries are cut into parts, so the long feature columns of a
-// Zipf-distributed F do not serialise on one warp.
+// max(128, nnz / (64 warps per SM)) entries are cut into parts, so the long feature columns of a
+// Zipf-distributed F do not serialise on one warp (16 or 32 entries are in flight per warp, so
+// a part of 128 is 4 to 8 gather latencies).
 struct SpmmSplit {
   DBuf<RowTask> tasks;
   DBuf<unsigned> cnt;
   DBuf<double> parts;
   void build(const std::vector<long long>& ptr, int num_sms, cudaStream_t s, DevCsr& A) {
     const long long nnz = ptr.empty() ? 0 : ptr.back();
-    const long long thr = std::max(256LL, nnz / ((long long)num_sms * 64));
+    const long long thr = std::max(128LL, nnz / ((long long)num_sms * 64));
     int nsplit = 0, nslots = 0;
     std::vector<RowTask> t = make_tasks(ptr, thr, 1, nsplit, nslots);
     tasks.upload(t.data(), t.size(), s);
