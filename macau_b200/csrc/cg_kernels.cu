@@ -12,6 +12,7 @@
 // residual replacement R = B - (F^T F + reg I) X every kReplaceEvery iterations.
 #include <cmath>
 
+#include "cg_small.cuh"
 #include "common.cuh"
 #include "kernels.h"
 #include "rng.cuh"
@@ -312,42 +313,6 @@ __device__ __forceinline__ double sum_part(const double* partials, int nparts, i
   return s;
 }
 
-// Left-looking lower Cholesky of the n x n matrix A (leading dimension ld) by one CTA, column by
-// column; thread i computes L(i, j).  On a non-positive pivot it stops and leaves column j and
-// the columns after it as they were, like the unchecked Eigen llt() the reference uses
-// (linop.h:287, 313): the caller's solves then read that partial factor.  Returns false then.
-__device__ bool cta_chol_n(double* A, int n, int ld) {
-  __syncthreads();
-  for (int j = 0; j < n; j++) {
-    double d = A[j + j * ld];
-    for (int p = 0; p < j; p++) d -= A[j + p * ld] * A[j + p * ld];
-    if (!(d > 0.0)) {
-      __syncthreads();
-      return false;
-    }
-    const double ljj = sqrt(d);
-    for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) {
-      double s = A[i + j * ld];
-      for (int p = 0; p < j; p++) s -= A[i + p * ld] * A[j + p * ld];
-      A[i + j * ld] = s / ljj;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) A[j + j * ld] = ljj;
-    __syncthreads();
-  }
-  return true;
-}
-
-// small layout (doubles): RtR[64*64] | RtR2[64*64] | M[64*64] | A[64*64] | Psi[64*64] | norms[64]
-//                         | inorms[64] | flags[4]
-constexpr int kSq = 64 * 64;
-struct SmallView {
-  double *RtR, *RtR2, *M, *A, *Psi, *norms, *inorms, *flags;
-  __host__ __device__ explicit SmallView(double* s)
-      : RtR(s), RtR2(s + kSq), M(s + 2 * kSq), A(s + 3 * kSq), Psi(s + 4 * kSq),
-        norms(s + 5 * kSq), inorms(s + 5 * kSq + 64), flags(s + 5 * kSq + 128) {}
-};
-
 // RtR = sum partials (full matrix from the lower triangle, A_mul_At_combo + makeSymmetric)
 __global__ void k_cg_rtr(const double* partials, int nparts, int NRP, int n, double* small) {
   SmallView v(small);
@@ -389,94 +354,12 @@ __global__ void k_cg_init(const double* __restrict__ B, int bstride, long long n
   }
 }
 
-// Out(c, i) = (M^{-T} M^{-1} Rhs)(i, c) for the n columns of Rhs, M the lower Cholesky factor
-// in v.M (leading dimension 64): thread c solves column c, forward then backward substitution in
-// the order of the reference's llt().solve.  The general path (n > 32, or a failed pivot).
-__device__ void cta_chol_solve_cols(const double* M, const double* Rhs, int n, double* Out) {
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    double y[64];
-    for (int i = 0; i < n; i++) y[i] = Rhs[i + c * 64];
-    for (int i = 0; i < n; i++) {
-      double s = y[i];
-      for (int p = 0; p < i; p++) s -= M[i + p * 64] * y[p];
-      y[i] = s / M[i + i * 64];
-    }
-    for (int i = n - 1; i >= 0; i--) {
-      double s = y[i];
-      for (int p = i + 1; p < n; p++) s -= M[p + i * 64] * y[p];
-      y[i] = s / M[i + i * 64];
-    }
-    for (int i = 0; i < n; i++) Out[c + i * 64] = y[i];
-  }
-}
-
 constexpr int kSolveThreads = 256;
-constexpr int kLcLd = 36;
-
-// The same solves for n <= 32 with the factor in registers: warp 0 factorises the SPD matrix Ms
-// (lower triangle, padded with the identity beyond n) by warp_factor, publishing L^T in Lc;
-// then warp w solves columns w, w + 8, ...: lane i holds L(i, j) for j <= i and L(j, i) for
-// j > i and runs each substitution as 32 shuffle steps.  Returns false, with Out untouched, when
-// a pivot is not positive (the caller then takes the general path).
-__device__ bool warp_chol_solve(const double (*Ms)[33], double* Lc, const double* Rhs, int n,
-                                double* Out, int* okf) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0) {
-    double a[32], rinv = 1.0, d0 = 1.0;
-#pragma unroll
-    for (int j = 0; j < 32; j++) {
-      double x;
-      if (lane < n && j < n) x = j <= lane ? Ms[lane][j] : Ms[j][lane];
-      else x = lane == j ? 1.0 : 0.0;
-      a[j] = x;
-      if (j == lane) d0 = x;
-    }
-    const bool ok = warp_factor<double, 32>(a, rinv, lane, 0.0, d0, Lc, kLcLd);
-    if (lane == 0) *okf = ok ? 1 : 0;
-  }
-  __syncthreads();
-  if (!*okf) return false;
-  double m[32], dinv = 1.0;
-#pragma unroll
-  for (int j = 0; j < 32; j++) {
-    m[j] = j <= lane ? Lc[j * kLcLd + lane] : Lc[lane * kLcLd + j];
-    if (j == lane) dinv = 1.0 / m[j];
-  }
-  for (int c = warp; c < n; c += kSolveThreads / 32) {
-    double y = lane < n ? Rhs[lane + c * 64] : 0.0;
-#pragma unroll
-    for (int j = 0; j < 32; j++) {
-      if (lane == j) y *= dinv;
-      const double yj = __shfl_sync(0xffffffffu, y, j);
-      if (lane > j) y = fma(-m[j], yj, y);
-    }
-#pragma unroll
-    for (int j = 31; j >= 0; j--) {
-      if (lane == j) y *= dinv;
-      const double xj = __shfl_sync(0xffffffffu, y, j);
-      if (lane < j) y = fma(-m[j], xj, y);
-    }
-    if (lane < n) Out[c + lane * 64] = y;
-  }
-  return true;
-}
-
 // A = (chol(PtKP) \ RtR)^T  (linop.h:286-289); PtKP from the lower triangle of sum P KP^T.
 __global__ void __launch_bounds__(kSolveThreads, 1)
     k_cg_solve_a(const double* partials, int nparts, int NRP, int n, double* small, Ctl* ctl) {
   if (ctl->cg_done) return;
-  __shared__ double Ms[32][33];
-  __shared__ __align__(16) double Lc[32 * kLcLd];
-  __shared__ int okf;
   SmallView v(small);
-  if (n <= 32) {
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-      const int i = e % n, j = e / n;
-      if (i >= j) Ms[i][j] = sum_part(partials, nparts, NRP, i, j);
-    }
-    __syncthreads();
-    if (warp_chol_solve(Ms, Lc, v.RtR, n, v.A, &okf)) return;
-  }
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
     const int i = e % n, j = e / n;
     if (i >= j) v.M[i + j * 64] = sum_part(partials, nparts, NRP, i, j);  // P(i) . KP(j)
@@ -492,9 +375,6 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
     k_cg_solve_psi(const double* partials, int nparts, int NRP, int n, double tolsq,
                    double* small, Ctl* ctl, int* flag_out, int iter) {
   if (ctl->cg_done) return;
-  __shared__ double Ms[32][33];
-  __shared__ __align__(16) double Lc[32 * kLcLd];
-  __shared__ int okf;
   SmallView v(small);
   __shared__ int conv;
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
@@ -530,24 +410,13 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
     }
   }
   if (conv) return;
-  bool fast = false;
-  if (n <= 32) {
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-      const int i = e % n, j = e / n;
-      if (i >= j) Ms[i][j] = v.RtR[i + j * 64];
-    }
-    __syncthreads();
-    fast = warp_chol_solve(Ms, Lc, v.RtR2, n, v.Psi, &okf);
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+    const int i = e % n, j = e / n;
+    v.M[i + j * 64] = v.RtR[i + j * 64];
   }
-  if (!fast) {
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-      const int i = e % n, j = e / n;
-      v.M[i + j * 64] = v.RtR[i + j * 64];
-    }
-    cta_chol_n(v.M, n, 64);
-    __syncthreads();
-    cta_chol_solve_cols(v.M, v.RtR2, n, v.Psi);
-  }
+  cta_chol_n(v.M, n, 64);
+  __syncthreads();
+  cta_chol_solve_cols(v.M, v.RtR2, n, v.Psi);
   __syncthreads();
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
     const int i = e % n, j = e / n;
@@ -796,20 +665,24 @@ int cg_core(const DevCsr& F, const DevCsr& Ft, double reg, const double* reg_dev
   if (n < NRP)
     MG_CUDA(cudaMemset2DAsync(Bn + n, NRP * sizeof(double), 0, (NRP - n) * sizeof(double),
                               nfeat, s));
-  outer<double, NRP>(Bn, Bn, nfeat, partials, nb, s);
-  sum_records(partials, nb, NRP * NRP, reduced, s);
-  k_cg_norms<<<1, 64, 0, s>>>(reduced, 1, NRP, n, small);
-  MG_CUDA(cudaGetLastError());
-  k_cg_init<V><<<eg, 256, 0, s>>>(Bn, NRP, nfeat, n, NRP, small, R, P, Xd,
-                                  sizeof(V) == 4 ? Bn : nullptr, ctl);
-  MG_CUDA(cudaGetLastError());
-  outer<V, NRP>(R, R, nfeat, partials, nb, s);
-  sum_records(partials, nb, NRP * NRP, reduced, s);
-  k_cg_rtr<<<1, 256, 0, s>>>(reduced, 1, NRP, n, small);
-  MG_CUDA(cudaGetLastError());
+  if constexpr (NRP == 32) {
+    Cg32<V>::start(Bn, nfeat, n, R, P, Xd, sizeof(V) == 4 ? Bn : nullptr, small, partials, ctl, s);
+  } else {
+    outer<double, NRP>(Bn, Bn, nfeat, partials, nb, s);
+    sum_records(partials, nb, NRP * NRP, reduced, s);
+    k_cg_norms<<<1, 64, 0, s>>>(reduced, 1, NRP, n, small);
+    MG_CUDA(cudaGetLastError());
+    k_cg_init<V><<<eg, 256, 0, s>>>(Bn, NRP, nfeat, n, NRP, small, R, P, Xd,
+                                    sizeof(V) == 4 ? Bn : nullptr, ctl);
+    MG_CUDA(cudaGetLastError());
+    outer<V, NRP>(R, R, nfeat, partials, nb, s);
+    sum_records(partials, nb, NRP * NRP, reduced, s);
+    k_cg_rtr<<<1, 256, 0, s>>>(reduced, 1, NRP, n, small);
+    MG_CUDA(cudaGetLastError());
+  }
   const double tolsq = tol * tol;
   const int rg = (int)((nfeat + kRowTile - 1) / kRowTile);
-  {
+  if constexpr (NRP != 32) {
     static bool configured[64] = {false};
     int dev = 0;
     MG_CUDA(cudaGetDevice(&dev));
@@ -833,27 +706,37 @@ int cg_core(const DevCsr& F, const DevCsr& Ft, double reg, const double* reg_dev
     for (int b = 0; b < kCgBatch && iter < max_iter; b++, iter++) {
       spmm_t<V, NRP>(F, P, NRP, inner, NRP, n, nullptr, 0, 0.0, nullptr, s, done);
       spmm_t<V, NRP>(Ft, inner, NRP, KPm, NRP, n, P, NRP, reg, reg_dev, s, done);
-      outer<V, NRP>(P, KPm, nfeat, partials, nb, s, done);
-      sum_records(partials, nb, NRP * NRP, reduced, s, done);
-      k_cg_solve_a<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, small, ctl);
-      MG_CUDA(cudaGetLastError());
-      k_cg_rows<V, NRP, true><<<rg, 256, rows_smem(NRP, true), s>>>(nfeat, n, small, P, KPm, R,
-                                                                    Xd, nullptr, done);
-      MG_CUDA(cudaGetLastError());
-      if (sizeof(V) == 4 && (iter + 1) % kReplaceEvery == 0) {
+      const bool replace = sizeof(V) == 4 && (iter + 1) % kReplaceEvery == 0;
+      if constexpr (NRP == 32) {
+        Cg32<V>::step_a(nfeat, n, P, KPm, R, Xd, small, partials, !replace, ctl, s);
+      } else {
+        outer<V, NRP>(P, KPm, nfeat, partials, nb, s, done);
+        sum_records(partials, nb, NRP * NRP, reduced, s, done);
+        k_cg_solve_a<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, small, ctl);
+        MG_CUDA(cudaGetLastError());
+        k_cg_rows<V, NRP, true><<<rg, 256, rows_smem(NRP, true), s>>>(nfeat, n, small, P, KPm, R,
+                                                                      Xd, nullptr, done);
+        MG_CUDA(cudaGetLastError());
+      }
+      if (replace) {
         spmm_t<double, NRP>(F, Xd, NRP, innerd, NRP, n, nullptr, 0, 0.0, nullptr, s, done);
         spmm_t<double, NRP>(Ft, innerd, NRP, KX, NRP, n, Xd, NRP, reg, reg_dev, s, done);
         k_cg_resid<V><<<eg, 256, 0, s>>>(nfeat * NRP, NRP, n, Bn, KX, R, done);
         MG_CUDA(cudaGetLastError());
+        if constexpr (NRP == 32) Cg32<V>::rr(nfeat, R, partials, ctl, s);
       }
-      outer<V, NRP>(R, R, nfeat, partials, nb, s, done);
-      sum_records(partials, nb, NRP * NRP, reduced, s, done);
-      k_cg_solve_psi<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, tolsq, small, ctl, flag_dev,
-                                                 iter);
-      MG_CUDA(cudaGetLastError());
-      k_cg_rows<V, NRP, false><<<rg, 256, rows_smem(NRP, false), s>>>(nfeat, n, small, P, nullptr,
-                                                                       R, nullptr, P, done);
-      MG_CUDA(cudaGetLastError());
+      if constexpr (NRP == 32) {
+        Cg32<V>::step_psi(nfeat, n, R, P, small, partials, tolsq, ctl, flag_dev, iter, s);
+      } else {
+        outer<V, NRP>(R, R, nfeat, partials, nb, s, done);
+        sum_records(partials, nb, NRP * NRP, reduced, s, done);
+        k_cg_solve_psi<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, tolsq, small, ctl, flag_dev,
+                                                   iter);
+        MG_CUDA(cudaGetLastError());
+        k_cg_rows<V, NRP, false><<<rg, 256, rows_smem(NRP, false), s>>>(nfeat, n, small, P, nullptr,
+                                                                         R, nullptr, P, done);
+        MG_CUDA(cudaGetLastError());
+      }
     }
     MG_CUDA(cudaStreamSynchronize(s));
     if (flag_host[0]) {

@@ -292,29 +292,7 @@ __global__ void __launch_bounds__(kNwThreads, 1)
     Y[tile_at(b, b) + tile_pos(r, c)] = Di[64 * b + tile_pos(c, r)];
   }
   __syncthreads();
-  // Below them: a warp per block column, Y(i, j) = -Y(i, i) sum_k M(i, k) Y(k, j)
-  for (int bj = warp; bj < nb; bj += kNwThreads / 32)
-    for (int bi = bj + 1; bi < nb; bi++) {
-      double s[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-      for (int k = bj; k < bi; k++) {
-        const double* A = M + tile_at(bi, k);
-        const double* B = Y + tile_at(k, bj);
-        mma_f64(s[0][0], s[0][1], A[tile_pos(g, t)], B[tile_pos(t, g)]);
-        mma_f64(s[1][0], s[1][1], A[tile_pos(g, t + 4)], B[tile_pos(t + 4, g)]);
-      }
-      double* out = Y + tile_at(bi, bj);
-      *reinterpret_cast<double2*>(out + tile_pos(g, 2 * t)) =
-          make_double2(s[0][0] + s[1][0], s[0][1] + s[1][1]);
-      __syncwarp();
-      const double* A = Y + tile_at(bi, bi);
-      const double b0 = out[tile_pos(t, g)], b1 = out[tile_pos(t + 4, g)];
-      double2 v = make_double2(0.0, 0.0);
-      __syncwarp();
-      mma_f64(v.x, v.y, -A[tile_pos(g, t)], b0);
-      mma_f64(v.x, v.y, -A[tile_pos(g, t + 4)], b1);
-      *reinterpret_cast<double2*>(out + tile_pos(g, 2 * t)) = v;
-      __syncwarp();
-    }
+  for (int bj = warp; bj < nb; bj += kNwThreads / 32) inverse_column(M, Y, bj, nb, lane);
   __syncthreads();
   // B = L c^T over M, L(i, j) = Y(n-1-j, n-1-i)
   for (int q = warp; q < nb * (nb + 1) / 2; q += kNwThreads / 32) {

@@ -296,4 +296,32 @@ __device__ __forceinline__ void wide_back(const F* M, F* y, const F* Di, F* x, i
   }
 }
 
+// Block column bj of Y = L^{-1} below its diagonal tile, by one warp: Y(i, j) = -Y(i, i) sum_k
+// L(i, k) Y(k, j).  Y's diagonal tiles are in place.
+__device__ __forceinline__ void inverse_column(const double* L, double* Y, int bj, int nb,
+                                               int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  for (int bi = bj + 1; bi < nb; bi++) {
+    double s[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    for (int k = bj; k < bi; k++) {
+      const double* A = L + tile_at(bi, k);
+      const double* B = Y + tile_at(k, bj);
+      mma_f64(s[0][0], s[0][1], A[tile_pos(g, t)], B[tile_pos(t, g)]);
+      mma_f64(s[1][0], s[1][1], A[tile_pos(g, t + 4)], B[tile_pos(t + 4, g)]);
+    }
+    double* out = Y + tile_at(bi, bj);
+    *reinterpret_cast<double2*>(out + tile_pos(g, 2 * t)) =
+        make_double2(s[0][0] + s[1][0], s[0][1] + s[1][1]);
+    __syncwarp();
+    const double* A = Y + tile_at(bi, bi);
+    const double b0 = out[tile_pos(t, g)], b1 = out[tile_pos(t + 4, g)];
+    double2 v = make_double2(0.0, 0.0);
+    __syncwarp();
+    mma_f64(v.x, v.y, -A[tile_pos(g, t)], b0);
+    mma_f64(v.x, v.y, -A[tile_pos(g, t + 4)], b1);
+    *reinterpret_cast<double2*>(out + tile_pos(g, 2 * t)) = v;
+    __syncwarp();
+  }
+}
+
 }  // namespace mg
