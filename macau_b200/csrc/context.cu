@@ -209,6 +209,9 @@ class Context {
     }
     MG_CUDA(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, dev_));
     MG_CUDA(cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking));
+    MG_CUDA(cudaStreamCreateWithFlags(&s_eval_, cudaStreamNonBlocking));
+    MG_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
+    MG_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
     ctl_.alloc_zero(1, s_);
     for (int m = 0; m < 2; m++) prior_[m].df = K_;
     MG_CUDA(cudaEventCreate(&ev0_));
@@ -219,6 +222,12 @@ class Context {
     drop_graphs();
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
+    if (s_eval_) {
+      cudaStreamSynchronize(s_eval_);  // its work reads buffers that are freed next
+      cudaStreamDestroy(s_eval_);
+    }
+    if (ev_fork_) cudaEventDestroy(ev_fork_);
+    if (ev_join_) cudaEventDestroy(ev_join_);
     if (s_) cudaStreamDestroy(s_);
   }
 
@@ -765,12 +774,13 @@ class Context {
                        cfg_.seed, mode, p.lambda_beta.p, s_);
   }
 
-  void eval(int n_fixed) {
+  void eval(int n_fixed) { eval_on(n_fixed, s_); }
+  void eval_on(int n_fixed, cudaStream_t s) {
     if (ntest_ == 0) return;
     launches_ += 2;
     launch_eval(trow_.p, tcol_.p, tval_.p, ntest_, latents(0), latents(1), mixed_, K_, KP_,
                 mean_, n_fixed, ctl_.p, pred_.p, pvar_.p, eval_partials_.p,
-                eval_blocks(ntest_), rmse_.p, s_);
+                eval_blocks(ntest_), rmse_.p, s);
   }
 
   // AdaptiveGaussianNoise::update (noisemodels.cpp:55-81); nothing under fixed noise.
@@ -828,6 +838,14 @@ class Context {
     if (ev) MG_CUDA(cudaEventRecord(ev[1], s_));
     sample(1, nullptr, false, ev ? ev[7] : nullptr);
     if (ev) MG_CUDA(cudaEventRecord(ev[2], s_));
+    // The evaluation reads the latents and the sweep index only, so it runs beside the prior and
+    // noise updates, whose chains of small kernels leave most of the GPU idle, and is joined
+    // before the sweep index moves on.  The phase-timed sweeps keep it on its own.
+    const bool beside = do_eval && !ev && ntest_ > 0;
+    if (beside) {
+      MG_CUDA(cudaEventRecord(ev_fork_, s_));
+      MG_CUDA(cudaStreamWaitEvent(s_eval_, ev_fork_, 0));
+    }
     if (!ev && pair_priors()) {
       update_priors_pair();
     } else {
@@ -837,7 +855,11 @@ class Context {
     }
     if (ev) MG_CUDA(cudaEventRecord(ev[4], s_));
     update_noise();  // noise.update between the priors and the evaluation (macau.cpp:130-132)
-    if (do_eval) eval(-1);
+    if (beside) {
+      eval_on(-1, s_eval_);
+      MG_CUDA(cudaEventRecord(ev_join_, s_eval_));
+      MG_CUDA(cudaStreamWaitEvent(s_, ev_join_, 0));
+    } else if (do_eval) eval(-1);
     launch_advance(ctl_.p, s_);
     launches_ += 1;
     if (ev) MG_CUDA(cudaEventRecord(ev[5], s_));
@@ -1409,6 +1431,9 @@ class Context {
   bool mixed_ = false;
   int dev_ = 0, num_sms_ = 148;
   cudaStream_t s_ = nullptr;
+  // evaluation beside the prior updates (sweep_body): forked from and joined to s_ in every sweep
+  cudaStream_t s_eval_ = nullptr;
+  cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
   long long dims_[2] = {0, 0};
   long long ntrain_ = 0, ntest_ = 0;

@@ -52,25 +52,60 @@ __global__ void k_lambda_beta(const double* __restrict__ bb_partials, int nparts
 
 constexpr int kEvalThreads = 256;
 
-// Groups of eight lanes take eight consecutive test entries at a time: for each entry the
-// group reads the two latent rows with vector loads (lane l: elements 4l .. 4l + 3, + 32 j) and
-// sums the partial dots with three shuffles; lane j keeps entry j's prediction and then does
-// the online mean / variance update of eval_rmse (bpmfutils.h:86-114) for it, so the updates
-// and their pred / pvar / value accesses run on all eight lanes.  Per block, the squared errors
-// are summed in lane and group order into partials[2 * block .. + 1].
+// Dots of eight consecutive entries by a group of eight lanes: entry j of the group has the rows
+// (r, c) of its lane j; the lanes read its two latent rows with vector loads (lane l: elements
+// 4l .. 4l + 3, + 32 i), four entries' loads in flight, and the 8 x 8 partial sums are transposed and
+// added in three exchange steps (7 shuffles instead of 24).  Returns the dot of the lane's entry.
 template <typename T>
 __device__ __forceinline__ double dot4(const T* u, const T* v) {
   if constexpr (sizeof(T) == 4) {
-    const float4 a = *reinterpret_cast<const float4*>(u), b = *reinterpret_cast<const float4*>(v);
+    const float4 a = __ldg(reinterpret_cast<const float4*>(u));
+    const float4 b = __ldg(reinterpret_cast<const float4*>(v));
     return (double)a.x * (double)b.x + (double)a.y * (double)b.y + (double)a.z * (double)b.z +
            (double)a.w * (double)b.w;
   } else {
-    const double2 a0 = *reinterpret_cast<const double2*>(u), a1 = *reinterpret_cast<const double2*>(u + 2);
-    const double2 b0 = *reinterpret_cast<const double2*>(v), b1 = *reinterpret_cast<const double2*>(v + 2);
+    const double2 a0 = __ldg(reinterpret_cast<const double2*>(u));
+    const double2 a1 = __ldg(reinterpret_cast<const double2*>(u + 2));
+    const double2 b0 = __ldg(reinterpret_cast<const double2*>(v));
+    const double2 b1 = __ldg(reinterpret_cast<const double2*>(v + 2));
     return a0.x * b0.x + a0.y * b0.y + a1.x * b1.x + a1.y * b1.y;
   }
 }
+template <typename T>
+__device__ __forceinline__ double group_dots(const T* __restrict__ U, const T* __restrict__ V,
+                                             int stride, int K, int r, int c, int l, unsigned mask) {
+  double d[8];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const T *u[4], *v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      u[j] = U + (size_t)__shfl_sync(mask, r, 4 * h + j, 8) * stride + 4 * l;
+      v[j] = V + (size_t)__shfl_sync(mask, c, 4 * h + j, 8) * stride + 4 * l;
+      d[4 * h + j] = 0.0;
+    }
+    for (int k0 = 4 * l; k0 < K; k0 += 32)
+#pragma unroll
+      for (int j = 0; j < 4; j++) d[4 * h + j] += dot4<T>(u[j] + (k0 - 4 * l), v[j] + (k0 - 4 * l));
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int j = 0; j < o; j++) {
+      const bool hi = (l & o) != 0;
+      const double keep = hi ? d[j + o] : d[j], send = hi ? d[j] : d[j + o];
+      d[j] = keep + __shfl_xor_sync(mask, send, o);
+    }
+  return d[0];
+}
 
+// Online mean / variance update of eval_rmse (bpmfutils.h:86-114): each lane keeps the entry whose
+// dot it holds, so the updates and their pred / pvar / value accesses run on all eight lanes.  Per
+// block, the squared errors are summed in lane and group order into partials[2 * block .. + 1].
+//   What bounds it: the gathers of the latent rows from L2.  The test arrays are read and written
+//   once a sweep, past the caches (ld.cs, st.cs): at 2M entries their 96 MB would push the latents
+//   and the samplers' entries out of L2, which cost the sweep more (160 us mixed, 257 us FP64 at
+//   K = 32) than this kernel takes.
 template <typename T>
 __global__ void __launch_bounds__(kEvalThreads)
     k_eval(const int* __restrict__ trow, const int* __restrict__ tcol,
@@ -85,37 +120,39 @@ __global__ void __launch_bounds__(kEvalThreads)
   const unsigned mask = 0xffu << (8 * ((threadIdx.x & 31) >> 3));
   double se = 0.0, sea = 0.0;
   const long long step = (long long)gridDim.x * kGroups * 8;
-  for (long long t0 = ((long long)blockIdx.x * kGroups + g) * 8; t0 < ntest; t0 += step) {
-    const long long t = t0 + l;  // this lane's entry
+  const bool first = n == 0;
+  // the next step's entry is loaded while this one's rows are gathered
+  int r = 0, c = 0;
+  double y = 0.0, old = 0.0, oldv = 0.0;
+  auto fetch = [&](long long t) {
     const bool own = t < ntest;
-    const int r = own ? trow[t] : 0, c = own ? tcol[t] : 0;
-    double mydot = 0.0;
-#pragma unroll 2
-    for (int j = 0; j < 8; j++) {
-      const int rj = __shfl_sync(mask, r, j, 8), cj = __shfl_sync(mask, c, j, 8);
-      const T* u = U + (size_t)rj * stride;
-      const T* v = V + (size_t)cj * stride;
-      double dot = 0.0;
-      for (int k0 = 4 * l; k0 < K; k0 += 32) dot += dot4<T>(u + k0, v + k0);
-      dot += __shfl_xor_sync(mask, dot, 4, 8);
-      dot += __shfl_xor_sync(mask, dot, 2, 8);
-      dot += __shfl_xor_sync(mask, dot, 1, 8);
-      if (l == j) mydot = dot;
-    }
-    if (own) {
+    r = own ? __ldcs(trow + t) : 0;
+    c = own ? __ldcs(tcol + t) : 0;
+    y = own ? __ldcs(tval + t) : 0.0;
+    old = own && !first ? __ldcs(pred + t) : 0.0;
+    oldv = own && !first ? __ldcs(pvar + t) : 0.0;
+  };
+  long long t0 = ((long long)blockIdx.x * kGroups + g) * 8;
+  if (t0 < ntest) fetch(t0 + l);
+  for (; t0 < ntest; t0 += step) {
+    const long long t = t0 + l;  // this lane's entry
+    const int r_t = r, c_t = c;
+    const double y_t = y, old_t = old, oldv_t = oldv;
+    if (t0 + step < ntest) fetch(t + step);
+    const double mydot = group_dots<T>(U, V, stride, K, r_t, c_t, l, mask);
+    if (t < ntest) {
       const double p = mydot + mean;
-      const double y = tval[t];
-      se += (y - p) * (y - p);
+      se += (y_t - p) * (y_t - p);
       double pavg;
-      if (n == 0) {
+      if (first) {
         pavg = p;
       } else {
-        const double delta = p - pred[t];
-        pavg = pred[t] + delta / (n + 1);
-        pvar[t] += delta * (p - pavg);
+        const double delta = p - old_t;
+        pavg = old_t + delta / (n + 1);
+        __stcs(pvar + t, oldv_t + delta * (p - pavg));
       }
-      sea += (y - pavg) * (y - pavg);
-      pred[t] = pavg;
+      sea += (y_t - pavg) * (y_t - pavg);
+      __stcs(pred + t, pavg);
     }
   }
   // group sums in lane order
@@ -181,8 +218,7 @@ __global__ void k_entry_rows(const long long* __restrict__ ptr, long long nrows,
 
 // Squared training residuals of AdaptiveGaussianNoise::update (noisemodels.cpp:55-72):
 // (U_i . V_j + mean - y)^2 over the entries (i = erow[e], j = col[e], y = val[e]).  Same
-// group layout as k_eval: eight lanes share the dot of one entry through vector loads and three
-// shuffles, lane l keeps entry t0 + l; the per-block sum goes to partials[block] in lane and
+// group layout as k_eval, lane l keeps entry t0 + l; the per-block sum goes to partials[block] in lane and
 // group order.
 template <typename T>
 __global__ void __launch_bounds__(kEvalThreads)
@@ -196,25 +232,24 @@ __global__ void __launch_bounds__(kEvalThreads)
   const unsigned mask = 0xffu << (8 * ((threadIdx.x & 31) >> 3));
   double se = 0.0;
   const long long step = (long long)gridDim.x * kGroups * 8;
-  for (long long t0 = ((long long)blockIdx.x * kGroups + g) * 8; t0 < nnz; t0 += step) {
-    const long long t = t0 + l;
+  // the next step's entry is loaded while this one's rows are gathered
+  int r = 0, c = 0;
+  double y = 0.0;
+  auto fetch = [&](long long t) {
     const bool own = t < nnz;
-    const int r = own ? erow[t] : 0, c = own ? col[t] : 0;
-    double mydot = 0.0;
-#pragma unroll 2
-    for (int j = 0; j < 8; j++) {
-      const int rj = __shfl_sync(mask, r, j, 8), cj = __shfl_sync(mask, c, j, 8);
-      const T* u = U + (size_t)rj * stride;
-      const T* v = V + (size_t)cj * stride;
-      double dot = 0.0;
-      for (int k0 = 4 * l; k0 < K; k0 += 32) dot += dot4<T>(u + k0, v + k0);
-      dot += __shfl_xor_sync(mask, dot, 4, 8);
-      dot += __shfl_xor_sync(mask, dot, 2, 8);
-      dot += __shfl_xor_sync(mask, dot, 1, 8);
-      if (l == j) mydot = dot;
-    }
-    if (own) {
-      const double d = (mydot + mean) - val[t];
+    r = own ? __ldcs(erow + t) : 0;
+    c = own ? __ldcs(col + t) : 0;
+    y = own ? __ldcs(val + t) : 0.0;
+  };
+  long long t0 = ((long long)blockIdx.x * kGroups + g) * 8;
+  if (t0 < nnz) fetch(t0 + l);
+  for (; t0 < nnz; t0 += step) {
+    const int r_t = r, c_t = c;
+    const double y_t = y;
+    if (t0 + step < nnz) fetch(t0 + step + l);
+    const double mydot = group_dots<T>(U, V, stride, K, r_t, c_t, l, mask);
+    if (t0 + l < nnz) {
+      const double d = (mydot + mean) - y_t;
       se += d * d;
     }
   }
