@@ -686,7 +686,7 @@ class Context {
   }
 
   // Both modes have the plain BPMF prior: the sweep updates them together
-  // (launch_prior_pair: three launches instead of six, the same result bit for bit).  The
+  // (launch_prior_pair: fewer launches, the same result bit for bit).  The
   // phase-timed sweeps keep one mode after the other, so each mode's prior is timed alone.
   bool pair_priors() const {
     return !prior_[0].macau && !prior_[0].one && !prior_[1].macau && !prior_[1].one;
@@ -708,24 +708,26 @@ class Context {
       pp.mu[m] = p.mu.p;
       pp.Lambda[m] = p.Lambda.p;
     }
-    launch_prior_pair(pp, mixed_, K_, KP_, ctl_.p, cfg_.seed, s_);
-    launches_ += 3;
+    launches_ += launch_prior_pair(pp, mixed_, K_, KP_, ctl_.p, cfg_.seed, s_);
   }
 
   void update_prior(int mode) {
     Prior& p = prior_[mode];
     const long long N = dims_[mode];
-    launches_ += p.macau ? 0 : 3;  // Macau launches are counted by kernels_in_cg below
     const int nb = stats_blocks(N);
+    const bool few = few_parts(nb, K_);
+    launches_ += p.macau ? 0 : few ? 2 : 3;  // Macau launches are counted by kernels_in_cg below
     const int rec = K_ + K_ * K_;
     launch_stats(latents(mode), mixed_, p.side() ? p.uhat.p : nullptr, N, K_, KP_, KP_,
                  stat_partials_.p, nb, s_);
-    launch_reduce_parts(stat_partials_.p, nb, rec, stat_final_.p, s_);
+    if (!few) launch_reduce_parts(stat_partials_.p, nb, rec, stat_final_.p, s_);
+    const double* stats = few ? stat_partials_.p : stat_final_.p;
+    const int nstats = few ? nb : 1;
     if (p.one) {
       // MacauOnePrior::update_prior (macauoneprior.cpp:189-194): sample_mu_lambda (Normal-Wishart
       // of U - Uhat with mu0 = 0, kappa = 2, W0 = I, nu = K, the BPMF defaults), sample_beta,
       // compute_uhat, sample_lambda_beta
-      launch_normal_wishart(stat_final_.p, 1, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr, 0,
+      launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr, 0,
                             nullptr, ctl_.p, cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
       launch_beta_one(p.Ft, p.colsq.p, p.lvl_ptr.p, p.lvl_feat.p, p.lvl_range.p, p.lvl_warp.p,
                       p.nlevels,
@@ -739,7 +741,7 @@ class Context {
       return;
     }
     if (!p.macau) {  // BPMFPrior::update_prior (latentprior.cpp:79-81)
-      launch_normal_wishart(stat_final_.p, 1, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr, 0,
+      launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr, 0,
                             nullptr, ctl_.p, cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
       return;
     }
@@ -747,7 +749,7 @@ class Context {
     const int nbb = stats_blocks(p.nfeat);
     launch_stats(p.beta.p, false, nullptr, p.nfeat, K_, CP_, 0, p.bb_partials.p, nbb, s_);
     launch_reduce_parts(p.bb_partials.p, nbb, rec, p.bb_final.p, s_);
-    launch_normal_wishart(stat_final_.p, 1, N, K_, p.mu0.p, p.b0, p.WI.p, p.df + (int)p.nfeat,
+    launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df + (int)p.nfeat,
                           p.bb_final.p, 1, p.lambda_beta.p, ctl_.p, cfg_.seed, mode, p.mu.p,
                           p.Lambda.p, s_);
     // sample_beta (latentprior.cpp:273-293)

@@ -2,8 +2,7 @@
 //
 //   k_stats32         per-block partial sums of x and x x^T over the rows of a latent matrix, K <=
 //                     32 (optionally x = U - Uhat, the Macau residual of latentprior.cpp:257);
-//                     FP64 accumulation from FP64 or FP32 latents, 4 x 4 register tiles of the
-//                     outer product (four row groups per block, summed in group order).
+//                     FP64 accumulation from FP64 or FP32 latents on the FP64 matrix instruction.
 //   k_nw32            one CTA, K <= 32: CondNormalWishart -> NormalWishart -> Wishart/WishartUnit
 //                     -> MvNormal_prec (mvnormal.cpp:169-184, 217-287, 314-336) in FP64 with keyed
 //                     draws; shared-memory matrices, warp-register Cholesky factors
@@ -14,6 +13,7 @@
 //                     the test predictions and the two RMSEs.
 #include "common.cuh"
 #include "kernels.h"
+#include "mma_tiles.cuh"
 #include "rng.cuh"
 #include "warp_finish.cuh"
 
@@ -21,7 +21,6 @@ namespace mg {
 namespace {
 
 constexpr int kStatThreads = 256;
-constexpr int kStatRows = 32;  // rows staged per step
 
 // lambda_beta ~ Gamma(nux/2, 2 mux/nux), nux = nu + K nfeat,
 // mux = mu nux / (nu + mu tr(B B^T Lambda))   (latentprior.cpp:317-331)
@@ -294,96 +293,96 @@ __global__ void k_set_sweep(Ctl* ctl, uint32_t sweep, int burnin) {
 
 __global__ void k_advance(Ctl* ctl) { ctl->sweep += 1u; }
 
-// Column sums and outer-product sums of rows r0 .. r1 - 1 of (U - Uhat) for K <= 32: thread t
-// owns the 4 x 4 tile (4 (t % 64) / 8 .., 4 (t % 8) ..) for the rows of row group t / 64 (every
-// fourth staged row); the four groups are summed in group order at the end.  The next 32 rows
-// are loaded into registers while the current ones are multiplied (double-buffered staging).
-template <typename T>
-__device__ __forceinline__ void stats_load(const T* U, const double* Uhat, long long b0, int cnt,
-                                           int K, int stride, int uhat_stride, int t,
-                                           double (&nx)[4]) {
+// One block's statistics (column sums and outer-product sums) over rows r0 .. r1 - 1 of (U - Uhat),
+// K <= 8 NB, into out[0 .. K + K*K) (k_stats32, k_stats32_pair and the batched k_stats_batch).  Warp
+// w takes the four rows 4 (w + 8 i) .. of the block, lane (g, t) = (lane / 4, lane % 4) component
+// 8 b + g of row t, which is the operand element of block b on either side of m8n8k4.f64: the
+// lower-triangle tiles take NB (NB + 1) / 2 matrix instructions per four rows, on operands loaded
+// straight from memory three steps ahead.  The warps' tiles are added in warp order.
+//   What bounds it: latency; 4 x 4 DFMA tiles over rows staged in shared memory took 42 us for both
+//   modes of 138,000 x 27,000 at K = 32, and 126 us on average for 64 problems of up to 4,000 rows.
+constexpr int kStatWarps = kStatThreads / 32;
+template <typename T, int NB>
+__device__ __forceinline__ void stats32_blocks(const T* __restrict__ U,
+                                               const double* __restrict__ Uhat, long long r0,
+                                               long long r1, int K, int stride, int uhat_stride,
+                                               double* __restrict__ out, double* buf) {
+  constexpr int TILES = NB * (NB + 1) / 2, R = 4, REC = TILES * 64 + 8 * NB;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double acc[TILES][2], su[NB], f[R][NB];
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int e = t + kStatThreads * q, r = e >> 5, k = e & 31;
-    double x = 0.0;
-    if (r < cnt && k < K) {
-      x = (double)U[(b0 + r) * stride + k];
-      if (Uhat) x -= Uhat[(b0 + r) * uhat_stride + k];
+  for (int q = 0; q < TILES; q++) acc[q][0] = acc[q][1] = 0.0;
+#pragma unroll
+  for (int b = 0; b < NB; b++) su[b] = 0.0;
+  auto load = [&](int stage, long long row) {
+    const T* u = U + row * stride + g;
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+      const bool ok = row < r1 && 8 * b + g < K;
+      double x = ok ? (double)__ldg(u + 8 * b) : 0.0;
+      if (Uhat) x -= ok ? __ldg(Uhat + row * uhat_stride + g + 8 * b) : 0.0;
+      f[stage][b] = x;
     }
-    nx[q] = x;
+  };
+  const long long first = r0 + 4 * warp + t;
+  constexpr int STEP = 4 * kStatWarps;
+#pragma unroll
+  for (int u = 0; u < R - 1; u++) load(u, first + STEP * u);
+  for (long long r = first - t; r < r1; r += R * STEP) {
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      load((u + R - 1) % R, r + t + STEP * (u + R - 1));
+      int q = 0;
+#pragma unroll
+      for (int a = 0; a < NB; a++) {
+        su[a] += f[u][a];
+#pragma unroll
+        for (int b = 0; b <= a; b++) {
+          mma_f64(acc[q][0], acc[q][1], f[u][a], f[u][b]);
+          q++;
+        }
+      }
+    }
+  }
+  double* mine = buf + warp * REC;
+#pragma unroll
+  for (int q = 0; q < TILES; q++)
+    *reinterpret_cast<double2*>(mine + q * 64 + g * 8 + 2 * t) = make_double2(acc[q][0], acc[q][1]);
+#pragma unroll
+  for (int b = 0; b < NB; b++) {
+    su[b] += __shfl_xor_sync(0xffffffffu, su[b], 1);
+    su[b] += __shfl_xor_sync(0xffffffffu, su[b], 2);
+    if (t == 0) mine[TILES * 64 + 8 * b + g] = su[b];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < REC; e += kStatThreads) {
+    double v = buf[e];
+#pragma unroll
+    for (int w = 1; w < kStatWarps; w++) v += buf[w * REC + e];
+    if (e >= TILES * 64) {
+      if (e - TILES * 64 < K) out[e - TILES * 64] = v;
+      continue;
+    }
+    int a = 0;
+    while ((a + 1) * (a + 2) / 2 <= (e >> 6)) a++;
+    const int b = (e >> 6) - a * (a + 1) / 2;
+    const int i = 8 * a + ((e >> 3) & 7), j = 8 * b + (e & 7);
+    if (i < K && j < K) {
+      out[K + i + j * K] = v;
+      if (a != b) out[K + j + i * K] = v;
+    }
   }
 }
 
-// One block's statistics over rows r0 .. r1 - 1 into out[0 .. K + K*K) (shared by k_stats32 and
-// the batched k_stats32_batch).
 template <typename T>
 __device__ __forceinline__ void stats32_rows(const T* __restrict__ U,
                                              const double* __restrict__ Uhat, long long r0,
                                              long long r1, int K, int stride, int uhat_stride,
                                              double* __restrict__ out) {
-  static_assert(kStatRows * 32 == 4 * kStatThreads, "four staged values per thread");
-  __shared__ __align__(16) double xs[2][kStatRows][36];
-  __shared__ double red[3][64][17];
-  const int KK = K * K;
-  const int t = threadIdx.x, tile = t & 63, rg = t >> 6;
-  const int ti = tile >> 3, tj = tile & 7;
-  double acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
-  double su = 0.0;
-  double nx[4];
-  stats_load(U, Uhat, r0, (int)max(0LL, min((long long)kStatRows, r1 - r0)), K, stride,
-             uhat_stride, t, nx);
-  int buf = 0;
-  for (long long b0 = r0; b0 < r1; b0 += kStatRows) {
-    const int cnt = (int)min((long long)kStatRows, r1 - b0);
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int e = t + kStatThreads * q;
-      xs[buf][e >> 5][e & 31] = nx[q];
-    }
-    __syncthreads();
-    const long long nb0 = b0 + kStatRows;
-    if (nb0 < r1)
-      stats_load(U, Uhat, nb0, (int)min((long long)kStatRows, r1 - nb0), K, stride, uhat_stride,
-                 t, nx);
-    if (t < K)
-      for (int r = 0; r < cnt; r++) su += xs[buf][r][t];
-#pragma unroll 2
-    for (int r = rg; r < kStatRows; r += 4) {
-      const double2 i01 = *reinterpret_cast<const double2*>(&xs[buf][r][4 * ti]);
-      const double2 i23 = *reinterpret_cast<const double2*>(&xs[buf][r][4 * ti + 2]);
-      const double2 j01 = *reinterpret_cast<const double2*>(&xs[buf][r][4 * tj]);
-      const double2 j23 = *reinterpret_cast<const double2*>(&xs[buf][r][4 * tj + 2]);
-      const double xi[4] = {i01.x, i01.y, i23.x, i23.y}, xj[4] = {j01.x, j01.y, j23.x, j23.y};
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = fma(xi[a], xj[b], acc[a][b]);
-    }
-    buf ^= 1;
-  }
-  __syncthreads();
-  if (rg > 0)
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-      for (int b = 0; b < 4; b++) red[rg - 1][tile][a * 4 + b] = acc[a][b];
-  __syncthreads();
-  if (t < K) out[t] = su;
-  if (rg == 0) {
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-      for (int b = 0; b < 4; b++) {
-        const double v = ((acc[a][b] + red[0][tile][a * 4 + b]) + red[1][tile][a * 4 + b]) +
-                         red[2][tile][a * 4 + b];
-        const int i = 4 * ti + a, j = 4 * tj + b;
-        if (i < K && j < K) out[K + i + j * K] = v;
-      }
-  }
+  __shared__ __align__(16) double buf[kStatWarps * (10 * 64 + 32)];
+  if (K <= 8) stats32_blocks<T, 1>(U, Uhat, r0, r1, K, stride, uhat_stride, out, buf);
+  else if (K <= 16) stats32_blocks<T, 2>(U, Uhat, r0, r1, K, stride, uhat_stride, out, buf);
+  else stats32_blocks<T, 4>(U, Uhat, r0, r1, K, stride, uhat_stride, out, buf);
 }
 
 template <typename T>
@@ -430,8 +429,17 @@ __global__ void __launch_bounds__(256)
 constexpr int kNwLd = 33;
 constexpr int kNwLc = 36;
 
-// T0 == null stands for the identity.
-__device__ __forceinline__ void nw32_run(const double* __restrict__ partials, int nparts,
+struct NwShared {
+  double A[32 * kNwLd], Bm[32 * kNwLd], C[32 * kNwLd], D[32 * kNwLd];
+  double Lc[32 * kNwLc];
+  double NU[32], muc[32], m0[32], rl[32], zs[32];
+  int flag;
+};
+
+// T0 == null stands for the identity.  The factor and the inverse run at the width KP = 8, 16 or 32
+// that holds K (nw32_run).
+template <int KP>
+__device__ __forceinline__ void nw32_width(NwShared& sh, const double* __restrict__ partials, int nparts,
                                          long long N, int K, const double* __restrict__ mu0,
                                          double kappa, const double* __restrict__ T0, int nu,
                                          const double* __restrict__ bb_partials, int bb_nparts,
@@ -439,10 +447,8 @@ __device__ __forceinline__ void nw32_run(const double* __restrict__ partials, in
                                          unsigned long long seed, int mode,
                                          double* __restrict__ mu_out,
                                          double* __restrict__ Lambda_out) {
-  __shared__ double A[32 * kNwLd], Bm[32 * kNwLd], C[32 * kNwLd], D[32 * kNwLd];
-  __shared__ __align__(16) double Lc[32 * kNwLc];
-  __shared__ double NU[32], muc[32], m0[32], rl[32], zs[32];
-  __shared__ int flag;
+  double *A = sh.A, *Bm = sh.Bm, *C = sh.C, *D = sh.D, *Lc = sh.Lc;
+  double *NU = sh.NU, *muc = sh.muc, *m0 = sh.m0, *rl = sh.rl, *zs = sh.zs;
   const int t = threadIdx.x, lane = t & 31;
   const int KK = K * K;
   const uint32_t sweep = ctl->sweep;
@@ -498,28 +504,33 @@ __device__ __forceinline__ void nw32_run(const double* __restrict__ partials, in
   __syncthreads();
   if (t < 32) {
     // 3a. M = chol(J X J), M^T rows into Lc
-    double a[32], d0 = 1.0, rinv = 1.0;
+    double a[KP], d0 = 1.0, rinv = 1.0;
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
+    for (int j = 0; j < KP; j++) {
       a[j] = (lane < K && j < K) ? A[(K - 1 - lane) * kNwLd + (K - 1 - j)] : (lane == j ? 1.0 : 0.0);
       if (j == lane) d0 = a[j];
     }
-    const bool ok = warp_factor<double, 32>(a, rinv, lane, 0.0, d0, Lc, kNwLc);
-    if (lane == 0) flag = ok ? 1 : 0;
-    // 3b. Y = M^{-1}: lane c solves M y = e_c; Y(i, c) into D
+    const bool ok = warp_factor<double, KP>(a, rinv, lane, 0.0, d0, Lc, kNwLc);
+    if (lane == 0) sh.flag = ok ? 1 : 0;
+    // 3b. Y = M^{-1}: lane c solves M y = e_c by columns (the updates of one column are
+    //     independent of one another); Y(i, c) into D
     if (ok) {
       rl[lane] = rinv;
       __syncwarp();
-      double y[32];
 #pragma unroll
-      for (int i = 0; i < 32; i++) {
-        double s = (lane == i) ? 1.0 : 0.0;
+      for (int i = 0; i < KP; i++) a[i] = lane == i ? 1.0 : 0.0;
 #pragma unroll
-        for (int q = 0; q < i; q++) s = fma(-Lc[q * kNwLc + i], y[q], s);
-        y[i] = s * rl[i];
+      for (int i = 0; i < KP; i++) {
+        const double y = a[i] * rl[i];
+        if (lane < KP) D[i * kNwLd + lane] = y;
+#pragma unroll
+        for (int q = (i + 1) / 4; q < KP / 4; q++) {
+          const Vec4<double> c = lds4(Lc + i * kNwLc + 4 * q);
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (4 * q + u > i) a[4 * q + u] = fma(-c.v[u], y, a[4 * q + u]);
+        }
       }
-#pragma unroll
-      for (int i = 0; i < 32; i++) D[i * kNwLd + lane] = y[i];
     }
   } else {
     // 3c. Bartlett factor c (upper) into C: c_ii = sqrt(2 Gamma((nu_c - i)/2)), c_ij ~ N(0,1);
@@ -538,7 +549,7 @@ __device__ __forceinline__ void nw32_run(const double* __restrict__ partials, in
     if (t - 32 < K) zs[t - 32] = normal_draw(seed, sweep, stream_id(kMuDraw, mode), 0u, (uint32_t)(t - 32));
   }
   __syncthreads();
-  if (!flag) {
+  if (!sh.flag) {
     if (t == 0) atomicOr(&ctl->status, kStatHyperFail);
     return;
   }
@@ -567,13 +578,34 @@ __device__ __forceinline__ void nw32_run(const double* __restrict__ partials, in
   // 7. mu = mu_c + B^{-T} z / sqrt(kappa_c)
   if (t < 32) {
     double x = lane < K ? zs[lane] / sqrt(kappa_c) : 0.0;
+    const double rb = lane < K ? 1.0 / Bm[lane * kNwLd + lane] : 0.0;
     for (int j = K - 1; j >= 0; j--) {
-      if (lane == j) x = x / Bm[j * kNwLd + j];
+      if (lane == j) x *= rb;
       const double xj = __shfl_sync(0xffffffffu, x, j);
       if (lane < j) x = fma(-Bm[j * kNwLd + lane], xj, x);
     }
     if (lane < K) mu_out[lane] = x + muc[lane];
   }
+}
+
+__device__ __forceinline__ void nw32_run(const double* __restrict__ partials, int nparts,
+                                         long long N, int K, const double* __restrict__ mu0,
+                                         double kappa, const double* __restrict__ T0, int nu,
+                                         const double* __restrict__ bb_partials, int bb_nparts,
+                                         const double* __restrict__ lambda_beta, Ctl* ctl,
+                                         unsigned long long seed, int mode,
+                                         double* __restrict__ mu_out,
+                                         double* __restrict__ Lambda_out) {
+  __shared__ __align__(16) NwShared sh;
+  if (K <= 8)
+    nw32_width<8>(sh, partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials, bb_nparts,
+                  lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
+  else if (K <= 16)
+    nw32_width<16>(sh, partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials, bb_nparts,
+                   lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
+  else
+    nw32_width<32>(sh, partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials, bb_nparts,
+                   lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
 }
 
 __global__ void __launch_bounds__(256)
@@ -622,16 +654,18 @@ __global__ void __launch_bounds__(256) k_reduce_parts_pair(PriorPair pp, int len
   }
 }
 
-__global__ void __launch_bounds__(256) k_nw32_pair(PriorPair pp, int K, Ctl* ctl,
+__global__ void __launch_bounds__(256) k_nw32_pair(PriorPair pp, int few, int K, Ctl* ctl,
                                                    unsigned long long seed) {
   const int m = blockIdx.x;
-  nw32_run(pp.final_[m], 1, pp.N[m], K, pp.mu0[m], pp.kappa[m], pp.T0[m], pp.nu[m], nullptr, 0,
-           nullptr, ctl, seed, m, pp.mu[m], pp.Lambda[m]);
+  const bool own = (few >> m) & 1;  // this block adds the mode's partials
+  nw32_run(own ? pp.partials[m] : pp.final_[m], own ? pp.nblocks[m] : 1, pp.N[m], K, pp.mu0[m],
+           pp.kappa[m], pp.T0[m], pp.nu[m], nullptr, 0, nullptr, ctl, seed, m, pp.mu[m],
+           pp.Lambda[m]);
 }
 
 }  // namespace
 
-void launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl,
+int launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl,
                        unsigned long long seed, cudaStream_t s) {
   const int nb = pp.nblocks[0] + pp.nblocks[1];
   if (K > 32)
@@ -641,13 +675,22 @@ void launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ct
   else
     k_stats32_pair<double><<<nb, kStatThreads, 0, s>>>(pp, K, stride);
   MG_CUDA(cudaGetLastError());
-  const int len = K + K * K;
-  k_reduce_parts_pair<<<2 * ((len + 31) / 32), 256, 0, s>>>(pp, len);
-  MG_CUDA(cudaGetLastError());
+  const int few = (few_parts(pp.nblocks[0], K) ? 1 : 0) | (few_parts(pp.nblocks[1], K) ? 2 : 0);
+  if (few != 3) {
+    const int len = K + K * K;
+    k_reduce_parts_pair<<<2 * ((len + 31) / 32), 256, 0, s>>>(pp, len);
+    MG_CUDA(cudaGetLastError());
+  }
   if (K > 32) launch_nw_wide_pair(pp, K, ctl, seed, s);
-  else k_nw32_pair<<<2, 256, 0, s>>>(pp, K, ctl, seed);
+  else k_nw32_pair<<<2, 256, 0, s>>>(pp, few, K, ctl, seed);
   MG_CUDA(cudaGetLastError());
+  return few == 3 ? 2 : 3;
 }
+
+// Up to 16 partials are added by the Normal-Wishart block itself: one CTA reads them in less time
+// than the reduction's launch takes (2,000 + 1,500 rows, 28 partials in all: a sweep of 47 us lost
+// 3 us); with more, its reads of up to 2.5 MB would cost more than they save.
+bool few_parts(int nblocks, int K) { return K <= 32 && nblocks <= 16; }
 
 int stats_blocks(long long N) {  // at most two blocks per SM: fewer partials to reduce
   long long b = (N + 127) / 128;

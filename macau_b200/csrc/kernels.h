@@ -81,6 +81,8 @@ bool launch_gram_tc(const SampleParams& p, float* gram, const int4* split_rows, 
 int stats_blocks(long long N);
 // Sums `nparts` records of `len` doubles (stats partials) into one record, in a fixed order.
 void launch_reduce_parts(const double* parts, int nparts, int len, double* out, cudaStream_t s);
+// Whether launch_normal_wishart is given the partials themselves (no launch_reduce_parts).
+bool few_parts(int nblocks, int K);
 void launch_stats(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
                   int uhat_stride, double* partials, int nblocks, cudaStream_t s);
 void launch_normal_wishart(const double* partials, int nparts, long long N, int K,
@@ -91,9 +93,10 @@ void launch_normal_wishart(const double* partials, int nparts, long long N, int 
 // Both modes' BPMF prior updates (BPMFPrior::update_prior, latentprior.cpp:79-81) at once:
 // statistics, reduction and Normal-Wishart draw of mode m from the latents U[m]
 // (N[m] rows, stride `stride`), partials[m] (nblocks[m] records, rows_per_block[m] rows each)
-// and final_[m] as work, into mu[m] / Lambda[m].  Three launches instead of six; each mode's
+// and final_[m] as work, into mu[m] / Lambda[m].  Two or three launches instead of up to six; each mode's
 // blocks compute what launch_stats / launch_reduce_parts / launch_normal_wishart compute, with
-// the same keyed draws, so the result is the same bit for bit.
+// the same keyed draws and the same few_parts rule, so the result is the same bit for bit.  Returns
+// the number of launches.
 struct PriorPair {
   const void* U[2];
   long long N[2];
@@ -108,7 +111,7 @@ struct PriorPair {
   double* mu[2];
   double* Lambda[2];
 };
-void launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl,
+int launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl,
                        unsigned long long seed, cudaStream_t s);
 // The K > 32 forms of the statistics and of the draw (hyper_wide.cu); the draw reads one record
 // of reduced statistics (and of beta beta^T, null without side information).
