@@ -193,29 +193,38 @@ __global__ void k_eval_batch(const int* __restrict__ trow, const int* __restrict
   }
 }
 
-// One warp per problem: RMSEs over its test segment (lane-strided sums, fixed xor tree);
-// rmse[2 p] = posterior mean, rmse[2 p + 1] = single sample (NaN without test entries).
-__global__ void k_rmse_batch(const long long* __restrict__ toff, int P,
-                             const double* __restrict__ se1, const double* __restrict__ sea,
-                             double* __restrict__ rmse) {
-  const int lane = threadIdx.x & 31;
-  for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < P;
-       p += (gridDim.x * blockDim.x) >> 5) {
-    double a = 0.0, b1 = 0.0;
-    for (long long t = toff[p] + lane; t < toff[p + 1]; t += 32) {
-      a += sea[t];
-      b1 += se1[t];
-    }
+// One block per problem: RMSEs over its test segment (thread-strided sums, a fixed xor tree per
+// warp, then the warps in order); rmse[2 p] = posterior mean, rmse[2 p + 1] = single sample (NaN
+// without test entries).  A warp per problem took 117 us for 64 problems of up to 17,000 entries.
+__global__ void __launch_bounds__(256)
+    k_rmse_batch(const long long* __restrict__ toff, const double* __restrict__ se1,
+                 const double* __restrict__ sea, double* __restrict__ rmse) {
+  __shared__ double ws[2][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = blockIdx.x;
+  double a = 0.0, b1 = 0.0;
+#pragma unroll 4
+  for (long long t = toff[p] + threadIdx.x; t < toff[p + 1]; t += 256) {
+    a += sea[t];
+    b1 += se1[t];
+  }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      b1 += __shfl_xor_sync(0xffffffffu, b1, o);
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b1 += __shfl_xor_sync(0xffffffffu, b1, o);
+  }
+  if (lane == 0) {
+    ws[0][warp] = a;
+    ws[1][warp] = b1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) {
+      a += ws[0][w];
+      b1 += ws[1][w];
     }
-    if (lane == 0) {
-      const double cnt = (double)(toff[p + 1] - toff[p]);
-      rmse[2 * p] = cnt > 0 ? sqrt(a / cnt) : NAN;
-      rmse[2 * p + 1] = cnt > 0 ? sqrt(b1 / cnt) : NAN;
-    }
+    const double cnt = (double)(toff[p + 1] - toff[p]);
+    rmse[2 * p] = cnt > 0 ? sqrt(a / cnt) : NAN;
+    rmse[2 * p + 1] = cnt > 0 ? sqrt(b1 / cnt) : NAN;
   }
 }
 
@@ -700,7 +709,7 @@ class Batch {
                                                            mean_d_.p, ctl_.p, pred_.p, pvar_.p,
                                                            se1_.p, sea_.p);
     MG_CUDA(cudaGetLastError());
-    k_rmse_batch<<<(P_ + 7) / 8, 256, 0, s_>>>(toff_.p, P_, se1_.p, sea_.p, rmse_.p);
+    k_rmse_batch<<<P_, 256, 0, s_>>>(toff_.p, se1_.p, sea_.p, rmse_.p);
     MG_CUDA(cudaGetLastError());
   }
 

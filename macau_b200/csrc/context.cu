@@ -387,13 +387,13 @@ class Context {
       for (int l = 0; l < nl; l++) lptr[l + 1] += lptr[l];
       std::vector<int> fill(lptr.begin(), lptr.end() - 1);
       for (int f = 0; f < nfeat; f++) order[fill[level[f]]++] = f;
-      // a level runs one warp per feature when it has many features or only short ones
+      // a level runs one warp per feature or each feature by the whole block
       std::vector<int> lwarp(nl, 1);
       for (int l = 0; l < nl; l++) {
         long long longest = 0;
         for (int q = lptr[l]; q < lptr[l + 1]; q++)
           longest = std::max(longest, t.ptr[order[q] + 1] - t.ptr[order[q]]);
-        lwarp[l] = (lptr[l + 1] - lptr[l] >= 8 || longest <= 1024) ? 1 : 0;
+        lwarp[l] = beta_one_warp_level(nrows, lptr[l + 1] - lptr[l], longest) ? 1 : 0;
       }
       p.colsq.upload(cs.data(), cs.size(), s_);
       p.lvl_warp.upload(lwarp.data(), lwarp.size(), s_);
@@ -736,8 +736,8 @@ class Context {
                       CP_, p.tmp.p, CP_, p.B.p, ctl_.p, cfg_.seed, mode, s_);
       launch_spmm(p.F, p.beta.p, CP_, p.uhat.p, KP_, K_, false, s_);
       launch_lambda_beta_one(p.beta.p, CP_, p.nfeat, K_, p.lb_a0, p.lb_b0, ctl_.p, cfg_.seed,
-                             mode, p.lb_one.p, s_);
-      launches_ += 4;  // draws, beta, spmm, lambda_beta (after the 3 of stats / reduce / NW)
+                             mode, p.B.p, p.lb_one.p, s_);
+      launches_ += 5;  // draws, beta, spmm, 2 of lambda_beta (after the 3 of stats / reduce / NW)
       return;
     }
     if (!p.macau) {  // BPMFPrior::update_prior (latentprior.cpp:79-81)

@@ -382,6 +382,7 @@ __device__ __forceinline__ void stats32_rows(const T* __restrict__ U,
   __shared__ __align__(16) double buf[kStatWarps * (10 * 64 + 32)];
   if (K <= 8) stats32_blocks<T, 1>(U, Uhat, r0, r1, K, stride, uhat_stride, out, buf);
   else if (K <= 16) stats32_blocks<T, 2>(U, Uhat, r0, r1, K, stride, uhat_stride, out, buf);
+  else if (K <= 24) stats32_blocks<T, 3>(U, Uhat, r0, r1, K, stride, uhat_stride, out, buf);
   else stats32_blocks<T, 4>(U, Uhat, r0, r1, K, stride, uhat_stride, out, buf);
 }
 

@@ -177,7 +177,8 @@ void launch_spmm(const DevCsr& A, const void* src, int src_stride, void* dst, in
 // Univariate prior (univariate_kernels.cu): MacauOnePrior::sample_beta over Ft (the columns of
 // F as CSR rows) with the feature levels lvl_ptr / lvl_feat (lvl_range: each listed feature's
 // entry range in Ft; lvl_warp: one warp per feature in that level), Z (N x zstride doubles) and draws
-// (nfeat x bstride doubles) as workspace; and sample_lambda_beta into lambda_beta[0 .. K).
+// (nfeat x bstride doubles) as workspace; and sample_lambda_beta into lambda_beta[0 .. K), with
+// `parts` (nfeat x bstride doubles) as workspace.
 void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
                      const int* lvl_feat, const longlong2* lvl_range, const int* lvl_warp,
                      int nlevels, const void* U, bool f32, int ustride,
@@ -187,7 +188,10 @@ void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
                      unsigned long long seed, int mode, cudaStream_t s);
 void launch_lambda_beta_one(const double* beta, int bstride, long long nfeat, int K, double a0,
                             double b0, const Ctl* ctl, unsigned long long seed, int mode,
-                            double* lambda_beta, cudaStream_t s);
+                            double* parts, double* lambda_beta, cudaStream_t s);
+// Whether a level of `nfeat` features, the longest of `longest` entries, runs a warp per feature
+// (lvl_warp) for a side matrix of N rows.
+bool beta_one_warp_level(long long N, long long nfeat, long long longest);
 
 // sample_beta pieces (latentprior.cpp:273-293)
 //   tmp[n] = U[n] + chol(Lambda)^{-T} z_n - mu      (n < N; z keyed (kMvnN, n))

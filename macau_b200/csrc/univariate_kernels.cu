@@ -143,43 +143,107 @@ __global__ void __launch_bounds__(kBetaThreads)
 
 // The same link sampler with one block per dimension d and this dimension's column of Z held in
 // shared memory (N doubles, N <= kZsMax), so the feature-by-feature chain reads and writes no
-// global memory but beta, with 32 warps per block and each feature's entry range (lvl_range)
-// read in one load.  The sums are formed as in k_beta_one (lane-strided then an xor tree in a
-// warp; thread-strided, per-warp trees, then the warps in order in a block).
+// global memory but beta, with 32 warps per block.
+//   What bounds it: the chain over the levels.  A level gives each of its features to a warp, or each
+// in turn to the whole block (lvl_warp, by the estimate of beta_one_warp_level).  While a feature is
+// processed, everything about the next one that no other feature changes is loaded: its entry
+// range, the first entries' rows, its coefficient and draw with the reciprocal and the square root
+// they are scaled by, and the next level's bounds.  The block's sum takes one barrier: every
+// warp adds the 32 warps' sums for itself by a shuffle tree.  (Reading each entry's row twice from
+// global memory, a warp for features of up to 1,024 entries and one thread to add the warps' sums,
+// 1,294 us for the 8,193 features, 250,000 entries and 32 dimensions of a 5,003-row matrix.)
 constexpr int kZsMax = 26 * 1024;
-
-// What a warp loads ahead about a feature: id, entry range, squared column norm, coefficient,
-// draw, and this lane's first entry (row, value).
-struct FeaturePre {
-  int f;
-  longlong2 rg;
-  double cs, b, z;
-  int i0;
-  double v0;
-};
-
-__device__ __forceinline__ FeaturePre fetch_feature(int q, int lane, int d,
-                                                   const int* __restrict__ lvl_feat,
-                                                   const longlong2* __restrict__ lvl_range,
-                                                   const double* __restrict__ colsq,
-                                                   const double* beta, int bstride,
-                                                   const double* __restrict__ draws,
-                                                   const int* __restrict__ tidx,
-                                                   const double* __restrict__ tval) {
-  FeaturePre r;
-  r.f = lvl_feat[q];
-  r.rg = lvl_range[q];
-  r.cs = colsq[r.f];
-  r.b = beta[(size_t)r.f * bstride + d];
-  r.z = draws[(size_t)r.f * bstride + d];
-  const long long e = r.rg.x + lane;
-  r.i0 = e < r.rg.y ? tidx[e] : 0;
-  r.v0 = e < r.rg.y ? (tval ? tval[e] : 1.0) : 0.0;
-  return r;
-}
 constexpr int kSmemThreads = 1024;
 constexpr int kSmemWarps = kSmemThreads / 32;
-template <typename T>
+
+// A feature's constants for one dimension, and the first NP entries of a thread that takes entries
+// first, first + stride, ...
+template <bool BINARY, int NP>
+struct FeaturePre {
+  int f, len;
+  long long begin;
+  double bcs, b, ainv, sz;
+  int i[NP];
+  double v[BINARY ? 1 : NP];
+};
+
+struct BetaOne {
+  const int* tidx;
+  const double* tval;
+  const double* colsq;
+  const int* lvl_feat;
+  const longlong2* lvl_range;
+  const double* draws;
+  double* beta;
+  int bstride;
+  double lam, lb;
+  int d;
+};
+
+template <bool BINARY, int NP>
+__device__ __forceinline__ FeaturePre<BINARY, NP> fetch_feature(const BetaOne& p, int q, int first,
+                                                               int stride) {
+  FeaturePre<BINARY, NP> r;
+  r.f = p.lvl_feat[q];
+  const longlong2 rg = p.lvl_range[q];
+  r.begin = rg.x;
+  r.len = (int)(rg.y - rg.x);
+  const double cs = p.colsq[r.f];
+  r.b = p.beta[(size_t)r.f * p.bstride + p.d];
+  r.bcs = r.b * cs;
+  r.ainv = 1.0 / (p.lb + p.lam * cs);
+  r.sz = sqrt(r.ainv) * p.draws[(size_t)r.f * p.bstride + p.d];
+#pragma unroll
+  for (int k = 0; k < NP; k++) {
+    const int e = first + k * stride;
+    r.i[k] = e < r.len ? p.tidx[r.begin + e] : -1;
+    if constexpr (!BINARY) r.v[k] = e < r.len ? p.tval[r.begin + e] : 0.0;
+  }
+  return r;
+}
+
+// sum of v Z over the thread's entries
+template <bool BINARY, int NP>
+__device__ __forceinline__ double feature_dot(const BetaOne& p, const FeaturePre<BINARY, NP>& r,
+                                              const double* Zs, int first, int stride) {
+  double zx = 0.0;
+#pragma unroll
+  for (int k = 0; k < NP; k++)
+    if (r.i[k] >= 0) zx = BINARY ? zx + Zs[r.i[k]] : fma(r.v[BINARY ? 0 : k], Zs[r.i[k]], zx);
+#pragma unroll 4
+  for (int e = first + NP * stride; e < r.len; e += stride) {
+    const double z = Zs[p.tidx[r.begin + e]];
+    zx = BINARY ? zx + z : fma(p.tval[r.begin + e], z, zx);
+  }
+  return zx;
+}
+// Z += v delta over the thread's entries (one entry per row of Z)
+template <bool BINARY, int NP>
+__device__ __forceinline__ void feature_add(const BetaOne& p, const FeaturePre<BINARY, NP>& r,
+                                            double* Zs, int first, int stride, double delta) {
+#pragma unroll
+  for (int k = 0; k < NP; k++)
+    if (r.i[k] >= 0)
+      Zs[r.i[k]] = BINARY ? Zs[r.i[k]] + delta : fma(r.v[BINARY ? 0 : k], delta, Zs[r.i[k]]);
+#pragma unroll 4
+  for (int e = first + NP * stride; e < r.len; e += stride) {
+    const int i = p.tidx[r.begin + e];
+    Zs[i] = BINARY ? Zs[i] + delta : fma(p.tval[r.begin + e], delta, Zs[i]);
+  }
+}
+// The new coefficient (macauoneprior.cpp:243-252) from the sum over the feature's entries.
+template <bool BINARY, int NP>
+__device__ __forceinline__ double new_coef(const BetaOne& p, const FeaturePre<BINARY, NP>& r,
+                                           double zx) {
+  return p.lam * (zx + r.bcs) * r.ainv + r.sz;
+}
+__device__ __forceinline__ double warp_sum(double x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+template <typename T, bool BINARY>
 __global__ void __launch_bounds__(kSmemThreads)
     k_beta_one_smem(const int* __restrict__ tidx, const double* __restrict__ tval,
                     const double* __restrict__ colsq, const int* __restrict__ lvl_ptr,
@@ -191,97 +255,79 @@ __global__ void __launch_bounds__(kSmemThreads)
                     int K, int N, double* __restrict__ beta, int bstride,
                     const double* __restrict__ draws) {
   extern __shared__ double Zs[];
-  __shared__ double red[kSmemWarps];
-  __shared__ double dl;
-  const int d = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double lam = Lambda[(size_t)d * (K + 1)], lb = lambda_beta[d];
-  for (int i = threadIdx.x; i < N; i += kSmemThreads)
+  __shared__ double red[2][kSmemWarps];
+  constexpr int NP = BINARY ? 4 : 2;  // entries held ahead per thread
+  const int d = blockIdx.x, tid = threadIdx.x;
+  const int warp = tid >> 5, lane = tid & 31;
+  const BetaOne p{tidx, tval, colsq, lvl_feat, lvl_range, draws, beta, bstride,
+                  Lambda[(size_t)d * (K + 1)], lambda_beta[d], d};
+  for (int i = tid; i < N; i += kSmemThreads)
     Zs[i] = (double)U[(size_t)i * ustride + d] - mu[d] - uhat[(size_t)i * hstride + d];
+  FeaturePre<BINARY, NP> cur{};
+  int cur_q = -1;  // the feature in `cur`, fetched for this thread's share of it, or -1
+  bool cur_block = false;
+  int buf = 0;
+  int f0 = 0, f1 = nlevels > 0 ? lvl_ptr[1] : 0, mode = nlevels > 0 ? lvl_warp[0] : 0;
   __syncthreads();
-  FeaturePre cur{};
-  int cur_q = -1;
-  bool have = false;
   for (int L = 0; L < nlevels; L++) {
-    const int f0 = lvl_ptr[L], f1 = lvl_ptr[L + 1];
-    if (lvl_warp[L]) {
-      // one feature per warp; while a feature is processed, the warp loads everything about its
-      // next one that no other feature changes (id, entry range, colsq, its coefficient and
-      // draw, the first 32 entries), including the first feature it takes in the next level
+    // the next level's bounds and mode
+    const bool more = L + 1 < nlevels;
+    const int f2 = more ? lvl_ptr[L + 2] : f1, mode2 = more ? lvl_warp[L + 1] : -1;
+    // the feature this thread meets first in the next level
+    const int q2 = !more ? -1 : mode2 == 0 ? f1 : (f1 + warp < f2 ? f1 + warp : -1);
+    const int first2 = mode2 == 0 ? tid : lane, stride2 = mode2 == 0 ? kSmemThreads : 32;
+    if (mode != 0) {
+      // one feature per warp
       int q = f0 + warp;
-      if (!(have && cur_q == q) && q < f1) {
-        cur = fetch_feature(q, lane, d, lvl_feat, lvl_range, colsq, beta, bstride, draws, tidx,
-                            tval);
+      if (q < f1 && (cur_q != q || cur_block)) {
+        cur = fetch_feature<BINARY, NP>(p, q, lane, 32);
         cur_q = q;
-        have = true;
+      }
+      if (q >= f1 && q2 >= 0) {  // nothing to do in this level
+        cur = fetch_feature<BINARY, NP>(p, q2, first2, stride2);
+        cur_q = q2;
+        cur_block = mode2 == 0;
       }
       for (; q < f1; q += kSmemWarps) {
-        int qn = q + kSmemWarps;
-        if (qn >= f1) {
-          qn = (L + 1 < nlevels && lvl_warp[L + 1] && f1 + warp < lvl_ptr[L + 2]) ? f1 + warp : -1;
-        }
-        FeaturePre nxt{};
+        const bool last = q + kSmemWarps >= f1;
+        const int qn = last ? q2 : q + kSmemWarps;
+        FeaturePre<BINARY, NP> nxt{};
         if (qn >= 0)
-          nxt = fetch_feature(qn, lane, d, lvl_feat, lvl_range, colsq, beta, bstride, draws, tidx,
-                              tval);
-        double zx = 0.0;
-        if (cur.rg.x + lane < cur.rg.y) zx = fma(cur.v0, Zs[cur.i0], zx);
-#pragma unroll 4
-        for (long long e = cur.rg.x + 32 + lane; e < cur.rg.y; e += 32)
-          zx = fma(tval ? tval[e] : 1.0, Zs[tidx[e]], zx);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) zx += __shfl_xor_sync(0xffffffffu, zx, o);
-        const double A = lb + lam * cur.cs;
-        const double B = lam * (zx + cur.b * cur.cs);
-        const double Ainv = 1.0 / A;
-        const double bn = B * Ainv + sqrt(Ainv) * cur.z;
-        const double my = cur.b - bn;
+          nxt = fetch_feature<BINARY, NP>(p, qn, last ? first2 : lane, last ? stride2 : 32);
+        const double bn = new_coef(p, cur, warp_sum(feature_dot(p, cur, Zs, lane, 32)));
         if (lane == 0) beta[(size_t)cur.f * bstride + d] = bn;
-        if (cur.rg.x + lane < cur.rg.y) Zs[cur.i0] = fma(cur.v0, my, Zs[cur.i0]);
-#pragma unroll 4
-        for (long long e = cur.rg.x + 32 + lane; e < cur.rg.y; e += 32)
-          Zs[tidx[e]] = fma(tval ? tval[e] : 1.0, my, Zs[tidx[e]]);
+        feature_add(p, cur, Zs, lane, 32, cur.b - bn);
         __syncwarp();
         cur = nxt;
         cur_q = qn;
-        have = qn >= 0;
+        cur_block = last && mode2 == 0;
       }
     } else {
+      // each feature by the whole block
       for (int q = f0; q < f1; q++) {
-        const int f = lvl_feat[q];
-        const longlong2 rg = lvl_range[q];
-        double cs = 0.0, bv = 0.0, zz = 0.0;  // thread 0 loads them before the reduction
-        if (threadIdx.x == 0) {
-          cs = colsq[f];
-          bv = beta[(size_t)f * bstride + d];
-          zz = draws[(size_t)f * bstride + d];
-        }
-        double zx = 0.0;
-#pragma unroll 4
-        for (long long e = rg.x + threadIdx.x; e < rg.y; e += kSmemThreads)
-          zx = fma(tval ? tval[e] : 1.0, Zs[tidx[e]], zx);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) zx += __shfl_xor_sync(0xffffffffu, zx, o);
-        if (lane == 0) red[warp] = zx;
+        if (cur_q != q || !cur_block) cur = fetch_feature<BINARY, NP>(p, q, tid, kSmemThreads);
+        const bool last = q + 1 == f1;
+        const int qn = last ? q2 : q + 1;
+        FeaturePre<BINARY, NP> nxt{};
+        if (qn >= 0)
+          nxt = fetch_feature<BINARY, NP>(p, qn, last ? first2 : tid,
+                                          last ? stride2 : kSmemThreads);
+        const double part = warp_sum(feature_dot(p, cur, Zs, tid, kSmemThreads));
+        if (lane == 0) red[buf][warp] = part;
         __syncthreads();
-        if (threadIdx.x == 0) {
-          double sum = 0.0;
-          for (int w = 0; w < kSmemWarps; w++) sum += red[w];
-          const double A = lb + lam * cs;
-          const double B = lam * (sum + bv * cs);
-          const double Ainv = 1.0 / A;
-          const double bn = B * Ainv + sqrt(Ainv) * zz;
-          beta[(size_t)f * bstride + d] = bn;
-          dl = bv - bn;
-        }
-        __syncthreads();
-        const double delta = dl;
-#pragma unroll 4
-        for (long long e = rg.x + threadIdx.x; e < rg.y; e += kSmemThreads)
-          Zs[tidx[e]] = fma(tval ? tval[e] : 1.0, delta, Zs[tidx[e]]);
+        const double bn = new_coef(p, cur, warp_sum(red[buf][lane]));
+        buf ^= 1;  // the next sum goes to the other half: one barrier between writes and reads
+        if (tid == 0) beta[(size_t)cur.f * bstride + d] = bn;
+        feature_add(p, cur, Zs, tid, kSmemThreads, cur.b - bn);
+        cur = nxt;
+        cur_q = qn;
+        cur_block = !last || mode2 == 0;
       }
     }
     __syncthreads();
+    f0 = f1;
+    f1 = f2;
+    mode = mode2;
   }
 }
 
@@ -305,26 +351,65 @@ __global__ void k_beta_draws(long long nfeat, int K, int stride, const Ctl* ctl,
 }
 
 // sample_lambda_beta (macauoneprior.cpp:267-290): lambda_beta_d ~ Gamma(a0 + nfeat / 2,
-// 1 / (b0 + sum_f beta_df^2 / 2)), one warp per dimension, keyed (kLambdaBeta, d).
-__global__ void k_lambda_beta_one(const double* __restrict__ beta, int bstride, long long nfeat,
+// 1 / (b0 + sum_f beta_df^2 / 2)), keyed (kLambdaBeta, d).  First the squares' sums per block of
+// features, rows read whole (thread (r, d): rows r, r + R, ... of the block), the block's row
+// groups added in order.  (One CTA, a warp per dimension reading a column of beta, took 148 us at
+// 8,193 features and 32 dimensions.)
+constexpr int kSqThreads = 256;
+__global__ void __launch_bounds__(kSqThreads)
+    k_beta_sq(const double* __restrict__ beta, int bstride, long long nfeat, int K,
+              long long rows_per_block, double* __restrict__ parts) {
+  __shared__ double s[kSqThreads];
+  const int W = K <= 32 ? 32 : 64, R = kSqThreads / W;
+  const int d = threadIdx.x % W, rg = threadIdx.x / W;
+  const long long r1 = min(nfeat, (blockIdx.x + 1) * rows_per_block);
+  double acc = 0.0;
+  if (d < K)
+#pragma unroll 4
+    for (long long f = blockIdx.x * rows_per_block + rg; f < r1; f += R) {
+      const double b = beta[f * bstride + d];
+      acc = fma(b, b, acc);
+    }
+  s[threadIdx.x] = acc;
+  __syncthreads();
+  if (rg == 0 && d < K) {
+    for (int q = 1; q < R; q++) acc += s[q * W + d];
+    parts[(size_t)blockIdx.x * K + d] = acc;
+  }
+}
+__global__ void k_lambda_beta_one(const double* __restrict__ parts, int nparts, long long nfeat,
                                   int K, double a0, double b0, const Ctl* ctl,
                                   unsigned long long seed, int mode,
                                   double* __restrict__ lambda_beta) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double a = a0 + (double)nfeat / 2.0;
-  for (int d = warp; d < K; d += blockDim.x >> 5) {
-    double s = 0.0;
-    for (long long f = lane; f < nfeat; f += 32) {
-      const double b = beta[f * bstride + d];
-      s = fma(b, b, s);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0)
-      lambda_beta[d] = gamma_draw(seed, ctl->sweep, stream_id(kLambdaBeta, (uint32_t)mode),
-                                  (uint32_t)d, a) *
-                       (1.0 / (b0 + s / 2.0));
+  const int d = threadIdx.x;
+  if (d >= K) return;
+  double s = 0.0;
+#pragma unroll 8
+  for (int b = 0; b < nparts; b++) s += parts[(size_t)b * K + d];
+  lambda_beta[d] = gamma_draw(seed, ctl->sweep, stream_id(kLambdaBeta, (uint32_t)mode), (uint32_t)d,
+                              a0 + (double)nfeat / 2.0) *
+                   (1.0 / (b0 + s / 2.0));
+}
+
+template <typename T, bool BINARY>
+void beta_smem(const DevCsr& Ft, const double* colsq, const int* lvl_ptr, const int* lvl_feat,
+               const longlong2* lvl_range, const int* lvl_warp, int nlevels, const void* U,
+               int ustride, const double* mu, const double* uhat, int hstride,
+               const double* Lambda, const double* lambda_beta, int K, long long N, double* beta,
+               int bstride, const double* draws, cudaStream_t s) {
+  static bool configured[64] = {false};
+  int dev = 0;
+  MG_CUDA(cudaGetDevice(&dev));
+  if (!configured[dev & 63]) {
+    MG_CUDA(cudaFuncSetAttribute(k_beta_one_smem<T, BINARY>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double) * kZsMax)));
+    configured[dev & 63] = true;
   }
+  k_beta_one_smem<T, BINARY><<<K, kSmemThreads, sizeof(double) * (size_t)N, s>>>(
+      Ft.idx, Ft.val, colsq, lvl_ptr, lvl_feat, lvl_range, lvl_warp, nlevels, (const T*)U, ustride,
+      mu, uhat, hstride, Lambda, lambda_beta, K, (int)N, beta, bstride, draws);
+  MG_CUDA(cudaGetLastError());
 }
 
 }  // namespace
@@ -341,30 +426,10 @@ void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
       Ft.nrow, K, bstride, ctl, seed, mode, draws);
   MG_CUDA(cudaGetLastError());
   if (N <= kZsMax) {  // one block per dimension, Z's column in shared memory
-    const size_t smem = sizeof(double) * (size_t)N;
-    static bool configured[64] = {false};
-    int dev = 0;
-    MG_CUDA(cudaGetDevice(&dev));
-    if (!configured[dev & 63]) {
-      MG_CUDA(cudaFuncSetAttribute(k_beta_one_smem<float>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(sizeof(double) * kZsMax)));
-      MG_CUDA(cudaFuncSetAttribute(k_beta_one_smem<double>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(sizeof(double) * kZsMax)));
-      configured[dev & 63] = true;
-    }
-    if (f32)
-      k_beta_one_smem<float><<<K, kSmemThreads, smem, s>>>(
-          Ft.idx, Ft.val, colsq, lvl_ptr, lvl_feat, lvl_range, lvl_warp, nlevels,
-          (const float*)U, ustride, mu, uhat, hstride, Lambda, lambda_beta, K, (int)N, beta,
-          bstride, draws);
-    else
-      k_beta_one_smem<double><<<K, kSmemThreads, smem, s>>>(
-          Ft.idx, Ft.val, colsq, lvl_ptr, lvl_feat, lvl_range, lvl_warp, nlevels,
-          (const double*)U, ustride, mu, uhat, hstride, Lambda, lambda_beta, K, (int)N, beta,
-          bstride, draws);
-    MG_CUDA(cudaGetLastError());
+    const auto run = f32 ? (Ft.val ? beta_smem<float, false> : beta_smem<float, true>)
+                         : (Ft.val ? beta_smem<double, false> : beta_smem<double, true>);
+    run(Ft, colsq, lvl_ptr, lvl_feat, lvl_range, lvl_warp, nlevels, U, ustride, mu, uhat, hstride,
+        Lambda, lambda_beta, K, N, beta, bstride, draws, s);
     return;
   }
   const int blocks = (K + 3) / 4;
@@ -379,11 +444,24 @@ void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
   MG_CUDA(cudaGetLastError());
 }
 
+// Cycles of a level by a warp per feature (32 at a time, a step of 32 entries read, summed and updated
+// in about 100 cycles beyond the four held ahead) against each feature by the whole block (about
+// 600 with its barrier and the two shuffle trees).
+bool beta_one_warp_level(long long N, long long nfeat, long long longest) {
+  if (N > kZsMax) return nfeat >= 8 || longest <= 1024;  // k_beta_one
+  const long long steps = (longest + 31) / 32;
+  const long long warp = (nfeat + kSmemWarps - 1) / kSmemWarps * (400 + 100 * std::max(0LL, steps - 4));
+  return warp <= 600 * nfeat;
+}
+
 void launch_lambda_beta_one(const double* beta, int bstride, long long nfeat, int K, double a0,
                             double b0, const Ctl* ctl, unsigned long long seed, int mode,
-                            double* lambda_beta, cudaStream_t s) {
-  k_lambda_beta_one<<<1, 256, 0, s>>>(beta, bstride, nfeat, K, a0, b0, ctl, seed, mode,
-                                      lambda_beta);
+                            double* parts, double* lambda_beta, cudaStream_t s) {
+  // `parts` holds nfeat * bstride doubles: at most one record of K per 64 features is written
+  const int nb = (int)std::min<long long>(148, (nfeat + 63) / 64);
+  k_beta_sq<<<nb, kSqThreads, 0, s>>>(beta, bstride, nfeat, K, (nfeat + nb - 1) / nb, parts);
+  MG_CUDA(cudaGetLastError());
+  k_lambda_beta_one<<<1, 64, 0, s>>>(parts, nb, nfeat, K, a0, b0, ctl, seed, mode, lambda_beta);
   MG_CUDA(cudaGetLastError());
 }
 
