@@ -727,7 +727,7 @@ class Context {
       // MacauOnePrior::update_prior (macauoneprior.cpp:189-194): sample_mu_lambda (Normal-Wishart
       // of U - Uhat with mu0 = 0, kappa = 2, W0 = I, nu = K, the BPMF defaults), sample_beta,
       // compute_uhat, sample_lambda_beta
-      launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr, 0,
+      launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr,
                             nullptr, ctl_.p, cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
       launch_beta_one(p.Ft, p.colsq.p, p.lvl_ptr.p, p.lvl_feat.p, p.lvl_range.p, p.lvl_warp.p,
                       p.nlevels,
@@ -741,7 +741,7 @@ class Context {
       return;
     }
     if (!p.macau) {  // BPMFPrior::update_prior (latentprior.cpp:79-81)
-      launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr, 0,
+      launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr,
                             nullptr, ctl_.p, cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
       return;
     }
@@ -750,7 +750,7 @@ class Context {
     launch_stats(p.beta.p, false, nullptr, p.nfeat, K_, CP_, 0, p.bb_partials.p, nbb, s_);
     launch_reduce_parts(p.bb_partials.p, nbb, rec, p.bb_final.p, s_);
     launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df + (int)p.nfeat,
-                          p.bb_final.p, 1, p.lambda_beta.p, ctl_.p, cfg_.seed, mode, p.mu.p,
+                          p.bb_final.p, p.lambda_beta.p, ctl_.p, cfg_.seed, mode, p.mu.p,
                           p.Lambda.p, s_);
     // sample_beta (latentprior.cpp:273-293)
     launch_small_chol(p.Lambda.p, K_, p.Lchol.p, ctl_.p, s_);

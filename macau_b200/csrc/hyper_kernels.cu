@@ -1,13 +1,9 @@
-// Normal-Wishart hyperprior update and test-set evaluation.
+// Hyperprior statistics, noise update and test-set evaluation.
 //
 //   k_stats32         per-block partial sums of x and x x^T over the rows of a latent matrix, K <=
 //                     32 (optionally x = U - Uhat, the Macau residual of latentprior.cpp:257);
 //                     FP64 accumulation from FP64 or FP32 latents on the FP64 matrix instruction.
-//   k_nw32            one CTA, K <= 32: CondNormalWishart -> NormalWishart -> Wishart/WishartUnit
-//                     -> MvNormal_prec (mvnormal.cpp:169-184, 217-287, 314-336) in FP64 with keyed
-//                     draws; shared-memory matrices, warp-register Cholesky factors
-//                     (warp_finish.cuh) and a warp-parallel triangular inverse.
-//   (K > 32: hyper_wide.cu)
+//   (K > 32, and the Normal-Wishart draw: hyper_wide.cu)
 //   k_lambda_beta     one CTA: posterior_lambda_beta + rgamma (latentprior.cpp:317-331).
 //   k_eval / k_eval_finish  eval_rmse (bpmfutils.h:86-114): online posterior mean / variance of
 //                     the test predictions and the two RMSEs.
@@ -418,207 +414,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// CondNormalWishart -> NormalWishart -> MvNormal_prec (mvnormal.cpp:169-184, 217-287, 314-336)
-// for K <= 32 in one CTA of 256 threads, matrices in shared memory (row-major, ld 33).  Two identities replace two of the reference's three Cholesky
-// factorisations (results agree to FP64 rounding):
-//   * chol(X^{-1}) = J M^{-T} J with M = chol(J X J), J the index reversal: one Cholesky of the
-//     reversed X (warp 0's registers, warp_factor) and one triangular inverse Y = M^{-1}
-//     (lane c solves M y = e_c), L(i, j) = Y(K-1-j, K-1-i);
-//   * Lambda = L c^T c L^T = B B^T with B = L c^T lower triangular with positive diagonal, so
-//     chol(kappa_c Lambda) = sqrt(kappa_c) B and mu = mu_c + B^{-T} z / sqrt(kappa_c).
-// The Bartlett factor c and z are drawn by warps 1-7 while warp 0 factorises.
-constexpr int kNwLd = 33;
-constexpr int kNwLc = 36;
-
-struct NwShared {
-  double A[32 * kNwLd], Bm[32 * kNwLd], C[32 * kNwLd], D[32 * kNwLd];
-  double Lc[32 * kNwLc];
-  double NU[32], muc[32], m0[32], rl[32], zs[32];
-  int flag;
-};
-
-// T0 == null stands for the identity.  The factor and the inverse run at the width KP = 8, 16 or 32
-// that holds K (nw32_run).
-template <int KP>
-__device__ __forceinline__ void nw32_width(NwShared& sh, const double* __restrict__ partials, int nparts,
-                                         long long N, int K, const double* __restrict__ mu0,
-                                         double kappa, const double* __restrict__ T0, int nu,
-                                         const double* __restrict__ bb_partials, int bb_nparts,
-                                         const double* __restrict__ lambda_beta, Ctl* ctl,
-                                         unsigned long long seed, int mode,
-                                         double* __restrict__ mu_out,
-                                         double* __restrict__ Lambda_out) {
-  double *A = sh.A, *Bm = sh.Bm, *C = sh.C, *D = sh.D, *Lc = sh.Lc;
-  double *NU = sh.NU, *muc = sh.muc, *m0 = sh.m0, *rl = sh.rl, *zs = sh.zs;
-  const int t = threadIdx.x, lane = t & 31;
-  const int KK = K * K;
-  const uint32_t sweep = ctl->sweep;
-  // 1. reduce partials in block order: NU = sum x, A = S = sum x x^T; Bm = T.  Thread t sums
-  //    elements t + 256 q (q < 5) together so that its loads of one partial are in flight at once.
-  {
-    double sv[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-#pragma unroll 4
-    for (int b = 0; b < nparts; b++) {
-      const double* pb = partials + (size_t)b * (K + KK);
-#pragma unroll
-      for (int q = 0; q < 5; q++)
-        if (t + 256 * q < K + KK) sv[q] += pb[t + 256 * q];
-    }
-#pragma unroll
-    for (int q = 0; q < 5; q++) {
-      const int e = t + 256 * q;
-      if (e < K) NU[e] = sv[q];
-      else if (e < K + KK) A[((e - K) % K) * kNwLd + (e - K) / K] = sv[q];
-    }
-  }
-  if (bb_partials) {  // T = WI + lambda_beta * beta beta^T  (latentprior.cpp:258-260)
-    const double lb = *lambda_beta;
-    double sv[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 4
-    for (int b = 0; b < bb_nparts; b++) {
-      const double* pb = bb_partials + (size_t)b * (K + KK) + K;
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-        if (t + 256 * q < KK) sv[q] += pb[t + 256 * q];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int e = t + 256 * q;
-      if (e < KK) Bm[(e % K) * kNwLd + e / K] = (T0 ? T0[e] : (e % K == e / K ? 1.0 : 0.0)) + lb * sv[q];
-    }
-  } else {
-    for (int e = t; e < KK; e += blockDim.x)
-      Bm[(e % K) * kNwLd + e / K] = T0 ? T0[e] : (e % K == e / K ? 1.0 : 0.0);
-  }
-  if (t < K) m0[t] = mu0 ? mu0[t] : 0.0;
-  __syncthreads();
-  const double kappa_c = kappa + (double)N;
-  const int nu_c = nu + (int)N;
-  if (t < K) muc[t] = (kappa * m0[t] + NU[t]) / kappa_c;
-  __syncthreads();
-  // 2. X = T + NS + kappa mu0 mu0^T - kappa_c mu_c mu_c^T   (into A)
-  for (int e = t; e < KK; e += blockDim.x) {
-    const int i = e % K, j = e / K;
-    A[i * kNwLd + j] =
-        Bm[i * kNwLd + j] + A[i * kNwLd + j] + kappa * m0[i] * m0[j] - kappa_c * muc[i] * muc[j];
-  }
-  __syncthreads();
-  if (t < 32) {
-    // 3a. M = chol(J X J), M^T rows into Lc
-    double a[KP], d0 = 1.0, rinv = 1.0;
-#pragma unroll
-    for (int j = 0; j < KP; j++) {
-      a[j] = (lane < K && j < K) ? A[(K - 1 - lane) * kNwLd + (K - 1 - j)] : (lane == j ? 1.0 : 0.0);
-      if (j == lane) d0 = a[j];
-    }
-    const bool ok = warp_factor<double, KP>(a, rinv, lane, 0.0, d0, Lc, kNwLc);
-    if (lane == 0) sh.flag = ok ? 1 : 0;
-    // 3b. Y = M^{-1}: lane c solves M y = e_c by columns (the updates of one column are
-    //     independent of one another); Y(i, c) into D
-    if (ok) {
-      rl[lane] = rinv;
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < KP; i++) a[i] = lane == i ? 1.0 : 0.0;
-#pragma unroll
-      for (int i = 0; i < KP; i++) {
-        const double y = a[i] * rl[i];
-        if (lane < KP) D[i * kNwLd + lane] = y;
-#pragma unroll
-        for (int q = (i + 1) / 4; q < KP / 4; q++) {
-          const Vec4<double> c = lds4(Lc + i * kNwLc + 4 * q);
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            if (4 * q + u > i) a[4 * q + u] = fma(-c.v[u], y, a[4 * q + u]);
-        }
-      }
-    }
-  } else {
-    // 3c. Bartlett factor c (upper) into C: c_ii = sqrt(2 Gamma((nu_c - i)/2)), c_ij ~ N(0,1);
-    //     z for the mean draw
-    for (int e = t - 32; e < KK; e += blockDim.x - 32) {
-      const int i = e % K, j = e / K;
-      double v = 0.0;
-      if (i == j)
-        v = sqrt(2.0 * gamma_draw(seed, sweep, stream_id(kWishartDiag, mode), (uint32_t)i,
-                                  0.5 * (double)(nu_c - i)));
-      else if (j > i)
-        v = normal_draw(seed, sweep, stream_id(kWishartOff, mode), (uint32_t)i,
-                        (uint32_t)(j - i - 1));
-      C[i * kNwLd + j] = v;
-    }
-    if (t - 32 < K) zs[t - 32] = normal_draw(seed, sweep, stream_id(kMuDraw, mode), 0u, (uint32_t)(t - 32));
-  }
-  __syncthreads();
-  if (!sh.flag) {
-    if (t == 0) atomicOr(&ctl->status, kStatHyperFail);
-    return;
-  }
-  // 4. L = chol(T_c) = chol(X^{-1}) into A: L(i, j) = Y(K-1-j, K-1-i), j <= i
-  for (int e = t; e < KK; e += blockDim.x) {
-    const int i = e % K, j = e / K;
-    A[i * kNwLd + j] = (j <= i) ? D[(K - 1 - j) * kNwLd + (K - 1 - i)] : 0.0;
-  }
-  __syncthreads();
-  // 5. B = L c^T (lower triangular): B(i, j) = sum_{q=j..i} L(i, q) c(j, q)
-  for (int e = t; e < KK; e += blockDim.x) {
-    const int i = e % K, j = e / K;
-    double s = 0.0;
-    for (int q = j; q <= i; q++) s += A[i * kNwLd + q] * C[j * kNwLd + q];
-    Bm[i * kNwLd + j] = (j <= i) ? s : 0.0;
-  }
-  __syncthreads();
-  // 6. Lambda = B B^T
-  for (int e = t; e < KK; e += blockDim.x) {
-    const int i = e % K, j = e / K;
-    const int m = min(i, j);
-    double s = 0.0;
-    for (int q = 0; q <= m; q++) s += Bm[i * kNwLd + q] * Bm[j * kNwLd + q];
-    Lambda_out[e] = s;
-  }
-  // 7. mu = mu_c + B^{-T} z / sqrt(kappa_c)
-  if (t < 32) {
-    double x = lane < K ? zs[lane] / sqrt(kappa_c) : 0.0;
-    const double rb = lane < K ? 1.0 / Bm[lane * kNwLd + lane] : 0.0;
-    for (int j = K - 1; j >= 0; j--) {
-      if (lane == j) x *= rb;
-      const double xj = __shfl_sync(0xffffffffu, x, j);
-      if (lane < j) x = fma(-Bm[j * kNwLd + lane], xj, x);
-    }
-    if (lane < K) mu_out[lane] = x + muc[lane];
-  }
-}
-
-__device__ __forceinline__ void nw32_run(const double* __restrict__ partials, int nparts,
-                                         long long N, int K, const double* __restrict__ mu0,
-                                         double kappa, const double* __restrict__ T0, int nu,
-                                         const double* __restrict__ bb_partials, int bb_nparts,
-                                         const double* __restrict__ lambda_beta, Ctl* ctl,
-                                         unsigned long long seed, int mode,
-                                         double* __restrict__ mu_out,
-                                         double* __restrict__ Lambda_out) {
-  __shared__ __align__(16) NwShared sh;
-  if (K <= 8)
-    nw32_width<8>(sh, partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials, bb_nparts,
-                  lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
-  else if (K <= 16)
-    nw32_width<16>(sh, partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials, bb_nparts,
-                   lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
-  else
-    nw32_width<32>(sh, partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials, bb_nparts,
-                   lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
-}
-
-__global__ void __launch_bounds__(256)
-    k_nw32(const double* __restrict__ partials, int nparts, long long N, int K,
-           const double* __restrict__ mu0, double kappa, const double* __restrict__ T0, int nu,
-           const double* __restrict__ bb_partials, int bb_nparts,
-           const double* __restrict__ lambda_beta, Ctl* ctl, unsigned long long seed, int mode,
-           double* __restrict__ mu_out, double* __restrict__ Lambda_out) {
-  nw32_run(partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials, bb_nparts, lambda_beta, ctl,
-           seed, mode, mu_out, Lambda_out);
-}
-
 // ---- both modes' BPMF prior updates in one launch per step: blocks of mode 0, then
 // of mode 1, each doing what the single-mode kernel's block does, so the results are the same
 // bit for bit; the two modes' steps only overlap ----
@@ -655,15 +450,6 @@ __global__ void __launch_bounds__(256) k_reduce_parts_pair(PriorPair pp, int len
   }
 }
 
-__global__ void __launch_bounds__(256) k_nw32_pair(PriorPair pp, int few, int K, Ctl* ctl,
-                                                   unsigned long long seed) {
-  const int m = blockIdx.x;
-  const bool own = (few >> m) & 1;  // this block adds the mode's partials
-  nw32_run(own ? pp.partials[m] : pp.final_[m], own ? pp.nblocks[m] : 1, pp.N[m], K, pp.mu0[m],
-           pp.kappa[m], pp.T0[m], pp.nu[m], nullptr, 0, nullptr, ctl, seed, m, pp.mu[m],
-           pp.Lambda[m]);
-}
-
 }  // namespace
 
 int launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl,
@@ -676,16 +462,14 @@ int launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl
   else
     k_stats32_pair<double><<<nb, kStatThreads, 0, s>>>(pp, K, stride);
   MG_CUDA(cudaGetLastError());
-  const int few = (few_parts(pp.nblocks[0], K) ? 1 : 0) | (few_parts(pp.nblocks[1], K) ? 2 : 0);
-  if (few != 3) {
+  const bool few = few_parts(pp.nblocks[0], K) && few_parts(pp.nblocks[1], K);
+  if (!few) {
     const int len = K + K * K;
     k_reduce_parts_pair<<<2 * ((len + 31) / 32), 256, 0, s>>>(pp, len);
     MG_CUDA(cudaGetLastError());
   }
-  if (K > 32) launch_nw_wide_pair(pp, K, ctl, seed, s);
-  else k_nw32_pair<<<2, 256, 0, s>>>(pp, few, K, ctl, seed);
-  MG_CUDA(cudaGetLastError());
-  return few == 3 ? 2 : 3;
+  launch_normal_wishart_pair(pp, K, ctl, seed, s);
+  return few ? 2 : 3;
 }
 
 // Up to 16 partials are added by the Normal-Wishart block itself: one CTA reads them in less time
@@ -726,60 +510,16 @@ __global__ void __launch_bounds__(kStatThreads)
                       partials + (size_t)p * (32 + 32 * 32));
 }
 
-// BPMFPrior::update_prior per problem with mu0 = 0, b0 = 2, W0 = I, df = K_p
-// (latentprior.cpp:79-99), keyed with the problem's seed; then the finish's operands: the FP32
-// Lambda (32 x 32, zero beyond K) and Lambda mu (FP64, summed in column order).
-__global__ void __launch_bounds__(256)
-    k_nw_batch(const double* __restrict__ partials, const int* __restrict__ row0,
-               const int* __restrict__ Kp, const unsigned long long* __restrict__ seed, Ctl* ctl,
-               int mode, double* __restrict__ mu, double* __restrict__ Lambda,
-               float* __restrict__ LamF, double* __restrict__ lmu) {
-  const int p = blockIdx.x, K = Kp[p];
-  double* L = Lambda + (size_t)p * 1024;
-  double* m = mu + (size_t)p * 32;
-  nw32_run(partials + (size_t)p * (32 + 32 * 32), 1, row0[p + 1] - row0[p], K, nullptr, 2.0,
-           nullptr, K, nullptr, 0, nullptr, ctl, seed[p], mode, m, L);
-  __syncthreads();
-  for (int e = threadIdx.x; e < 1024; e += blockDim.x) {
-    const int i = e >> 5, j = e & 31;
-    LamF[(size_t)p * 1024 + e] = (i < K && j < K) ? (float)L[i + j * K] : 0.f;
-  }
-  if (threadIdx.x < 32) {
-    double acc = 0.0;
-    if ((int)threadIdx.x < K)
-      for (int j = 0; j < K; j++) acc += L[threadIdx.x + j * K] * m[j];
-    lmu[(size_t)p * 32 + threadIdx.x] = acc;
-  }
-}
-
 void launch_prior_batch(const float* U, const int* row0, const int* Kp,
                         const unsigned long long* seed, int P, double* partials, Ctl* ctl, int mode,
                         double* mu, double* Lambda, float* LamF, double* lmu, cudaStream_t s) {
   k_stats_batch<<<P, kStatThreads, 0, s>>>(U, row0, Kp, partials);
   MG_CUDA(cudaGetLastError());
-  k_nw_batch<<<P, 256, 0, s>>>(partials, row0, Kp, seed, ctl, mode, mu, Lambda, LamF, lmu);
-  MG_CUDA(cudaGetLastError());
+  launch_nw_batch(partials, row0, Kp, seed, P, ctl, mode, mu, Lambda, LamF, lmu, s);
 }
 
 void launch_reduce_parts(const double* parts, int nparts, int len, double* out, cudaStream_t s) {
   k_reduce_parts<<<(len + 31) / 32, 256, 0, s>>>(parts, nparts, len, out);
-  MG_CUDA(cudaGetLastError());
-}
-
-void launch_normal_wishart(const double* partials, int nparts, long long N, int K,
-                           const double* mu0, double kappa, const double* T0, int nu,
-                           const double* bb_partials, int bb_nparts, const double* lambda_beta,
-                           Ctl* ctl, unsigned long long seed, int mode, double* mu_out,
-                           double* Lambda_out, cudaStream_t s) {
-  if (K > 32) {  // the wide kernel reads reduced statistics
-    if (nparts != 1 || (bb_partials && bb_nparts != 1))
-      throw MgError(MG_ERR_STATE, "Normal-Wishart update of unreduced statistics at K > 32");
-    launch_nw_wide(partials, N, K, mu0, kappa, T0, nu, bb_partials, lambda_beta, ctl, seed, mode,
-                   mu_out, Lambda_out, s);
-    return;
-  }
-  k_nw32<<<1, 256, 0, s>>>(partials, nparts, N, K, mu0, kappa, T0, nu, bb_partials, bb_nparts,
-                           lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
   MG_CUDA(cudaGetLastError());
 }
 

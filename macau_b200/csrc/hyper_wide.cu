@@ -1,16 +1,17 @@
-// Normal-Wishart hyperprior update for 32 < K <= 128, FP64 on the matrix instruction m8n8k4.f64.
+// Normal-Wishart hyperprior update on the FP64 matrix instruction m8n8k4.f64.
 //
-//   k_stats_wide  per-block partial sums of x and x x^T over the rows of a latent matrix (x = U, or
-//                 U - Uhat): the lower-triangle tiles spread over the block's warps as in the row
-//                 sampler, rows read straight into fragments.
-//   k_nw_wide     one block per update: CondNormalWishart -> NormalWishart -> Wishart ->
-//                 MvNormal_prec (mvnormal.cpp:169-184, 217-287, 314-336), all matrices in shared
-//                 memory as 8 x 8 tiles of their lower triangles.
+//   k_nw          one block per update, every K <= 128: CondNormalWishart -> NormalWishart -> Wishart
+//                 -> MvNormal_prec (mvnormal.cpp:169-184, 217-287, 314-336), all matrices in shared
+//                 memory as 8 x 8 tiles of their lower triangles, keyed draws beside the factor.
+//   k_stats_wide  32 < K <= 128: per-block partial sums of x and x x^T over the rows of a latent
+//                 matrix (x = U, or U - Uhat): the lower-triangle tiles spread over the block's
+//                 warps as in the row sampler, rows read straight into fragments.
 //
-// What bounds k_nw_wide: the chain of the panel factor, about 1,900 cycles per 8 columns; the
-// triangular inverse and the three products that follow are matrix instructions on 16 warps.  The
-// version this replaces kept the matrices in global memory and gave one thread a dot product (or a
-// whole substitution) at a time: 4.28 ms at K = 128 and 0.81 ms at K = 64.
+// What bounds k_nw: the chain of the panel factor, about 1,500 to 2,500 cycles per 8 columns; the
+// triangular inverse and the three products that follow are matrix instructions on 16 warps.  With
+// the matrices in global memory and one thread to a dot product (or a whole substitution) a draw
+// took 4.28 ms at K = 128 and 0.81 ms at K = 64; with a matrix row per lane of one warp 25 us at
+// K = 32 (450 cycles a column, and 1,024 separate normal draws).
 #include "common.cuh"
 #include "kernels.h"
 #include "rng.cuh"
@@ -158,11 +159,12 @@ void stats_launch(const StatsArgs& a, int K, int stride, int uhat_stride, cudaSt
 
 // ---- the Normal-Wishart draw ----
 struct NwArgs {
-  const double* stats;  // sums (K), then x x^T (K x K)
-  const double* bb;     // beta beta^T statistics of a Macau prior (same layout), or null
+  const double* stats;  // `nparts` records of sums (K), then x x^T (K x K), added in order
+  int nparts;
+  const double* bb;     // beta beta^T statistics of a Macau prior (one such record), or null
   const double* lambda_beta;
-  const double* mu0;
-  const double* T0;
+  const double* mu0;    // null: zero
+  const double* T0;     // null: the identity
   double kappa;
   long long N;
   int nu, mode;
@@ -188,14 +190,16 @@ struct NwW {
 __device__ __forceinline__ void bartlett(double* Ct, double* z, int K, int n, int nu_c,
                                          unsigned long long seed, uint32_t sweep, uint32_t mode,
                                          int tid, int nt) {
-  for (int i = tid; i < K; i += nt) {
+  // the three kinds of draws start at different threads, so that at small K they are different
+  // warps' work: gammas from the first, z from the middle, pairs from the last
+  for (int i = tid; i < K; i += nt)
     Ct[elem_at(i, i)] = sqrt(2.0 * gamma_draw(seed, sweep, stream_id(kWishartDiag, mode),
                                               (uint32_t)i, 0.5 * (double)(nu_c - i)));
+  for (int i = (tid + nt / 2) % nt; i < K; i += nt)
     z[i] = normal_draw(seed, sweep, stream_id(kMuDraw, mode), 0u, (uint32_t)i);
-  }
   // off-diagonal draws two to a block: rows i and K - 2 - i together have at most K / 2 + 1 pairs
   const int slots = K / 2 + 1;
-  for (int e = tid; e < slots * (K / 2); e += nt) {
+  for (int e = nt - 1 - tid; e < slots * (K / 2); e += nt) {
     const int s = e / slots, first = (K - s) / 2;  // pairs of row s
     int i = s, q = e % slots;
     if (q >= first) {
@@ -225,12 +229,10 @@ __device__ __forceinline__ void bartlett(double* Ct, double* z, int K, int n, in
 //   Lambda = L c^T c L^T = B B^T with B = L c^T lower triangular, so chol(kappa_c Lambda) =
 //   sqrt(kappa_c) B and mu = mu_c + B^{-T} z / sqrt(kappa_c).
 template <int KP>
-__global__ void __launch_bounds__(kNwThreads, 1)
-    k_nw_wide(const NwPair args, int K, Ctl* ctl, unsigned long long seed) {
+__device__ __forceinline__ void nw_tiles(const NwArgs& p, int K, Ctl* ctl, unsigned long long seed,
+                                         double* smem) {
   using C = NwW<KP>;
-  extern __shared__ __align__(16) double nsm[];
-  const NwArgs& p = args.m[blockIdx.x];
-  double* M = nsm;
+  double* M = smem;
   double* Y = M + (size_t)C::TRI * 64;
   double* Ct = Y + (size_t)C::TRI * 64;
   double* Di = Ct + (size_t)C::TRI * 64;
@@ -249,8 +251,18 @@ __global__ void __launch_bounds__(kNwThreads, 1)
     while (q >= (a + 1) * (a + 2) / 2) a++;
     tri[q] = (unsigned char)((a << 4) | (q - a * (a + 1) / 2));
   }
+  const size_t rec = K + (size_t)K * K;
+  auto stat = [&](size_t at) {
+    double v = p.stats[at];
+#pragma unroll 8
+    for (int b = 1; b < p.nparts; b++) v += p.stats[b * rec + at];
+    return v;
+  };
+  // x holds mu0 until the mean is solved for
   for (int i = tid; i < n; i += kNwThreads) {
-    muc[i] = i < K ? (p.kappa * p.mu0[i] + p.stats[i]) / kappa_c : 0.0;
+    const double m0 = i < K && p.mu0 ? p.mu0[i] : 0.0;
+    muc[i] = i < K ? (p.kappa * m0 + stat(i)) / kappa_c : 0.0;
+    x[i] = m0;
     y[i] = zero[i] = 0.0;
   }
   __syncthreads();
@@ -267,9 +279,9 @@ __global__ void __launch_bounds__(kNwThreads, 1)
       v[e] = a == b ? 1.0 : 0.0;
       if (a >= pad && b >= pad) {
         const size_t at = j + (size_t)i * K;
-        double T = p.T0[at];
+        double T = p.T0 ? p.T0[at] : (a == b ? 1.0 : 0.0);
         if (p.bb) T += lb * p.bb[K + at];
-        v[e] = T + p.stats[K + at] + p.kappa * p.mu0[i] * p.mu0[j] - kappa_c * muc[i] * muc[j];
+        v[e] = T + stat(K + at) + p.kappa * x[i] * x[j] - kappa_c * muc[i] * muc[j];
       }
     }
     *reinterpret_cast<double2*>(M + tile_at(tri[q] >> 4, tri[q] & 15) + tile_pos(g, 2 * t)) =
@@ -314,13 +326,17 @@ __global__ void __launch_bounds__(kNwThreads, 1)
       // column c of the inverse of diagonal tile b
       const int b = tid >> 3, c = tid & 7;
       const double* D = M + tile_at(b, b);
-      double v[8];
+      double v[8], ri[8];
 #pragma unroll
       for (int r = 0; r < 8; r++) {
-        double s = r == c ? 1.0 : 0.0;
+        ri[r] = 1.0 / D[tile_pos(r, r)];
+        v[r] = r == c ? 1.0 : 0.0;
+      }
 #pragma unroll
-        for (int k = 0; k < r; k++) s = fma(-D[tile_pos(r, k)], v[k], s);
-        v[r] = r < c ? 0.0 : s / D[tile_pos(r, r)];
+      for (int r = 0; r < 8; r++) {
+        v[r] *= ri[r];
+#pragma unroll
+        for (int k = r + 1; k < 8; k++) v[k] = fma(-D[tile_pos(k, r)], v[r], v[k]);
       }
       store_row8(Di + 64 * b, c, v);
       y[tid] = z[tid] / sqrt(kappa_c);
@@ -353,6 +369,41 @@ __global__ void __launch_bounds__(kNwThreads, 1)
 }
 
 template <int KP>
+__global__ void __launch_bounds__(kNwThreads, 1)
+    k_nw(const NwPair args, int K, Ctl* ctl, unsigned long long seed) {
+  extern __shared__ __align__(16) double nsm[];
+  nw_tiles<KP>(args.m[blockIdx.x], K, ctl, seed, nsm);
+}
+
+// BPMFPrior::update_prior per problem with mu0 = 0, b0 = 2, W0 = I, df = K_p
+// (latentprior.cpp:79-99), keyed with the problem's seed; then the finish's operands: the FP32
+// Lambda (32 x 32, zero beyond K) and Lambda mu (FP64, summed in column order).
+__global__ void __launch_bounds__(kNwThreads, 1)
+    k_nw_batch(const double* __restrict__ partials, const int* __restrict__ row0,
+               const int* __restrict__ Kp, const unsigned long long* __restrict__ seed, Ctl* ctl,
+               int mode, double* __restrict__ mu, double* __restrict__ Lambda,
+               float* __restrict__ LamF, double* __restrict__ lmu) {
+  __shared__ __align__(16) double nsm[NwW<32>::kDoubles];
+  const int p = blockIdx.x, K = Kp[p];
+  double* L = Lambda + (size_t)p * 1024;
+  double* m = mu + (size_t)p * 32;
+  const NwArgs a{partials + (size_t)p * (32 + 32 * 32), 1, nullptr, nullptr, nullptr, nullptr, 2.0,
+                 row0[p + 1] - row0[p], K, mode, m, L};
+  nw_tiles<32>(a, K, ctl, seed[p], nsm);
+  __syncthreads();
+  for (int e = threadIdx.x; e < 1024; e += kNwThreads) {
+    const int i = e >> 5, j = e & 31;
+    LamF[(size_t)p * 1024 + e] = (i < K && j < K) ? (float)L[i + j * K] : 0.f;
+  }
+  if (threadIdx.x < 32) {
+    double acc = 0.0;
+    if ((int)threadIdx.x < K)
+      for (int j = 0; j < K; j++) acc += L[threadIdx.x + j * K] * m[j];
+    lmu[(size_t)p * 32 + threadIdx.x] = acc;
+  }
+}
+
+template <int KP>
 void nw_launch(const NwPair& a, int count, int K, Ctl* ctl, unsigned long long seed,
                cudaStream_t s) {
   constexpr size_t smem = sizeof(double) * NwW<KP>::kDoubles;
@@ -361,17 +412,17 @@ void nw_launch(const NwPair& a, int count, int K, Ctl* ctl, unsigned long long s
   int dev = 0;
   MG_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    MG_CUDA(cudaFuncSetAttribute(k_nw_wide<KP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+    MG_CUDA(cudaFuncSetAttribute(k_nw<KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured[dev & 63] = true;
   }
-  k_nw_wide<KP><<<count, kNwThreads, smem, s>>>(a, K, ctl, seed);
+  k_nw<KP><<<count, kNwThreads, smem, s>>>(a, K, ctl, seed);
   MG_CUDA(cudaGetLastError());
 }
 
 void nw_dispatch(const NwPair& a, int count, int K, Ctl* ctl, unsigned long long seed,
                  cudaStream_t s) {
-  if (K <= 64) nw_launch<64>(a, count, K, ctl, seed, s);
+  if (K <= 32) nw_launch<32>(a, count, K, ctl, seed, s);
+  else if (K <= 64) nw_launch<64>(a, count, K, ctl, seed, s);
   else nw_launch<128>(a, count, K, ctl, seed, s);
 }
 
@@ -394,22 +445,34 @@ void launch_stats_wide_pair(const PriorPair& pp, bool f32, int K, int stride, cu
   else stats_launch<double>(a, K, stride, 0, s);
 }
 
-void launch_nw_wide(const double* stats, long long N, int K, const double* mu0, double kappa,
-                    const double* T0, int nu, const double* bb, const double* lambda_beta, Ctl* ctl,
-                    unsigned long long seed, int mode, double* mu, double* Lambda,
-                    cudaStream_t s) {
+void launch_normal_wishart(const double* partials, int nparts, long long N, int K,
+                           const double* mu0, double kappa, const double* T0, int nu,
+                           const double* bb, const double* lambda_beta, Ctl* ctl,
+                           unsigned long long seed, int mode, double* mu_out, double* Lambda_out,
+                           cudaStream_t s) {
   NwPair a{};
-  a.m[0] = NwArgs{stats, bb, lambda_beta, mu0, T0, kappa, N, nu, mode, mu, Lambda};
+  a.m[0] = NwArgs{partials, nparts, bb, lambda_beta, mu0, T0, kappa, N, nu, mode, mu_out,
+                  Lambda_out};
   nw_dispatch(a, 1, K, ctl, seed, s);
 }
 
-void launch_nw_wide_pair(const PriorPair& pp, int K, Ctl* ctl, unsigned long long seed,
-                         cudaStream_t s) {
+void launch_normal_wishart_pair(const PriorPair& pp, int K, Ctl* ctl, unsigned long long seed,
+                                cudaStream_t s) {
   NwPair a{};
-  for (int m = 0; m < 2; m++)
-    a.m[m] = NwArgs{pp.final_[m], nullptr, nullptr, pp.mu0[m], pp.T0[m], pp.kappa[m], pp.N[m],
-                    pp.nu[m], m, pp.mu[m], pp.Lambda[m]};
+  for (int m = 0; m < 2; m++) {
+    const bool few = few_parts(pp.nblocks[m], K);
+    a.m[m] = NwArgs{few ? pp.partials[m] : pp.final_[m], few ? pp.nblocks[m] : 1, nullptr, nullptr,
+                    pp.mu0[m], pp.T0[m], pp.kappa[m], pp.N[m], pp.nu[m], m, pp.mu[m],
+                    pp.Lambda[m]};
+  }
   nw_dispatch(a, 2, K, ctl, seed, s);
+}
+
+void launch_nw_batch(const double* partials, const int* row0, const int* Kp,
+                     const unsigned long long* seed, int P, Ctl* ctl, int mode, double* mu,
+                     double* Lambda, float* LamF, double* lmu, cudaStream_t s) {
+  k_nw_batch<<<P, kNwThreads, 0, s>>>(partials, row0, Kp, seed, ctl, mode, mu, Lambda, LamF, lmu);
+  MG_CUDA(cudaGetLastError());
 }
 
 }  // namespace mg

@@ -85,11 +85,13 @@ void launch_reduce_parts(const double* parts, int nparts, int len, double* out, 
 bool few_parts(int nblocks, int K);
 void launch_stats(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
                   int uhat_stride, double* partials, int nblocks, cudaStream_t s);
+// One Normal-Wishart draw (hyper_wide.cu) from `nparts` statistics records, added in order; bb: one
+// record of beta beta^T (null without side information).
 void launch_normal_wishart(const double* partials, int nparts, long long N, int K,
                            const double* mu0, double kappa, const double* T0, int nu,
-                           const double* bb_partials, int bb_nparts, const double* lambda_beta,
-                           Ctl* ctl, unsigned long long seed, int mode, double* mu_out,
-                           double* Lambda_out, cudaStream_t s);
+                           const double* bb, const double* lambda_beta, Ctl* ctl,
+                           unsigned long long seed, int mode, double* mu_out, double* Lambda_out,
+                           cudaStream_t s);
 // Both modes' BPMF prior updates (BPMFPrior::update_prior, latentprior.cpp:79-81) at once:
 // statistics, reduction and Normal-Wishart draw of mode m from the latents U[m]
 // (N[m] rows, stride `stride`), partials[m] (nblocks[m] records, rows_per_block[m] rows each)
@@ -113,17 +115,15 @@ struct PriorPair {
 };
 int launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl,
                        unsigned long long seed, cudaStream_t s);
-// The K > 32 forms of the statistics and of the draw (hyper_wide.cu); the draw reads one record
-// of reduced statistics (and of beta beta^T, null without side information).
+// The K > 32 forms of the statistics, and the pair's and the batch's draws (hyper_wide.cu).
 void launch_stats_wide(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
                        int uhat_stride, double* partials, int nblocks, cudaStream_t s);
 void launch_stats_wide_pair(const PriorPair& pp, bool f32, int K, int stride, cudaStream_t s);
-void launch_nw_wide(const double* stats, long long N, int K, const double* mu0, double kappa,
-                    const double* T0, int nu, const double* bb, const double* lambda_beta, Ctl* ctl,
-                    unsigned long long seed, int mode, double* mu, double* Lambda,
-                    cudaStream_t s);
-void launch_nw_wide_pair(const PriorPair& pp, int K, Ctl* ctl, unsigned long long seed,
-                         cudaStream_t s);
+void launch_normal_wishart_pair(const PriorPair& pp, int K, Ctl* ctl, unsigned long long seed,
+                                cudaStream_t s);
+void launch_nw_batch(const double* partials, const int* row0, const int* Kp,
+                     const unsigned long long* seed, int P, Ctl* ctl, int mode, double* mu,
+                     double* Lambda, float* LamF, double* lmu, cudaStream_t s);
 void launch_lambda_beta(const double* bb_partials, int nparts, int K, long long nfeat,
                         const double* Lambda, double nu, double mu, const Ctl* ctl,
                         unsigned long long seed, int mode, double* lambda_beta, cudaStream_t s);

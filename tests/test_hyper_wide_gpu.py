@@ -1,5 +1,6 @@
-"""The hyperprior update for 32 < K <= 128 (hyper_wide.cu) at the edges of its 8 x 8 tiles, of its
-four-row steps and of its row blocks (128 rows each), FP64 and mixed, one mode and both."""
+"""The hyperprior update (hyper_wide.cu, k_stats32) at the edges of its 8 x 8 tiles, of its four-row
+steps, of its row blocks (128 rows each) and of the partials the draw adds itself (16 blocks), FP64
+and mixed, one mode and both."""
 import numpy as np
 import pytest
 
@@ -17,8 +18,8 @@ def matrix(rows, cols):
                 vals=rng.normal(size=rows), shape=(rows, cols))
 
 
-@pytest.mark.parametrize("K", [33, 40, 63, 64, 65, 100, 128])
-@pytest.mark.parametrize("rows", [1, 130, 517])
+@pytest.mark.parametrize("K", [1, 2, 7, 8, 9, 20, 32, 33, 40, 63, 64, 65, 100, 128])
+@pytest.mark.parametrize("rows", [1, 130, 517, 2100])
 @pytest.mark.parametrize("compute", [_lib.MG_COMPUTE_FP64, _lib.MG_COMPUTE_MIXED])
 def test_draw_matches_oracle(K, rows, compute):
     rng = np.random.default_rng(K + rows)
@@ -36,7 +37,7 @@ def test_draw_matches_oracle(K, rows, compute):
     s.close()
 
 
-@pytest.mark.parametrize("K", [40, 128])
+@pytest.mark.parametrize("K", [10, 40, 128])
 def test_both_modes_at_once_match_one_at_a_time(K):
     rng = np.random.default_rng(K)
     w = matrix(300, 170)
