@@ -23,6 +23,7 @@
 #include "mma_tiles.cuh"
 #include "rng.cuh"
 #include "warp_finish.cuh"
+#include "wide_tiles.cuh"
 
 namespace mg {
 namespace {
@@ -41,8 +42,11 @@ struct Warp64 {
   static constexpr int TILES = NB * (NB + 1) / 2;
   static constexpr int LD = KP + 1;             // Gram tile in shared memory
   static constexpr int kRing = 4;               // gather stages: loads run three steps ahead
-  // Gram (KP x LD), later the factor's L^T (KP x (KP + 4)); then the rhs
-  static constexpr size_t kWarpDoubles = (size_t)KP * (KP + 4) + KP;
+  // MM's tiles and the inverses of the diagonal ones, or the whole Gram of the univariate draws
+  // (KP x LD); then the rhs
+  static constexpr size_t kTiles = (size_t)(TILES + NB) * 64;
+  static constexpr size_t kWork = kTiles > (size_t)KP * LD ? kTiles : (size_t)KP * LD;
+  static constexpr size_t kWarpDoubles = kWork + KP;
   static constexpr size_t kCtaDoubles = (size_t)KP * (KP + 1) + KP;  // Lambda, Lambda mu
 };
 
@@ -74,7 +78,7 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
   double* lmu_s = Lam_s + KP * (KP + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* Gs = smem_d + C::kCtaDoubles + (size_t)warp * C::kWarpDoubles;
-  double* rhs_s = Gs + KP * (KP + 4);
+  double* rhs_s = Gs + C::kWork;
   const int g = lane >> 2, t = lane & 3;
   const int K = p.K, ntasks = p.ntasks;
   // the first task is claimed while Lambda is staged
@@ -193,29 +197,30 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
     }
 
     if (finish) {
-      // the Gram (both triangles) and the rhs to shared memory; then lane i owns row i
-      int q = 0;
-#pragma unroll
-      for (int bi = 0; bi < NB; bi++)
-#pragma unroll
-        for (int bj = 0; bj <= bi; bj++) {
-          const int i = comp_of<KP>(bi, g), j0 = comp_of<KP>(bj, 2 * t),
-                    j1 = comp_of<KP>(bj, 2 * t + 1);
-          Gs[i * LD + j0] = acc[q][0];
-          Gs[i * LD + j1] = acc[q][1];
-          if (bi != bj) {
-            Gs[j0 * LD + i] = acc[q][0];
-            Gs[j1 * LD + i] = acc[q][1];
-          }
-          q++;
-        }
-      if (t == 0)
-#pragma unroll
-        for (int b = 0; b < NB; b++) rhs_s[comp_of<KP>(b, g)] = racc[b];
-      __syncwarp();
       const int row = tk.row;
-      const double rac = lane < KP ? rhs_s[lane] : 0.0;
-      if (p.one) {  // univariate prior: coordinate draws from the Gram (warp_finish.cuh)
+      if (p.one) {
+        // univariate prior: the Gram (both triangles) to shared memory, coordinate draws from it by
+        // the lane of its row (warp_finish.cuh)
+        int q = 0;
+#pragma unroll
+        for (int bi = 0; bi < NB; bi++)
+#pragma unroll
+          for (int bj = 0; bj <= bi; bj++) {
+            const int i = comp_of<KP>(bi, g), j0 = comp_of<KP>(bj, 2 * t),
+                      j1 = comp_of<KP>(bj, 2 * t + 1);
+            Gs[i * LD + j0] = acc[q][0];
+            Gs[i * LD + j1] = acc[q][1];
+            if (bi != bj) {
+              Gs[j0 * LD + i] = acc[q][0];
+              Gs[j1 * LD + i] = acc[q][1];
+            }
+            q++;
+          }
+        if (t == 0)
+#pragma unroll
+          for (int b = 0; b < NB; b++) rhs_s[comp_of<KP>(b, g)] = racc[b];
+        __syncwarp();
+        const double rac = lane < KP ? rhs_s[lane] : 0.0;
         double gr[KP];
 #pragma unroll
         for (int j = 0; j < KP; j++) gr[j] = lane < K ? Gs[lane * LD + j] : 0.0;
@@ -223,6 +228,31 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
         const double un = one_gs_warp<KP, double>(gr, rac, u0, p, row, sweep, lane);
         if (lane < K) p.out_f64[(size_t)row * KP + lane] = un;
       } else {
+        const double z = row_noise(p, row, K, lane, sweep);
+        // MM = Lambda + alpha G as tiles, each unordered pair of components once (the blocks hold
+        // the components in another order), the identity beyond K; the rhs by component
+        auto put = [&](int i, int j, double gram) {
+          const int hi = max(i, j), lo = min(i, j);
+          Gs[elem_at(hi, lo)] = hi < K ? Lam_s[hi * (KP + 1) + lo] + alpha * gram
+                                       : (hi == lo ? 1.0 : 0.0);
+        };
+        int q = 0;
+#pragma unroll
+        for (int bi = 0; bi < NB; bi++)
+#pragma unroll
+          for (int bj = 0; bj <= bi; bj++) {
+            const int i = comp_of<KP>(bi, g);
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+              const int j = comp_of<KP>(bj, 2 * t + e);
+              if (bi != bj || i >= j) put(i, j, acc[q][e]);
+            }
+            q++;
+          }
+        if (t == 0)
+#pragma unroll
+          for (int b = 0; b < NB; b++) rhs_s[comp_of<KP>(b, g)] = racc[b];
+        __syncwarp();
         double lm;
         if (p.uhat) {  // Macau prior mean mu + Uhat[row]
           const double mun = lane < K ? p.mu[lane] + p.uhat[(size_t)row * KP + lane] : 0.0;
@@ -234,9 +264,12 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
         } else {
           lm = lane < KP ? lmu_s[lane] : 0.0;
         }
-        const bool ok = warp_finish_f64_body<KP, double>(
-            Gs, LD, Lam_s, rac + lm, p, row, sweep, reinterpret_cast<unsigned char*>(Gs));
-        if (!ok && lane == 0) {
+        if (lane < KP) rhs_s[lane] += lm;
+        __syncwarp();
+        double x;
+        if (warp_tiles_solve<NB>(Gs, Gs + C::TILES * 64, rhs_s, (K + 7) / 8, z, lane, x)) {
+          if (lane < K) p.out_f64[(size_t)row * KP + lane] = x;
+        } else if (lane == 0) {
           atomicOr(&p.ctl->status, kStatCholFail);
           atomicCAS(&p.ctl->bad_row, -1, row);
         }

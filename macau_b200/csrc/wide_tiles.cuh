@@ -163,6 +163,11 @@ __device__ __forceinline__ bool diag_factor(F (&x)[8], const F* diag0, F rel_flo
   return ok;
 }
 
+__device__ __forceinline__ bool diag_factor(double (&x)[8]) {
+  const double zero[8] = {};
+  return diag_factor(x, zero, 0.0);
+}
+
 // Tile T <- T L^{-T}, Di the transposed inverse of L, by one warp.
 __device__ __forceinline__ void solve_tile(double* T, const double* Di, int lane) {
   const int g = lane >> 2, t = lane & 3;
@@ -322,6 +327,114 @@ __device__ __forceinline__ void inverse_column(const double* L, double* Y, int b
     *reinterpret_cast<double2*>(out + tile_pos(g, 2 * t)) = v;
     __syncwarp();
   }
+}
+
+// ---- the same for one warp and at most 32 rows (NB <= 4 blocks): factor, forward substitution,
+// the draw z added, backward substitution.  y: right-hand side by component; returns x of component
+// `lane`.  False when a pivot is not positive.
+template <int NB>
+__device__ __forceinline__ bool warp_tiles_solve(double* M, double* Di, double* y, int nb, double z,
+                                                 int lane, double& x_out) {
+  const int g = lane >> 2, t = lane & 3, r8 = lane & 7;
+  const int p0 = tile_pos(g, t), p1 = tile_pos(g, t + 4), pc = tile_pos(g, 2 * t);
+#pragma unroll 1
+  for (int pn = 0; pn < nb; pn++) {
+    if (pn > 0) {
+      // y's components from the panel on by the panel before; the panel's tiles by all before it
+      double s = 0.0, s1 = 0.0;
+      const bool on = lane >= 8 * pn && lane < 8 * nb;
+      if (on) {
+        double v[8];
+        load_row8(M + tile_at(lane >> 3, pn - 1), r8, v);
+        s = y[lane];
+#pragma unroll
+        for (int c = 0; c < 8; c += 2) {
+          s = fma(-v[c], y[8 * pn - 8 + c], s);
+          s1 = fma(-v[c + 1], y[8 * pn - 7 + c], s1);
+        }
+      }
+      double2 acc[NB];
+#pragma unroll
+      for (int bi = 1; bi < NB; bi++)
+        if (bi >= pn && bi < nb) acc[bi] = *reinterpret_cast<double2*>(M + tile_at(bi, pn) + pc);
+      for (int k = 0; k < pn; k++) {
+        const double* B = M + tile_at(pn, k);
+        const double b0 = -B[p0], b1 = -B[p1];
+#pragma unroll
+        for (int bi = 1; bi < NB; bi++)
+          if (bi >= pn && bi < nb) {
+            const double* A = M + tile_at(bi, k);
+            mma_f64(acc[bi].x, acc[bi].y, A[p0], b0);
+            mma_f64(acc[bi].x, acc[bi].y, A[p1], b1);
+          }
+      }
+      __syncwarp();
+      if (on) y[lane] = s + s1;
+#pragma unroll
+      for (int bi = 1; bi < NB; bi++)
+        if (bi >= pn && bi < nb) *reinterpret_cast<double2*>(M + tile_at(bi, pn) + pc) = acc[bi];
+      __syncwarp();
+    }
+    // lanes 0-7: the diagonal tile's rows, 8-15: the identity's, 16: y
+    double* row = lane < 8 ? M + tile_at(pn, pn) : (lane < 16 ? Di + 64 * pn : y + 8 * pn);
+    const int r = lane < 16 ? r8 : 0;
+    double x[8];
+    if (lane < 8 || lane == 16) {
+      load_row8(row, r, x);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 8; c++) x[c] = lane - 8 == c ? 1.0 : 0.0;
+    }
+    if (!diag_factor(x)) return false;
+    if (lane >= 8 && lane <= 16) store_row8(row, r, x);
+    __syncwarp();
+    if (pn + 1 < nb) {
+      const double* D = Di + 64 * pn;
+      const double d0 = D[tile_pos(t, g)], d1 = D[tile_pos(t + 4, g)];
+      double2 acc[NB];
+#pragma unroll
+      for (int bi = 1; bi < NB; bi++)
+        if (bi > pn && bi < nb) {
+          const double* T = M + tile_at(bi, pn);
+          acc[bi] = make_double2(0.0, 0.0);
+          mma_f64(acc[bi].x, acc[bi].y, T[p0], d0);
+          mma_f64(acc[bi].x, acc[bi].y, T[p1], d1);
+        }
+      __syncwarp();
+#pragma unroll
+      for (int bi = 1; bi < NB; bi++)
+        if (bi > pn && bi < nb) *reinterpret_cast<double2*>(M + tile_at(bi, pn) + pc) = acc[bi];
+      __syncwarp();
+    }
+  }
+  // backward: lane's component of b = y + z stays in a register, the panel's x go round by shuffles
+  double b = lane < 8 * nb ? y[lane] + z : 0.0;
+  x_out = 0.0;
+#pragma unroll 1
+  for (int pn = nb - 1; pn >= 0; pn--) {
+    double d[8], u0 = 0.0, u1 = 0.0;
+    load_row8(Di + 64 * pn, r8, d);
+    const bool on = lane < 8 * pn;
+    const double* P = M + tile_at(pn, on ? lane >> 3 : 0);
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      u0 = fma(d[c], wshfl(b, 8 * pn + c), u0);
+      u1 = fma(d[c + 1], wshfl(b, 8 * pn + c + 1), u1);
+    }
+    const double xr = u0 + u1;  // x of component 8 pn + lane % 8
+    if ((lane >> 3) == pn) x_out = xr;
+    double s1 = 0.0;
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      const double x0 = wshfl(xr, c), x1 = wshfl(xr, c + 1);
+      if (on) {
+        b = fma(-P[tile_pos(c, r8)], x0, b);
+        s1 = fma(-P[tile_pos(c + 1, r8)], x1, s1);
+      }
+    }
+    b += s1;
+  }
+  return true;
 }
 
 }  // namespace mg
