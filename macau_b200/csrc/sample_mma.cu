@@ -28,14 +28,6 @@
 namespace mg {
 namespace {
 
-// Component of fragment block b held by lane group g.  Two blocks share one 16-byte load, so that
-// the eight groups read 128 contiguous bytes of a gathered row: blocks 2c and 2c + 1 hold the
-// even and odd components of 16c .. 16c + 15.
-template <int KP>
-__device__ __forceinline__ int comp_of(int b, int g) {
-  return KP == 8 ? g : 16 * (b >> 1) + 2 * g + (b & 1);
-}
-
 template <int KP>
 struct Warp64 {
   static constexpr int NB = KP / 8;             // component blocks
@@ -47,25 +39,16 @@ struct Warp64 {
   static constexpr size_t kTiles = (size_t)(TILES + NB) * 64;
   static constexpr size_t kWork = kTiles > (size_t)KP * LD ? kTiles : (size_t)KP * LD;
   static constexpr size_t kWarpDoubles = kWork + KP;
-  static constexpr size_t kCtaDoubles = (size_t)KP * (KP + 1) + KP;  // Lambda, Lambda mu
+  static constexpr size_t kCtaDoubles = (size_t)TILES * 64 + KP;  // Lambda's tiles, Lambda mu
 };
 
-// Fragment blocks of one entry (lane's group g) of the gathered row `row`, zero when !ok.
+// Fragment blocks of one entry (component g of each block) of the gathered row `row`, zero when !ok.
 template <int KP>
 __device__ __forceinline__ void gather_frag(double (&f)[KP / 8], const double* __restrict__ other,
                                             int row, int g, bool ok) {
-  const double* src = other + (size_t)row * KP;
-  if constexpr (KP == 8) {
-    f[0] = ok ? __ldg(src + g) : 0.0;
-  } else {
+  const double* src = other + (size_t)row * KP + g;
 #pragma unroll
-    for (int c = 0; c < KP / 16; c++) {
-      const double2 v = ok ? __ldg(reinterpret_cast<const double2*>(src + 16 * c) + g)
-                           : make_double2(0.0, 0.0);
-      f[2 * c] = v.x;
-      f[2 * c + 1] = v.y;
-    }
-  }
+  for (int b = 0; b < KP / 8; b++) f[b] = ok ? __ldg(src + 8 * b) : 0.0;
 }
 
 // G warps (row groups) per CTA; 16 warps per SM in every shape.
@@ -74,8 +57,8 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
   using C = Warp64<KP>;
   constexpr int NB = C::NB, LD = C::LD, R = C::kRing;
   extern __shared__ __align__(16) double smem_d[];
-  double* Lam_s = smem_d;  // Lambda (row-major, ld KP + 1), then Lambda mu
-  double* lmu_s = Lam_s + KP * (KP + 1);
+  double* Lam_s = smem_d;  // Lambda's lower-triangle tiles, the identity beyond K; then Lambda mu
+  double* lmu_s = Lam_s + C::TILES * 64;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* Gs = smem_d + C::kCtaDoubles + (size_t)warp * C::kWarpDoubles;
   double* rhs_s = Gs + C::kWork;
@@ -86,14 +69,15 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
   if (lane == 0) ti = (int)atomicAdd(&p.ctl->queue[p.qslot], 1u);
   ti = __shfl_sync(0xffffffffu, ti, 0);
   for (int e = threadIdx.x; e < KP * KP; e += blockDim.x) {
-    const int i = e / KP, j = e % KP;
-    Lam_s[i * (KP + 1) + j] = (i < K && j < K) ? p.Lambda[i + j * K] : 0.0;
+    const int i = e % KP, j = e / KP;
+    if ((i >> 3) >= (j >> 3))
+      Lam_s[tile_at(i >> 3, j >> 3) + tile_pos(i & 7, j & 7)] =
+          i < K && j < K ? p.Lambda[i + j * K] : (i == j ? 1.0 : 0.0);
   }
-  __syncthreads();
   if (threadIdx.x < KP) {
     double s = 0.0;
     if ((int)threadIdx.x < K)
-      for (int j = 0; j < K; j++) s += Lam_s[threadIdx.x * (KP + 1) + j] * p.mu[j];
+      for (int j = 0; j < K; j++) s += p.Lambda[threadIdx.x + j * K] * p.mu[j];
     lmu_s[threadIdx.x] = s;
   }
   __syncthreads();
@@ -101,10 +85,23 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
   const double* other = reinterpret_cast<const double*>(p.other);
   const double alpha = noise_alpha(p);
 
+  // entries in chunks of 32 (lane l: entry l of the chunk), steps of four entries
+  auto load_chunk = [&](const RowTask& task, int off, int& c, double& w) {
+    const bool in = off + lane < task.len;
+    c = in ? __ldcs(p.colidx + task.begin + off + lane) : 0;
+    w = in ? (__ldcs(p.vals + task.begin + off + lane) - p.mean) * alpha : 0.0;
+  };
+  RowTask tk{};
+  int c_cur = 0, c_nxt = 0, c_nn = 0;  // this chunk's columns, the next one's and the one after's
+  double w_cur = 0.0, w_nxt = 0.0, w_nn = 0.0;
+  if (ti < ntasks) {
+    tk = p.tasks[ti];
+    load_chunk(tk, 0, c_cur, w_cur);
+  }
   while (ti < ntasks) {
-    const RowTask tk = p.tasks[ti];
     int ti_next = 0;  // claimed early: its latency passes behind this row
     if (lane == 0) ti_next = (int)atomicAdd(&p.ctl->queue[p.qslot], 1u);
+    load_chunk(tk, 32, c_nxt, w_nxt);
 
     double acc[C::TILES][2];
     double racc[NB];
@@ -113,22 +110,13 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
 #pragma unroll
     for (int b = 0; b < NB; b++) racc[b] = 0.0;
 
-    // entries in chunks of 32 (lane l: entry l of the chunk), steps of four entries
-    auto load_chunk = [&](int off, int& c, double& w) {
-      const bool in = off + lane < tk.len;
-      c = in ? p.colidx[tk.begin + off + lane] : 0;
-      w = in ? (p.vals[tk.begin + off + lane] - p.mean) * alpha : 0.0;
-    };
-    int c_cur, c_nxt = 0;
-    double w_cur, w_nxt = 0.0;
-    load_chunk(0, c_cur, w_cur);
     double f[R][NB];
 #pragma unroll
     for (int u = 0; u < R - 1; u++)
       gather_frag<KP>(f[u], other, __shfl_sync(0xffffffffu, c_cur, 4 * u + t), g,
                       4 * u + t < tk.len);
     for (int off = 0; off < tk.len; off += 32) {
-      load_chunk(off + 32, c_nxt, w_nxt);
+      load_chunk(tk, off + 64, c_nn, w_nn);
 #pragma unroll
       for (int u = 0; u < 8; u++) {
         if (off + 4 * u < tk.len) {
@@ -151,6 +139,15 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
       }
       c_cur = c_nxt;
       w_cur = w_nxt;
+      c_nxt = c_nn;
+      w_nxt = w_nn;
+    }
+    // the next row's task and first chunk are loaded behind this row's finish
+    ti = __shfl_sync(0xffffffffu, ti_next, 0);
+    RowTask tk_next{};
+    if (ti < ntasks) {
+      tk_next = p.tasks[ti];
+      load_chunk(tk_next, 0, c_cur, w_cur);
     }
     // the rhs: the four entry lanes of a group hold partial sums
 #pragma unroll
@@ -206,8 +203,7 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
         for (int bi = 0; bi < NB; bi++)
 #pragma unroll
           for (int bj = 0; bj <= bi; bj++) {
-            const int i = comp_of<KP>(bi, g), j0 = comp_of<KP>(bj, 2 * t),
-                      j1 = comp_of<KP>(bj, 2 * t + 1);
+            const int i = 8 * bi + g, j0 = 8 * bj + 2 * t, j1 = j0 + 1;
             Gs[i * LD + j0] = acc[q][0];
             Gs[i * LD + j1] = acc[q][1];
             if (bi != bj) {
@@ -218,7 +214,7 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
           }
         if (t == 0)
 #pragma unroll
-          for (int b = 0; b < NB; b++) rhs_s[comp_of<KP>(b, g)] = racc[b];
+          for (int b = 0; b < NB; b++) rhs_s[8 * b + g] = racc[b];
         __syncwarp();
         const double rac = lane < KP ? rhs_s[lane] : 0.0;
         double gr[KP];
@@ -229,29 +225,21 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
         if (lane < K) p.out_f64[(size_t)row * KP + lane] = un;
       } else {
         const double z = row_noise(p, row, K, lane, sweep);
-        // MM = Lambda + alpha G as tiles, each unordered pair of components once (the blocks hold
-        // the components in another order), the identity beyond K; the rhs by component
-        auto put = [&](int i, int j, double gram) {
-          const int hi = max(i, j), lo = min(i, j);
-          Gs[elem_at(hi, lo)] = hi < K ? Lam_s[hi * (KP + 1) + lo] + alpha * gram
-                                       : (hi == lo ? 1.0 : 0.0);
-        };
+        // MM = Lambda + alpha G as tiles (the Gram is zero beyond K), the rhs by component
         int q = 0;
 #pragma unroll
         for (int bi = 0; bi < NB; bi++)
 #pragma unroll
           for (int bj = 0; bj <= bi; bj++) {
-            const int i = comp_of<KP>(bi, g);
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-              const int j = comp_of<KP>(bj, 2 * t + e);
-              if (bi != bj || i >= j) put(i, j, acc[q][e]);
-            }
+            const int at = tile_at(bi, bj) + tile_pos(g, 2 * t);
+            const double2 lam = *reinterpret_cast<const double2*>(Lam_s + at);
+            *reinterpret_cast<double2*>(Gs + at) =
+                make_double2(lam.x + alpha * acc[q][0], lam.y + alpha * acc[q][1]);
             q++;
           }
         if (t == 0)
 #pragma unroll
-          for (int b = 0; b < NB; b++) rhs_s[comp_of<KP>(b, g)] = racc[b];
+          for (int b = 0; b < NB; b++) rhs_s[8 * b + g] = racc[b];
         __syncwarp();
         double lm;
         if (p.uhat) {  // Macau prior mean mu + Uhat[row]
@@ -259,16 +247,16 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
           lm = 0.0;
           for (int j = 0; j < K; j++) {
             const double mj = wshfl(mun, j);
-            if (lane < K) lm += Lam_s[lane * (KP + 1) + j] * mj;
+            if (lane < K) lm += p.Lambda[lane + j * K] * mj;
           }
         } else {
           lm = lane < KP ? lmu_s[lane] : 0.0;
         }
         if (lane < KP) rhs_s[lane] += lm;
         __syncwarp();
-        double x;
-        if (warp_tiles_solve<NB>(Gs, Gs + C::TILES * 64, rhs_s, (K + 7) / 8, z, lane, x)) {
-          if (lane < K) p.out_f64[(size_t)row * KP + lane] = x;
+        if (warp_tiles_solve<NB>(Gs, Gs + C::TILES * 64, rhs_s, (K + 7) / 8, z, lane)) {
+          __syncwarp();
+          if (lane < K) p.out_f64[(size_t)row * KP + lane] = rhs_s[lane];
         } else if (lane == 0) {
           atomicOr(&p.ctl->status, kStatCholFail);
           atomicCAS(&p.ctl->bad_row, -1, row);
@@ -276,7 +264,7 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
       }
       __syncwarp();
     }
-    ti = __shfl_sync(0xffffffffu, ti_next, 0);
+    tk = tk_next;
   }
 }
 

@@ -330,36 +330,30 @@ __device__ __forceinline__ void inverse_column(const double* L, double* Y, int b
 }
 
 // ---- the same for one warp and at most 32 rows (NB <= 4 blocks): factor, forward substitution,
-// the draw z added, backward substitution.  y: right-hand side by component; returns x of component
-// `lane`.  False when a pivot is not positive.
+// the draw z added, backward substitution.  y: right-hand side by component, overwritten by x.
+// False when a pivot is not positive.
+//   What bounds it: the shared-memory pipe (loads, stores and shuffles), so the vectors go through
+// the matrix instruction as well, as a row that every lane group repeats: a tile's fragment costs
+// two conflict-free loads where a row or a column per lane cost eight conflicting ones.
 template <int NB>
 __device__ __forceinline__ bool warp_tiles_solve(double* M, double* Di, double* y, int nb, double z,
-                                                 int lane, double& x_out) {
+                                                 int lane) {
   const int g = lane >> 2, t = lane & 3, r8 = lane & 7;
   const int p0 = tile_pos(g, t), p1 = tile_pos(g, t + 4), pc = tile_pos(g, 2 * t);
+  const int q0 = tile_pos(t, g), q1 = tile_pos(t + 4, g);
+  auto pair_at = [&](double* v, int b) { return reinterpret_cast<double2*>(v + 8 * b + 2 * t); };
 #pragma unroll 1
   for (int pn = 0; pn < nb; pn++) {
     if (pn > 0) {
-      // y's components from the panel on by the panel before; the panel's tiles by all before it
-      double s = 0.0, s1 = 0.0;
-      const bool on = lane >= 8 * pn && lane < 8 * nb;
-      if (on) {
-        double v[8];
-        load_row8(M + tile_at(lane >> 3, pn - 1), r8, v);
-        s = y[lane];
-#pragma unroll
-        for (int c = 0; c < 8; c += 2) {
-          s = fma(-v[c], y[8 * pn - 8 + c], s);
-          s1 = fma(-v[c + 1], y[8 * pn - 7 + c], s1);
-        }
-      }
-      double2 acc[NB];
+      // the panel's tiles and y's components by all panels before it
+      double2 acc[NB], ya = *pair_at(y, pn);
 #pragma unroll
       for (int bi = 1; bi < NB; bi++)
         if (bi >= pn && bi < nb) acc[bi] = *reinterpret_cast<double2*>(M + tile_at(bi, pn) + pc);
       for (int k = 0; k < pn; k++) {
         const double* B = M + tile_at(pn, k);
         const double b0 = -B[p0], b1 = -B[p1];
+        mma_f64(ya.x, ya.y, y[8 * k + t], b0);
 #pragma unroll
         for (int bi = 1; bi < NB; bi++)
           if (bi >= pn && bi < nb) {
@@ -367,9 +361,10 @@ __device__ __forceinline__ bool warp_tiles_solve(double* M, double* Di, double* 
             mma_f64(acc[bi].x, acc[bi].y, A[p0], b0);
             mma_f64(acc[bi].x, acc[bi].y, A[p1], b1);
           }
+        mma_f64(ya.x, ya.y, y[8 * k + 4 + t], b1);
       }
       __syncwarp();
-      if (on) y[lane] = s + s1;
+      if (g == 0) *pair_at(y, pn) = ya;
 #pragma unroll
       for (int bi = 1; bi < NB; bi++)
         if (bi >= pn && bi < nb) *reinterpret_cast<double2*>(M + tile_at(bi, pn) + pc) = acc[bi];
@@ -389,8 +384,7 @@ __device__ __forceinline__ bool warp_tiles_solve(double* M, double* Di, double* 
     if (lane >= 8 && lane <= 16) store_row8(row, r, x);
     __syncwarp();
     if (pn + 1 < nb) {
-      const double* D = Di + 64 * pn;
-      const double d0 = D[tile_pos(t, g)], d1 = D[tile_pos(t + 4, g)];
+      const double d0 = Di[64 * pn + q0], d1 = Di[64 * pn + q1];
       double2 acc[NB];
 #pragma unroll
       for (int bi = 1; bi < NB; bi++)
@@ -407,32 +401,33 @@ __device__ __forceinline__ bool warp_tiles_solve(double* M, double* Di, double* 
       __syncwarp();
     }
   }
-  // backward: lane's component of b = y + z stays in a register, the panel's x go round by shuffles
-  double b = lane < 8 * nb ? y[lane] + z : 0.0;
-  x_out = 0.0;
+  if (lane < 8 * nb) y[lane] += z;
+  __syncwarp();
 #pragma unroll 1
   for (int pn = nb - 1; pn >= 0; pn--) {
-    double d[8], u0 = 0.0, u1 = 0.0;
-    load_row8(Di + 64 * pn, r8, d);
-    const bool on = lane < 8 * pn;
-    const double* P = M + tile_at(pn, on ? lane >> 3 : 0);
+    double2 v = make_double2(0.0, 0.0);
+    mma_f64(v.x, v.y, y[8 * pn + t], Di[64 * pn + p0]);
+    mma_f64(v.x, v.y, y[8 * pn + 4 + t], Di[64 * pn + p1]);
+    __syncwarp();
+    if (g == 0) *pair_at(y, pn) = v;
+    __syncwarp();
+    if (pn > 0) {
+      const double x0 = -y[8 * pn + t], x1 = -y[8 * pn + 4 + t];
+      double2 acc[NB];
 #pragma unroll
-    for (int c = 0; c < 8; c += 2) {
-      u0 = fma(d[c], wshfl(b, 8 * pn + c), u0);
-      u1 = fma(d[c + 1], wshfl(b, 8 * pn + c + 1), u1);
-    }
-    const double xr = u0 + u1;  // x of component 8 pn + lane % 8
-    if ((lane >> 3) == pn) x_out = xr;
-    double s1 = 0.0;
+      for (int bj = 0; bj < NB - 1; bj++)
+        if (bj < pn) {
+          const double* P = M + tile_at(pn, bj);
+          acc[bj] = *pair_at(y, bj);
+          mma_f64(acc[bj].x, acc[bj].y, x0, P[q0]);
+          mma_f64(acc[bj].x, acc[bj].y, x1, P[q1]);
+        }
+      __syncwarp();
 #pragma unroll
-    for (int c = 0; c < 8; c += 2) {
-      const double x0 = wshfl(xr, c), x1 = wshfl(xr, c + 1);
-      if (on) {
-        b = fma(-P[tile_pos(c, r8)], x0, b);
-        s1 = fma(-P[tile_pos(c + 1, r8)], x1, s1);
-      }
+      for (int bj = 0; bj < NB - 1; bj++)
+        if (bj < pn && g == 0) *pair_at(y, bj) = acc[bj];
+      __syncwarp();
     }
-    b += s1;
   }
   return true;
 }
