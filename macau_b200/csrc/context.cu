@@ -371,7 +371,6 @@ class Context {
       // level of an earlier feature sharing a row with f (0 when none)
       std::vector<double> cs(nfeat, 0.0);
       std::vector<int> level(nfeat, 0), last(nrows, -1);
-      int nl = 0;
       for (int f = 0; f < nfeat; f++) {
         int lv = 0;
         for (long long e = t.ptr[f]; e < t.ptr[f + 1]; e++) {
@@ -380,21 +379,9 @@ class Context {
         }
         for (long long e = t.ptr[f]; e < t.ptr[f + 1]; e++) last[t.idx[e]] = lv;
         level[f] = lv;
-        nl = std::max(nl, lv + 1);
       }
-      std::vector<int> lptr(nl + 1, 0), order(nfeat);
-      for (int f = 0; f < nfeat; f++) lptr[level[f] + 1]++;
-      for (int l = 0; l < nl; l++) lptr[l + 1] += lptr[l];
-      std::vector<int> fill(lptr.begin(), lptr.end() - 1);
-      for (int f = 0; f < nfeat; f++) order[fill[level[f]]++] = f;
-      // a level runs one warp per feature or each feature by the whole block
-      std::vector<int> lwarp(nl, 1);
-      for (int l = 0; l < nl; l++) {
-        long long longest = 0;
-        for (int q = lptr[l]; q < lptr[l + 1]; q++)
-          longest = std::max(longest, t.ptr[order[q] + 1] - t.ptr[order[q]]);
-        lwarp[l] = beta_one_warp_level(nrows, lptr[l + 1] - lptr[l], longest) ? 1 : 0;
-      }
+      std::vector<int> lptr, order, lwarp;
+      beta_one_levels(nrows, level, t.ptr, lptr, order, lwarp);
       p.colsq.upload(cs.data(), cs.size(), s_);
       p.lvl_warp.upload(lwarp.data(), lwarp.size(), s_);
       p.lvl_ptr.upload(lptr.data(), lptr.size(), s_);
@@ -403,7 +390,7 @@ class Context {
       for (int q = 0; q < nfeat; q++)
         range[q] = make_longlong2(t.ptr[order[q]], t.ptr[order[q] + 1]);
       p.lvl_range.upload(range.data(), range.size(), s_);
-      p.nlevels = nl;
+      p.nlevels = (int)lwarp.size();
     }
     MG_CUDA(cudaStreamSynchronize(s_));
     drop_graphs();

@@ -189,9 +189,11 @@ void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
 void launch_lambda_beta_one(const double* beta, int bstride, long long nfeat, int K, double a0,
                             double b0, const Ctl* ctl, unsigned long long seed, int mode,
                             double* parts, double* lambda_beta, cudaStream_t s);
-// Whether a level of `nfeat` features, the longest of `longest` entries, runs a warp per feature
-// (lvl_warp) for a side matrix of N rows.
-bool beta_one_warp_level(long long N, long long nfeat, long long longest);
+// Level tables of the link sampler for a side matrix of N rows from each feature's level and the column
+// pointers: features in level order, the bounds of the (possibly split) levels and lvl_warp.
+void beta_one_levels(long long N, const std::vector<int>& level, const std::vector<long long>& ptr,
+                     std::vector<int>& lvl_ptr, std::vector<int>& order,
+                     std::vector<int>& lvl_warp);
 
 // sample_beta pieces (latentprior.cpp:273-293)
 //   tmp[n] = U[n] + chol(Lambda)^{-T} z_n - mu      (n < N; z keyed (kMvnN, n))

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <numeric>
+#include <vector>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -143,26 +145,39 @@ __global__ void __launch_bounds__(kBetaThreads)
 
 // The same link sampler with one block per dimension d and this dimension's column of Z held in
 // shared memory (N doubles, N <= kZsMax), so the feature-by-feature chain reads and writes no
-// global memory but beta, with 32 warps per block.
+// global memory but beta, with 16 warps per block (with 32 the idle ones' instructions cost more than
+// their share of the work saves, with 8 the long features take longer).
 //   What bounds it: the chain over the levels.  A level gives each of its features to a warp, or each
-// in turn to the whole block (lvl_warp, by the estimate of beta_one_warp_level).  While a feature is
-// processed, everything about the next one that no other feature changes is loaded: its entry
-// range, the first entries' rows, its coefficient and draw with the reciprocal and the square root
-// they are scaled by, and the next level's bounds.  The block's sum takes one barrier: every
-// warp adds the 32 warps' sums for itself by a shuffle tree.  (Reading each entry's row twice from
-// global memory, a warp for features of up to 1,024 entries and one thread to add the warps' sums,
-// 1,294 us for the 8,193 features, 250,000 entries and 32 dimensions of a 5,003-row matrix.)
+// in turn to the whole block (lvl_warp, beta_one_levels).  Nothing that a feature needs is more than
+// one memory latency behind when its level begins: the bounds of a level are loaded three levels
+// ahead, the id and entry range of the feature that a warp takes in it two ahead, its first
+// entries' rows, coefficient, draw and squared norm one ahead.  The
+// block's sum takes one barrier: every warp adds the warps' sums for itself by a shuffle tree.
+// 32,768 features, 20,000 rows, 1M entries, 32 dimensions: 6.0 -> 3.0 ms; 8,193 features in 615
+// levels, 5,003 rows, 250,000 entries: 1.29 -> 1.10 ms.
 constexpr int kZsMax = 26 * 1024;
-constexpr int kSmemThreads = 1024;
+constexpr int kSmemThreads = 512;
+constexpr int kNp = 6;  // entries held ahead per thread
 constexpr int kSmemWarps = kSmemThreads / 32;
 
+// A level: features f0 .. f1 - 1 of the level order, a warp each or the block for each in turn.
+struct LevelPre {
+  int f0, f1, warp;
+};
+// The id and entry range of the feature a thread takes (f < 0: none).  These and FeaturePre hold what
+// the loads return and nothing computed from it: an instruction that used a value here would
+// hold the warp until it arrives.
+struct FeatureId {
+  int f;
+  longlong2 rg;
+};
 // A feature's constants for one dimension, and the first NP entries of a thread that takes entries
 // first, first + stride, ...
 template <bool BINARY, int NP>
 struct FeaturePre {
   int f, len;
   long long begin;
-  double bcs, b, ainv, sz;
+  double b, cs, z;
   int i[NP];
   double v[BINARY ? 1 : NP];
 };
@@ -171,33 +186,51 @@ struct BetaOne {
   const int* tidx;
   const double* tval;
   const double* colsq;
+  const int* lvl_ptr;
   const int* lvl_feat;
   const longlong2* lvl_range;
+  const int* lvl_warp;
   const double* draws;
   double* beta;
-  int bstride;
+  int bstride, nlevels;
   double lam, lb;
   int d;
 };
 
+__device__ __forceinline__ LevelPre fetch_level(const BetaOne& p, int L) {
+  if (L >= p.nlevels) return {0, 0, 1};
+  return {p.lvl_ptr[L], p.lvl_ptr[L + 1], p.lvl_warp[L]};
+}
+__device__ __forceinline__ FeatureId fetch_id(const BetaOne& p, int q, int end) {
+  FeatureId id{-1, make_longlong2(0, 0)};
+  if (q < end) {
+    id.f = p.lvl_feat[q];
+    id.rg = p.lvl_range[q];
+  }
+  return id;
+}
 template <bool BINARY, int NP>
-__device__ __forceinline__ FeaturePre<BINARY, NP> fetch_feature(const BetaOne& p, int q, int first,
-                                                               int stride) {
+__device__ __forceinline__ FeaturePre<BINARY, NP> fetch_feature(const BetaOne& p, const FeatureId& id,
+                                                               int first, int stride) {
   FeaturePre<BINARY, NP> r;
-  r.f = p.lvl_feat[q];
-  const longlong2 rg = p.lvl_range[q];
-  r.begin = rg.x;
-  r.len = (int)(rg.y - rg.x);
-  const double cs = p.colsq[r.f];
-  r.b = p.beta[(size_t)r.f * p.bstride + p.d];
-  r.bcs = r.b * cs;
-  r.ainv = 1.0 / (p.lb + p.lam * cs);
-  r.sz = sqrt(r.ainv) * p.draws[(size_t)r.f * p.bstride + p.d];
+  r.f = id.f;
+  r.begin = id.rg.x;
+  r.len = (int)(id.rg.y - id.rg.x);
+  r.b = r.cs = r.z = 0.0;
 #pragma unroll
   for (int k = 0; k < NP; k++) {
     const int e = first + k * stride;
-    r.i[k] = e < r.len ? p.tidx[r.begin + e] : -1;
-    if constexpr (!BINARY) r.v[k] = e < r.len ? p.tval[r.begin + e] : 0.0;
+    r.i[k] = -1;
+    if (e < r.len) r.i[k] = p.tidx[r.begin + e];
+    if constexpr (!BINARY) {
+      r.v[k] = 0.0;
+      if (e < r.len) r.v[k] = p.tval[r.begin + e];
+    }
+  }
+  if (id.f >= 0) {
+    r.cs = p.colsq[id.f];
+    r.b = p.beta[(size_t)id.f * p.bstride + p.d];
+    r.z = p.draws[(size_t)id.f * p.bstride + p.d];
   }
   return r;
 }
@@ -235,7 +268,8 @@ __device__ __forceinline__ void feature_add(const BetaOne& p, const FeaturePre<B
 template <bool BINARY, int NP>
 __device__ __forceinline__ double new_coef(const BetaOne& p, const FeaturePre<BINARY, NP>& r,
                                            double zx) {
-  return p.lam * (zx + r.bcs) * r.ainv + r.sz;
+  const double ainv = 1.0 / (p.lb + p.lam * r.cs);
+  return p.lam * (zx + r.b * r.cs) * ainv + sqrt(ainv) * r.z;
 }
 __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
@@ -255,79 +289,64 @@ __global__ void __launch_bounds__(kSmemThreads)
                     int K, int N, double* __restrict__ beta, int bstride,
                     const double* __restrict__ draws) {
   extern __shared__ double Zs[];
-  __shared__ double red[2][kSmemWarps];
-  constexpr int NP = BINARY ? 4 : 2;  // entries held ahead per thread
+  __shared__ double red[2][32];
+  constexpr int NP = kNp;
   const int d = blockIdx.x, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
-  const BetaOne p{tidx, tval, colsq, lvl_feat, lvl_range, draws, beta, bstride,
-                  Lambda[(size_t)d * (K + 1)], lambda_beta[d], d};
+  const BetaOne p{tidx, tval, colsq, lvl_ptr, lvl_feat, lvl_range, lvl_warp, draws, beta, bstride,
+                  nlevels, Lambda[(size_t)d * (K + 1)], lambda_beta[d], d};
   for (int i = tid; i < N; i += kSmemThreads)
     Zs[i] = (double)U[(size_t)i * ustride + d] - mu[d] - uhat[(size_t)i * hstride + d];
-  FeaturePre<BINARY, NP> cur{};
-  int cur_q = -1;  // the feature in `cur`, fetched for this thread's share of it, or -1
-  bool cur_block = false;
+  // this thread's first feature of a level, and its share of the entries
+  auto first_id = [&](const LevelPre& l) { return fetch_id(p, l.warp ? l.f0 + warp : l.f0, l.f1); };
+  auto share = [&](const LevelPre& l, const FeatureId& id) {
+    return fetch_feature<BINARY, NP>(p, id, l.warp ? lane : tid, l.warp ? 32 : kSmemThreads);
+  };
+  // rings by level: bounds, ids and features; the loop runs four levels at a time so that every
+  // ring index is a constant (a register that a load is still to fill is never moved)
+  LevelPre lev[4] = {fetch_level(p, 0), fetch_level(p, 1), fetch_level(p, 2), {0, 0, 1}};
+  FeatureId id[2] = {{-1, make_longlong2(0, 0)}, first_id(lev[1])};
+  FeaturePre<BINARY, NP> pre[2];
+  pre[0] = share(lev[0], first_id(lev[0]));
   int buf = 0;
-  int f0 = 0, f1 = nlevels > 0 ? lvl_ptr[1] : 0, mode = nlevels > 0 ? lvl_warp[0] : 0;
   __syncthreads();
-  for (int L = 0; L < nlevels; L++) {
-    // the next level's bounds and mode
-    const bool more = L + 1 < nlevels;
-    const int f2 = more ? lvl_ptr[L + 2] : f1, mode2 = more ? lvl_warp[L + 1] : -1;
-    // the feature this thread meets first in the next level
-    const int q2 = !more ? -1 : mode2 == 0 ? f1 : (f1 + warp < f2 ? f1 + warp : -1);
-    const int first2 = mode2 == 0 ? tid : lane, stride2 = mode2 == 0 ? kSmemThreads : 32;
-    if (mode != 0) {
-      // one feature per warp
-      int q = f0 + warp;
-      if (q < f1 && (cur_q != q || cur_block)) {
-        cur = fetch_feature<BINARY, NP>(p, q, lane, 32);
-        cur_q = q;
+  for (int L0 = 0; L0 < nlevels; L0 += 4) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (L0 + u >= nlevels) break;
+      const LevelPre& l = lev[u];
+      lev[(u + 3) & 3] = fetch_level(p, L0 + u + 3);
+      id[u & 1] = first_id(lev[(u + 2) & 3]);
+      pre[(u + 1) & 1] = share(lev[(u + 1) & 3], id[(u + 1) & 1]);
+      FeaturePre<BINARY, NP> cur = pre[u & 1];
+      if (l.warp) {
+        // one feature per warp
+        for (int q = l.f0 + warp; q < l.f1; q += kSmemWarps) {
+          FeaturePre<BINARY, NP> next{};
+          if (q + kSmemWarps < l.f1) next = share(l, fetch_id(p, q + kSmemWarps, l.f1));
+          const double bn = new_coef(p, cur, warp_sum(feature_dot(p, cur, Zs, lane, 32)));
+          if (lane == 0) beta[(size_t)cur.f * bstride + d] = bn;
+          feature_add(p, cur, Zs, lane, 32, cur.b - bn);
+          cur = next;
+        }
+      } else {
+        // each feature by the whole block
+        for (int q = l.f0; q < l.f1; q++) {
+          FeaturePre<BINARY, NP> next{};
+          if (q + 1 < l.f1) next = share(l, fetch_id(p, q + 1, l.f1));
+          const double part = warp_sum(feature_dot(p, cur, Zs, tid, kSmemThreads));
+          if (lane == 0) red[buf][warp] = part;
+          __syncthreads();
+          const double bn =
+              new_coef(p, cur, warp_sum(lane < kSmemWarps ? red[buf][lane] : 0.0));
+          buf ^= 1;  // the next sum goes to the other half: one barrier between writes and reads
+          if (tid == 0) beta[(size_t)cur.f * bstride + d] = bn;
+          feature_add(p, cur, Zs, tid, kSmemThreads, cur.b - bn);
+          cur = next;
+        }
       }
-      if (q >= f1 && q2 >= 0) {  // nothing to do in this level
-        cur = fetch_feature<BINARY, NP>(p, q2, first2, stride2);
-        cur_q = q2;
-        cur_block = mode2 == 0;
-      }
-      for (; q < f1; q += kSmemWarps) {
-        const bool last = q + kSmemWarps >= f1;
-        const int qn = last ? q2 : q + kSmemWarps;
-        FeaturePre<BINARY, NP> nxt{};
-        if (qn >= 0)
-          nxt = fetch_feature<BINARY, NP>(p, qn, last ? first2 : lane, last ? stride2 : 32);
-        const double bn = new_coef(p, cur, warp_sum(feature_dot(p, cur, Zs, lane, 32)));
-        if (lane == 0) beta[(size_t)cur.f * bstride + d] = bn;
-        feature_add(p, cur, Zs, lane, 32, cur.b - bn);
-        __syncwarp();
-        cur = nxt;
-        cur_q = qn;
-        cur_block = last && mode2 == 0;
-      }
-    } else {
-      // each feature by the whole block
-      for (int q = f0; q < f1; q++) {
-        if (cur_q != q || !cur_block) cur = fetch_feature<BINARY, NP>(p, q, tid, kSmemThreads);
-        const bool last = q + 1 == f1;
-        const int qn = last ? q2 : q + 1;
-        FeaturePre<BINARY, NP> nxt{};
-        if (qn >= 0)
-          nxt = fetch_feature<BINARY, NP>(p, qn, last ? first2 : tid,
-                                          last ? stride2 : kSmemThreads);
-        const double part = warp_sum(feature_dot(p, cur, Zs, tid, kSmemThreads));
-        if (lane == 0) red[buf][warp] = part;
-        __syncthreads();
-        const double bn = new_coef(p, cur, warp_sum(red[buf][lane]));
-        buf ^= 1;  // the next sum goes to the other half: one barrier between writes and reads
-        if (tid == 0) beta[(size_t)cur.f * bstride + d] = bn;
-        feature_add(p, cur, Zs, tid, kSmemThreads, cur.b - bn);
-        cur = nxt;
-        cur_q = qn;
-        cur_block = !last || mode2 == 0;
-      }
+      __syncthreads();
     }
-    __syncthreads();
-    f0 = f1;
-    f1 = f2;
-    mode = mode2;
   }
 }
 
@@ -444,14 +463,53 @@ void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
   MG_CUDA(cudaGetLastError());
 }
 
-// Cycles of a level by a warp per feature (32 at a time, a step of 32 entries read, summed and updated
-// in about 100 cycles beyond the four held ahead) against each feature by the whole block (about
-// 600 with its barrier and the two shuffle trees).
-bool beta_one_warp_level(long long N, long long nfeat, long long longest) {
-  if (N > kZsMax) return nfeat >= 8 || longest <= 1024;  // k_beta_one
-  const long long steps = (longest + 31) / 32;
-  const long long warp = (nfeat + kSmemWarps - 1) / kSmemWarps * (400 + 100 * std::max(0LL, steps - 4));
-  return warp <= 600 * nfeat;
+// Orders the features by level and splits each level into at most two: the long features, each taken by
+// the whole block in turn, and the others, a warp each.  The features of a level touch
+// disjoint rows, so any order and grouping of them gives the same sums.  With Z in shared memory
+// the split minimises the estimate: 700 cycles per feature of the block (two shuffle trees and a
+// barrier), 600 per 32 features of the warps plus 60 for every 32 entries of the longest one beyond
+// the first 128.  k_beta_one gives a level to the warps unless it has few features and a long one.
+void beta_one_levels(long long N, const std::vector<int>& level, const std::vector<long long>& ptr,
+                     std::vector<int>& lvl_ptr, std::vector<int>& order,
+                     std::vector<int>& lvl_warp) {
+  const int nfeat = (int)level.size();
+  auto len = [&](int f) { return ptr[f + 1] - ptr[f]; };
+  order.resize(nfeat);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return level[a] != level[b] ? level[a] < level[b] : len(a) > len(b);
+  });
+  lvl_ptr.assign(1, 0);
+  lvl_warp.clear();
+  for (int s = 0; s < nfeat;) {
+    int e = s;
+    while (e < nfeat && level[order[e]] == level[order[s]]) e++;
+    const long long n = e - s, longest = len(order[s]);
+    int cut = s;  // features s .. cut - 1 by the block
+    if (N > kZsMax) {
+      if (n < 8 && longest > 1024) cut = e;
+    } else {
+      long long best = -1;
+      for (int c = s; c <= e && c <= s + 64; c++) {
+        const long long rest = e - c, steps = rest ? (len(order[c]) + 31) / 32 : 0;
+        const long long cost = 700 * (c - s) + (rest + kSmemWarps - 1) / kSmemWarps * 600 +
+                               60 * std::max(0LL, steps - 4);
+        if (best < 0 || cost < best) {
+          best = cost;
+          cut = c;
+        }
+      }
+    }
+    if (cut > s) {
+      lvl_ptr.push_back(cut);
+      lvl_warp.push_back(0);
+    }
+    if (e > cut) {
+      lvl_ptr.push_back(e);
+      lvl_warp.push_back(1);
+    }
+    s = e;
+  }
 }
 
 void launch_lambda_beta_one(const double* beta, int bstride, long long nfeat, int K, double a0,
