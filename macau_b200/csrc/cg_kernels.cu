@@ -12,7 +12,6 @@
 // residual replacement R = B - (F^T F + reg I) X every kReplaceEvery iterations.
 #include <cmath>
 
-#include "cg_small.cuh"
 #include "common.cuh"
 #include "kernels.h"
 #include "rng.cuh"
@@ -76,111 +75,91 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------- SpMM over a work split (DevCsr::tasks) ----------------
-// One warp per task (a whole row, or one part of a long row).  LPE lanes share an entry, each with
-// two components (one 16-byte load in FP64), so 32 / LPE entries are read per load instruction and
-// eight such loads are in flight; the indices come 32 at a time by one coalesced load, the next 32
-// ahead.  A part stores its FP64 partial row in A.parts; the last part of a row to finish (arrival
-// counter) adds the parts in a fixed order and writes the row.
-//   What bounds it: for short tasks the latency of index and gather, for the others the gathers
-//   from L2 (256 bytes per entry at 32 components).  One 8-byte load per lane and entry, four in
-//   flight behind scalar index loads, took 52 us for the 4,099 columns (150,000 entries, parts
-//   of 256) of a 5,003-row feature matrix.
-template <typename V>
-struct Vec2;
-template <>
-struct Vec2<double> {
-  using T = double2;
-};
-template <>
-struct Vec2<float> {
-  using T = float2;
-};
-
-template <typename V, int LPE>
+// One warp per task (a whole row, or one part of a long row).  Entries are read four at a time
+// (independent gathers in flight) and added in CSR order.  A part stores its FP64 partial row in
+// A.parts; the last part of a row to finish (arrival counter) adds the parts in part order and
+// writes the row.  Whole rows give the same sums as k_spmm.
+template <typename V, int NRP>
 __global__ void __launch_bounds__(256)
     k_spmm_split(const DevCsr A, const V* __restrict__ src, int sstride, V* __restrict__ dst,
                  int dstride, int ncomp, const V* __restrict__ add, int astride, double reg,
                  const double* __restrict__ reg_dev, const uint32_t* __restrict__ done) {
   if (done && *done) return;
-  using T2 = typename Vec2<V>::T;
-  constexpr int EPS = 32 / LPE, U = 8;  // entries per load, loads in flight
-  static_assert(EPS * U <= 32, "a step stays inside its chunk of 32 entries");
-  const int lane = threadIdx.x & 31, grp = lane / LPE, k0 = 2 * (lane % LPE);
+  constexpr int C = NRP / 32;
+  const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (blockDim.x >> 5);
   const bool weighted = sizeof(V) == 8 ? A.val != nullptr : A.valf != nullptr;
-  const V* base = src + k0;
-  auto combine = [](T2& v) {  // the groups' sums, by a fixed tree
-#pragma unroll
-    for (int o = LPE; o < 32; o <<= 1) {
-      v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-      v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-    }
-  };
   for (int ti = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); ti < A.ntasks; ti += nw) {
     const RowTask tk = A.tasks[ti];
-    T2 acc{};
-    auto load_chunk = [&](int off, int& c, V& w) {
-      const bool in = off + lane < tk.len;
-      c = in ? A.idx[tk.begin + off + lane] : 0;
-      w = (V)1;
-      if (weighted && in) {
-        if constexpr (sizeof(V) == 8) w = (V)A.val[tk.begin + off + lane];
-        else w = (V)A.valf[tk.begin + off + lane];
+    V acc[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) acc[c] = (V)0;
+    const long long b = tk.begin, e = tk.begin + tk.len;
+    long long q = b;
+    for (; q + 4 <= e; q += 4) {
+      const V* s0 = src + (size_t)A.idx[q] * sstride;
+      const V* s1 = src + (size_t)A.idx[q + 1] * sstride;
+      const V* s2 = src + (size_t)A.idx[q + 2] * sstride;
+      const V* s3 = src + (size_t)A.idx[q + 3] * sstride;
+      V w0 = (V)1, w1 = (V)1, w2 = (V)1, w3 = (V)1;
+      if (weighted) {
+        if constexpr (sizeof(V) == 8) {
+          w0 = (V)A.val[q]; w1 = (V)A.val[q + 1]; w2 = (V)A.val[q + 2]; w3 = (V)A.val[q + 3];
+        } else {
+          w0 = (V)A.valf[q]; w1 = (V)A.valf[q + 1]; w2 = (V)A.valf[q + 2]; w3 = (V)A.valf[q + 3];
+        }
       }
-    };
-    int c_cur, c_nxt = 0;
-    V w_cur, w_nxt = (V)1;
-    load_chunk(0, c_cur, w_cur);
-    for (int off = 0; off < tk.len; off += 32) {
-      load_chunk(off + 32, c_nxt, w_nxt);
 #pragma unroll
-      for (int u = 0; u < 32; u += EPS * U) {
-        if (off + u < tk.len) {
-          T2 x[U];
-#pragma unroll
-          for (int i = 0; i < U; i++) {
-            const int en = u + i * EPS + grp;
-            const int col = __shfl_sync(0xffffffffu, c_cur, en);
-            x[i] = T2{};
-            if (off + en < tk.len)
-              x[i] = *reinterpret_cast<const T2*>(base + (size_t)col * sstride);
-          }
-#pragma unroll
-          for (int i = 0; i < U; i++) {
-            if (weighted) {
-              const V w = __shfl_sync(0xffffffffu, w_cur, u + i * EPS + grp);
-              acc.x += x[i].x * w;
-              acc.y += x[i].y * w;
-            } else {
-              acc.x += x[i].x;
-              acc.y += x[i].y;
-            }
+      for (int c = 0; c < C; c++) {
+        const int k = lane + 32 * c;
+        if (k < ncomp) {
+          const V x0 = s0[k], x1 = s1[k], x2 = s2[k], x3 = s3[k];
+          if (weighted) {
+            acc[c] += x0 * w0;
+            acc[c] += x1 * w1;
+            acc[c] += x2 * w2;
+            acc[c] += x3 * w3;
+          } else {
+            acc[c] += x0;
+            acc[c] += x1;
+            acc[c] += x2;
+            acc[c] += x3;
           }
         }
       }
-      c_cur = c_nxt;
-      w_cur = w_nxt;
     }
-    combine(acc);
-    const V r = (V)(reg_dev ? *reg_dev : reg);
-    auto write = [&](V x, V y) {
-      if (grp != 0) return;
-      const V o[2] = {x, y};
+    for (; q < e; q++) {
+      const V* s0 = src + (size_t)A.idx[q] * sstride;
+      V w0 = (V)1;
+      if (weighted) {
+        if constexpr (sizeof(V) == 8) w0 = (V)A.val[q];
+        else w0 = (V)A.valf[q];
+      }
 #pragma unroll
-      for (int c = 0; c < 2; c++)
-        if (k0 + c < ncomp) {
-          V v = o[c];
-          if (add) v += r * add[(size_t)tk.row * astride + k0 + c];
-          dst[(size_t)tk.row * dstride + k0 + c] = v;
-        }
-    };
+      for (int c = 0; c < C; c++) {
+        const int k = lane + 32 * c;
+        if (k < ncomp) acc[c] += weighted ? s0[k] * w0 : s0[k];
+      }
+    }
+    const V r = (V)(reg_dev ? *reg_dev : reg);
     if (tk.nparts == 1) {
-      write(acc.x, acc.y);
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        const int k = lane + 32 * c;
+        if (k < ncomp) {
+          V o = acc[c];
+          if (add) o += r * add[(size_t)tk.row * astride + k];
+          dst[(size_t)tk.row * dstride + k] = o;
+        }
+      }
       continue;
     }
-    if (grp == 0)
-      *reinterpret_cast<double2*>(A.parts + (size_t)(tk.slot + tk.part) * 64 + k0) =
-          make_double2((double)acc.x, (double)acc.y);
+    double* pp = A.parts + (size_t)(tk.slot + tk.part) * 64;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      const int k = lane + 32 * c;
+      if (k < ncomp) pp[k] = (double)acc[c];
+    }
     __threadfence();
     __syncwarp();
     unsigned last = 0;
@@ -188,20 +167,18 @@ __global__ void __launch_bounds__(256)
     last = __shfl_sync(0xffffffffu, last, 0);
     if (!last) continue;
     __threadfence();
-    const double* p0 = A.parts + (size_t)tk.slot * 64 + k0;
-    double2 t = make_double2(0.0, 0.0);
-#pragma unroll 8
-    for (int pt = grp; pt < tk.nparts; pt += EPS) {
-      const double2 v = __ldcg(reinterpret_cast<const double2*>(p0 + (size_t)pt * 64));
-      t.x += v.x;
-      t.y += v.y;
-    }
+    const double* p0 = A.parts + (size_t)tk.slot * 64;
 #pragma unroll
-    for (int o = LPE; o < 32; o <<= 1) {
-      t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
-      t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+    for (int c = 0; c < C; c++) {
+      const int k = lane + 32 * c;
+      if (k < ncomp) {
+        double t = 0.0;
+        for (int pt = 0; pt < tk.nparts; pt++) t += __ldcg(p0 + (size_t)pt * 64 + k);
+        V o = (V)t;
+        if (add) o += r * add[(size_t)tk.row * astride + k];
+        dst[(size_t)tk.row * dstride + k] = o;
+      }
     }
-    write((V)t.x, (V)t.y);
     if (lane == 0) A.split_cnt[tk.split] = 0u;
   }
 }
@@ -313,6 +290,42 @@ __device__ __forceinline__ double sum_part(const double* partials, int nparts, i
   return s;
 }
 
+// Left-looking lower Cholesky of the n x n matrix A (leading dimension ld) by one CTA, column by
+// column; thread i computes L(i, j).  On a non-positive pivot it stops and leaves column j and
+// the columns after it as they were, like the unchecked Eigen llt() the reference uses
+// (linop.h:287, 313): the caller's solves then read that partial factor.  Returns false then.
+__device__ bool cta_chol_n(double* A, int n, int ld) {
+  __syncthreads();
+  for (int j = 0; j < n; j++) {
+    double d = A[j + j * ld];
+    for (int p = 0; p < j; p++) d -= A[j + p * ld] * A[j + p * ld];
+    if (!(d > 0.0)) {
+      __syncthreads();
+      return false;
+    }
+    const double ljj = sqrt(d);
+    for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) {
+      double s = A[i + j * ld];
+      for (int p = 0; p < j; p++) s -= A[i + p * ld] * A[j + p * ld];
+      A[i + j * ld] = s / ljj;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) A[j + j * ld] = ljj;
+    __syncthreads();
+  }
+  return true;
+}
+
+// small layout (doubles): RtR[64*64] | RtR2[64*64] | M[64*64] | A[64*64] | Psi[64*64] | norms[64]
+//                         | inorms[64] | flags[4]
+constexpr int kSq = 64 * 64;
+struct SmallView {
+  double *RtR, *RtR2, *M, *A, *Psi, *norms, *inorms, *flags;
+  __host__ __device__ explicit SmallView(double* s)
+      : RtR(s), RtR2(s + kSq), M(s + 2 * kSq), A(s + 3 * kSq), Psi(s + 4 * kSq),
+        norms(s + 5 * kSq), inorms(s + 5 * kSq + 64), flags(s + 5 * kSq + 128) {}
+};
+
 // RtR = sum partials (full matrix from the lower triangle, A_mul_At_combo + makeSymmetric)
 __global__ void k_cg_rtr(const double* partials, int nparts, int NRP, int n, double* small) {
   SmallView v(small);
@@ -354,12 +367,94 @@ __global__ void k_cg_init(const double* __restrict__ B, int bstride, long long n
   }
 }
 
+// Out(c, i) = (M^{-T} M^{-1} Rhs)(i, c) for the n columns of Rhs, M the lower Cholesky factor
+// in v.M (leading dimension 64): thread c solves column c, forward then backward substitution in
+// the order of the reference's llt().solve.  The general path (n > 32, or a failed pivot).
+__device__ void cta_chol_solve_cols(const double* M, const double* Rhs, int n, double* Out) {
+  for (int c = threadIdx.x; c < n; c += blockDim.x) {
+    double y[64];
+    for (int i = 0; i < n; i++) y[i] = Rhs[i + c * 64];
+    for (int i = 0; i < n; i++) {
+      double s = y[i];
+      for (int p = 0; p < i; p++) s -= M[i + p * 64] * y[p];
+      y[i] = s / M[i + i * 64];
+    }
+    for (int i = n - 1; i >= 0; i--) {
+      double s = y[i];
+      for (int p = i + 1; p < n; p++) s -= M[p + i * 64] * y[p];
+      y[i] = s / M[i + i * 64];
+    }
+    for (int i = 0; i < n; i++) Out[c + i * 64] = y[i];
+  }
+}
+
 constexpr int kSolveThreads = 256;
+constexpr int kLcLd = 36;
+
+// The same solves for n <= 32 with the factor in registers: warp 0 factorises the SPD matrix Ms
+// (lower triangle, padded with the identity beyond n) by warp_factor, publishing L^T in Lc;
+// then warp w solves columns w, w + 8, ...: lane i holds L(i, j) for j <= i and L(j, i) for
+// j > i and runs each substitution as 32 shuffle steps.  Returns false, with Out untouched, when
+// a pivot is not positive (the caller then takes the general path).
+__device__ bool warp_chol_solve(const double (*Ms)[33], double* Lc, const double* Rhs, int n,
+                                double* Out, int* okf) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0) {
+    double a[32], rinv = 1.0, d0 = 1.0;
+#pragma unroll
+    for (int j = 0; j < 32; j++) {
+      double x;
+      if (lane < n && j < n) x = j <= lane ? Ms[lane][j] : Ms[j][lane];
+      else x = lane == j ? 1.0 : 0.0;
+      a[j] = x;
+      if (j == lane) d0 = x;
+    }
+    const bool ok = warp_factor<double, 32>(a, rinv, lane, 0.0, d0, Lc, kLcLd);
+    if (lane == 0) *okf = ok ? 1 : 0;
+  }
+  __syncthreads();
+  if (!*okf) return false;
+  double m[32], dinv = 1.0;
+#pragma unroll
+  for (int j = 0; j < 32; j++) {
+    m[j] = j <= lane ? Lc[j * kLcLd + lane] : Lc[lane * kLcLd + j];
+    if (j == lane) dinv = 1.0 / m[j];
+  }
+  for (int c = warp; c < n; c += kSolveThreads / 32) {
+    double y = lane < n ? Rhs[lane + c * 64] : 0.0;
+#pragma unroll
+    for (int j = 0; j < 32; j++) {
+      if (lane == j) y *= dinv;
+      const double yj = __shfl_sync(0xffffffffu, y, j);
+      if (lane > j) y = fma(-m[j], yj, y);
+    }
+#pragma unroll
+    for (int j = 31; j >= 0; j--) {
+      if (lane == j) y *= dinv;
+      const double xj = __shfl_sync(0xffffffffu, y, j);
+      if (lane < j) y = fma(-m[j], xj, y);
+    }
+    if (lane < n) Out[c + lane * 64] = y;
+  }
+  return true;
+}
+
 // A = (chol(PtKP) \ RtR)^T  (linop.h:286-289); PtKP from the lower triangle of sum P KP^T.
 __global__ void __launch_bounds__(kSolveThreads, 1)
     k_cg_solve_a(const double* partials, int nparts, int NRP, int n, double* small, Ctl* ctl) {
   if (ctl->cg_done) return;
+  __shared__ double Ms[32][33];
+  __shared__ __align__(16) double Lc[32 * kLcLd];
+  __shared__ int okf;
   SmallView v(small);
+  if (n <= 32) {
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+      const int i = e % n, j = e / n;
+      if (i >= j) Ms[i][j] = sum_part(partials, nparts, NRP, i, j);
+    }
+    __syncthreads();
+    if (warp_chol_solve(Ms, Lc, v.RtR, n, v.A, &okf)) return;
+  }
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
     const int i = e % n, j = e / n;
     if (i >= j) v.M[i + j * 64] = sum_part(partials, nparts, NRP, i, j);  // P(i) . KP(j)
@@ -375,6 +470,9 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
     k_cg_solve_psi(const double* partials, int nparts, int NRP, int n, double tolsq,
                    double* small, Ctl* ctl, int* flag_out, int iter) {
   if (ctl->cg_done) return;
+  __shared__ double Ms[32][33];
+  __shared__ __align__(16) double Lc[32 * kLcLd];
+  __shared__ int okf;
   SmallView v(small);
   __shared__ int conv;
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
@@ -410,13 +508,24 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
     }
   }
   if (conv) return;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int i = e % n, j = e / n;
-    v.M[i + j * 64] = v.RtR[i + j * 64];
+  bool fast = false;
+  if (n <= 32) {
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+      const int i = e % n, j = e / n;
+      if (i >= j) Ms[i][j] = v.RtR[i + j * 64];
+    }
+    __syncthreads();
+    fast = warp_chol_solve(Ms, Lc, v.RtR2, n, v.Psi, &okf);
   }
-  cta_chol_n(v.M, n, 64);
-  __syncthreads();
-  cta_chol_solve_cols(v.M, v.RtR2, n, v.Psi);
+  if (!fast) {
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+      const int i = e % n, j = e / n;
+      v.M[i + j * 64] = v.RtR[i + j * 64];
+    }
+    cta_chol_n(v.M, n, 64);
+    __syncthreads();
+    cta_chol_solve_cols(v.M, v.RtR2, n, v.Psi);
+  }
   __syncthreads();
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
     const int i = e % n, j = e / n;
@@ -633,13 +742,8 @@ void spmm_t(const DevCsr& A, const V* src, int sstride, V* dst, int dstride, int
             const V* add, int astride, double reg, const double* reg_dev, cudaStream_t s,
             const uint32_t* done = nullptr) {
   if (A.tasks) {
-    // lanes per entry: two components each, rounded up to a power of two (the rows are padded to
-    // 32 or 64 components, so the lanes past ncomp read padding and write nothing)
-    const auto kern = ncomp <= 16   ? k_spmm_split<V, 8>
-                      : ncomp <= 32 ? k_spmm_split<V, 16>
-                                    : k_spmm_split<V, 32>;
-    kern<<<grid_for(A.ntasks, 8), 256, 0, s>>>(A, src, sstride, dst, dstride, ncomp, add, astride,
-                                               reg, reg_dev, done);
+    k_spmm_split<V, NRP><<<grid_for(A.ntasks, 8), 256, 0, s>>>(
+        A, src, sstride, dst, dstride, ncomp, add, astride, reg, reg_dev, done);
     MG_CUDA(cudaGetLastError());
     return;
   }
@@ -665,24 +769,20 @@ int cg_core(const DevCsr& F, const DevCsr& Ft, double reg, const double* reg_dev
   if (n < NRP)
     MG_CUDA(cudaMemset2DAsync(Bn + n, NRP * sizeof(double), 0, (NRP - n) * sizeof(double),
                               nfeat, s));
-  if constexpr (NRP == 32) {
-    Cg32<V>::start(Bn, nfeat, n, R, P, Xd, sizeof(V) == 4 ? Bn : nullptr, small, partials, ctl, s);
-  } else {
-    outer<double, NRP>(Bn, Bn, nfeat, partials, nb, s);
-    sum_records(partials, nb, NRP * NRP, reduced, s);
-    k_cg_norms<<<1, 64, 0, s>>>(reduced, 1, NRP, n, small);
-    MG_CUDA(cudaGetLastError());
-    k_cg_init<V><<<eg, 256, 0, s>>>(Bn, NRP, nfeat, n, NRP, small, R, P, Xd,
-                                    sizeof(V) == 4 ? Bn : nullptr, ctl);
-    MG_CUDA(cudaGetLastError());
-    outer<V, NRP>(R, R, nfeat, partials, nb, s);
-    sum_records(partials, nb, NRP * NRP, reduced, s);
-    k_cg_rtr<<<1, 256, 0, s>>>(reduced, 1, NRP, n, small);
-    MG_CUDA(cudaGetLastError());
-  }
+  outer<double, NRP>(Bn, Bn, nfeat, partials, nb, s);
+  sum_records(partials, nb, NRP * NRP, reduced, s);
+  k_cg_norms<<<1, 64, 0, s>>>(reduced, 1, NRP, n, small);
+  MG_CUDA(cudaGetLastError());
+  k_cg_init<V><<<eg, 256, 0, s>>>(Bn, NRP, nfeat, n, NRP, small, R, P, Xd,
+                                  sizeof(V) == 4 ? Bn : nullptr, ctl);
+  MG_CUDA(cudaGetLastError());
+  outer<V, NRP>(R, R, nfeat, partials, nb, s);
+  sum_records(partials, nb, NRP * NRP, reduced, s);
+  k_cg_rtr<<<1, 256, 0, s>>>(reduced, 1, NRP, n, small);
+  MG_CUDA(cudaGetLastError());
   const double tolsq = tol * tol;
   const int rg = (int)((nfeat + kRowTile - 1) / kRowTile);
-  if constexpr (NRP != 32) {
+  {
     static bool configured[64] = {false};
     int dev = 0;
     MG_CUDA(cudaGetDevice(&dev));
@@ -706,37 +806,27 @@ int cg_core(const DevCsr& F, const DevCsr& Ft, double reg, const double* reg_dev
     for (int b = 0; b < kCgBatch && iter < max_iter; b++, iter++) {
       spmm_t<V, NRP>(F, P, NRP, inner, NRP, n, nullptr, 0, 0.0, nullptr, s, done);
       spmm_t<V, NRP>(Ft, inner, NRP, KPm, NRP, n, P, NRP, reg, reg_dev, s, done);
-      const bool replace = sizeof(V) == 4 && (iter + 1) % kReplaceEvery == 0;
-      if constexpr (NRP == 32) {
-        Cg32<V>::step_a(nfeat, n, P, KPm, R, Xd, small, partials, !replace, ctl, s);
-      } else {
-        outer<V, NRP>(P, KPm, nfeat, partials, nb, s, done);
-        sum_records(partials, nb, NRP * NRP, reduced, s, done);
-        k_cg_solve_a<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, small, ctl);
-        MG_CUDA(cudaGetLastError());
-        k_cg_rows<V, NRP, true><<<rg, 256, rows_smem(NRP, true), s>>>(nfeat, n, small, P, KPm, R,
-                                                                      Xd, nullptr, done);
-        MG_CUDA(cudaGetLastError());
-      }
-      if (replace) {
+      outer<V, NRP>(P, KPm, nfeat, partials, nb, s, done);
+      sum_records(partials, nb, NRP * NRP, reduced, s, done);
+      k_cg_solve_a<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, small, ctl);
+      MG_CUDA(cudaGetLastError());
+      k_cg_rows<V, NRP, true><<<rg, 256, rows_smem(NRP, true), s>>>(nfeat, n, small, P, KPm, R,
+                                                                    Xd, nullptr, done);
+      MG_CUDA(cudaGetLastError());
+      if (sizeof(V) == 4 && (iter + 1) % kReplaceEvery == 0) {
         spmm_t<double, NRP>(F, Xd, NRP, innerd, NRP, n, nullptr, 0, 0.0, nullptr, s, done);
         spmm_t<double, NRP>(Ft, innerd, NRP, KX, NRP, n, Xd, NRP, reg, reg_dev, s, done);
         k_cg_resid<V><<<eg, 256, 0, s>>>(nfeat * NRP, NRP, n, Bn, KX, R, done);
         MG_CUDA(cudaGetLastError());
-        if constexpr (NRP == 32) Cg32<V>::rr(nfeat, R, partials, ctl, s);
       }
-      if constexpr (NRP == 32) {
-        Cg32<V>::step_psi(nfeat, n, R, P, small, partials, tolsq, ctl, flag_dev, iter, s);
-      } else {
-        outer<V, NRP>(R, R, nfeat, partials, nb, s, done);
-        sum_records(partials, nb, NRP * NRP, reduced, s, done);
-        k_cg_solve_psi<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, tolsq, small, ctl, flag_dev,
-                                                   iter);
-        MG_CUDA(cudaGetLastError());
-        k_cg_rows<V, NRP, false><<<rg, 256, rows_smem(NRP, false), s>>>(nfeat, n, small, P, nullptr,
-                                                                         R, nullptr, P, done);
-        MG_CUDA(cudaGetLastError());
-      }
+      outer<V, NRP>(R, R, nfeat, partials, nb, s, done);
+      sum_records(partials, nb, NRP * NRP, reduced, s, done);
+      k_cg_solve_psi<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, tolsq, small, ctl, flag_dev,
+                                                 iter);
+      MG_CUDA(cudaGetLastError());
+      k_cg_rows<V, NRP, false><<<rg, 256, rows_smem(NRP, false), s>>>(nfeat, n, small, P, nullptr,
+                                                                       R, nullptr, P, done);
+      MG_CUDA(cudaGetLastError());
     }
     MG_CUDA(cudaStreamSynchronize(s));
     if (flag_host[0]) {

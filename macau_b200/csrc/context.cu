@@ -132,16 +132,15 @@ struct ModeData {
 };
 
 // Work split of a CSR for the side-information SpMMs (k_spmm_split): rows longer than
-// max(128, nnz / (64 warps per SM)) entries are cut into parts, so the long feature columns of a
-// Zipf-distributed F do not serialise on one warp (16 or 32 entries are in flight per warp, so
-// a part of 128 is 4 to 8 gather latencies).
+// max(256, nnz / (64 warps per SM)) entries are cut into parts, so the long feature columns of a
+// Zipf-distributed F do not serialise on one warp.
 struct SpmmSplit {
   DBuf<RowTask> tasks;
   DBuf<unsigned> cnt;
   DBuf<double> parts;
   void build(const std::vector<long long>& ptr, int num_sms, cudaStream_t s, DevCsr& A) {
     const long long nnz = ptr.empty() ? 0 : ptr.back();
-    const long long thr = std::max(128LL, nnz / ((long long)num_sms * 64));
+    const long long thr = std::max(256LL, nnz / ((long long)num_sms * 64));
     int nsplit = 0, nslots = 0;
     std::vector<RowTask> t = make_tasks(ptr, thr, 1, nsplit, nslots);
     tasks.upload(t.data(), t.size(), s);
@@ -511,6 +510,7 @@ class Context {
     sp.Lambda = p.Lambda.p;
     sp.mu = p.mu.p;
     sp.uhat = p.side() ? p.uhat.p : nullptr;
+    sp.ordered = link_chain();
     sp.one = p.one ? 1 : 0;
     sp.out_f64 = lat64_[mode].p;
     sp.out_f32 = lat32_[mode].p;
@@ -698,24 +698,38 @@ class Context {
     launches_ += launch_prior_pair(pp, mixed_, K_, KP_, ctl_.p, cfg_.seed, s_);
   }
 
+  // A chain with a block-CG link at K <= 32: statistics, draws and FP64 rows of both modes in a fixed
+  // order of summation (link_hyper.cu says why).
+  bool link_chain() const { return K_ <= 32 && (prior_[0].macau || prior_[1].macau); }
+
   void update_prior(int mode) {
     Prior& p = prior_[mode];
     const long long N = dims_[mode];
     const int nb = stats_blocks(N);
-    const bool few = few_parts(nb, K_);
+    const bool link = link_chain();
+    const auto stats_of = link ? launch_link_stats : launch_stats;
+    const bool few = !link && few_parts(nb, K_);
     launches_ += p.macau ? 0 : few ? 2 : 3;  // Macau launches are counted by kernels_in_cg below
     const int rec = K_ + K_ * K_;
-    launch_stats(latents(mode), mixed_, p.side() ? p.uhat.p : nullptr, N, K_, KP_, KP_,
-                 stat_partials_.p, nb, s_);
+    stats_of(latents(mode), mixed_, p.side() ? p.uhat.p : nullptr, N, K_, KP_, KP_,
+             stat_partials_.p, nb, s_);
     if (!few) launch_reduce_parts(stat_partials_.p, nb, rec, stat_final_.p, s_);
     const double* stats = few ? stat_partials_.p : stat_final_.p;
     const int nstats = few ? nb : 1;
+    auto draw = [&](int nu, const double* bb) {
+      const double* lb = bb ? p.lambda_beta.p : nullptr;
+      if (link)
+        launch_link_wishart(stats, N, K_, p.mu0.p, p.b0, p.WI.p, nu, bb, lb, ctl_.p, cfg_.seed, mode,
+                            p.mu.p, p.Lambda.p, s_);
+      else
+        launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, nu, bb, lb, ctl_.p,
+                              cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
+    };
     if (p.one) {
       // MacauOnePrior::update_prior (macauoneprior.cpp:189-194): sample_mu_lambda (Normal-Wishart
       // of U - Uhat with mu0 = 0, kappa = 2, W0 = I, nu = K, the BPMF defaults), sample_beta,
       // compute_uhat, sample_lambda_beta
-      launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr,
-                            nullptr, ctl_.p, cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
+      draw(p.df, nullptr);
       launch_beta_one(p.Ft, p.colsq.p, p.lvl_ptr.p, p.lvl_feat.p, p.lvl_range.p, p.lvl_warp.p,
                       p.nlevels,
                       latents(mode),
@@ -728,17 +742,14 @@ class Context {
       return;
     }
     if (!p.macau) {  // BPMFPrior::update_prior (latentprior.cpp:79-81)
-      launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df, nullptr,
-                            nullptr, ctl_.p, cfg_.seed, mode, p.mu.p, p.Lambda.p, s_);
+      draw(p.df, nullptr);
       return;
     }
     // MacauPrior::update_prior (latentprior.cpp:255-264)
     const int nbb = stats_blocks(p.nfeat);
-    launch_stats(p.beta.p, false, nullptr, p.nfeat, K_, CP_, 0, p.bb_partials.p, nbb, s_);
+    stats_of(p.beta.p, false, nullptr, p.nfeat, K_, CP_, 0, p.bb_partials.p, nbb, s_);
     launch_reduce_parts(p.bb_partials.p, nbb, rec, p.bb_final.p, s_);
-    launch_normal_wishart(stats, nstats, N, K_, p.mu0.p, p.b0, p.WI.p, p.df + (int)p.nfeat,
-                          p.bb_final.p, p.lambda_beta.p, ctl_.p, cfg_.seed, mode, p.mu.p,
-                          p.Lambda.p, s_);
+    draw(p.df + (int)p.nfeat, p.bb_final.p);
     // sample_beta (latentprior.cpp:273-293)
     launch_small_chol(p.Lambda.p, K_, p.Lchol.p, ctl_.p, s_);
     launch_beta_rhs_tmp(latents(mode), mixed_, KP_, N, K_, p.Lchol.p, p.mu.p, ctl_.p, cfg_.seed,
@@ -757,7 +768,7 @@ class Context {
     // compute_uhat (linop.h:196-198): Uhat = beta F^T, one K-vector per row of F
     launch_spmm(p.F, p.beta.p, CP_, p.uhat.p, KP_, K_, false, s_);
     // sample_lambda_beta with the new beta and Lambda (latentprior.cpp:263)
-    launch_stats(p.beta.p, false, nullptr, p.nfeat, K_, CP_, 0, p.bb_partials.p, nbb, s_);
+    stats_of(p.beta.p, false, nullptr, p.nfeat, K_, CP_, 0, p.bb_partials.p, nbb, s_);
     launch_reduce_parts(p.bb_partials.p, nbb, rec, p.bb_final.p, s_);
     launch_lambda_beta(p.bb_final.p, 1, K_, p.nfeat, p.Lambda.p, p.lb_nu0, p.lb_mu0, ctl_.p,
                        cfg_.seed, mode, p.lambda_beta.p, s_);

@@ -92,6 +92,14 @@ void launch_normal_wishart(const double* partials, int nparts, long long N, int 
                            const double* bb, const double* lambda_beta, Ctl* ctl,
                            unsigned long long seed, int mode, double* mu_out, double* Lambda_out,
                            cudaStream_t s);
+// The same two for a chain with a block-CG link at K <= 32 (link_hyper.cu), in a fixed order of summation;
+// `stats` is one record, `bb` one or null.
+void launch_link_stats(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
+                       int uhat_stride, double* partials, int nblocks, cudaStream_t s);
+void launch_link_wishart(const double* stats, long long N, int K, const double* mu0, double kappa,
+                         const double* T0, int nu, const double* bb, const double* lambda_beta,
+                         Ctl* ctl, unsigned long long seed, int mode, double* mu_out,
+                         double* Lambda_out, cudaStream_t s);
 // Both modes' BPMF prior updates (BPMFPrior::update_prior, latentprior.cpp:79-81) at once:
 // statistics, reduction and Normal-Wishart draw of mode m from the latents U[m]
 // (N[m] rows, stride `stride`), partials[m] (nblocks[m] records, rows_per_block[m] rows each)
@@ -208,24 +216,6 @@ void launch_beta_rhs_b(const DevCsr& Ft, const double* tmp, int tstride, int K,
                        cudaStream_t s);
 // one-CTA Cholesky of a K x K matrix into L (lower, zero upper); status on failure
 void launch_small_chol(const double* A, int K, double* L, Ctl* ctl, cudaStream_t s);
-
-// Pieces of a block-CG solve of up to 32 right-hand sides (cg_tiles.cu): R, P, KP, X and Bn are nfeat
-// x 32, `small` the K x K workspace (SmallView), `recs` the partial sums' records.
-template <typename V>
-struct Cg32 {
-  // norms of the right-hand sides Bn, R = P = Bn / norms (kept in Bsave too unless null), X = 0,
-  // R^T R, ctl->cg_done = 0
-  static void start(const double* Bn, long long nfeat, int n, V* R, V* P, double* X, double* Bsave,
-                    double* small, double* recs, Ctl* ctl, cudaStream_t s);
-  // A from P^T KP, then X += A P and R -= A KP; with_rr: also the records of the new R^T R
-  static void step_a(long long nfeat, int n, const V* P, const V* KP, V* R, double* X,
-                     double* small, double* recs, bool with_rr, Ctl* ctl, cudaStream_t s);
-  // the records of R^T R alone (after a residual replacement)
-  static void rr(long long nfeat, const V* R, double* recs, Ctl* ctl, cudaStream_t s);
-  // convergence test and Psi from the records, then P = R + Psi P
-  static void step_psi(long long nfeat, int n, const V* R, V* P, double* small, double* recs,
-                       double tolsq, Ctl* ctl, int* flag, int iter, cudaStream_t s);
-};
 
 class BlockCg {
  public:

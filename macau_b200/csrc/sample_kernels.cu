@@ -586,10 +586,19 @@ void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStre
     if (gram == kGeTf32) return launch_mixed<kGeTf32>(p, KP, groups, s, num_sms);
     return launch_mixed<kGeBf16>(p, KP, groups, s, num_sms);
   } else {
+    // K <= 32: Grams on the FP64 matrix instruction, except in a chain with a block-CG link, whose rows
+    // keep the order of summation of k_sample (link_hyper.cu says why)
+    if (KP <= 32 && (p.one || !p.ordered)) return launch_sample_f64(p, KP, s, num_sms, groups);
     switch (KP) {
       case 8:
+        if (groups == 2) return launch_t<8, 1, 2, false>(p, s, num_sms);
+        return launch_t<8, 1, 4, false>(p, s, num_sms);
       case 16:
-      case 32: return launch_sample_f64(p, KP, s, num_sms, groups);
+        if (groups == 2) return launch_t<16, 1, 2, false>(p, s, num_sms);
+        return launch_t<16, 1, 4, false>(p, s, num_sms);
+      case 32:
+        if (groups == 2) return launch_t<32, 1, 2, false>(p, s, num_sms);
+        return launch_t<32, 1, 4, false>(p, s, num_sms);
       case 64:
         if (groups == 1) return launch_t<64, 4, 1, false>(p, s, num_sms);
         return launch_t<64, 4, 2, false>(p, s, num_sms);
