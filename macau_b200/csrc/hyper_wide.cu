@@ -289,7 +289,7 @@ __device__ __forceinline__ void nw_tiles(const NwArgs& p, int K, Ctl* ctl, unsig
   }
   __syncthreads();
   if (warp < 8) {
-    wide_factor<double, KP, kNwHalf>(M, y, Di, zero, nb, 0.0, tid, 0, bad);
+    wide_factor<KP, kNwHalf>(M, y, Di, nb, tid, 0, bad);
   } else {
     bartlett(Ct, z, K, n, nu_c, seed, sweep, (uint32_t)p.mode, tid - kNwHalf, kNwHalf);
   }
@@ -342,7 +342,7 @@ __device__ __forceinline__ void nw_tiles(const NwArgs& p, int K, Ctl* ctl, unsig
       y[tid] = z[tid] / sqrt(kappa_c);
     }
     group_sync<kNwHalf>(0);
-    wide_back<double, KP, kNwHalf>(M, y, Di, x, nb, tid, 0);
+    wide_back<KP, kNwHalf>(M, y, Di, x, nb, tid, 0);
     if (tid < K) p.mu[tid] = x[tid] + muc[tid];
   } else {
     // Lambda = B B^T

@@ -38,11 +38,12 @@ void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStre
 // Its FP64 form for KP <= 32, a warp per row with the Grams on the FP64 matrix instruction
 // (sample_mma.cu); groups = 2 or 4 (default) warps per CTA.
 void launch_sample_f64(const SampleParams& p, int KP, cudaStream_t s, int num_sms, int groups);
-// Its form for KP = 64 and 128 without the univariate prior, FP64 or mixed with BF16 gathers
-// (sample_wide.cu): a group of warps per row, matrix-instruction Grams, panel factor; groups = 1
-// or 2 (default) rows per CTA at KP = 64.
-void launch_sample_wide(const SampleParams& p, int KP, bool mixed, cudaStream_t s, int num_sms,
-                        int groups);
+// Its forms for KP = 64 and 128 without the univariate prior, a group of warps per row and a panel
+// factor: FP64 with matrix-instruction Grams (sample_wide.cu), mixed with BF16 gathers
+// (sample_wide_mixed.cu); groups = 1 or 2 (default) rows per CTA at KP = 64.
+void launch_sample_wide(const SampleParams& p, int KP, cudaStream_t s, int num_sms, int groups);
+void launch_sample_wide_mixed(const SampleParams& p, int KP, cudaStream_t s, int num_sms,
+                              int groups);
 // The default CTA shape of the CUDA-core sampler at KP, and the shapes the autotuner may pick
 // from (the default first).
 int sample_default_groups(int KP);

@@ -580,7 +580,8 @@ void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStre
   // K > 32: the group sampler with matrix-instruction Grams; the univariate prior and the FP16
   // and TF32 Grams, which need other operands or the whole Gram, keep k_sample
   if (KP > 32 && !p.one && (!mixed || gram == kGeBf16))
-    return launch_sample_wide(p, KP, mixed, s, num_sms, groups);
+    return mixed ? launch_sample_wide_mixed(p, KP, s, num_sms, groups)
+                 : launch_sample_wide(p, KP, s, num_sms, groups);
   if (mixed) {
     if (gram == kGeFp16) return launch_mixed<kGeFp16>(p, KP, groups, s, num_sms);
     if (gram == kGeTf32) return launch_mixed<kGeTf32>(p, KP, groups, s, num_sms);

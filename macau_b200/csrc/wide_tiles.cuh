@@ -1,4 +1,4 @@
-// FP64 and FP32 triangular matrices of 33 to 128 rows in shared memory as 8 x 8 tiles, for a group of
+// Triangular matrices of 33 to 128 rows in shared memory as 8 x 8 tiles, for a group of
 // warps: the panel Cholesky factor with a right-hand side, the backward substitution, and the split
 // of a Gram's lower-triangle tiles over the warps (sample_wide.cu, hyper_wide.cu).
 #pragma once
@@ -110,6 +110,7 @@ __device__ __forceinline__ void update_tile(double* M, int bi, int bj, int k0, i
   }
   *c = make_double2(v.x + w.x, v.y + w.y);
 }
+// FP32: one fused multiply-add per column, in column order.
 __device__ __forceinline__ void update_tile(float* M, int bi, int bj, int k0, int k1, int lane) {
   const int g = lane >> 2, t = lane & 3;
   const float* A = M + tile_at(bi, 0);
@@ -134,38 +135,28 @@ __device__ __forceinline__ void update_tile(float* M, int bi, int bj, int k0, in
 // Factor of a diagonal tile by one warp: lanes 0-7 hold its rows (x[j], j <= lane, in; the factor's
 // rows out), any other lane a row v that becomes v L^{-T}.  What a column needs of the other rows
 // is shuffled before its pivot is known (unscaled), so the chain from pivot to pivot is one
-// reciprocal square root, one product and one fma.  False when a pivot is not positive, or
-// not above rel_floor times its original diagonal.
-template <typename F>
-__device__ __forceinline__ bool diag_factor(F (&x)[8], const F* diag0, F rel_floor) {
+// reciprocal square root, one product and one fma.  False when a pivot is not positive.
+__device__ __forceinline__ bool diag_factor(double (&x)[8]) {
   bool ok = true;
-  F low[8];
-#pragma unroll
-  for (int c = 0; c < 8; c++) low[c] = rel_floor * diag0[c];
-  F d = wshfl(x[0], 0);
+  double d = wshfl(x[0], 0);
 #pragma unroll
   for (int c = 0; c < 8; c++) {
-    F w[8], v = (F)0;
+    double w[8], v = 0.0;
 #pragma unroll
     for (int j = c + 1; j < 8; j++) w[j] = wshfl(x[c], j);
     if (c < 7) v = wshfl(x[c + 1], c + 1);
-    ok = ok & (d > (F)0) & (d > low[c]);
-    const F r = mrsqrt(d);
+    ok = ok & (d > 0.0);
+    const double r = mrsqrt(d);
     if (c < 7) {
-      const F l = w[c + 1] * r;
-      d = mfma(-l, l, v);
+      const double l = w[c + 1] * r;
+      d = fma(-l, l, v);
     }
-    const F s = x[c] * (r * r);
+    const double s = x[c] * (r * r);
     x[c] *= r;
 #pragma unroll
-    for (int j = c + 1; j < 8; j++) x[j] = mfma(-s, w[j], x[j]);
+    for (int j = c + 1; j < 8; j++) x[j] = fma(-s, w[j], x[j]);
   }
   return ok;
-}
-
-__device__ __forceinline__ bool diag_factor(double (&x)[8]) {
-  const double zero[8] = {};
-  return diag_factor(x, zero, 0.0);
 }
 
 // Tile T <- T L^{-T}, Di the transposed inverse of L, by one warp.
@@ -178,49 +169,34 @@ __device__ __forceinline__ void solve_tile(double* T, const double* Di, int lane
   mma_f64(v.x, v.y, a1, Di[tile_pos(t + 4, g)]);
   *reinterpret_cast<double2*>(T + tile_pos(g, 2 * t)) = v;
 }
-__device__ __forceinline__ void solve_tile(float* T, const float* Di, int lane) {
-  const int g = lane >> 2, t = lane & 3;
-  float a[8];
-  load_row8(T, g, a);
-  float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const float2 b = *reinterpret_cast<const float2*>(Di + tile_pos(k, 2 * t));
-    v.x = fmaf(a[k], b.x, v.x);
-    v.y = fmaf(a[k], b.y, v.y);
-  }
-  __syncwarp();
-  *reinterpret_cast<float2*>(T + tile_pos(g, 2 * t)) = v;
-}
 
 // Factorises MM (nb blocks) in place by panels of 8 columns, left-looking, y (the right-hand side)
 // along with it, and leaves the transposed inverse of each diagonal tile in Di (a tile per panel).
-// A pivot that is not positive, or not above rel_floor times its original diagonal, fails the
-// group (all threads return false).
+// A pivot that is not positive fails the group (all threads return false).
 //   Per panel: warp 0 subtracts the last panel's product from the diagonal tile and factors it, with
 //   the identity's rows and y's among its lanes, while the other warps subtract all earlier
 //   panels' from the tiles below and from the next diagonal tile; barrier; the tiles below times the
 //   transposed inverse; barrier.  (Every row's owner factoring the diagonal tile for itself,
 //   without the second step, took 2,800 cycles a panel at K = 64 in FP64: 244 FP64 instructions
 //   a thread, in every warp.)
-template <typename F, int KP, int T>
-__device__ __forceinline__ bool wide_factor(F* M, F* y, F* Di, const F* diag0, int nb,
-                                            F rel_floor, int tid, int grp, volatile int* bad) {
+template <int KP, int T>
+__device__ __forceinline__ bool wide_factor(double* M, double* y, double* Di, int nb, int tid,
+                                            int grp, volatile int* bad) {
   constexpr int W = T / 32;
   const int warp = tid >> 5, lane = tid & 31;
   for (int pn = 0; pn < nb; pn++) {
     // y's components by the panel before: the panel's own by warp 0, the others by warps 1 ..
     const int j = warp == 0 ? 8 * pn + (lane & 7) : 8 * pn + 8 + tid - 32;
-    F s = (F)0;
+    double s = 0.0;
     if (pn > 0 && j < 8 * nb) {
-      F v[8];
+      double v[8];
       load_row8(M + tile_at(j >> 3, pn - 1), j & 7, v);
       s = y[j];
-      F s1 = (F)0;
+      double s1 = 0.0;
 #pragma unroll
       for (int c = 0; c < 8; c += 2) {
-        s = mfma(-v[c], y[8 * pn - 8 + c], s);
-        s1 = mfma(-v[c + 1], y[8 * pn - 7 + c], s1);
+        s = fma(-v[c], y[8 * pn - 8 + c], s);
+        s1 = fma(-v[c + 1], y[8 * pn - 7 + c], s1);
       }
       s += s1;
     }
@@ -231,17 +207,17 @@ __device__ __forceinline__ bool wide_factor(F* M, F* y, F* Di, const F* diag0, i
       }
       __syncwarp();
       // lanes 0-7: the tile's rows, 8-15: the identity's, 16: y
-      F* row = lane < 8 ? M + tile_at(pn, pn) : (lane < 16 ? Di + 64 * pn : y + 8 * pn);
+      double* row = lane < 8 ? M + tile_at(pn, pn) : (lane < 16 ? Di + 64 * pn : y + 8 * pn);
       const int r = lane < 16 ? lane & 7 : 0;
-      F x[8];
+      double x[8];
       if (lane < 8 || lane == 16) {
         load_row8(row, r, x);
       } else {
 #pragma unroll
-        for (int c = 0; c < 8; c++) x[c] = lane - 8 == c ? (F)1 : (F)0;
+        for (int c = 0; c < 8; c++) x[c] = lane - 8 == c ? 1.0 : 0.0;
       }
       __syncwarp();
-      const bool ok = diag_factor(x, diag0 + 8 * pn, rel_floor);
+      const bool ok = diag_factor(x);
       if (lane <= 16) store_row8(row, r, x);
       if (!ok && lane == 0) *bad = 1;
     } else {
@@ -264,35 +240,35 @@ __device__ __forceinline__ bool wide_factor(F* M, F* y, F* Di, const F* diag0, i
 
 // x = L^{-T} b over the panels from the last, b in y (overwritten), Di the diagonal tiles'
 // transposed inverses; one barrier a panel.  Each warp forms the panel's eight x for itself.
-template <typename F, int KP, int T>
-__device__ __forceinline__ void wide_back(const F* M, F* y, const F* Di, F* x, int nb, int tid,
-                                          int grp) {
+template <int KP, int T>
+__device__ __forceinline__ void wide_back(const double* M, double* y, const double* Di, double* x,
+                                          int nb, int tid, int grp) {
   const int warp = tid >> 5, r = tid & 7;
   for (int pn = nb - 1; pn >= 0; pn--) {
     if (warp == 0 || 32 * warp < 8 * pn) {
-      F d[8], b[8], p[8];
+      double d[8], b[8], p[8];
       load_row8(Di + 64 * pn, r, d);
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const Vec4<F> q = lds4(y + 8 * pn + 4 * h);
+        const Vec4<double> q = lds4(y + 8 * pn + 4 * h);
 #pragma unroll
         for (int u = 0; u < 4; u++) b[4 * h + u] = q.v[u];
       }
       const bool on = tid < 8 * pn;
-      const F* P = M + tile_at(pn, on ? tid >> 3 : 0);
+      const double* P = M + tile_at(pn, on ? tid >> 3 : 0);
 #pragma unroll
       for (int c = 0; c < 8; c++) p[c] = P[tile_pos(c, r)];
-      F s = on ? y[tid] : (F)0, u0 = (F)0, u1 = (F)0, s1 = (F)0;
+      double s = on ? y[tid] : 0.0, u0 = 0.0, u1 = 0.0, s1 = 0.0;
 #pragma unroll
       for (int c = 0; c < 8; c += 2) {
-        u0 = mfma(d[c], b[c], u0);
-        u1 = mfma(d[c + 1], b[c + 1], u1);
+        u0 = fma(d[c], b[c], u0);
+        u1 = fma(d[c + 1], b[c + 1], u1);
       }
-      const F xr = u0 + u1;
+      const double xr = u0 + u1;
 #pragma unroll
       for (int c = 0; c < 8; c += 2) {
-        s = mfma(-p[c], wshfl(xr, c), s);
-        s1 = mfma(-p[c + 1], wshfl(xr, c + 1), s1);
+        s = fma(-p[c], wshfl(xr, c), s);
+        s1 = fma(-p[c + 1], wshfl(xr, c + 1), s1);
       }
       if (on) y[tid] = s + s1;
       if (tid < 8) x[8 * pn + tid] = xr;
