@@ -32,6 +32,11 @@
 namespace mg {
 namespace {
 
+// FP32 tiles 72 floats apart: threads that hold the same element of neighbouring tiles then touch
+// different banks.
+constexpr int kTile = 72;
+__device__ __forceinline__ int ftile(int bi, int bj) { return (bi * (bi + 1) / 2 + bj) * kTile; }
+
 template <int KP>
 struct Mixed {
   static constexpr int W = KP == 64 ? 4 : 8;  // warps of a row group
@@ -44,13 +49,13 @@ struct Mixed {
   static constexpr int kChunk = 32;        // entries per stage
   static constexpr int VPR = KP / 8;       // 16-byte vectors per gathered row
   static constexpr int NV = kChunk * VPR / T;
-  static constexpr bool kLamShared = KP == 64;  // at 128 it would halve the rows in flight
   // group's shared memory in doubles: tiles (FP64 for the redo; the stages before the finish) |
   // inverses of the redo's diagonal tiles | rhs, y | draws | x | diagonal | flags
   static constexpr size_t kGroupDoubles = (size_t)(TRI + NB) * 64 + 4 * KP + 2;
-  static constexpr size_t kCtaDoubles = KP + (kLamShared ? TRI * 32 : 0);  // Lambda mu | Lambda
+  static constexpr size_t kCtaDoubles = KP + TRI * kTile / 2;  // Lambda mu | Lambda
   static_assert(2 * kChunk * KP * sizeof(float) <= TRI * 64 * sizeof(double), "stages");
   static_assert(NTILE <= T - 32 && KP * KP >= 8 * TC * T, "tiles, scratch slot");
+  static_assert(TRI * kTile * sizeof(float) <= TRI * 64 * sizeof(double), "tiles");
 };
 
 // Accumulates the thread's tile (and the last warp's right-hand side) over a task's entries.
@@ -148,7 +153,25 @@ __device__ __forceinline__ void gram_mixed(const SampleParams& p, const RowTask&
   }
 }
 
-// Row r (8 values) of tile (bi, pn) -> x L^{-T}, L the factored diagonal tile: one thread.
+// x[c] -= sum_{k < 8 pn} L(i, k) L(8 pn + c, k) of one row per thread: row = row i of its block's first
+// tile; one fused multiply-add per column, in column order.
+__device__ __forceinline__ void update_row(float (&x)[8], const float* row_tile, const float* diag_row,
+                                           int r, int pn) {
+  for (int k = 0; k < pn; k++) {
+    float a[8];
+    load_row8(row_tile + k * kTile, r, a);
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        const Vec4<float> b = lds4(diag_row + k * kTile + c * 8 + 4 * (h ^ ((c >> 1) & 1)));
+#pragma unroll
+        for (int q = 0; q < 4; q++) x[c] = fmaf(-a[4 * h + q], b.v[q], x[c]);
+      }
+  }
+}
+
+// x -> x L^{-T}, L the factored diagonal tile.
 __device__ __forceinline__ void solve_row(float (&x)[8], const float* L) {
 #pragma unroll
   for (int c = 0; c < 8; c++) {
@@ -162,31 +185,38 @@ __device__ __forceinline__ void solve_row(float (&x)[8], const float* L) {
 
 // Factorises MM (nb blocks) in place, y along with it; df: MM's diagonal.  A pivot that is not
 // positive, or not above 2^-20 of its original diagonal, fails the group.
+//   Per panel: warp 0 subtracts the last panel's product from the diagonal tile and factors it; a
+// thread per row below subtracts all earlier panels' products, and the last warp those of the next
+// diagonal tile; barrier; the rows below are solved in their threads' registers; barrier.
 template <int T>
 __device__ __forceinline__ bool factor_mixed(float* M, float* y, const float* df, int nb, int tid,
                                              int grp, volatile int* bad) {
   constexpr int W = T / 32;
-  const int warp = tid >> 5, lane = tid & 31;
+  const int warp = tid >> 5, lane = tid & 31, r = tid & 7;
   for (int pn = 0; pn < nb; pn++) {
-    // y's components by the panel before: the panel's own by warp 0, the others by warps 1 ..
-    const int j = warp == 0 ? 8 * pn + (lane & 7) : 8 * pn + 8 + tid - 32;
-    float s = 0.f;
-    if (pn > 0 && j < 8 * nb) {
+    float* D = M + ftile(pn, pn);
+    // row of the panel: warp 0 the panel's own, the others those below
+    const int j = warp == 0 ? 8 * pn + r : 8 * pn + 8 + tid - 32;
+    const bool below = warp > 0 && j < 8 * nb;
+    float* tile = M + ftile(below ? j >> 3 : pn, 0);  // the row's block
+    float s = 0.f, x[8];
+    if (pn > 0 && (warp == 0 || below)) {  // y by the panel before
       float v[8];
-      load_row8(M + tile_at(j >> 3, pn - 1), j & 7, v);
+      load_row8(tile + (pn - 1) * kTile, r, v);
       s = y[j];
 #pragma unroll
       for (int c = 0; c < 8; c++) s = fmaf(-v[c], y[8 * pn - 8 + c], s);
     }
     if (warp == 0) {
       if (pn > 0) {
-        update_tile(M, pn, pn, pn - 1, pn, lane);
+        update_tile(D, M + ftile(pn, 0), M + ftile(pn, 0), pn - 1, pn, kTile, lane);
         if (lane < 8) y[j] = s;
       }
       __syncwarp();
       // lanes 0-7: the tile's rows, 8: y (the others repeat it)
-      float x[8];
-      load_row8(lane < 8 ? M + tile_at(pn, pn) : y + 8 * pn, lane < 8 ? lane : 0, x);
+      float* own = lane < 8 ? D : y + 8 * pn;
+      const int at = lane < 8 ? r : 0;
+      load_row8(own, at, x);
       __syncwarp();
       bool ok = true;
 #pragma unroll
@@ -198,23 +228,24 @@ __device__ __forceinline__ bool factor_mixed(float* M, float* y, const float* df
 #pragma unroll
         for (int k = c + 1; k < 8; k++) x[k] = fmaf(-x[c], wshfl(x[c], k), x[k]);
       }
-      if (lane <= 8) store_row8(lane < 8 ? M + tile_at(pn, pn) : y + 8 * pn, lane < 8 ? lane : 0, x);
+      if (lane <= 8) store_row8(own, at, x);
       if (!ok && lane == 0) *bad = 1;
-    } else if (pn > 0) {
-      if (j < 8 * nb) y[j] = s;
-      for (int bi = pn + warp; bi < nb; bi += W - 1) update_tile(M, bi, pn, 0, pn, lane);
-      // the next diagonal tile, by the warp whose turn is next
-      if (pn + 1 < nb && warp == 1 + (nb - pn - 1) % (W - 1))
-        update_tile(M, pn + 1, pn + 1, 0, pn, lane);
+    } else {
+      if (below) {
+        if (pn > 0) y[j] = s;
+        load_row8(tile + pn * kTile, r, x);
+        update_row(x, tile, M + ftile(pn, 0), r, pn);
+      }
+      if (warp == W - 1 && pn > 0 && pn + 1 < nb) {
+        const float* next = M + ftile(pn + 1, 0);
+        update_tile(M + ftile(pn + 1, pn + 1), next, next, 0, pn, kTile, lane);
+      }
     }
     group_sync<T>(grp);
     if (*bad) return false;
-    if (tid < 8 * (nb - pn - 1)) {
-      float* tile = M + tile_at(pn + 1 + (tid >> 3), pn);
-      float x[8];
-      load_row8(tile, tid & 7, x);
-      solve_row(x, M + tile_at(pn, pn));
-      store_row8(tile, tid & 7, x);
+    if (below) {
+      solve_row(x, D);
+      store_row8(tile + pn * kTile, r, x);
     }
     group_sync<T>(grp);
   }
@@ -228,9 +259,9 @@ __device__ __forceinline__ void back_mixed(const float* M, float* y, float* x, i
   const int warp = tid >> 5, r = tid & 7;
   for (int pn = nb - 1; pn >= 0; pn--) {
     if (warp == 0 || 32 * warp < 8 * pn) {
-      const float* D = M + tile_at(pn, pn);
+      const float* D = M + ftile(pn, pn);
       const bool on = tid < 8 * pn;
-      const float* P = M + tile_at(pn, on ? tid >> 3 : 0);
+      const float* P = M + ftile(pn, on ? tid >> 3 : 0);
       float d[8], l[8], p[8], b = y[8 * pn + r], s = on ? y[tid] : 0.f;
 #pragma unroll
       for (int c = 0; c < 8; c++) {
@@ -289,11 +320,12 @@ __global__ void __launch_bounds__(Mixed<KP>::T* G, (KP == 64 ? 6 : 2) / G)
       for (int j = 0; j < K; j++) s += p.Lambda[i + (size_t)j * K] * p.mu[j];
     lmu_s[i] = s;
   }
-  if constexpr (C::kLamShared)
-    for (int e = threadIdx.x; e < KP * KP; e += blockDim.x) {
-      const int i = e % KP, j = e / KP;
-      if (i >= j && i < K) lam_s[elem_at(i, j)] = (float)p.Lambda[i + (size_t)j * K];
-    }
+  for (int e = threadIdx.x; e < KP * KP; e += blockDim.x) {  // both triangles of a diagonal tile
+    const int i = e % KP, j = e / KP, hi = max(i, j), lo = min(i, j);
+    if (i >> 3 >= j >> 3)
+      lam_s[ftile(i >> 3, j >> 3) + tile_pos(i & 7, j & 7)] =
+          hi < K ? (float)p.Lambda[hi + (size_t)lo * K] : (i == j ? 1.f : 0.f);
+  }
   __syncthreads();
   // the thread's tile: rows 8 rt .., columns TC ct ..
   int rt = 0, ct = vt < C::NTILE ? vt : 0;
@@ -309,37 +341,42 @@ __global__ void __launch_bounds__(Mixed<KP>::T* G, (KP == 64 ? 6 : 2) / G)
     const RowTask tk = p.tasks[ti];
     int ti_next = 0;  // claimed early: its latency passes behind this row
     if (tid == 0) ti_next = (int)atomicAdd(&p.ctl->queue[p.qslot], 1u);
-    float acc[8][TC], racc[C::RC];
+    // The second pass is the FP64 redo of a row whose FP32 pivot failed; it forms the Gram again (or
+    // adds the parts again), so that the factor need not keep it in registers.
+    for (bool redo = false;;) {
+      float acc[8][TC], racc[C::RC];
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+      for (int i = 0; i < 8; i++)
 #pragma unroll
-      for (int j = 0; j < TC; j++) acc[i][j] = 0.f;
+        for (int j = 0; j < TC; j++) acc[i][j] = 0.f;
 #pragma unroll
-    for (int c = 0; c < C::RC; c++) racc[c] = 0.f;
-    gram_mixed<KP>(p, tk, wscale, Mf, tid, vt, rt, ct, grp, acc, racc);
-    if (vt >= T - 32)
+      for (int c = 0; c < C::RC; c++) racc[c] = 0.f;
+      if (!redo || tk.nparts == 1) {
+        gram_mixed<KP>(p, tk, wscale, Mf, tid, vt, rt, ct, grp, acc, racc);
+        if (vt >= T - 32)
 #pragma unroll
-      for (int c = 0; c < C::RC; c++) rhs_s[lane + 32 * c] = (double)racc[c];
-    group_sync<T>(grp);
-
-    bool finish = true;
-    if (tk.nparts > 1) {  // a part of a split row: the last part to arrive adds them in order
-      constexpr size_t kSlot = (size_t)KP * KP + KP;
-      double* sp = p.scratch + (size_t)(tk.slot + tk.part) * kSlot;
-      if (vt < C::NTILE)
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-#pragma unroll
-          for (int j = 0; j < TC; j++) sp[(i * TC + j) * T + vt] = (double)acc[i][j];
-      if (tid < KP) sp[KP * KP + tid] = rhs_s[tid];
-      __threadfence();
+          for (int c = 0; c < C::RC; c++) rhs_s[lane + 32 * c] = (double)racc[c];
+      }
       group_sync<T>(grp);
-      if (tid == 0)
-        bcast[1] = atomicAdd(&p.split_cnt[tk.split], 1u) == (unsigned)(tk.nparts - 1) ? 1 : 0;
-      group_sync<T>(grp);
-      finish = bcast[1] != 0;
-      if (finish) {
-        __threadfence();
+      if (tk.nparts > 1) {  // a part of a split row: the last part to arrive adds them in order
+        constexpr size_t kSlot = (size_t)KP * KP + KP;
+        if (!redo) {
+          double* sp = p.scratch + (size_t)(tk.slot + tk.part) * kSlot;
+          if (vt < C::NTILE)
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+              for (int j = 0; j < TC; j++) sp[(i * TC + j) * T + vt] = (double)acc[i][j];
+          if (tid < KP) sp[KP * KP + tid] = rhs_s[tid];
+          __threadfence();
+          group_sync<T>(grp);
+          if (tid == 0)
+            bcast[1] = atomicAdd(&p.split_cnt[tk.split], 1u) == (unsigned)(tk.nparts - 1) ? 1 : 0;
+          group_sync<T>(grp);
+          if (!bcast[1]) break;
+          __threadfence();
+          if (tid == 0) p.split_cnt[tk.split] = 0u;
+        }
         const double* s0 = p.scratch + (size_t)tk.slot * kSlot;
         if (vt < C::NTILE)
 #pragma unroll
@@ -357,35 +394,39 @@ __global__ void __launch_bounds__(Mixed<KP>::T* G, (KP == 64 ? 6 : 2) / G)
             r += __ldcg(s0 + (size_t)part * kSlot + KP * KP + tid);
           rhs_s[tid] = (double)(float)r;
         }
-        if (tid == 0) p.split_cnt[tk.split] = 0u;
         group_sync<T>(grp);
       }
-    }
 
-    if (finish) {
       const int row = tk.row;
-      // MM = Lambda + alpha G, the identity beyond K, in F
-      auto store_mm = [&](auto* dst, auto af) {
-        using F = decltype(af);
-        if (vt >= C::NTILE) return;
+      // MM = Lambda + alpha G, the identity beyond K (FP32: a diagonal tile's upper half mirrors its lower)
+      if (vt < C::NTILE && rt < nb) {
+        if (!redo) {
+          const float af = (float)alpha;
 #pragma unroll
-        for (int i = 0; i < 8; i++)
+          for (int i = 0; i < 8; i++)
 #pragma unroll
-          for (int j = 0; j < TC; j++) {
-            const int gi = 8 * rt + i, gj = TC * ct + j;
-            if (gi >= gj && gi < 8 * nb) {
-              F v = gi == gj ? (F)1 : (F)0;
-              if (gi < K) {
-                if constexpr (C::kLamShared && sizeof(F) == 4) v = lam_s[elem_at(gi, gj)];
-                else v = (F)p.Lambda[gi + (size_t)gj * K];
-                v = mfma(af, (F)acc[i][j], v);
-              }
-              dst[elem_at(gi, gj)] = v;
-              if constexpr (sizeof(F) == 4)
-                if (gi == gj) df[gi] = v;
+            for (int h = 0; h < TC / 4; h++) {
+              const int half = TC == 4 ? ct & 1 : h;
+              const int at = ftile(rt, TC * ct >> 3) + i * 8 + 4 * (half ^ ((i >> 1) & 1));
+              Vec4<float> v = lds4(lam_s + at);
+              if (8 * rt + i < K)
+#pragma unroll
+                for (int u = 0; u < 4; u++) v.v[u] = fmaf(af, acc[i][4 * h + u], v.v[u]);
+              *reinterpret_cast<float4*>(Mf + at) = make_float4(v.v[0], v.v[1], v.v[2], v.v[3]);
             }
-          }
-      };
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j < TC; j++) {
+              const int gi = 8 * rt + i, gj = TC * ct + j;
+              if (gi >= gj)
+                M[elem_at(gi, gj)] =
+                    gi < K ? fma(alpha, (double)acc[i][j], p.Lambda[gi + (size_t)gj * K])
+                           : (gi == gj ? 1.0 : 0.0);
+            }
+        }
+      }
       // the row's draws and the right-hand side Lambda (mu + Uhat[row]) + Gram rhs
       if (p.znoise) {
         if (tid < KP) z_s[tid] = tid < K ? p.znoise[(size_t)row * K + tid] : 0.0;
@@ -396,7 +437,6 @@ __global__ void __launch_bounds__(Mixed<KP>::T* G, (KP == 64 ? 6 : 2) / G)
         z_s[2 * tid] = 2 * tid < K ? z0 : 0.0;
         z_s[2 * tid + 1] = 2 * tid + 1 < K ? z1 : 0.0;
       }
-      store_mm(Mf, (float)alpha);
       double lm = 0.0;
       if (p.uhat) {
         if (tid < K) x_s[tid] = p.mu[tid] + p.uhat[(size_t)row * KP + tid];
@@ -407,28 +447,30 @@ __global__ void __launch_bounds__(Mixed<KP>::T* G, (KP == 64 ? 6 : 2) / G)
       } else {
         if (tid < KP) lm = lmu_s[tid];
       }
-      const double rr = tid < KP ? rhs_s[tid] + lm : 0.0;
-      if (tid < KP) yf[tid] = (float)rr;
+      if (tid < KP) {
+        const double rr = rhs_s[tid] + lm;
+        if (redo) rhs_s[tid] = rr;
+        else yf[tid] = (float)rr;
+      }
       if (tid == 0) *bad = 0;
       group_sync<T>(grp);
-      bool done = factor_mixed<T>(Mf, yf, df, nb, tid, grp, bad);
-      if (done) {
-        if (tid < 8 * nb) yf[tid] += (float)z_s[tid];
+      if (!redo) {
+        if (tid < 8 * nb) df[tid] = Mf[ftile(tid >> 3, tid >> 3) + tile_pos(tid & 7, tid & 7)];
         group_sync<T>(grp);
-        back_mixed<T>(Mf, yf, xf, nb, tid, grp);
-        if (tid < K) {
-          p.out_f32[(size_t)row * KP + tid] = xf[tid];
-          store_copy(p, (size_t)row * KP + tid, xf[tid]);
+        if (factor_mixed<T>(Mf, yf, df, nb, tid, grp, bad)) {
+          if (tid < 8 * nb) yf[tid] += (float)z_s[tid];
+          group_sync<T>(grp);
+          back_mixed<T>(Mf, yf, xf, nb, tid, grp);
+          if (tid < K) {
+            p.out_f32[(size_t)row * KP + tid] = xf[tid];
+            store_copy(p, (size_t)row * KP + tid, xf[tid]);
+          }
+          break;
         }
-      } else {  // the whole row again in FP64
+        if (tid == 0) atomicAdd(&p.ctl->retries[p.mode], 1u);
+        redo = true;
         group_sync<T>(grp);  // every thread has seen the flag
-        if (tid == 0) {
-          atomicAdd(&p.ctl->retries[p.mode], 1u);
-          *bad = 0;
-        }
-        store_mm(M, alpha);
-        if (tid < KP) rhs_s[tid] = rr;
-        group_sync<T>(grp);
+      } else {
         if (wide_factor_redo<KP, T>(M, rhs_s, Di, nb, tid, grp, bad)) {
           if (tid < 8 * nb) rhs_s[tid] += z_s[tid];
           group_sync<T>(grp);
@@ -441,6 +483,7 @@ __global__ void __launch_bounds__(Mixed<KP>::T* G, (KP == 64 ? 6 : 2) / G)
           atomicOr(&p.ctl->status, kStatCholFail);
           atomicCAS(&p.ctl->bad_row, -1, row);
         }
+        break;
       }
     }
     if (tid == 0) bcast[0] = ti_next;
@@ -473,7 +516,7 @@ void launch_mixed(const SampleParams& p, cudaStream_t s, int num_sms) {
 
 void launch_sample_wide_mixed(const SampleParams& p, int KP, cudaStream_t s, int num_sms,
                               int groups) {
-  if (KP == 128) return launch_mixed<128, 1>(p, s, num_sms);
+  if (KP == 128) return launch_mixed<128, 2>(p, s, num_sms);
   if (groups == 1) return launch_mixed<64, 1>(p, s, num_sms);
   return launch_mixed<64, 2>(p, s, num_sms);
 }

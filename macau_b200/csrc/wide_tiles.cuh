@@ -110,19 +110,19 @@ __device__ __forceinline__ void update_tile(double* M, int bi, int bj, int k0, i
   }
   *c = make_double2(v.x + w.x, v.y + w.y);
 }
-// FP32: one fused multiply-add per column, in column order.
-__device__ __forceinline__ void update_tile(float* M, int bi, int bj, int k0, int k1, int lane) {
+// FP32 (c -= sum over tiles A + k stride, B + k stride): one fused multiply-add per column, in column
+// order.
+__device__ __forceinline__ void update_tile(float* tile, const float* A, const float* B, int k0,
+                                            int k1, int stride, int lane) {
   const int g = lane >> 2, t = lane & 3;
-  const float* A = M + tile_at(bi, 0);
-  const float* B = M + tile_at(bj, 0);
-  float2* c = reinterpret_cast<float2*>(M + tile_at(bi, bj) + tile_pos(g, 2 * t));
+  float2* c = reinterpret_cast<float2*>(tile + tile_pos(g, 2 * t));
   float2 v = *c;
 #pragma unroll 2
   for (int k = k0; k < k1; k++) {
     float a[8], b0[8], b1[8];
-    load_row8(A + 64 * k, g, a);
-    load_row8(B + 64 * k, 2 * t, b0);
-    load_row8(B + 64 * k, 2 * t + 1, b1);
+    load_row8(A + stride * k, g, a);
+    load_row8(B + stride * k, 2 * t, b0);
+    load_row8(B + stride * k, 2 * t + 1, b1);
 #pragma unroll
     for (int q = 0; q < 8; q++) {
       v.x = fmaf(-a[q], b0[q], v.x);
