@@ -699,7 +699,7 @@ class Context {
   }
 
   // A chain with a block-CG link at K <= 32: statistics, draws and FP64 rows of both modes in a fixed
-  // order of summation (link_hyper.cu says why).
+  // order of summation (hyper_ordered.cu says why).
   bool link_chain() const { return K_ <= 32 && (prior_[0].macau || prior_[1].macau); }
 
   void update_prior(int mode) {

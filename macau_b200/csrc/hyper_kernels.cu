@@ -500,24 +500,6 @@ void launch_stats(const void* U, bool f32, const double* Uhat, long long N, int 
   launch_stats_wide(U, f32, Uhat, N, K, stride, uhat_stride, partials, nblocks, s);
 }
 
-// ---- batched problems (batch.cu): one statistics block and one Normal-Wishart block per
-// problem; problem p owns rows row0[p] .. row0[p + 1] - 1 of U (stride 32), K = Kp[p] ----
-__global__ void __launch_bounds__(kStatThreads)
-    k_stats_batch(const float* __restrict__ U, const int* __restrict__ row0,
-                  const int* __restrict__ Kp, double* __restrict__ partials) {
-  const int p = blockIdx.x;
-  stats32_rows<float>(U, nullptr, row0[p], row0[p + 1], Kp[p], 32, 0,
-                      partials + (size_t)p * (32 + 32 * 32));
-}
-
-void launch_prior_batch(const float* U, const int* row0, const int* Kp,
-                        const unsigned long long* seed, int P, double* partials, Ctl* ctl, int mode,
-                        double* mu, double* Lambda, float* LamF, double* lmu, cudaStream_t s) {
-  k_stats_batch<<<P, kStatThreads, 0, s>>>(U, row0, Kp, partials);
-  MG_CUDA(cudaGetLastError());
-  launch_nw_batch(partials, row0, Kp, seed, P, ctl, mode, mu, Lambda, LamF, lmu, s);
-}
-
 void launch_reduce_parts(const double* parts, int nparts, int len, double* out, cudaStream_t s) {
   k_reduce_parts<<<(len + 31) / 32, 256, 0, s>>>(parts, nparts, len, out);
   MG_CUDA(cudaGetLastError());

@@ -1,15 +1,19 @@
-// Hyperprior of a chain with a block-CG link matrix at K <= 32: statistics and Normal-Wishart draw in a
-// fixed order of summation.
+// Hyperprior in a fixed order of summation, K <= 32: statistics and Normal-Wishart draw of chains with a
+// block-CG link matrix, and of the batched problems.
 //
-// Why these modes do not use the matrix-instruction kernels of hyper_kernels.cu and hyper_wide.cu: a
-// link solve stops at a tolerance (1e-6 by default), and its result within that tolerance depends on
-// the last bit of its right-hand side: latents that differ by one unit in the last place give link
-// matrices that differ by 2e-7 to 8e-7 (3,814 rows, 1,847 features, 8 to 20 components; 5,003 rows,
-// 4,099 features, 16 components), in FP64 too.  So a chain with side information repeats a
-// recorded one only if everything that reaches the solve is summed in the order it was recorded
-// with: the rows (launch_sample), these two, and the SpMMs and solves of cg_kernels.cu.
-//   What bounds them: nothing that matters beside the solve (the draw 25 us on one SM, the
-// statistics 21 us at 138,000 rows; a solve takes milliseconds).
+// Why these do not use the matrix-instruction kernels of hyper_kernels.cu and hyper_wide.cu:
+//   * A link solve stops at a tolerance (1e-6 by default), and its result within that tolerance
+//     depends on the last bit of its right-hand side: latents that differ by one unit in the last
+//     place give link matrices that differ by 2e-7 to 8e-7 (3,814 rows, 1,847 features, 8 to 20
+//     components; 5,003 rows, 4,099 features, 16 components), in FP64 too.  So a chain with side
+//     information repeats a recorded one only if everything that reaches the solve is summed in the
+//     order it was recorded with: the rows (launch_sample), these, and the SpMMs and solves of
+//     cg_kernels.cu.
+//   * A batch runs many mixed-precision chains for many sweeps, each rounding Lambda to FP32 and its
+//     latents to BF16: of 64 problems over 40 sweeps about one met a Lambda whose last FP64 bit
+//     decided its FP32 rounding, and its latents were then 0.04 apart.
+//   What bounds them: nothing that matters beside a solve (the draw 25 us on one SM, the
+// statistics 21 us at 138,000 rows); in a batch the longest problem's statistics.
 #include "common.cuh"
 #include "kernels.h"
 #include "rng.cuh"
@@ -41,13 +45,12 @@ __device__ __forceinline__ void stats_load(const T* U, const double* Uhat, long 
   }
 }
 
+// One block's statistics over rows r0 .. r1 - 1 into out[0 .. K + K*K).
 template <typename T>
-__global__ void __launch_bounds__(kStatThreads)
-    k_link_stats(const T* __restrict__ U, const double* __restrict__ Uhat, long long N, int K,
-                 int stride, int uhat_stride, long long rows_per_block,
-                 double* __restrict__ partials) {
-  const long long r0 = (long long)blockIdx.x * rows_per_block, r1 = min(N, r0 + rows_per_block);
-  double* out = partials + (size_t)blockIdx.x * (K + K * K);
+__device__ __forceinline__ void stats32_rows(const T* __restrict__ U,
+                                             const double* __restrict__ Uhat, long long r0,
+                                             long long r1, int K, int stride, int uhat_stride,
+                                             double* __restrict__ out) {
   static_assert(kStatRows * 32 == 4 * kStatThreads, "four staged values per thread");
   __shared__ __align__(16) double xs[2][kStatRows][36];
   __shared__ double red[3][64][17];
@@ -113,6 +116,25 @@ __global__ void __launch_bounds__(kStatThreads)
   }
 }
 
+template <typename T>
+__global__ void __launch_bounds__(kStatThreads)
+    k_link_stats(const T* __restrict__ U, const double* __restrict__ Uhat, long long N, int K,
+                 int stride, int uhat_stride, long long rows_per_block,
+                 double* __restrict__ partials) {
+  const long long r0 = (long long)blockIdx.x * rows_per_block;
+  stats32_rows(U, Uhat, r0, min(N, r0 + rows_per_block), K, stride, uhat_stride,
+               partials + (size_t)blockIdx.x * (K + K * K));
+}
+
+// Problem p owns rows row0[p] .. row0[p + 1] - 1 of U (stride 32), K = Kp[p]; one block per problem.
+__global__ void __launch_bounds__(kStatThreads)
+    k_stats_batch(const float* __restrict__ U, const int* __restrict__ row0,
+                  const int* __restrict__ Kp, double* __restrict__ partials) {
+  const int p = blockIdx.x;
+  stats32_rows<float>(U, nullptr, row0[p], row0[p + 1], Kp[p], 32, 0,
+                      partials + (size_t)p * (32 + 32 * 32));
+}
+
 // CondNormalWishart -> NormalWishart -> MvNormal_prec (mvnormal.cpp:169-184, 217-287, 314-336)
 // for K <= 32 in one CTA of 256 threads, matrices in shared memory (row-major, ld 33), the
 // draws of k_nw.  Two identities replace two of the reference's three Cholesky
@@ -126,12 +148,15 @@ __global__ void __launch_bounds__(kStatThreads)
 constexpr int kNwLd = 33;
 constexpr int kNwLc = 36;
 
-__global__ void __launch_bounds__(256)
-    k_link_wishart(const double* __restrict__ stats, long long N, int K,
-                   const double* __restrict__ mu0, double kappa, const double* __restrict__ T0,
-                   int nu, const double* __restrict__ bb, const double* __restrict__ lambda_beta,
-                   Ctl* ctl, unsigned long long seed, int mode, double* __restrict__ mu_out,
-                   double* __restrict__ Lambda_out) {
+// mu0 == null stands for zeros, T0 == null for the identity, bb == null for no link matrix.
+__device__ __forceinline__ void nw32_run(const double* __restrict__ stats, long long N, int K,
+                                         const double* __restrict__ mu0, double kappa,
+                                         const double* __restrict__ T0, int nu,
+                                         const double* __restrict__ bb,
+                                         const double* __restrict__ lambda_beta, Ctl* ctl,
+                                         unsigned long long seed, int mode,
+                                         double* __restrict__ mu_out,
+                                         double* __restrict__ Lambda_out) {
   __shared__ double A[32 * kNwLd], Bm[32 * kNwLd], C[32 * kNwLd], D[32 * kNwLd];
   __shared__ __align__(16) double Lc[32 * kNwLc];
   __shared__ double NU[32], muc[32], m0[32], rl[32], zs[32];
@@ -144,9 +169,10 @@ __global__ void __launch_bounds__(256)
   for (int e = t; e < K; e += 256) NU[e] = stats[e];
   for (int e = t; e < KK; e += 256) {
     A[(e % K) * kNwLd + e / K] = stats[K + e];
-    Bm[(e % K) * kNwLd + e / K] = bb ? T0[e] + lb * bb[K + e] : T0[e];
+    const double w0 = T0 ? T0[e] : (e % K == e / K ? 1.0 : 0.0);
+    Bm[(e % K) * kNwLd + e / K] = bb ? w0 + lb * bb[K + e] : w0;
   }
-  if (t < K) m0[t] = mu0[t];
+  if (t < K) m0[t] = mu0 ? mu0[t] : 0.0;
   __syncthreads();
   const double kappa_c = kappa + (double)N;
   const int nu_c = nu + (int)N;
@@ -238,6 +264,41 @@ __global__ void __launch_bounds__(256)
     if (lane < K) mu_out[lane] = x + muc[lane];
   }
 }
+__global__ void __launch_bounds__(256)
+    k_link_wishart(const double* __restrict__ stats, long long N, int K,
+                   const double* __restrict__ mu0, double kappa, const double* __restrict__ T0,
+                   int nu, const double* __restrict__ bb, const double* __restrict__ lambda_beta,
+                   Ctl* ctl, unsigned long long seed, int mode, double* __restrict__ mu_out,
+                   double* __restrict__ Lambda_out) {
+  nw32_run(stats, N, K, mu0, kappa, T0, nu, bb, lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
+}
+
+// BPMFPrior::update_prior per problem with mu0 = 0, b0 = 2, W0 = I, df = K_p
+// (latentprior.cpp:79-99), keyed with the problem's seed; then the finish's operands: the FP32
+// Lambda (32 x 32, zero beyond K) and Lambda mu (FP64, summed in column order).
+__global__ void __launch_bounds__(256)
+    k_nw_batch(const double* __restrict__ partials, const int* __restrict__ row0,
+               const int* __restrict__ Kp, const unsigned long long* __restrict__ seed, Ctl* ctl,
+               int mode, double* __restrict__ mu, double* __restrict__ Lambda,
+               float* __restrict__ LamF, double* __restrict__ lmu) {
+  const int p = blockIdx.x, K = Kp[p];
+  double* L = Lambda + (size_t)p * 1024;
+  double* m = mu + (size_t)p * 32;
+  nw32_run(partials + (size_t)p * (32 + 32 * 32), row0[p + 1] - row0[p], K, nullptr, 2.0, nullptr, K,
+           nullptr, nullptr, ctl, seed[p], mode, m, L);
+  __syncthreads();
+  for (int e = threadIdx.x; e < 1024; e += blockDim.x) {
+    const int i = e >> 5, j = e & 31;
+    LamF[(size_t)p * 1024 + e] = (i < K && j < K) ? (float)L[i + j * K] : 0.f;
+  }
+  if (threadIdx.x < 32) {
+    double acc = 0.0;
+    if ((int)threadIdx.x < K)
+      for (int j = 0; j < K; j++) acc += L[threadIdx.x + j * K] * m[j];
+    lmu[(size_t)p * 32 + threadIdx.x] = acc;
+  }
+}
+
 }  // namespace
 
 void launch_link_stats(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
@@ -258,6 +319,15 @@ void launch_link_wishart(const double* stats, long long N, int K, const double* 
                          double* Lambda_out, cudaStream_t s) {
   k_link_wishart<<<1, 256, 0, s>>>(stats, N, K, mu0, kappa, T0, nu, bb, lambda_beta, ctl, seed, mode,
                                    mu_out, Lambda_out);
+  MG_CUDA(cudaGetLastError());
+}
+
+void launch_prior_batch(const float* U, const int* row0, const int* Kp,
+                        const unsigned long long* seed, int P, double* partials, Ctl* ctl, int mode,
+                        double* mu, double* Lambda, float* LamF, double* lmu, cudaStream_t s) {
+  k_stats_batch<<<P, kStatThreads, 0, s>>>(U, row0, Kp, partials);
+  MG_CUDA(cudaGetLastError());
+  k_nw_batch<<<P, 256, 0, s>>>(partials, row0, Kp, seed, ctl, mode, mu, Lambda, LamF, lmu);
   MG_CUDA(cudaGetLastError());
 }
 

@@ -375,34 +375,6 @@ __global__ void __launch_bounds__(kNwThreads, 1)
   nw_tiles<KP>(args.m[blockIdx.x], K, ctl, seed, nsm);
 }
 
-// BPMFPrior::update_prior per problem with mu0 = 0, b0 = 2, W0 = I, df = K_p
-// (latentprior.cpp:79-99), keyed with the problem's seed; then the finish's operands: the FP32
-// Lambda (32 x 32, zero beyond K) and Lambda mu (FP64, summed in column order).
-__global__ void __launch_bounds__(kNwThreads, 1)
-    k_nw_batch(const double* __restrict__ partials, const int* __restrict__ row0,
-               const int* __restrict__ Kp, const unsigned long long* __restrict__ seed, Ctl* ctl,
-               int mode, double* __restrict__ mu, double* __restrict__ Lambda,
-               float* __restrict__ LamF, double* __restrict__ lmu) {
-  __shared__ __align__(16) double nsm[NwW<32>::kDoubles];
-  const int p = blockIdx.x, K = Kp[p];
-  double* L = Lambda + (size_t)p * 1024;
-  double* m = mu + (size_t)p * 32;
-  const NwArgs a{partials + (size_t)p * (32 + 32 * 32), 1, nullptr, nullptr, nullptr, nullptr, 2.0,
-                 row0[p + 1] - row0[p], K, mode, m, L};
-  nw_tiles<32>(a, K, ctl, seed[p], nsm);
-  __syncthreads();
-  for (int e = threadIdx.x; e < 1024; e += kNwThreads) {
-    const int i = e >> 5, j = e & 31;
-    LamF[(size_t)p * 1024 + e] = (i < K && j < K) ? (float)L[i + j * K] : 0.f;
-  }
-  if (threadIdx.x < 32) {
-    double acc = 0.0;
-    if ((int)threadIdx.x < K)
-      for (int j = 0; j < K; j++) acc += L[threadIdx.x + j * K] * m[j];
-    lmu[(size_t)p * 32 + threadIdx.x] = acc;
-  }
-}
-
 template <int KP>
 void nw_launch(const NwPair& a, int count, int K, Ctl* ctl, unsigned long long seed,
                cudaStream_t s) {
@@ -466,13 +438,6 @@ void launch_normal_wishart_pair(const PriorPair& pp, int K, Ctl* ctl, unsigned l
                     pp.Lambda[m]};
   }
   nw_dispatch(a, 2, K, ctl, seed, s);
-}
-
-void launch_nw_batch(const double* partials, const int* row0, const int* Kp,
-                     const unsigned long long* seed, int P, Ctl* ctl, int mode, double* mu,
-                     double* Lambda, float* LamF, double* lmu, cudaStream_t s) {
-  k_nw_batch<<<P, kNwThreads, 0, s>>>(partials, row0, Kp, seed, ctl, mode, mu, Lambda, LamF, lmu);
-  MG_CUDA(cudaGetLastError());
 }
 
 }  // namespace mg

@@ -93,7 +93,7 @@ void launch_normal_wishart(const double* partials, int nparts, long long N, int 
                            const double* bb, const double* lambda_beta, Ctl* ctl,
                            unsigned long long seed, int mode, double* mu_out, double* Lambda_out,
                            cudaStream_t s);
-// The same two for a chain with a block-CG link at K <= 32 (link_hyper.cu), in a fixed order of summation;
+// The same two for a chain with a block-CG link at K <= 32 (hyper_ordered.cu), in a fixed order of summation;
 // `stats` is one record, `bb` one or null.
 void launch_link_stats(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
                        int uhat_stride, double* partials, int nblocks, cudaStream_t s);
@@ -124,15 +124,12 @@ struct PriorPair {
 };
 int launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl,
                        unsigned long long seed, cudaStream_t s);
-// The K > 32 forms of the statistics, and the pair's and the batch's draws (hyper_wide.cu).
+// The K > 32 forms of the statistics, and the pair's draws (hyper_wide.cu).
 void launch_stats_wide(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
                        int uhat_stride, double* partials, int nblocks, cudaStream_t s);
 void launch_stats_wide_pair(const PriorPair& pp, bool f32, int K, int stride, cudaStream_t s);
 void launch_normal_wishart_pair(const PriorPair& pp, int K, Ctl* ctl, unsigned long long seed,
                                 cudaStream_t s);
-void launch_nw_batch(const double* partials, const int* row0, const int* Kp,
-                     const unsigned long long* seed, int P, Ctl* ctl, int mode, double* mu,
-                     double* Lambda, float* LamF, double* lmu, cudaStream_t s);
 void launch_lambda_beta(const double* bb_partials, int nparts, int K, long long nfeat,
                         const double* Lambda, double nu, double mu, const Ctl* ctl,
                         unsigned long long seed, int mode, double* lambda_beta, cudaStream_t s);

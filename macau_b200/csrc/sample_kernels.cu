@@ -588,7 +588,7 @@ void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStre
     return launch_mixed<kGeBf16>(p, KP, groups, s, num_sms);
   } else {
     // K <= 32: Grams on the FP64 matrix instruction, except in a chain with a block-CG link, whose rows
-    // keep the order of summation of k_sample (link_hyper.cu says why)
+    // keep the order of summation of k_sample (hyper_ordered.cu says why)
     if (KP <= 32 && (p.one || !p.ordered)) return launch_sample_f64(p, KP, s, num_sms, groups);
     switch (KP) {
       case 8:
