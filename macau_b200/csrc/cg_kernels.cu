@@ -75,17 +75,21 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------- SpMM over a work split (DevCsr::tasks) ----------------
-// One warp per task (a whole row, or one part of a long row).  Entries are read four at a time
-// (independent gathers in flight) and added in CSR order.  A part stores its FP64 partial row in
-// A.parts; the last part of a row to finish (arrival counter) adds the parts in part order and
-// writes the row.  Whole rows give the same sums as k_spmm.
+// One warp per task (a whole row, or one part of a long row), a component per lane.  Entries are
+// added in CSR order; the indices come 32 at a time by one coalesced load, the next 32 ahead, and U
+// entries' gathers are in flight.  A part stores its FP64 partial row in A.parts; the last part of a row to
+// finish (arrival counter) adds the parts in part order and writes the row.  Whole rows give the
+// same sums as k_spmm.
+//   What bounds it: for short tasks the latency of index and gather, for the others the gathers
+//   from L2 (256 bytes per entry at 32 components).  (Several lane groups per entry, each summing
+//   every second or fourth entry, are faster, but sum in another order: hyper_ordered.cu.)
 template <typename V, int NRP>
 __global__ void __launch_bounds__(256)
     k_spmm_split(const DevCsr A, const V* __restrict__ src, int sstride, V* __restrict__ dst,
                  int dstride, int ncomp, const V* __restrict__ add, int astride, double reg,
                  const double* __restrict__ reg_dev, const uint32_t* __restrict__ done) {
   if (done && *done) return;
-  constexpr int C = NRP / 32;
+  constexpr int C = NRP / 32, U = 16 / C;
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (blockDim.x >> 5);
   const bool weighted = sizeof(V) == 8 ? A.val != nullptr : A.valf != nullptr;
@@ -94,52 +98,48 @@ __global__ void __launch_bounds__(256)
     V acc[C];
 #pragma unroll
     for (int c = 0; c < C; c++) acc[c] = (V)0;
-    const long long b = tk.begin, e = tk.begin + tk.len;
-    long long q = b;
-    for (; q + 4 <= e; q += 4) {
-      const V* s0 = src + (size_t)A.idx[q] * sstride;
-      const V* s1 = src + (size_t)A.idx[q + 1] * sstride;
-      const V* s2 = src + (size_t)A.idx[q + 2] * sstride;
-      const V* s3 = src + (size_t)A.idx[q + 3] * sstride;
-      V w0 = (V)1, w1 = (V)1, w2 = (V)1, w3 = (V)1;
-      if (weighted) {
-        if constexpr (sizeof(V) == 8) {
-          w0 = (V)A.val[q]; w1 = (V)A.val[q + 1]; w2 = (V)A.val[q + 2]; w3 = (V)A.val[q + 3];
-        } else {
-          w0 = (V)A.valf[q]; w1 = (V)A.valf[q + 1]; w2 = (V)A.valf[q + 2]; w3 = (V)A.valf[q + 3];
-        }
+    auto load_chunk = [&](int off, int& col, V& w) {
+      const bool in = off + lane < tk.len;
+      col = in ? A.idx[tk.begin + off + lane] : 0;
+      w = (V)1;
+      if (weighted && in) {
+        if constexpr (sizeof(V) == 8) w = (V)A.val[tk.begin + off + lane];
+        else w = (V)A.valf[tk.begin + off + lane];
       }
+    };
+    int c_cur, c_nxt;
+    V w_cur, w_nxt;
+    load_chunk(0, c_cur, w_cur);
+    for (int off = 0; off < tk.len; off += 32) {
+      load_chunk(off + 32, c_nxt, w_nxt);
 #pragma unroll
-      for (int c = 0; c < C; c++) {
-        const int k = lane + 32 * c;
-        if (k < ncomp) {
-          const V x0 = s0[k], x1 = s1[k], x2 = s2[k], x3 = s3[k];
-          if (weighted) {
-            acc[c] += x0 * w0;
-            acc[c] += x1 * w1;
-            acc[c] += x2 * w2;
-            acc[c] += x3 * w3;
-          } else {
-            acc[c] += x0;
-            acc[c] += x1;
-            acc[c] += x2;
-            acc[c] += x3;
+      for (int u = 0; u < 32; u += U) {
+        if (off + u < tk.len) {
+          V x[U][C];
+#pragma unroll
+          for (int i = 0; i < U; i++) {
+            const V* s0 = src + (size_t)__shfl_sync(0xffffffffu, c_cur, u + i) * sstride;
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+              const int k = lane + 32 * c;
+              x[i][c] = off + u + i < tk.len && k < ncomp ? s0[k] : (V)0;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < U; i++) {
+            const V w = weighted ? __shfl_sync(0xffffffffu, w_cur, u + i) : (V)1;
+            if (off + u + i < tk.len) {
+#pragma unroll
+              for (int c = 0; c < C; c++) {
+                if (weighted) acc[c] += x[i][c] * w;
+                else acc[c] += x[i][c];
+              }
+            }
           }
         }
       }
-    }
-    for (; q < e; q++) {
-      const V* s0 = src + (size_t)A.idx[q] * sstride;
-      V w0 = (V)1;
-      if (weighted) {
-        if constexpr (sizeof(V) == 8) w0 = (V)A.val[q];
-        else w0 = (V)A.valf[q];
-      }
-#pragma unroll
-      for (int c = 0; c < C; c++) {
-        const int k = lane + 32 * c;
-        if (k < ncomp) acc[c] += weighted ? s0[k] * w0 : s0[k];
-      }
+      c_cur = c_nxt;
+      w_cur = w_nxt;
     }
     const V r = (V)(reg_dev ? *reg_dev : reg);
     if (tk.nparts == 1) {
@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(256)
       const int k = lane + 32 * c;
       if (k < ncomp) {
         double t = 0.0;
+#pragma unroll 8
         for (int pt = 0; pt < tk.nparts; pt++) t += __ldcg(p0 + (size_t)pt * 64 + k);
         V o = (V)t;
         if (add) o += r * add[(size_t)tk.row * astride + k];
