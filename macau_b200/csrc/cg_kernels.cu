@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256)
   const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, l = threadIdx.x & 7;
   double s = 0.0;
   if (g < len)
-#pragma unroll 4
+#pragma unroll 16
     for (int b = l; b < nparts; b += 8) s += parts[(size_t)b * len + g];
   s += __shfl_xor_sync(0xffffffffu, s, 4, 8);
   s += __shfl_xor_sync(0xffffffffu, s, 2, 8);
@@ -394,8 +394,8 @@ constexpr int kLcLd = 36;
 
 // The same solves for n <= 32 with the factor in registers: warp 0 factorises the SPD matrix Ms
 // (lower triangle, padded with the identity beyond n) by warp_factor, publishing L^T in Lc;
-// then warp w solves columns w, w + 8, ...: lane i holds L(i, j) for j <= i and L(j, i) for
-// j > i and runs each substitution as 32 shuffle steps.  Returns false, with Out untouched, when
+// then warp w solves columns w, w + 8, ... side by side: lane i holds L(i, j) for j <= i and L(j, i)
+// for j > i and runs each substitution as 32 shuffle steps.  Returns false, with Out untouched, when
 // a pivot is not positive (the caller then takes the general path).
 __device__ bool warp_chol_solve(const double (*Ms)[33], double* Lc, const double* Rhs, int n,
                                 double* Out, int* okf) {
@@ -415,27 +415,40 @@ __device__ bool warp_chol_solve(const double (*Ms)[33], double* Lc, const double
   }
   __syncthreads();
   if (!*okf) return false;
-  double m[32], dinv = 1.0;
+  double m[32], d = 1.0;
 #pragma unroll
   for (int j = 0; j < 32; j++) {
     m[j] = j <= lane ? Lc[j * kLcLd + lane] : Lc[lane * kLcLd + j];
-    if (j == lane) dinv = 1.0 / m[j];
+    if (j == lane) d = m[j];
   }
-  for (int c = warp; c < n; c += kSolveThreads / 32) {
-    double y = lane < n ? Rhs[lane + c * 64] : 0.0;
+  const double dinv = 1.0 / d;
+  constexpr int kWarps = kSolveThreads / 32, C = 32 / kWarps;  // columns of a warp, side by side
+  double y[C];
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
-      if (lane == j) y *= dinv;
-      const double yj = __shfl_sync(0xffffffffu, y, j);
-      if (lane > j) y = fma(-m[j], yj, y);
+  for (int u = 0; u < C; u++) {
+    const int c = warp + kWarps * u;
+    y[u] = lane < n && c < n ? Rhs[lane + c * 64] : 0.0;
+  }
+#pragma unroll
+  for (int j = 0; j < 32; j++)
+#pragma unroll
+    for (int u = 0; u < C; u++) {
+      if (lane == j) y[u] *= dinv;
+      const double yj = __shfl_sync(0xffffffffu, y[u], j);
+      if (lane > j) y[u] = fma(-m[j], yj, y[u]);
     }
 #pragma unroll
-    for (int j = 31; j >= 0; j--) {
-      if (lane == j) y *= dinv;
-      const double xj = __shfl_sync(0xffffffffu, y, j);
-      if (lane < j) y = fma(-m[j], xj, y);
+  for (int j = 31; j >= 0; j--)
+#pragma unroll
+    for (int u = 0; u < C; u++) {
+      if (lane == j) y[u] *= dinv;
+      const double xj = __shfl_sync(0xffffffffu, y[u], j);
+      if (lane < j) y[u] = fma(-m[j], xj, y[u]);
     }
-    if (lane < n) Out[c + lane * 64] = y;
+#pragma unroll
+  for (int u = 0; u < C; u++) {
+    const int c = warp + kWarps * u;
+    if (lane < n && c < n) Out[c + lane * 64] = y[u];
   }
   return true;
 }
