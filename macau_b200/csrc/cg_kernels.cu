@@ -14,6 +14,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "mma_tiles.cuh"
 #include "rng.cuh"
 #include "warp_finish.cuh"
 
@@ -279,6 +280,79 @@ __global__ void __launch_bounds__(kOuterThreads, 2)
 #pragma unroll
           for (int g = 0; g < G - 1; g++) v += red[g][tile][x * 4 + y];
         out[(4 * ti + x) + (4 * tj + y) * NRP] = v;
+      }
+  }
+}
+
+// The same for NRP = 32 on the FP64 matrix instruction, which adds its four products one by one in
+// order (bit for bit a chain of fma), so the sums are k_outer's: warp rg takes every fourth row
+// of the block from r0 + rg on, four of them per instruction, and the warps' tiles are added in order.
+//   What bounds it: memory latency (about 28 rows a warp, two steps of four rows in flight), where
+//   k_outer staged every row in shared memory for 16 fma a thread.
+constexpr int kOuter32Threads = 128;
+template <typename V>
+__global__ void __launch_bounds__(kOuter32Threads)
+    k_outer32(const V* __restrict__ A, const V* __restrict__ B, long long nrow,
+              long long rows_per_block, double* __restrict__ partials,
+              const uint32_t* __restrict__ done) {
+  if (done && *done) return;
+  __shared__ __align__(16) double red[3][32 * 32];
+  const int rg = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const long long r0 = (long long)blockIdx.x * rows_per_block;
+  const long long r1 = min(nrow, r0 + rows_per_block);
+  double acc[4][4][2] = {};
+  double a[2][4], b[2][4];
+  auto load = [&](int stage, long long row) {
+    const bool in = row < r1;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      a[stage][k] = in ? (double)A[row * 32 + 8 * k + g] : 0.0;
+      b[stage][k] = in ? (double)B[row * 32 + 8 * k + g] : 0.0;
+    }
+  };
+  load(0, r0 + rg + 4 * t);
+  load(1, r0 + rg + 4 * t + 16);
+  for (long long r = r0 + rg; r < r1; r += 32) {
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      double ca[4], cb[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        ca[k] = a[u][k];
+        cb[k] = b[u][k];
+      }
+      load(u, r + 4 * t + 16 * u + 32);
+#pragma unroll
+      for (int bi = 0; bi < 4; bi++)
+#pragma unroll
+        for (int bj = 0; bj < 4; bj++)
+          mma_f64(acc[bi][bj][0], acc[bi][bj][1], ca[bi], cb[bj]);
+    }
+  }
+  auto at = [&](int bi, int bj) { return (8 * bi + g) * 32 + 8 * bj + 2 * t; };
+  if (rg > 0)
+#pragma unroll
+    for (int bi = 0; bi < 4; bi++)
+#pragma unroll
+      for (int bj = 0; bj < 4; bj++)
+        *reinterpret_cast<double2*>(&red[rg - 1][at(bi, bj)]) =
+            make_double2(acc[bi][bj][0], acc[bi][bj][1]);
+  __syncthreads();
+  if (rg == 0) {
+    double* out = partials + (size_t)blockIdx.x * 32 * 32;
+#pragma unroll
+    for (int bi = 0; bi < 4; bi++)
+#pragma unroll
+      for (int bj = 0; bj < 4; bj++) {
+        double2 v = make_double2(acc[bi][bj][0], acc[bi][bj][1]);
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+          const double2 x = *reinterpret_cast<const double2*>(&red[q][at(bi, bj)]);
+          v.x += x.x;
+          v.y += x.y;
+        }
+        out[(8 * bi + g) + (8 * bj + 2 * t) * 32] = v.x;
+        out[(8 * bi + g) + (8 * bj + 2 * t + 1) * 32] = v.y;
       }
   }
 }
@@ -629,6 +703,76 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// The same for NRP = 32 on the FP64 matrix instruction (a chain of fma over k in order, as above): a
+// warp takes 8 rows at a time, M's operands held in registers.
+//   What bounds it: the passes over X, R, P and KP from L2 (8.4 MB each at 32,768 rows).
+template <typename V, bool UPDATE>
+__global__ void __launch_bounds__(256)
+    k_cg_rows32(long long nfeat, int n, const double* small, const V* __restrict__ P,
+                const V* __restrict__ KPm, V* __restrict__ R, double* __restrict__ X,
+                V* __restrict__ Pout, const uint32_t* __restrict__ done) {
+  if (*done) return;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  SmallView v(const_cast<double*>(small));
+  const double* M = UPDATE ? v.A : v.Psi;
+  double m[4][8];  // M(8 b + g, 4 s + t)
+#pragma unroll
+  for (int b = 0; b < 4; b++)
+#pragma unroll
+    for (int s = 0; s < 8; s++) {
+      const int i = 8 * b + g, k = 4 * s + t;
+      m[b][s] = i < n && k < n ? M[i + k * 64] : 0.0;
+    }
+  const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long f = 8 * ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) + g;
+       f - g < nfeat; f += 8 * nw) {
+    const bool in = f < nfeat;
+    double a[8], q[UPDATE ? 8 : 1];
+#pragma unroll
+    for (int s = 0; s < 8; s++) {
+      const bool ok = in && 4 * s + t < n;
+      a[s] = ok ? (double)P[f * 32 + 4 * s + t] : 0.0;
+      if constexpr (UPDATE) q[s] = ok ? (double)KPm[f * 32 + 4 * s + t] : 0.0;
+    }
+    double sp[4][2] = {}, sq[4][2] = {};
+#pragma unroll
+    for (int s = 0; s < 8; s++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) {
+        mma_f64(sp[b][0], sp[b][1], a[s], m[b][s]);
+        if constexpr (UPDATE) mma_f64(sq[b][0], sq[b][1], q[s], m[b][s]);
+      }
+    if (!in) continue;
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int i = 8 * b + 2 * t + e;
+        if (i >= n) continue;
+        if constexpr (UPDATE) {
+          X[f * 32 + i] += sp[b][e];
+          R[f * 32 + i] = (V)((double)R[f * 32 + i] - sq[b][e]);
+        } else {
+          Pout[f * 32 + i] = (V)((double)R[f * 32 + i] + sp[b][e]);
+        }
+      }
+  }
+}
+
+template <typename V, int NRP, bool UPDATE>
+void cg_rows(long long nfeat, int n, const double* small, const V* P, const V* KPm, V* R, double* X,
+             V* Pout, const uint32_t* done, cudaStream_t s) {
+  if constexpr (NRP == 32) {
+    const int blocks = (int)std::min<long long>((nfeat + 63) / 64, 296);
+    k_cg_rows32<V, UPDATE><<<blocks, 256, 0, s>>>(nfeat, n, small, P, KPm, R, X, Pout, done);
+  } else {
+    k_cg_rows<V, NRP, UPDATE><<<(int)((nfeat + kRowTile - 1) / kRowTile), 256,
+                                rows_smem(NRP, UPDATE), s>>>(nfeat, n, small, P, KPm, R, X, Pout,
+                                                             done);
+  }
+  MG_CUDA(cudaGetLastError());
+}
+
 // R = Bn - KX (FP64 residual replacement, rounded to V)
 template <typename V>
 __global__ void k_cg_resid(long long total, int NRP, int n, const double* __restrict__ Bn,
@@ -747,7 +891,10 @@ template <typename V, int NRP>
 void outer(const V* A, const V* B, long long nrow, double* partials, int nb, cudaStream_t s,
            const uint32_t* done = nullptr) {
   const long long rpb = (nrow + nb - 1) / nb;
-  k_outer<V, NRP><<<nb, kOuterThreads, 0, s>>>(A, B, NRP, nrow, rpb, partials, done);
+  if constexpr (NRP == 32)
+    k_outer32<V><<<nb, kOuter32Threads, 0, s>>>(A, B, nrow, rpb, partials, done);
+  else
+    k_outer<V, NRP><<<nb, kOuterThreads, 0, s>>>(A, B, NRP, nrow, rpb, partials, done);
   MG_CUDA(cudaGetLastError());
 }
 
@@ -795,8 +942,7 @@ int cg_core(const DevCsr& F, const DevCsr& Ft, double reg, const double* reg_dev
   k_cg_rtr<<<1, 256, 0, s>>>(reduced, 1, NRP, n, small);
   MG_CUDA(cudaGetLastError());
   const double tolsq = tol * tol;
-  const int rg = (int)((nfeat + kRowTile - 1) / kRowTile);
-  {
+  if constexpr (NRP != 32) {
     static bool configured[64] = {false};
     int dev = 0;
     MG_CUDA(cudaGetDevice(&dev));
@@ -824,9 +970,7 @@ int cg_core(const DevCsr& F, const DevCsr& Ft, double reg, const double* reg_dev
       sum_records(partials, nb, NRP * NRP, reduced, s, done);
       k_cg_solve_a<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, small, ctl);
       MG_CUDA(cudaGetLastError());
-      k_cg_rows<V, NRP, true><<<rg, 256, rows_smem(NRP, true), s>>>(nfeat, n, small, P, KPm, R,
-                                                                    Xd, nullptr, done);
-      MG_CUDA(cudaGetLastError());
+      cg_rows<V, NRP, true>(nfeat, n, small, P, KPm, R, Xd, nullptr, done, s);
       if (sizeof(V) == 4 && (iter + 1) % kReplaceEvery == 0) {
         spmm_t<double, NRP>(F, Xd, NRP, innerd, NRP, n, nullptr, 0, 0.0, nullptr, s, done);
         spmm_t<double, NRP>(Ft, innerd, NRP, KX, NRP, n, Xd, NRP, reg, reg_dev, s, done);
@@ -838,9 +982,7 @@ int cg_core(const DevCsr& F, const DevCsr& Ft, double reg, const double* reg_dev
       k_cg_solve_psi<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, tolsq, small, ctl, flag_dev,
                                                  iter);
       MG_CUDA(cudaGetLastError());
-      k_cg_rows<V, NRP, false><<<rg, 256, rows_smem(NRP, false), s>>>(nfeat, n, small, P, nullptr,
-                                                                       R, nullptr, P, done);
-      MG_CUDA(cudaGetLastError());
+      cg_rows<V, NRP, false>(nfeat, n, small, P, nullptr, R, nullptr, P, done, s);
     }
     MG_CUDA(cudaStreamSynchronize(s));
     if (flag_host[0]) {
