@@ -466,37 +466,39 @@ __device__ void cta_chol_solve_cols(const double* M, const double* Rhs, int n, d
 constexpr int kSolveThreads = 256;
 constexpr int kLcLd = 36;
 
-// The same solves for n <= 32 with the factor in registers: warp 0 factorises the SPD matrix Ms
+// The same solves for n <= KP <= 32 with the factor in registers (KP = 8, 16 or 32, the least that
+// holds n: a column costs 450 cycles in the factor and 50 in each substitution, padding or not): warp 0 factorises the SPD matrix Ms
 // (lower triangle, padded with the identity beyond n) by warp_factor, publishing L^T in Lc;
 // then warp w solves columns w, w + 8, ... side by side: lane i holds L(i, j) for j <= i and L(j, i)
 // for j > i and runs each substitution as 32 shuffle steps.  Returns false, with Out untouched, when
 // a pivot is not positive (the caller then takes the general path).
+template <int KP>
 __device__ bool warp_chol_solve(const double (*Ms)[33], double* Lc, const double* Rhs, int n,
                                 double* Out, int* okf) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
-    double a[32], rinv = 1.0, d0 = 1.0;
+    double a[KP], rinv = 1.0, d0 = 1.0;
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
+    for (int j = 0; j < KP; j++) {
       double x;
       if (lane < n && j < n) x = j <= lane ? Ms[lane][j] : Ms[j][lane];
       else x = lane == j ? 1.0 : 0.0;
       a[j] = x;
       if (j == lane) d0 = x;
     }
-    const bool ok = warp_factor<double, 32>(a, rinv, lane, 0.0, d0, Lc, kLcLd);
+    const bool ok = warp_factor<double, KP>(a, rinv, lane, 0.0, d0, Lc, kLcLd);
     if (lane == 0) *okf = ok ? 1 : 0;
   }
   __syncthreads();
   if (!*okf) return false;
-  double m[32], d = 1.0;
+  double m[KP], d = 1.0;
 #pragma unroll
-  for (int j = 0; j < 32; j++) {
+  for (int j = 0; j < KP; j++) {
     m[j] = j <= lane ? Lc[j * kLcLd + lane] : Lc[lane * kLcLd + j];
     if (j == lane) d = m[j];
   }
   const double dinv = 1.0 / d;
-  constexpr int kWarps = kSolveThreads / 32, C = 32 / kWarps;  // columns of a warp, side by side
+  constexpr int kWarps = kSolveThreads / 32, C = KP / kWarps;  // columns of a warp, side by side
   double y[C];
 #pragma unroll
   for (int u = 0; u < C; u++) {
@@ -504,7 +506,7 @@ __device__ bool warp_chol_solve(const double (*Ms)[33], double* Lc, const double
     y[u] = lane < n && c < n ? Rhs[lane + c * 64] : 0.0;
   }
 #pragma unroll
-  for (int j = 0; j < 32; j++)
+  for (int j = 0; j < KP; j++)
 #pragma unroll
     for (int u = 0; u < C; u++) {
       if (lane == j) y[u] *= dinv;
@@ -512,7 +514,7 @@ __device__ bool warp_chol_solve(const double (*Ms)[33], double* Lc, const double
       if (lane > j) y[u] = fma(-m[j], yj, y[u]);
     }
 #pragma unroll
-  for (int j = 31; j >= 0; j--)
+  for (int j = KP - 1; j >= 0; j--)
 #pragma unroll
     for (int u = 0; u < C; u++) {
       if (lane == j) y[u] *= dinv;
@@ -528,6 +530,7 @@ __device__ bool warp_chol_solve(const double (*Ms)[33], double* Lc, const double
 }
 
 // A = (chol(PtKP) \ RtR)^T  (linop.h:286-289); PtKP from the lower triangle of sum P KP^T.
+template <int KP>
 __global__ void __launch_bounds__(kSolveThreads, 1)
     k_cg_solve_a(const double* partials, int nparts, int NRP, int n, double* small, Ctl* ctl) {
   if (ctl->cg_done) return;
@@ -541,7 +544,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
       if (i >= j) Ms[i][j] = sum_part(partials, nparts, NRP, i, j);
     }
     __syncthreads();
-    if (warp_chol_solve(Ms, Lc, v.RtR, n, v.A, &okf)) return;
+    if (warp_chol_solve<KP>(Ms, Lc, v.RtR, n, v.A, &okf)) return;
   }
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
     const int i = e % n, j = e / n;
@@ -554,6 +557,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
 }
 
 // RtR2 = sum R R^T; converged = all diag < tol^2; Psi = (chol(RtR) \ RtR2)^T; RtR <- RtR2.
+template <int KP>
 __global__ void __launch_bounds__(kSolveThreads, 1)
     k_cg_solve_psi(const double* partials, int nparts, int NRP, int n, double tolsq,
                    double* small, Ctl* ctl, int* flag_out, int iter) {
@@ -603,7 +607,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
       if (i >= j) Ms[i][j] = v.RtR[i + j * 64];
     }
     __syncthreads();
-    fast = warp_chol_solve(Ms, Lc, v.RtR2, n, v.Psi, &okf);
+    fast = warp_chol_solve<KP>(Ms, Lc, v.RtR2, n, v.Psi, &okf);
   }
   if (!fast) {
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
@@ -968,7 +972,8 @@ int cg_core(const DevCsr& F, const DevCsr& Ft, double reg, const double* reg_dev
       spmm_t<V, NRP>(Ft, inner, NRP, KPm, NRP, n, P, NRP, reg, reg_dev, s, done);
       outer<V, NRP>(P, KPm, nfeat, partials, nb, s, done);
       sum_records(partials, nb, NRP * NRP, reduced, s, done);
-      k_cg_solve_a<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, small, ctl);
+      (n <= 8 ? k_cg_solve_a<8> : n <= 16 ? k_cg_solve_a<16> : k_cg_solve_a<32>)
+          <<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, small, ctl);
       MG_CUDA(cudaGetLastError());
       cg_rows<V, NRP, true>(nfeat, n, small, P, KPm, R, Xd, nullptr, done, s);
       if (sizeof(V) == 4 && (iter + 1) % kReplaceEvery == 0) {
@@ -979,8 +984,8 @@ int cg_core(const DevCsr& F, const DevCsr& Ft, double reg, const double* reg_dev
       }
       outer<V, NRP>(R, R, nfeat, partials, nb, s, done);
       sum_records(partials, nb, NRP * NRP, reduced, s, done);
-      k_cg_solve_psi<<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, tolsq, small, ctl, flag_dev,
-                                                 iter);
+      (n <= 8 ? k_cg_solve_psi<8> : n <= 16 ? k_cg_solve_psi<16> : k_cg_solve_psi<32>)
+          <<<1, kSolveThreads, 0, s>>>(reduced, 1, NRP, n, tolsq, small, ctl, flag_dev, iter);
       MG_CUDA(cudaGetLastError());
       cg_rows<V, NRP, false>(nfeat, n, small, P, nullptr, R, nullptr, P, done, s);
     }
