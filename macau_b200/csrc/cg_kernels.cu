@@ -204,22 +204,19 @@ __global__ void __launch_bounds__(256)
 
 // ---------------- per-block partial of sum_f a_f b_f^T (NRP x NRP, full) ----------------
 // Rows staged 32 at a time in shared memory (the next 32 prefetched into registers); each thread
-// accumulates a 4 x 4 tile (i in 4 ti .., j in 4 tj ..) over the rows of its row group (every
-// G-th staged row; G = 4 for NRP = 32, 1 for NRP = 64), and the groups' tiles are added in group
-// order at the end.  partials[block][i + j * NRP] = sum over the block's rows of a_i b_j.
+// accumulates a 4 x 4 tile (i in 4 ti .., j in 4 tj ..).  partials[block][i + j * NRP] = sum over the
+// block's rows of a_i b_j.  NRP = 64; for 32: k_outer32.
 template <typename V, int NRP>
 __global__ void __launch_bounds__(kOuterThreads, 2)
     k_outer(const V* __restrict__ A, const V* __restrict__ B, int stride, long long nrow,
             long long rows_per_block, double* __restrict__ partials,
             const uint32_t* __restrict__ done) {
   if (done && *done) return;
-  constexpr int T4 = NRP / 4, TILES = T4 * T4, G = kOuterThreads / TILES;
+  constexpr int T4 = NRP / 4;
   constexpr int LD = NRP + 4, PRE = kOuterRows * NRP / kOuterThreads;  // staged values / thread
-  static_assert(G >= 1 && TILES * G == kOuterThreads, "tile layout");
+  static_assert(T4 * T4 == kOuterThreads, "tile layout");
   __shared__ __align__(16) double as[kOuterRows][LD], bs[kOuterRows][LD];
-  __shared__ double red[G > 1 ? G - 1 : 1][G > 1 ? TILES : 1][16];
-  const int t = threadIdx.x, tile = t % TILES, rg = t / TILES;
-  const int ti = tile / T4, tj = tile % T4;
+  const int t = threadIdx.x, ti = t / T4, tj = t % T4;
   const long long r0 = (long long)blockIdx.x * rows_per_block;
   const long long r1 = min(nrow, r0 + rows_per_block);
   double acc[4][4];
@@ -249,7 +246,7 @@ __global__ void __launch_bounds__(kOuterThreads, 2)
     }
     __syncthreads();
     if (b0 + kOuterRows < r1) fetch(b0 + kOuterRows);
-    for (int r = rg; r < cnt; r += G) {
+    for (int r = 0; r < cnt; r++) {
       const double2 i01 = *reinterpret_cast<const double2*>(&as[r][4 * ti]);
       const double2 i23 = *reinterpret_cast<const double2*>(&as[r][4 * ti + 2]);
       const double2 j01 = *reinterpret_cast<const double2*>(&bs[r][4 * tj]);
@@ -261,34 +258,19 @@ __global__ void __launch_bounds__(kOuterThreads, 2)
         for (int y = 0; y < 4; y++) acc[x][y] = fma(xi[x], xj[y], acc[x][y]);
     }
   }
-  if constexpr (G > 1) {
-    if (rg > 0)
+  double* out = partials + (size_t)blockIdx.x * NRP * NRP;
 #pragma unroll
-      for (int x = 0; x < 4; x++)
+  for (int x = 0; x < 4; x++)
 #pragma unroll
-        for (int y = 0; y < 4; y++) red[rg - 1][tile][x * 4 + y] = acc[x][y];
-    __syncthreads();
-  }
-  if (rg == 0) {
-    double* out = partials + (size_t)blockIdx.x * NRP * NRP;
-#pragma unroll
-    for (int x = 0; x < 4; x++)
-#pragma unroll
-      for (int y = 0; y < 4; y++) {
-        double v = acc[x][y];
-        if constexpr (G > 1)
-#pragma unroll
-          for (int g = 0; g < G - 1; g++) v += red[g][tile][x * 4 + y];
-        out[(4 * ti + x) + (4 * tj + y) * NRP] = v;
-      }
-  }
+    for (int y = 0; y < 4; y++) out[(4 * ti + x) + (4 * tj + y) * NRP] = acc[x][y];
 }
 
 // The same for NRP = 32 on the FP64 matrix instruction, which adds its four products one by one in
-// order (bit for bit a chain of fma), so the sums are k_outer's: warp rg takes every fourth row
-// of the block from r0 + rg on, four of them per instruction, and the warps' tiles are added in order.
-//   What bounds it: memory latency (about 28 rows a warp, two steps of four rows in flight), where
-//   k_outer staged every row in shared memory for 16 fma a thread.
+// order (bit for bit a chain of fma): warp rg takes every fourth row of the block from r0 + rg on,
+// four of them per instruction, and the warps' tiles are added in order, which is the order of
+// summation of recorded chains (hyper_ordered.cu).
+//   What bounds it: memory latency (about 28 rows a warp, two steps of four rows in flight).  With
+//   every row staged in shared memory for 4 x 4 tiles of fma it took 13.8 us at 32,768 rows.
 constexpr int kOuter32Threads = 128;
 template <typename V>
 __global__ void __launch_bounds__(kOuter32Threads)
@@ -709,7 +691,8 @@ __global__ void __launch_bounds__(256)
 
 // The same for NRP = 32 on the FP64 matrix instruction (a chain of fma over k in order, as above): a
 // warp takes 8 rows at a time, M's operands held in registers.
-//   What bounds it: the passes over X, R, P and KP from L2 (8.4 MB each at 32,768 rows).
+//   What bounds it: the passes over X, R, P and KP from L2 (8.4 MB each at 32,768 rows).  Through
+//   shared memory, as k_cg_rows, they took 24 and 13 us there.
 template <typename V, bool UPDATE>
 __global__ void __launch_bounds__(256)
     k_cg_rows32(long long nfeat, int n, const double* small, const V* __restrict__ P,

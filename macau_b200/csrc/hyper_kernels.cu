@@ -290,7 +290,7 @@ __global__ void k_set_sweep(Ctl* ctl, uint32_t sweep, int burnin) {
 __global__ void k_advance(Ctl* ctl) { ctl->sweep += 1u; }
 
 // One block's statistics (column sums and outer-product sums) over rows r0 .. r1 - 1 of (U - Uhat),
-// K <= 8 NB, into out[0 .. K + K*K) (k_stats32, k_stats32_pair and the batched k_stats_batch).  Warp
+// K <= 8 NB, into out[0 .. K + K*K) (k_stats32 and k_stats32_pair).  Warp
 // w takes the four rows 4 (w + 8 i) .. of the block, lane (g, t) = (lane / 4, lane % 4) component
 // 8 b + g of row t, which is the operand element of block b on either side of m8n8k4.f64: the
 // lower-triangle tiles take NB (NB + 1) / 2 matrix instructions per four rows, on operands loaded

@@ -1,7 +1,7 @@
 // Hyperprior in a fixed order of summation, K <= 32: statistics and Normal-Wishart draw of chains with a
 // block-CG link matrix, and of the batched problems.
 //
-// Why these do not use the matrix-instruction kernels of hyper_kernels.cu and hyper_wide.cu:
+// Why these do not use the kernels of hyper_kernels.cu and hyper_wide.cu:
 //   * A link solve stops at a tolerance (1e-6 by default), and its result within that tolerance
 //     depends on the last bit of its right-hand side: latents that differ by one unit in the last
 //     place give link matrices that differ by 2e-7 to 8e-7 (3,814 rows, 1,847 features, 8 to 20
@@ -12,108 +12,129 @@
 //   * A batch runs many mixed-precision chains for many sweeps, each rounding Lambda to FP32 and its
 //     latents to BF16: of 64 problems over 40 sweeps about one met a Lambda whose last FP64 bit
 //     decided its FP32 rounding, and its latents were then 0.04 apart.
-//   What bounds them: nothing that matters beside a solve (the draw 25 us on one SM, the
-// statistics 21 us at 138,000 rows); in a batch the longest problem's statistics.
+//   What bounds them: beside a solve nothing that matters (the draw takes 36 us on one SM); in a batch the
+// longest problem's statistics.
 #include "common.cuh"
 #include "kernels.h"
+#include "mma_tiles.cuh"
 #include "rng.cuh"
 #include "warp_finish.cuh"
 
 namespace mg {
 namespace {
 
-constexpr int kStatThreads = 256;
-constexpr int kStatRows = 32;  // rows staged per step
+constexpr int kStatThreads = 160;  // four warps of products, one of sums
 
-// Column sums and outer-product sums of rows r0 .. r1 - 1 of (U - Uhat): thread t
-// owns the 4 x 4 tile (4 (t % 64) / 8 .., 4 (t % 8) ..) for the rows of row group t / 64 (every
-// fourth staged row); the four groups are summed in group order at the end.  The next 32 rows
-// are loaded into registers while the current ones are multiplied (double-buffered staging).
-template <typename T>
-__device__ __forceinline__ void stats_load(const T* U, const double* Uhat, long long b0, int cnt,
-                                           int K, int stride, int uhat_stride, int t,
-                                           double (&nx)[4]) {
+// Column sums of rows r0 .. r1 - 1 of (U - Uhat), row after row, column `lane`; two batches of loads in
+// flight.
+template <typename T, bool HAT>
+__device__ __forceinline__ double ordered_sums(const T* __restrict__ U,
+                                               const double* __restrict__ Uhat, long long r0,
+                                               long long r1, int K, int stride, int uhat_stride,
+                                               int lane) {
+  constexpr int B = HAT || sizeof(T) == 8 ? 16 : 32;
+  T u[2][B];
+  double h[HAT ? 2 : 1][B];
+  auto load = [&](int stage, long long row) {
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int e = t + kStatThreads * q, r = e >> 5, k = e & 31;
-    double x = 0.0;
-    if (r < cnt && k < K) {
-      x = (double)U[(b0 + r) * stride + k];
-      if (Uhat) x -= Uhat[(b0 + r) * uhat_stride + k];
+    for (int i = 0; i < B; i++) {
+      const bool in = row + i < r1 && lane < K;
+      u[stage][i] = in ? U[(row + i) * stride + lane] : (T)0;
+      if constexpr (HAT) h[stage][i] = in ? Uhat[(row + i) * uhat_stride + lane] : 0.0;
     }
-    nx[q] = x;
+  };
+  double s = 0.0;
+  load(0, r0);
+  for (long long r = r0; r < r1; r += 2 * B) {
+#pragma unroll
+    for (int v = 0; v < 2; v++) {
+      load(v ^ 1, r + (v + 1) * B);
+#pragma unroll
+      for (int i = 0; i < B; i++) {
+        double x = (double)u[v][i];
+        if constexpr (HAT) x -= h[v][i];
+        s += x;
+      }
+    }
   }
+  return s;
 }
 
-// One block's statistics over rows r0 .. r1 - 1 into out[0 .. K + K*K).
+// One block's statistics over rows r0 .. r1 - 1 of (U - Uhat) into out[0 .. K + K*K).  The product sum
+// of a pair of columns is four sums over every fourth row, added in order; warp w < 4 forms the
+// w-th of them for all lower-triangle tiles by m8n8k4.f64, which adds its four products one by
+// one in order (bit for bit a chain of fma).
+//   What bounds it: 16 cycles of a sub-partition per instruction, 10 of them per 16 rows and warp
+//   at K = 32, on one SM per block.  (4 x 4 tiles of fma over rows staged in shared memory: 126 us on
+//   average for 64 problems of up to 4,000 rows.)
 template <typename T>
 __device__ __forceinline__ void stats32_rows(const T* __restrict__ U,
                                              const double* __restrict__ Uhat, long long r0,
                                              long long r1, int K, int stride, int uhat_stride,
                                              double* __restrict__ out) {
-  static_assert(kStatRows * 32 == 4 * kStatThreads, "four staged values per thread");
-  __shared__ __align__(16) double xs[2][kStatRows][36];
-  __shared__ double red[3][64][17];
-  const int KK = K * K;
-  const int t = threadIdx.x, tile = t & 63, rg = t >> 6;
-  const int ti = tile >> 3, tj = tile & 7;
-  double acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
-  double su = 0.0;
-  double nx[4];
-  stats_load(U, Uhat, r0, (int)max(0LL, min((long long)kStatRows, r1 - r0)), K, stride,
-             uhat_stride, t, nx);
-  int buf = 0;
-  for (long long b0 = r0; b0 < r1; b0 += kStatRows) {
-    const int cnt = (int)min((long long)kStatRows, r1 - b0);
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int e = t + kStatThreads * q;
-      xs[buf][e >> 5][e & 31] = nx[q];
-    }
-    __syncthreads();
-    const long long nb0 = b0 + kStatRows;
-    if (nb0 < r1)
-      stats_load(U, Uhat, nb0, (int)min((long long)kStatRows, r1 - nb0), K, stride, uhat_stride,
-                 t, nx);
-    if (t < K)
-      for (int r = 0; r < cnt; r++) su += xs[buf][r][t];
-#pragma unroll 2
-    for (int r = rg; r < kStatRows; r += 4) {
-      const double2 i01 = *reinterpret_cast<const double2*>(&xs[buf][r][4 * ti]);
-      const double2 i23 = *reinterpret_cast<const double2*>(&xs[buf][r][4 * ti + 2]);
-      const double2 j01 = *reinterpret_cast<const double2*>(&xs[buf][r][4 * tj]);
-      const double2 j23 = *reinterpret_cast<const double2*>(&xs[buf][r][4 * tj + 2]);
-      const double xi[4] = {i01.x, i01.y, i23.x, i23.y}, xj[4] = {j01.x, j01.y, j23.x, j23.y};
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = fma(xi[a], xj[b], acc[a][b]);
-    }
-    buf ^= 1;
-  }
-  __syncthreads();
-  if (rg > 0)
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-      for (int b = 0; b < 4; b++) red[rg - 1][tile][a * 4 + b] = acc[a][b];
-  __syncthreads();
-  if (t < K) out[t] = su;
-  if (rg == 0) {
-#pragma unroll
-    for (int a = 0; a < 4; a++)
+  constexpr int R = 4;  // steps of four rows in flight
+  __shared__ __align__(16) double red[3][10 * 64];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int nb = (K + 7) / 8;
+  double acc[10][2] = {};
+  if (warp == 4) {
+    const double s =
+        Uhat ? ordered_sums<T, true>(U, Uhat, r0, r1, K, stride, uhat_stride, lane)
+             : ordered_sums<T, false>(U, Uhat, r0, r1, K, stride, uhat_stride, lane);
+    if (lane < K) out[lane] = s;
+  } else {
+    double f[R][4];
+    auto load = [&](int stage, long long row) {
 #pragma unroll
       for (int b = 0; b < 4; b++) {
-        const double v = ((acc[a][b] + red[0][tile][a * 4 + b]) + red[1][tile][a * 4 + b]) +
-                         red[2][tile][a * 4 + b];
-        const int i = 4 * ti + a, j = 4 * tj + b;
-        if (i < K && j < K) out[K + i + j * K] = v;
+        const int k = 8 * b + g;
+        const bool in = row < r1 && k < K;
+        f[stage][b] = in ? (double)U[row * stride + k] : 0.0;
+        if (Uhat && in) f[stage][b] -= Uhat[row * uhat_stride + k];
       }
+    };
+    const long long first = r0 + warp + 4 * t;
+#pragma unroll
+    for (int v = 0; v < R - 1; v++) load(v, first + 16 * v);
+    for (long long r = r0; r < r1; r += 16 * R) {
+#pragma unroll
+      for (int v = 0; v < R; v++) {
+        load((v + R - 1) % R, r - r0 + first + 16 * (v + R - 1));
+        int q = 0;
+#pragma unroll
+        for (int bi = 0; bi < 4; bi++)
+#pragma unroll
+          for (int bj = 0; bj <= bi; bj++) {
+            if (bi < nb) mma_f64(acc[q][0], acc[q][1], f[v][bi], f[v][bj]);
+            q++;
+          }
+      }
+    }
+    if (warp > 0)
+#pragma unroll
+      for (int q = 0; q < 10; q++)
+        *reinterpret_cast<double2*>(&red[warp - 1][q * 64 + g * 8 + 2 * t]) =
+            make_double2(acc[q][0], acc[q][1]);
   }
+  __syncthreads();
+  if (warp > 0) return;
+  int q = 0;
+#pragma unroll
+  for (int bi = 0; bi < 4; bi++)
+#pragma unroll
+    for (int bj = 0; bj <= bi; bj++) {
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int at = q * 64 + g * 8 + 2 * t + e;
+        const double v = ((acc[q][e] + red[0][at]) + red[1][at]) + red[2][at];
+        const int i = 8 * bi + g, j = 8 * bj + 2 * t + e;
+        if (i < K && j < K) {
+          out[K + i + j * K] = v;
+          out[K + j + i * K] = v;
+        }
+      }
+      q++;
+    }
 }
 
 template <typename T>

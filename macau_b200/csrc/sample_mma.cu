@@ -14,8 +14,9 @@
 // TFLOP/s per GPU) for long rows, and the latency of the row finish for short ones; 16 warps per
 // SM at 128 registers keep four rows per sub-partition in flight, and the gathers run three
 // steps (12 entries) ahead of the products.  138,000 x 27,000 with 18M entries at K = 32: both
-// half-sweeps took 8.5 ms of an 8.97 ms sweep with the DFMA tiles, 2.5 of 2.98 ms here; 2,000 x
-// 1,500 with 54,000 entries at K = 10: a sweep of 112 us became 95 us.
+// half-sweeps took 8.5 ms of an 8.97 ms sweep with the DFMA tiles; the sweep takes 2.44 ms now, of
+// which the Grams are 1.25 ms of matrix instructions and most of the rest the row finishes.  2,000 x 1,500
+// with 54,000 entries at K = 10: a sweep of 112 us became 77 us.
 #include <algorithm>
 
 #include "common.cuh"
