@@ -296,7 +296,7 @@ __global__ void k_advance(Ctl* ctl) { ctl->sweep += 1u; }
 // lower-triangle tiles take NB (NB + 1) / 2 matrix instructions per four rows, on operands loaded
 // straight from memory three steps ahead.  The warps' tiles are added in warp order.
 //   What bounds it: latency; 4 x 4 DFMA tiles over rows staged in shared memory took 42 us for both
-//   modes of 138,000 x 27,000 at K = 32, and 126 us on average for 64 problems of up to 4,000 rows.
+//   modes of 138,000 x 27,000 at K = 32, this 17.
 constexpr int kStatWarps = kStatThreads / 32;
 template <typename T, int NB>
 __device__ __forceinline__ void stats32_blocks(const T* __restrict__ U,
