@@ -81,7 +81,7 @@ struct SampleParams {
   int mode;                    // 0 = rows of Y, 1 = columns
   unsigned long long seed;
   const double* znoise;        // optional injected N(0,1) draws (nrows x K), tests only
-  int ordered;                 // FP64, K <= 32: rows summed in k_sample's order (hyper_ordered.cu)
+  int ordered;                 // chain with a block-CG link: rows in k_sample's order of summation
   int one;                     // univariate prior (MacauOnePrior): coordinate-wise draws from
                                // the row's Gram with the precisions on Lambda's diagonal
   int half_copy;               // mixed: the 16-bit gather copy (out_bf16) holds FP16, not BF16

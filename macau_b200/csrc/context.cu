@@ -698,9 +698,9 @@ class Context {
     launches_ += launch_prior_pair(pp, mixed_, K_, KP_, ctl_.p, cfg_.seed, s_);
   }
 
-  // A chain with a block-CG link at K <= 32: statistics, draws and FP64 rows of both modes in a fixed
-  // order of summation (hyper_ordered.cu says why).
-  bool link_chain() const { return K_ <= 32 && (prior_[0].macau || prior_[1].macau); }
+  // A chain with a block-CG link: statistics, draws and rows of both modes in a fixed order of
+  // summation (hyper_ordered.cu says why).
+  bool link_chain() const { return prior_[0].macau || prior_[1].macau; }
 
   void update_prior(int mode) {
     Prior& p = prior_[mode];
@@ -710,6 +710,7 @@ class Context {
     const auto stats_of = link ? launch_link_stats : launch_stats;
     const bool few = !link && few_parts(nb, K_);
     launches_ += p.macau ? 0 : few ? 2 : 3;  // Macau launches are counted by kernels_in_cg below
+    if (link && K_ > 32) launches_ += p.macau ? 3 : 1;  // the ordered column sums of each statistics
     const int rec = K_ + K_ * K_;
     stats_of(latents(mode), mixed_, p.side() ? p.uhat.p : nullptr, N, K_, KP_, KP_,
              stat_partials_.p, nb, s_);

@@ -1,19 +1,19 @@
-// Hyperprior in a fixed order of summation, K <= 32: statistics and Normal-Wishart draw of chains with a
-// block-CG link matrix, and of the batched problems.
+// Hyperprior in a fixed order of summation: statistics and Normal-Wishart draw of chains with a
+// block-CG link matrix (K <= 64), and of the batched problems (K <= 32).
 //
 // Why these do not use the kernels of hyper_kernels.cu and hyper_wide.cu:
 //   * A link solve stops at a tolerance (1e-6 by default), and its result within that tolerance
 //     depends on the last bit of its right-hand side: latents that differ by one unit in the last
-//     place give link matrices that differ by 2e-7 to 8e-7 (3,814 rows, 1,847 features, 8 to 20
-//     components; 5,003 rows, 4,099 features, 16 components), in FP64 too.  So a chain with side
-//     information repeats a recorded one only if everything that reaches the solve is summed in the
-//     order it was recorded with: the rows (launch_sample), these, and the SpMMs and solves of
-//     cg_kernels.cu.
+//     place give link matrices that differ by 1e-7 to 2e-6 (1,203 to 5,003 rows, 517 to 4,099
+//     features, 7 to 64 components), in FP64 too, and mixed latents that differ by 2e-4 a sweep
+//     later.  So a chain with side information repeats a recorded one only if everything that
+//     reaches the solve is summed in the order it was recorded with: the rows (launch_sample),
+//     these, and the SpMMs and solves of cg_kernels.cu.
 //   * A batch runs many mixed-precision chains for many sweeps, each rounding Lambda to FP32 and its
 //     latents to BF16: of 64 problems over 40 sweeps about one met a Lambda whose last FP64 bit
 //     decided its FP32 rounding, and its latents were then 0.04 apart.
-//   What bounds them: beside a solve nothing that matters (the draw takes 36 us on one SM); in a batch the
-// longest problem's statistics.
+//   What bounds them: beside a solve nothing that matters (the draw takes 36 us on one SM at K <= 32);
+// in a batch the longest problem's statistics.
 #include "common.cuh"
 #include "kernels.h"
 #include "mma_tiles.cuh"
@@ -145,6 +145,22 @@ __global__ void __launch_bounds__(kStatThreads)
   const long long r0 = (long long)blockIdx.x * rows_per_block;
   stats32_rows(U, Uhat, r0, min(N, r0 + rows_per_block), K, stride, uhat_stride,
                partials + (size_t)blockIdx.x * (K + K * K));
+}
+
+// K > 32: k_stats_wide's products are chains of fma over the rows already (one warp takes a tile
+// through all of a block's rows); its column sums, four partial sums each, are replaced by these.
+// One warp per 32 columns.
+template <typename T>
+__global__ void __launch_bounds__(64)
+    k_link_sums(const T* __restrict__ U, const double* __restrict__ Uhat, long long N, int K,
+                int stride, int uhat_stride, long long rows_per_block,
+                double* __restrict__ partials) {
+  const long long r0 = (long long)blockIdx.x * rows_per_block, r1 = min(N, r0 + rows_per_block);
+  const int c0 = threadIdx.x & ~31, lane = threadIdx.x & 31;
+  const double s =
+      Uhat ? ordered_sums<T, true>(U + c0, Uhat + c0, r0, r1, K - c0, stride, uhat_stride, lane)
+           : ordered_sums<T, false>(U + c0, nullptr, r0, r1, K - c0, stride, uhat_stride, lane);
+  if (c0 + lane < K) partials[(size_t)blockIdx.x * (K + K * K) + c0 + lane] = s;
 }
 
 // Problem p owns rows row0[p] .. row0[p + 1] - 1 of U (stride 32), K = Kp[p]; one block per problem.
@@ -294,6 +310,130 @@ __global__ void __launch_bounds__(256)
   nw32_run(stats, N, K, mu0, kappa, T0, nu, bb, lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
 }
 
+// ---- the draw for 32 < K <= 64 ----
+// Left-looking lower Cholesky of the K x K column-major matrix A (shared memory) by the block,
+// thread i forming L(i, j); the strict upper triangle is zeroed.  False on a pivot that is not
+// positive (the same value in every thread).
+__device__ bool block_chol(double* A, int K) {
+  __syncthreads();
+  for (int j = 0; j < K; j++) {
+    double d = A[j + j * K];
+    for (int p = 0; p < j; p++) d = fma(-A[j + p * K], A[j + p * K], d);
+    if (!(d > 0.0)) {
+      __syncthreads();
+      return false;
+    }
+    const double ljj = sqrt(d);
+    for (int i = j + 1 + threadIdx.x; i < K; i += blockDim.x) {
+      double s = A[i + j * K];
+      for (int p = 0; p < j; p++) s = fma(-A[i + p * K], A[j + p * K], s);
+      A[i + j * K] = s / ljj;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) A[j + j * K] = ljj;
+    __syncthreads();
+  }
+  for (int q = threadIdx.x; q < K * K; q += blockDim.x)
+    if (q % K < q / K) A[q] = 0.0;
+  __syncthreads();
+  return true;
+}
+
+// CondNormalWishart -> NormalWishart -> Wishart -> MvNormal_prec (mvnormal.cpp:169-184, 217-287,
+// 314-336) step by step, each matrix element one chain of fma over its index: T_c by the factor of X
+// and two substitutions per column, its factor L, Lambda = L (c^T c) L^T, the mean through the
+// factor of kappa_c Lambda.  The matrices are in shared memory.
+//   What bounds it: the substitutions, a thread per column.
+__global__ void __launch_bounds__(256)
+    k_link_wishart_wide(const double* __restrict__ stats, long long N, int K,
+                        const double* __restrict__ mu0, double kappa, const double* __restrict__ T0,
+                        int nu, const double* __restrict__ bb,
+                        const double* __restrict__ lambda_beta, Ctl* ctl, unsigned long long seed,
+                        int mode, double* __restrict__ mu_out, double* __restrict__ Lambda_out) {
+  extern __shared__ __align__(16) double wsm[];
+  __shared__ double muc[64], z[64];
+  const int KK = K * K;
+  const uint32_t sweep = ctl->sweep;
+  double *X = wsm, *Tc = X + KK, *c = Tc + KK, *W = c + KK;
+  const double lb = bb ? *lambda_beta : 0.0;
+  const double kappa_c = kappa + (double)N;
+  const int nu_c = nu + (int)N;
+  for (int i = threadIdx.x; i < K; i += blockDim.x) muc[i] = fma(kappa, mu0[i], stats[i]) / kappa_c;
+  __syncthreads();
+  for (int e = threadIdx.x; e < KK; e += blockDim.x) {
+    const int i = e % K, j = e / K;
+    const double T = bb ? fma(lb, bb[K + e], T0[e]) : T0[e];  // latentprior.cpp:258-260
+    X[e] = fma(-(kappa_c * muc[i]), muc[j], fma(kappa * mu0[i], mu0[j], T + stats[K + e]));
+  }
+  bool ok = block_chol(X, K);
+  if (ok) {
+    for (int q = threadIdx.x; q < K; q += blockDim.x) {  // column q of X^{-1}
+      double* x = Tc + q * K;
+      for (int i = 0; i < K; i++) {
+        double s = i == q ? 1.0 : 0.0;
+        for (int p = 0; p < i; p++) s = fma(-X[i + p * K], x[p], s);
+        x[i] = s / X[i + i * K];
+      }
+      for (int i = K - 1; i >= 0; i--) {
+        double s = x[i];
+        for (int p = i + 1; p < K; p++) s = fma(-X[p + i * K], x[p], s);
+        x[i] = s / X[i + i * K];
+      }
+    }
+    ok = block_chol(Tc, K);
+  }
+  if (ok) {
+    // Bartlett factor: c_ii = sqrt(2 Gamma((nu_c - i) / 2)), c_ij ~ N(0, 1) for j > i
+    for (int e = threadIdx.x; e < KK; e += blockDim.x) {
+      const int i = e % K, j = e / K;
+      double v = 0.0;
+      if (i == j)
+        v = sqrt(2.0 * gamma_draw(seed, sweep, stream_id(kWishartDiag, mode), (uint32_t)i,
+                                  0.5 * (double)(nu_c - i)));
+      else if (j > i)
+        v = normal_draw(seed, sweep, stream_id(kWishartOff, mode), (uint32_t)i,
+                        (uint32_t)(j - i - 1));
+      c[e] = v;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < KK; e += blockDim.x) {  // W = c^T c
+      double s = 0.0;
+      for (int p = 0; p < K; p++) s = fma(c[p + e % K * K], c[p + e / K * K], s);
+      W[e] = s;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < KK; e += blockDim.x) {  // X = L W
+      double s = 0.0;
+      for (int p = 0; p < K; p++) s = fma(Tc[e % K + p * K], W[p + e / K * K], s);
+      X[e] = s;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < KK; e += blockDim.x) {  // Lambda = X L^T
+      double s = 0.0;
+      for (int p = 0; p < K; p++) s = fma(X[e % K + p * K], Tc[e / K + p * K], s);
+      Lambda_out[e] = s;
+      c[e] = s * kappa_c;
+    }
+    ok = block_chol(c, K);
+  }
+  if (!ok) {
+    if (threadIdx.x == 0) atomicOr(&ctl->status, kStatHyperFail);
+    return;
+  }
+  // mu = mu_c + chol(kappa_c Lambda)^{-T} z
+  for (int i = threadIdx.x; i < K; i += blockDim.x)
+    z[i] = normal_draw(seed, sweep, stream_id(kMuDraw, mode), 0u, (uint32_t)i);
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int i = K - 1; i >= 0; i--) {
+      double s = z[i];
+      for (int p = i + 1; p < K; p++) s = fma(-c[p + i * K], z[p], s);
+      z[i] = s / c[i + i * K];
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < K; i += blockDim.x) mu_out[i] = z[i] + muc[i];
+}
+
 // BPMFPrior::update_prior per problem with mu0 = 0, b0 = 2, W0 = I, df = K_p
 // (latentprior.cpp:79-99), keyed with the problem's seed; then the finish's operands: the FP32
 // Lambda (32 x 32, zero beyond K) and Lambda mu (FP64, summed in column order).
@@ -325,6 +465,17 @@ __global__ void __launch_bounds__(256)
 void launch_link_stats(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
                        int uhat_stride, double* partials, int nblocks, cudaStream_t s) {
   const long long rpb = (N + nblocks - 1) / nblocks;
+  if (K > 32) {
+    launch_stats_wide(U, f32, Uhat, N, K, stride, uhat_stride, partials, nblocks, s);
+    if (f32)
+      k_link_sums<float><<<nblocks, 64, 0, s>>>((const float*)U, Uhat, N, K, stride, uhat_stride,
+                                                rpb, partials);
+    else
+      k_link_sums<double><<<nblocks, 64, 0, s>>>((const double*)U, Uhat, N, K, stride, uhat_stride,
+                                                 rpb, partials);
+    MG_CUDA(cudaGetLastError());
+    return;
+  }
   if (f32)
     k_link_stats<float><<<nblocks, kStatThreads, 0, s>>>((const float*)U, Uhat, N, K, stride,
                                                          uhat_stride, rpb, partials);
@@ -338,6 +489,20 @@ void launch_link_wishart(const double* stats, long long N, int K, const double* 
                          const double* T0, int nu, const double* bb, const double* lambda_beta,
                          Ctl* ctl, unsigned long long seed, int mode, double* mu_out,
                          double* Lambda_out, cudaStream_t s) {
+  if (K > 32) {
+    static bool configured[64] = {false};
+    int dev = 0;
+    MG_CUDA(cudaGetDevice(&dev));
+    if (!configured[dev & 63]) {
+      MG_CUDA(cudaFuncSetAttribute(k_link_wishart_wide, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(4 * 64 * 64 * sizeof(double))));
+      configured[dev & 63] = true;
+    }
+    k_link_wishart_wide<<<1, 256, 4 * sizeof(double) * K * K, s>>>(
+        stats, N, K, mu0, kappa, T0, nu, bb, lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
+    MG_CUDA(cudaGetLastError());
+    return;
+  }
   k_link_wishart<<<1, 256, 0, s>>>(stats, N, K, mu0, kappa, T0, nu, bb, lambda_beta, ctl, seed, mode,
                                    mu_out, Lambda_out);
   MG_CUDA(cudaGetLastError());

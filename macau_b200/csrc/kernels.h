@@ -93,8 +93,8 @@ void launch_normal_wishart(const double* partials, int nparts, long long N, int 
                            const double* bb, const double* lambda_beta, Ctl* ctl,
                            unsigned long long seed, int mode, double* mu_out, double* Lambda_out,
                            cudaStream_t s);
-// The same two for a chain with a block-CG link at K <= 32 (hyper_ordered.cu), in a fixed order of summation;
-// `stats` is one record, `bb` one or null.
+// The same two for a chain with a block-CG link (hyper_ordered.cu; K <= 64), in a fixed order of
+// summation; `stats` is one record, `bb` one or null.
 void launch_link_stats(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
                        int uhat_stride, double* partials, int nblocks, cudaStream_t s);
 void launch_link_wishart(const double* stats, long long N, int K, const double* mu0, double kappa,

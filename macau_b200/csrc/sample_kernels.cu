@@ -577,9 +577,11 @@ std::vector<int> sample_group_options(int KP, bool mixed, int gram) {
 
 void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStream_t s,
                    int num_sms, int groups) {
-  // K > 32: the group sampler with matrix-instruction Grams; the univariate prior and the FP16
-  // and TF32 Grams, which need other operands or the whole Gram, keep k_sample
-  if (KP > 32 && !p.one && (!mixed || gram == kGeBf16))
+  // K > 32: a group of warps per row and a panel factor.  The univariate prior and the FP16 and TF32
+  // Grams, which need the whole Gram or other operands, keep k_sample, and so do FP64 rows of a
+  // chain with a block-CG link, for their order of summation (hyper_ordered.cu says why; the mixed
+  // group sampler keeps that order by itself).
+  if (KP > 32 && !p.one && (mixed ? gram == kGeBf16 : !p.ordered))
     return mixed ? launch_sample_wide_mixed(p, KP, s, num_sms, groups)
                  : launch_sample_wide(p, KP, s, num_sms, groups);
   if (mixed) {
