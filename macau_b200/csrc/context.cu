@@ -178,6 +178,8 @@ struct Prior {
   DBuf<double> colsq, lb_one;
   DBuf<int> lvl_ptr, lvl_feat, lvl_warp;
   DBuf<longlong2> lvl_range;
+  std::vector<int> level;           // each feature's level, and Ft's row pointers, on the host
+  std::vector<long long> tptr_host;
   int nlevels = 0;
   double lb_a0 = 0.1, lb_b0 = 0.1;
   bool side() const { return macau || one; }
@@ -379,21 +381,31 @@ class Context {
         for (long long e = t.ptr[f]; e < t.ptr[f + 1]; e++) last[t.idx[e]] = lv;
         level[f] = lv;
       }
-      std::vector<int> lptr, order, lwarp;
-      beta_one_levels(nrows, level, t.ptr, lptr, order, lwarp);
       p.colsq.upload(cs.data(), cs.size(), s_);
-      p.lvl_warp.upload(lwarp.data(), lwarp.size(), s_);
-      p.lvl_ptr.upload(lptr.data(), lptr.size(), s_);
-      p.lvl_feat.upload(order.data(), order.size(), s_);
-      std::vector<longlong2> range(nfeat);
-      for (int q = 0; q < nfeat; q++)
-        range[q] = make_longlong2(t.ptr[order[q]], t.ptr[order[q] + 1]);
-      p.lvl_range.upload(range.data(), range.size(), s_);
-      p.nlevels = (int)lwarp.size();
+      p.level = std::move(level);
+      p.tptr_host = std::move(t.ptr);
     }
+    for (int m = 0; m < 2; m++)  // also the other mode's: whether a link chain is ordered may change
+      if (prior_[m].one) build_levels(m);
     MG_CUDA(cudaStreamSynchronize(s_));
     drop_graphs();
     initialised_ = false;
+  }
+
+  // Level tables of a univariate mode's link sampler.
+  void build_levels(int mode) {
+    Prior& p = prior_[mode];
+    std::vector<int> lptr, order, lwarp;
+    beta_one_levels(p.F.nrow, link_chain(), p.level, p.tptr_host, lptr, order, lwarp);
+    p.lvl_warp.upload(lwarp.data(), lwarp.size(), s_);
+    p.lvl_ptr.upload(lptr.data(), lptr.size(), s_);
+    p.lvl_feat.upload(order.data(), order.size(), s_);
+    std::vector<longlong2> range(order.size());
+    for (size_t q = 0; q < order.size(); q++)
+      range[q] = make_longlong2(p.tptr_host[order[q]], p.tptr_host[order[q] + 1]);
+    p.lvl_range.upload(range.data(), range.size(), s_);
+    p.nlevels = (int)lwarp.size();
+    MG_CUDA(cudaStreamSynchronize(s_));  // the host tables go out of scope
   }
 
   void set_samples(int burnin, int nsamples) {
@@ -735,11 +747,12 @@ class Context {
                       p.nlevels,
                       latents(mode),
                       mixed_, KP_, p.mu.p, p.uhat.p, KP_, p.Lambda.p, p.lb_one.p, K_, N, p.beta.p,
-                      CP_, p.tmp.p, CP_, p.B.p, ctl_.p, cfg_.seed, mode, s_);
+                      CP_, p.tmp.p, CP_, p.B.p, link, ctl_.p, cfg_.seed, mode, s_);
       launch_spmm(p.F, p.beta.p, CP_, p.uhat.p, KP_, K_, false, s_);
       launch_lambda_beta_one(p.beta.p, CP_, p.nfeat, K_, p.lb_a0, p.lb_b0, ctl_.p, cfg_.seed,
-                             mode, p.B.p, p.lb_one.p, s_);
-      launches_ += 5;  // draws, beta, spmm, 2 of lambda_beta (after the 3 of stats / reduce / NW)
+                             mode, link, p.B.p, p.lb_one.p, s_);
+      // draws, beta, spmm, 1 or 2 of lambda_beta (after the 3 of stats / reduce / NW)
+      launches_ += link ? 4 : 5;
       return;
     }
     if (!p.macau) {  // BPMFPrior::update_prior (latentprior.cpp:79-81)

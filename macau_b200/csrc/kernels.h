@@ -184,22 +184,23 @@ void launch_spmm(const DevCsr& A, const void* src, int src_stride, void* dst, in
 // F as CSR rows) with the feature levels lvl_ptr / lvl_feat (lvl_range: each listed feature's
 // entry range in Ft; lvl_warp: one warp per feature in that level), Z (N x zstride doubles) and draws
 // (nfeat x bstride doubles) as workspace; and sample_lambda_beta into lambda_beta[0 .. K), with
-// `parts` (nfeat x bstride doubles) as workspace.
+// `parts` (nfeat x bstride doubles) as workspace.  ordered: a chain whose other mode has a block-CG
+// link, sums in the order of recorded chains.
 void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
                      const int* lvl_feat, const longlong2* lvl_range, const int* lvl_warp,
                      int nlevels, const void* U, bool f32, int ustride,
                      const double* mu, const double* uhat, int hstride, const double* Lambda,
                      const double* lambda_beta, int K, long long N, double* beta, int bstride,
-                     double* Z, int zstride, double* draws, const Ctl* ctl,
+                     double* Z, int zstride, double* draws, bool ordered, const Ctl* ctl,
                      unsigned long long seed, int mode, cudaStream_t s);
 void launch_lambda_beta_one(const double* beta, int bstride, long long nfeat, int K, double a0,
                             double b0, const Ctl* ctl, unsigned long long seed, int mode,
-                            double* parts, double* lambda_beta, cudaStream_t s);
+                            bool ordered, double* parts, double* lambda_beta, cudaStream_t s);
 // Level tables of the link sampler for a side matrix of N rows from each feature's level and the column
 // pointers: features in level order, the bounds of the (possibly split) levels and lvl_warp.
-void beta_one_levels(long long N, const std::vector<int>& level, const std::vector<long long>& ptr,
-                     std::vector<int>& lvl_ptr, std::vector<int>& order,
-                     std::vector<int>& lvl_warp);
+void beta_one_levels(long long N, bool ordered, const std::vector<int>& level,
+                     const std::vector<long long>& ptr, std::vector<int>& lvl_ptr,
+                     std::vector<int>& order, std::vector<int>& lvl_warp);
 
 // sample_beta pieces (latentprior.cpp:273-293)
 //   tmp[n] = U[n] + chol(Lambda)^{-T} z_n - mu      (n < N; z keyed (kMvnN, n))

@@ -591,7 +591,7 @@ void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStre
   } else {
     // K <= 32: Grams on the FP64 matrix instruction, except in a chain with a block-CG link, whose rows
     // keep the order of summation of k_sample (hyper_ordered.cu says why)
-    if (KP <= 32 && (p.one || !p.ordered)) return launch_sample_f64(p, KP, s, num_sms, groups);
+    if (KP <= 32 && !p.ordered) return launch_sample_f64(p, KP, s, num_sms, groups);
     switch (KP) {
       case 8:
         if (groups == 2) return launch_t<8, 1, 2, false>(p, s, num_sms);

@@ -159,6 +159,9 @@ constexpr int kZsMax = 26 * 1024;
 constexpr int kSmemThreads = 512;
 constexpr int kNp = 6;  // entries held ahead per thread
 constexpr int kSmemWarps = kSmemThreads / 32;
+// A chain whose other mode has a block-CG link (hyper_ordered.cu): each feature's sum as it was
+// recorded, a block's over 1,024 threads and its warps' sums added one after the other.
+constexpr int kOrderedThreads = 1024;
 
 // A level: features f0 .. f1 - 1 of the level order, a warp each or the block for each in turn.
 struct LevelPre {
@@ -277,8 +280,8 @@ __device__ __forceinline__ double warp_sum(double x) {
   return x;
 }
 
-template <typename T, bool BINARY>
-__global__ void __launch_bounds__(kSmemThreads)
+template <typename T, bool BINARY, int THREADS, int NP>
+__global__ void __launch_bounds__(THREADS)
     k_beta_one_smem(const int* __restrict__ tidx, const double* __restrict__ tval,
                     const double* __restrict__ colsq, const int* __restrict__ lvl_ptr,
                     const int* __restrict__ lvl_feat, const longlong2* __restrict__ lvl_range,
@@ -290,17 +293,17 @@ __global__ void __launch_bounds__(kSmemThreads)
                     const double* __restrict__ draws) {
   extern __shared__ double Zs[];
   __shared__ double red[2][32];
-  constexpr int NP = kNp;
+  constexpr int WARPS = THREADS / 32;
   const int d = blockIdx.x, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const BetaOne p{tidx, tval, colsq, lvl_ptr, lvl_feat, lvl_range, lvl_warp, draws, beta, bstride,
                   nlevels, Lambda[(size_t)d * (K + 1)], lambda_beta[d], d};
-  for (int i = tid; i < N; i += kSmemThreads)
+  for (int i = tid; i < N; i += THREADS)
     Zs[i] = (double)U[(size_t)i * ustride + d] - mu[d] - uhat[(size_t)i * hstride + d];
   // this thread's first feature of a level, and its share of the entries
   auto first_id = [&](const LevelPre& l) { return fetch_id(p, l.warp ? l.f0 + warp : l.f0, l.f1); };
   auto share = [&](const LevelPre& l, const FeatureId& id) {
-    return fetch_feature<BINARY, NP>(p, id, l.warp ? lane : tid, l.warp ? 32 : kSmemThreads);
+    return fetch_feature<BINARY, NP>(p, id, l.warp ? lane : tid, l.warp ? 32 : THREADS);
   };
   // rings by level: bounds, ids and features; the loop runs four levels at a time so that every
   // ring index is a constant (a register that a load is still to fill is never moved)
@@ -321,9 +324,9 @@ __global__ void __launch_bounds__(kSmemThreads)
       FeaturePre<BINARY, NP> cur = pre[u & 1];
       if (l.warp) {
         // one feature per warp
-        for (int q = l.f0 + warp; q < l.f1; q += kSmemWarps) {
+        for (int q = l.f0 + warp; q < l.f1; q += WARPS) {
           FeaturePre<BINARY, NP> next{};
-          if (q + kSmemWarps < l.f1) next = share(l, fetch_id(p, q + kSmemWarps, l.f1));
+          if (q + WARPS < l.f1) next = share(l, fetch_id(p, q + WARPS, l.f1));
           const double bn = new_coef(p, cur, warp_sum(feature_dot(p, cur, Zs, lane, 32)));
           if (lane == 0) beta[(size_t)cur.f * bstride + d] = bn;
           feature_add(p, cur, Zs, lane, 32, cur.b - bn);
@@ -334,14 +337,20 @@ __global__ void __launch_bounds__(kSmemThreads)
         for (int q = l.f0; q < l.f1; q++) {
           FeaturePre<BINARY, NP> next{};
           if (q + 1 < l.f1) next = share(l, fetch_id(p, q + 1, l.f1));
-          const double part = warp_sum(feature_dot(p, cur, Zs, tid, kSmemThreads));
+          const double part = warp_sum(feature_dot(p, cur, Zs, tid, THREADS));
           if (lane == 0) red[buf][warp] = part;
           __syncthreads();
-          const double bn =
-              new_coef(p, cur, warp_sum(lane < kSmemWarps ? red[buf][lane] : 0.0));
+          double sum;
+          if constexpr (THREADS == kOrderedThreads) {
+            sum = 0.0;
+            for (int w = 0; w < WARPS; w++) sum += red[buf][w];
+          } else {
+            sum = warp_sum(lane < WARPS ? red[buf][lane] : 0.0);
+          }
+          const double bn = new_coef(p, cur, sum);
           buf ^= 1;  // the next sum goes to the other half: one barrier between writes and reads
           if (tid == 0) beta[(size_t)cur.f * bstride + d] = bn;
-          feature_add(p, cur, Zs, tid, kSmemThreads, cur.b - bn);
+          feature_add(p, cur, Zs, tid, THREADS, cur.b - bn);
           cur = next;
         }
       }
@@ -410,7 +419,29 @@ __global__ void k_lambda_beta_one(const double* __restrict__ parts, int nparts, 
                    (1.0 / (b0 + s / 2.0));
 }
 
-template <typename T, bool BINARY>
+// The same with the squares summed as recorded chains with a block-CG link had them: a warp per
+// dimension, a lane's features in order, then a shuffle tree.
+__global__ void __launch_bounds__(256)
+    k_lambda_beta_ordered(const double* __restrict__ beta, int bstride, long long nfeat, int K,
+                          double a0, double b0, const Ctl* ctl, unsigned long long seed, int mode,
+                          double* __restrict__ lambda_beta) {
+  const int lane = threadIdx.x & 31;
+  for (int d = threadIdx.x >> 5; d < K; d += blockDim.x >> 5) {
+    double s = 0.0;
+#pragma unroll 4
+    for (long long f = lane; f < nfeat; f += 32) {
+      const double b = beta[f * bstride + d];
+      s = fma(b, b, s);
+    }
+    s = warp_sum(s);
+    if (lane == 0)
+      lambda_beta[d] = gamma_draw(seed, ctl->sweep, stream_id(kLambdaBeta, (uint32_t)mode),
+                                  (uint32_t)d, a0 + (double)nfeat / 2.0) *
+                       (1.0 / (b0 + s / 2.0));
+  }
+}
+
+template <typename T, bool BINARY, int THREADS, int NP>
 void beta_smem(const DevCsr& Ft, const double* colsq, const int* lvl_ptr, const int* lvl_feat,
                const longlong2* lvl_range, const int* lvl_warp, int nlevels, const void* U,
                int ustride, const double* mu, const double* uhat, int hstride,
@@ -420,12 +451,12 @@ void beta_smem(const DevCsr& Ft, const double* colsq, const int* lvl_ptr, const 
   int dev = 0;
   MG_CUDA(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    MG_CUDA(cudaFuncSetAttribute(k_beta_one_smem<T, BINARY>,
+    MG_CUDA(cudaFuncSetAttribute(k_beta_one_smem<T, BINARY, THREADS, NP>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(double) * kZsMax)));
     configured[dev & 63] = true;
   }
-  k_beta_one_smem<T, BINARY><<<K, kSmemThreads, sizeof(double) * (size_t)N, s>>>(
+  k_beta_one_smem<T, BINARY, THREADS, NP><<<K, THREADS, sizeof(double) * (size_t)N, s>>>(
       Ft.idx, Ft.val, colsq, lvl_ptr, lvl_feat, lvl_range, lvl_warp, nlevels, (const T*)U, ustride,
       mu, uhat, hstride, Lambda, lambda_beta, K, (int)N, beta, bstride, draws);
   MG_CUDA(cudaGetLastError());
@@ -438,15 +469,21 @@ void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
                      int nlevels, const void* U, bool f32, int ustride,
                      const double* mu, const double* uhat, int hstride, const double* Lambda,
                      const double* lambda_beta, int K, long long N, double* beta, int bstride,
-                     double* Z, int zstride, double* draws, const Ctl* ctl,
+                     double* Z, int zstride, double* draws, bool ordered, const Ctl* ctl,
                      unsigned long long seed, int mode, cudaStream_t s) {
   const long long work = Ft.nrow * ((K + 1) / 2);
   k_beta_draws<<<(int)std::min<long long>(4736, (work + 255) / 256), 256, 0, s>>>(
       Ft.nrow, K, bstride, ctl, seed, mode, draws);
   MG_CUDA(cudaGetLastError());
   if (N <= kZsMax) {  // one block per dimension, Z's column in shared memory
-    const auto run = f32 ? (Ft.val ? beta_smem<float, false> : beta_smem<float, true>)
-                         : (Ft.val ? beta_smem<double, false> : beta_smem<double, true>);
+    const auto pick = [&](auto u) {
+      using T = decltype(u);
+      if (ordered)
+        return Ft.val ? beta_smem<T, false, kOrderedThreads, 1>
+                      : beta_smem<T, true, kOrderedThreads, 1>;
+      return Ft.val ? beta_smem<T, false, kSmemThreads, kNp> : beta_smem<T, true, kSmemThreads, kNp>;
+    };
+    const auto run = f32 ? pick(0.f) : pick(0.0);
     run(Ft, colsq, lvl_ptr, lvl_feat, lvl_range, lvl_warp, nlevels, U, ustride, mu, uhat, hstride,
         Lambda, lambda_beta, K, N, beta, bstride, draws, s);
     return;
@@ -465,11 +502,13 @@ void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
 
 // Orders the features by level and splits each level into at most two: the long features, each taken by
 // the whole block in turn, and the others, a warp each.  The features of a level touch
-// disjoint rows, so any order and grouping of them gives the same sums.  With Z in shared memory
-// the split minimises the estimate: 700 cycles per feature of the block (two shuffle trees and a
-// barrier), 600 per 32 features of the warps plus 60 for every 32 entries of the longest one beyond
-// the first 128.  k_beta_one gives a level to the warps unless it has few features and a long one.
-void beta_one_levels(long long N, const std::vector<int>& level, const std::vector<long long>& ptr,
+// disjoint rows, so their order does not matter; who takes a feature decides the order in which its
+// entries are added.  With Z in shared memory the split minimises the estimate: 700 cycles per
+// feature of the block (two shuffle trees and a barrier), 600 per 32 features of the warps plus 60
+// for every 32 entries of the longest one beyond the first 128.  k_beta_one, and every chain with a
+// block-CG link (`ordered`), gives a level to the warps unless it has few features and a long one.
+void beta_one_levels(long long N, bool ordered, const std::vector<int>& level,
+                     const std::vector<long long>& ptr,
                      std::vector<int>& lvl_ptr, std::vector<int>& order,
                      std::vector<int>& lvl_warp) {
   const int nfeat = (int)level.size();
@@ -486,7 +525,7 @@ void beta_one_levels(long long N, const std::vector<int>& level, const std::vect
     while (e < nfeat && level[order[e]] == level[order[s]]) e++;
     const long long n = e - s, longest = len(order[s]);
     int cut = s;  // features s .. cut - 1 by the block
-    if (N > kZsMax) {
+    if (ordered || N > kZsMax) {
       if (n < 8 && longest > 1024) cut = e;
     } else {
       long long best = -1;
@@ -514,7 +553,13 @@ void beta_one_levels(long long N, const std::vector<int>& level, const std::vect
 
 void launch_lambda_beta_one(const double* beta, int bstride, long long nfeat, int K, double a0,
                             double b0, const Ctl* ctl, unsigned long long seed, int mode,
-                            double* parts, double* lambda_beta, cudaStream_t s) {
+                            bool ordered, double* parts, double* lambda_beta, cudaStream_t s) {
+  if (ordered) {
+    k_lambda_beta_ordered<<<1, 256, 0, s>>>(beta, bstride, nfeat, K, a0, b0, ctl, seed, mode,
+                                            lambda_beta);
+    MG_CUDA(cudaGetLastError());
+    return;
+  }
   // `parts` holds nfeat * bstride doubles: at most one record of K per 64 features is written
   const int nb = (int)std::min<long long>(148, (nfeat + 63) / 64);
   k_beta_sq<<<nb, kSqThreads, 0, s>>>(beta, bstride, nfeat, K, (nfeat + nb - 1) / nb, parts);

@@ -114,7 +114,7 @@ def batch():
 
 
 CHAINS = [(K, mixed, kind, weighted) for K in (1, 7, 8, 16, 31, 32, 33, 40, 64) for mixed in (0, 1)
-          for kind in ("one", "both") for weighted in (0, 1)]
+          for kind in ("one", "both", "univariate") for weighted in (0, 1)]
 SOLVES = [(n, mixed, weighted) for n in (1, 8, 9, 16, 17, 32, 33, 64) for mixed in (0, 1)
           for weighted in (0, 1)]
 
