@@ -33,9 +33,12 @@ namespace mg {
 namespace {
 
 // FP32 tiles 72 floats apart: threads that hold the same element of neighbouring tiles then touch
-// different banks.
+// different banks.  The FP64 redo's are packed.
 constexpr int kTile = 72;
-__device__ __forceinline__ int ftile(int bi, int bj) { return (bi * (bi + 1) / 2 + bj) * kTile; }
+template <typename F>
+constexpr int kLd = sizeof(F) == 4 ? kTile : 64;
+template <typename F = float>
+__device__ __forceinline__ int ftile(int bi, int bj) { return (bi * (bi + 1) / 2 + bj) * kLd<F>; }
 
 template <int KP>
 struct Mixed {
@@ -50,8 +53,8 @@ struct Mixed {
   static constexpr int VPR = KP / 8;       // 16-byte vectors per gathered row
   static constexpr int NV = kChunk * VPR / T;
   // group's shared memory in doubles: tiles (FP64 for the redo; the stages before the finish) |
-  // inverses of the redo's diagonal tiles | rhs, y | draws | x | diagonal | flags
-  static constexpr size_t kGroupDoubles = (size_t)(TRI + NB) * 64 + 4 * KP + 2;
+  // rhs, y | draws | x | diagonal | flags
+  static constexpr size_t kGroupDoubles = (size_t)TRI * 64 + 4 * KP + 2;
   static constexpr size_t kCtaDoubles = KP + TRI * kTile / 2;  // Lambda mu | Lambda
   static_assert(2 * kChunk * KP * sizeof(float) <= TRI * 64 * sizeof(double), "stages");
   static_assert(NTILE <= T - 32 && KP * KP >= 8 * TC * T, "tiles, scratch slot");
@@ -155,97 +158,100 @@ __device__ __forceinline__ void gram_mixed(const SampleParams& p, const RowTask&
 
 // x[c] -= sum_{k < 8 pn} L(i, k) L(8 pn + c, k) of one row per thread: row = row i of its block's first
 // tile; one fused multiply-add per column, in column order.
-__device__ __forceinline__ void update_row(float (&x)[8], const float* row_tile, const float* diag_row,
-                                           int r, int pn) {
+template <typename F>
+__device__ __forceinline__ void update_row(F (&x)[8], const F* row_tile, const F* diag_row, int r,
+                                           int pn) {
   for (int k = 0; k < pn; k++) {
-    float a[8];
-    load_row8(row_tile + k * kTile, r, a);
+    F a[8];
+    load_row8(row_tile + k * kLd<F>, r, a);
 #pragma unroll
     for (int h = 0; h < 2; h++)
 #pragma unroll
       for (int c = 0; c < 8; c++) {
-        const Vec4<float> b = lds4(diag_row + k * kTile + c * 8 + 4 * (h ^ ((c >> 1) & 1)));
+        const Vec4<F> b = lds4(diag_row + k * kLd<F> + c * 8 + 4 * (h ^ ((c >> 1) & 1)));
 #pragma unroll
-        for (int q = 0; q < 4; q++) x[c] = fmaf(-a[4 * h + q], b.v[q], x[c]);
+        for (int q = 0; q < 4; q++) x[c] = mfma(-a[4 * h + q], b.v[q], x[c]);
       }
   }
 }
 
 // x -> x L^{-T}, L the factored diagonal tile.
-__device__ __forceinline__ void solve_row(float (&x)[8], const float* L) {
+template <typename F>
+__device__ __forceinline__ void solve_row(F (&x)[8], const F* L) {
 #pragma unroll
   for (int c = 0; c < 8; c++) {
-    float l[8];
+    F l[8];
     load_row8(L, c, l);
 #pragma unroll
-    for (int k = 0; k < c; k++) x[c] = fmaf(-x[k], l[k], x[c]);
+    for (int k = 0; k < c; k++) x[c] = mfma(-x[k], l[k], x[c]);
     x[c] = x[c] / l[c];
   }
 }
 
 // Factorises MM (nb blocks) in place, y along with it; df: MM's diagonal.  A pivot that is not
-// positive, or not above 2^-20 of its original diagonal, fails the group.
+// positive, or in FP32 not above 2^-20 of its original diagonal, fails the group.
 //   Per panel: warp 0 subtracts the last panel's product from the diagonal tile and factors it; a
 // thread per row below subtracts all earlier panels' products, and the last warp those of the next
 // diagonal tile; barrier; the rows below are solved in their threads' registers; barrier.
-template <int T>
-__device__ __forceinline__ bool factor_mixed(float* M, float* y, const float* df, int nb, int tid,
-                                             int grp, volatile int* bad) {
+template <int T, typename F>
+__device__ __forceinline__ bool factor_mixed(F* M, F* y, const float* df, int nb, int tid, int grp,
+                                             volatile int* bad) {
   constexpr int W = T / 32;
   const int warp = tid >> 5, lane = tid & 31, r = tid & 7;
   for (int pn = 0; pn < nb; pn++) {
-    float* D = M + ftile(pn, pn);
+    F* D = M + ftile<F>(pn, pn);
     // row of the panel: warp 0 the panel's own, the others those below
     const int j = warp == 0 ? 8 * pn + r : 8 * pn + 8 + tid - 32;
     const bool below = warp > 0 && j < 8 * nb;
-    float* tile = M + ftile(below ? j >> 3 : pn, 0);  // the row's block
-    float s = 0.f, x[8];
+    F* tile = M + ftile<F>(below ? j >> 3 : pn, 0);  // the row's block
+    F s = (F)0, x[8];
     if (pn > 0 && (warp == 0 || below)) {  // y by the panel before
-      float v[8];
-      load_row8(tile + (pn - 1) * kTile, r, v);
+      F v[8];
+      load_row8(tile + (pn - 1) * kLd<F>, r, v);
       s = y[j];
 #pragma unroll
-      for (int c = 0; c < 8; c++) s = fmaf(-v[c], y[8 * pn - 8 + c], s);
+      for (int c = 0; c < 8; c++) s = mfma(-v[c], y[8 * pn - 8 + c], s);
     }
     if (warp == 0) {
       if (pn > 0) {
-        update_tile(D, M + ftile(pn, 0), M + ftile(pn, 0), pn - 1, pn, kTile, lane);
+        update_tile(D, M + ftile<F>(pn, 0), M + ftile<F>(pn, 0), pn - 1, pn, kLd<F>, lane);
         if (lane < 8) y[j] = s;
       }
       __syncwarp();
       // lanes 0-7: the tile's rows, 8: y (the others repeat it)
-      float* own = lane < 8 ? D : y + 8 * pn;
+      F* own = lane < 8 ? D : y + 8 * pn;
       const int at = lane < 8 ? r : 0;
       load_row8(own, at, x);
       __syncwarp();
       bool ok = true;
 #pragma unroll
       for (int c = 0; c < 8; c++) {
-        const float d = wshfl(x[c], c);
-        ok = ok & (d > 0.f) & (d > 0x1p-20f * df[8 * pn + c]);
-        const float l = sqrtf(d), q = (lane > c ? x[c] : d) / l;  // above the diagonal: anything
+        const F d = wshfl(x[c], c);
+        ok = ok & (d > (F)0);
+        if constexpr (sizeof(F) == 4) ok = ok & (d > 0x1p-20f * df[8 * pn + c]);
+        const F l = msqrt(d), q = (lane > c ? x[c] : d) / l;  // above the diagonal: anything
         x[c] = lane == c ? l : q;
 #pragma unroll
-        for (int k = c + 1; k < 8; k++) x[k] = fmaf(-x[c], wshfl(x[c], k), x[k]);
+        for (int k = c + 1; k < 8; k++) x[k] = mfma(-x[c], wshfl(x[c], k), x[k]);
       }
       if (lane <= 8) store_row8(own, at, x);
       if (!ok && lane == 0) *bad = 1;
     } else {
       if (below) {
         if (pn > 0) y[j] = s;
-        load_row8(tile + pn * kTile, r, x);
-        update_row(x, tile, M + ftile(pn, 0), r, pn);
+        load_row8(tile + pn * kLd<F>, r, x);
+        update_row(x, tile, M + ftile<F>(pn, 0), r, pn);
       }
       if (warp == W - 1 && pn > 0 && pn + 1 < nb) {
-        const float* next = M + ftile(pn + 1, 0);
-        update_tile(M + ftile(pn + 1, pn + 1), next, next, 0, pn, kTile, lane);
+        const F* next = M + ftile<F>(pn + 1, 0);
+        update_tile(M + ftile<F>(pn + 1, pn + 1), next, next, 0, pn, kLd<F>, lane);
       }
     }
     group_sync<T>(grp);
     if (*bad) return false;
     if (below) {
       solve_row(x, D);
-      store_row8(tile + pn * kTile, r, x);
+      store_row8(tile + pn * kLd<F>, r, x);
     }
     group_sync<T>(grp);
   }
@@ -253,16 +259,15 @@ __device__ __forceinline__ bool factor_mixed(float* M, float* y, const float* df
 }
 
 // x = L^{-T} y over the panels from the last (y is overwritten).
-template <int T>
-__device__ __forceinline__ void back_mixed(const float* M, float* y, float* x, int nb, int tid,
-                                           int grp) {
+template <int T, typename F>
+__device__ __forceinline__ void back_mixed(const F* M, F* y, F* x, int nb, int tid, int grp) {
   const int warp = tid >> 5, r = tid & 7;
   for (int pn = nb - 1; pn >= 0; pn--) {
     if (warp == 0 || 32 * warp < 8 * pn) {
-      const float* D = M + ftile(pn, pn);
+      const F* D = M + ftile<F>(pn, pn);
       const bool on = tid < 8 * pn;
-      const float* P = M + ftile(pn, on ? tid >> 3 : 0);
-      float d[8], l[8], p[8], b = y[8 * pn + r], s = on ? y[tid] : 0.f;
+      const F* P = M + ftile<F>(pn, on ? tid >> 3 : 0);
+      F d[8], l[8], p[8], b = y[8 * pn + r], s = on ? y[tid] : (F)0;
 #pragma unroll
       for (int c = 0; c < 8; c++) {
         d[c] = D[tile_pos(c, r)];
@@ -271,10 +276,10 @@ __device__ __forceinline__ void back_mixed(const float* M, float* y, float* x, i
       }
 #pragma unroll
       for (int c = 7; c >= 0; c--) {
-        const float xc = wshfl(b, c) / l[c];
-        if (r < c) b = fmaf(-d[c], xc, b);
+        const F xc = wshfl(b, c) / l[c];
+        if (r < c) b = mfma(-d[c], xc, b);
         if (r == c) b = xc;
-        s = fmaf(-p[c], xc, s);
+        s = mfma(-p[c], xc, s);
       }
       if (on) y[tid] = s;
       if (tid < 8) x[8 * pn + tid] = b;
@@ -283,11 +288,16 @@ __device__ __forceinline__ void back_mixed(const float* M, float* y, float* x, i
   }
 }
 
-// The FP64 redo, kept out of line for its registers.
-template <int KP, int T>
-__device__ __noinline__ bool wide_factor_redo(double* M, double* y, double* Di, int nb, int tid,
-                                              int grp, volatile int* bad) {
-  return wide_factor<KP, T>(M, y, Di, nb, tid, grp, bad);
+// The FP64 redo of a row from MM and the right-hand side, in the same order; kept out of line for its
+// registers.
+template <int T>
+__device__ __noinline__ bool redo_solve(double* M, double* y, const double* z, double* x, int nb,
+                                        int tid, int grp, volatile int* bad) {
+  if (!factor_mixed<T>(M, y, nullptr, nb, tid, grp, bad)) return false;
+  if (tid < 8 * nb) y[tid] += z[tid];
+  group_sync<T>(grp);
+  back_mixed<T>(M, y, x, nb, tid, grp);
+  return true;
 }
 
 template <int KP, int G>
@@ -302,8 +312,7 @@ __global__ void __launch_bounds__(Mixed<KP>::T* G, (KP == 64 ? 6 : 2) / G)
   const int lane = tid & 31;
   const int vt = (tid + 32 * (grp + 2 * (int)(blockIdx.x / 148))) % T;
   double* M = smem_m + C::kCtaDoubles + (size_t)grp * C::kGroupDoubles;
-  double* Di = M + (size_t)C::TRI * 64;
-  double* rhs_s = Di + (size_t)C::NB * 64;
+  double* rhs_s = M + (size_t)C::TRI * 64;
   double* z_s = rhs_s + KP;
   double* x_s = z_s + KP;
   float* df = reinterpret_cast<float*>(x_s + KP);
@@ -471,10 +480,7 @@ __global__ void __launch_bounds__(Mixed<KP>::T* G, (KP == 64 ? 6 : 2) / G)
         redo = true;
         group_sync<T>(grp);  // every thread has seen the flag
       } else {
-        if (wide_factor_redo<KP, T>(M, rhs_s, Di, nb, tid, grp, bad)) {
-          if (tid < 8 * nb) rhs_s[tid] += z_s[tid];
-          group_sync<T>(grp);
-          wide_back<KP, T>(M, rhs_s, Di, x_s, nb, tid, grp);
+        if (redo_solve<T>(M, rhs_s, z_s, x_s, nb, tid, grp, bad)) {
           if (tid < K) {
             p.out_f32[(size_t)row * KP + tid] = (float)x_s[tid];
             store_copy(p, (size_t)row * KP + tid, (float)x_s[tid]);

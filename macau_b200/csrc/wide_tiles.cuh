@@ -110,26 +110,28 @@ __device__ __forceinline__ void update_tile(double* M, int bi, int bj, int k0, i
   }
   *c = make_double2(v.x + w.x, v.y + w.y);
 }
-// FP32 (c -= sum over tiles A + k stride, B + k stride): one fused multiply-add per column, in column
-// order.
-__device__ __forceinline__ void update_tile(float* tile, const float* A, const float* B, int k0,
-                                            int k1, int stride, int lane) {
+// Scalar form (c -= sum over tiles A + k stride, B + k stride): one fused multiply-add per column, in
+// column order.
+template <typename F>
+__device__ __forceinline__ void update_tile(F* tile, const F* A, const F* B, int k0, int k1,
+                                            int stride, int lane) {
   const int g = lane >> 2, t = lane & 3;
-  float2* c = reinterpret_cast<float2*>(tile + tile_pos(g, 2 * t));
-  float2 v = *c;
+  F* c = tile + tile_pos(g, 2 * t);
+  F v0 = c[0], v1 = c[1];
 #pragma unroll 2
   for (int k = k0; k < k1; k++) {
-    float a[8], b0[8], b1[8];
+    F a[8], b0[8], b1[8];
     load_row8(A + stride * k, g, a);
     load_row8(B + stride * k, 2 * t, b0);
     load_row8(B + stride * k, 2 * t + 1, b1);
 #pragma unroll
     for (int q = 0; q < 8; q++) {
-      v.x = fmaf(-a[q], b0[q], v.x);
-      v.y = fmaf(-a[q], b1[q], v.y);
+      v0 = mfma(-a[q], b0[q], v0);
+      v1 = mfma(-a[q], b1[q], v1);
     }
   }
-  *c = v;
+  c[0] = v0;
+  c[1] = v1;
 }
 
 // Factor of a diagonal tile by one warp: lanes 0-7 hold its rows (x[j], j <= lane, in; the factor's

@@ -1,8 +1,9 @@
-"""Chains with a block-CG link, block-CG solves and batches against recorded ones, bit for bit.
+"""Chains with a block-CG link, block-CG solves, batches and wide mixed rows against recorded ones, bit
+for bit.
 
 A link solve ends at a tolerance, so one rounding in what reaches it moves the link matrix by 1e-7 to
-1e-6, and a batch's mixed chains part after a rounding that falls the other way: these paths keep one
-order of summation (macau_b200/csrc/hyper_ordered.cu).  golden/recorded_chains.json holds digests of
+1e-6, and a batch's mixed chains and mixed rows at K > 32 part after a rounding that falls the other
+way: these paths keep one order of summation (macau_b200/csrc/hyper_ordered.cu, sample_wide_mixed.cu).  golden/recorded_chains.json holds digests of
 their outputs, recorded on a B200 with the scalar kernels that the matrix-instruction and pipelined
 ones replaced; a change of the order, of the matrix instruction's rounding or of its place in a row
 shows as another digest, whatever its size.
@@ -113,6 +114,26 @@ def batch():
     return out
 
 
+def wide_rows(K):
+    """Mixed rows of every length up to 700, those shorter than K redone in FP64: Lambda = 1e-7 I, so
+    that their FP32 pivots are rounding alone."""
+    lengths = (0, 1, 3, 4, 5, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 129, 255, 256, 257, 700)
+    rng = np.random.default_rng(K)
+    r = np.repeat(np.arange(len(lengths), dtype=np.int32), lengths)
+    c = np.concatenate([rng.permutation(720)[:n] for n in lengths]).astype(np.int32)
+    s = _lib.Sampler(K, 1.5, seed=2, compute=_lib.MG_COMPUTE_MIXED)
+    s.set_relation_data(r, c, rng.normal(size=len(r)), (len(lengths), 720))
+    s.set_samples(0, 1)
+    s.init()
+    s.set_option("split_threshold", 256)  # rows of 257 and 700 entries in parts
+    s.set_latents(1, rng.integers(-4, 5, size=(720, K)) / 4.0)
+    s.set_hyper(0, np.zeros(K), 1e-7 * np.eye(K))
+    s.sample_latents(0, 4)
+    out = {"rows": digest(s.latents(0)), "redone": s.stats()["retries"][0]}
+    s.close()
+    return out
+
+
 CHAINS = [(K, mixed, kind, weighted) for K in (1, 7, 8, 16, 31, 32, 33, 40, 64) for mixed in (0, 1)
           for kind in ("one", "both", "univariate") for weighted in (0, 1)]
 SOLVES = [(n, mixed, weighted) for n in (1, 8, 9, 16, 17, 32, 33, 64) for mixed in (0, 1)
@@ -131,6 +152,11 @@ def test_solve(n, mixed, weighted):
 @pytest.mark.parametrize("K,mixed,kind,weighted", CHAINS)
 def test_chain(K, mixed, kind, weighted):
     assert chain(K, mixed, kind, weighted) == recorded("chain %d %d %s %d" % (K, mixed, kind, weighted))
+
+
+@pytest.mark.parametrize("K", [33, 48, 64, 65, 100, 128])
+def test_wide_rows(K):
+    assert wide_rows(K) == recorded("rows %d" % K)
 
 
 def test_batch():
