@@ -157,7 +157,10 @@ __global__ void __launch_bounds__(kBetaThreads)
 // levels, 5,003 rows, 250,000 entries: 1.29 -> 1.10 ms.
 constexpr int kZsMax = 26 * 1024;
 constexpr int kSmemThreads = 512;
-constexpr int kNp = 6;  // entries held ahead per thread
+// entries held ahead per thread: with weights more than one leave no registers for the rings (six
+// spilled 260 bytes in the level chain: 1,506 us a link draw of 5,003 rows and 8,193 features at 32
+// components for 1,061; 1,436 us with the kernel of 1,024 threads and one feature ahead)
+constexpr int kNp = 6, kNpWeighted = 1;
 constexpr int kSmemWarps = kSmemThreads / 32;
 // A chain whose other mode has a block-CG link (hyper_ordered.cu): each feature's sum as it was
 // recorded, a block's over 1,024 threads and its warps' sums added one after the other.
@@ -481,7 +484,8 @@ void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
       if (ordered)
         return Ft.val ? beta_smem<T, false, kOrderedThreads, 1>
                       : beta_smem<T, true, kOrderedThreads, 1>;
-      return Ft.val ? beta_smem<T, false, kSmemThreads, kNp> : beta_smem<T, true, kSmemThreads, kNp>;
+      return Ft.val ? beta_smem<T, false, kSmemThreads, kNpWeighted>
+                    : beta_smem<T, true, kSmemThreads, kNp>;
     };
     const auto run = f32 ? pick(0.f) : pick(0.0);
     run(Ft, colsq, lvl_ptr, lvl_feat, lvl_range, lvl_warp, nlevels, U, ustride, mu, uhat, hstride,
