@@ -182,7 +182,7 @@ void launch_spmm(const DevCsr& A, const void* src, int src_stride, void* dst, in
 
 // Univariate prior (univariate_kernels.cu): MacauOnePrior::sample_beta over Ft (the columns of
 // F as CSR rows) with the feature levels lvl_ptr / lvl_feat (lvl_range: each listed feature's
-// entry range in Ft; lvl_warp: one warp per feature in that level), Z (N x zstride doubles) and draws
+// entry range in Ft; lvl_warp: who takes that level's features), Z (N x zstride doubles) and draws
 // (nfeat x bstride doubles) as workspace; and sample_lambda_beta into lambda_beta[0 .. K), with
 // `parts` (nfeat x bstride doubles) as workspace.  ordered: a chain whose other mode has a block-CG
 // link, sums in the order of recorded chains.

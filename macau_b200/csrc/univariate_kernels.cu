@@ -147,28 +147,31 @@ __global__ void __launch_bounds__(kBetaThreads)
 // shared memory (N doubles, N <= kZsMax), so the feature-by-feature chain reads and writes no
 // global memory but beta, with 16 warps per block (with 32 the idle ones' instructions cost more than
 // their share of the work saves, with 8 the long features take longer).
-//   What bounds it: the chain over the levels.  A level gives each of its features to a warp, or each
-// in turn to the whole block (lvl_warp, beta_one_levels).  Nothing that a feature needs is more than
-// one memory latency behind when its level begins: the bounds of a level are loaded three levels
-// ahead, the id and entry range of the feature that a warp takes in it two ahead, its first
-// entries' rows, coefficient, draw and squared norm one ahead.  The
-// block's sum takes one barrier: every warp adds the warps' sums for itself by a shuffle tree.
-// 32,768 features, 20,000 rows, 1M entries, 32 dimensions: 6.0 -> 3.0 ms; 8,193 features in 615
-// levels, 5,003 rows, 250,000 entries: 1.29 -> 1.10 ms.
+//   What bounds it: the chain over the levels, and in wide levels the instructions per feature.  A
+// level gives its features to the block, each in turn, to a warp each or to a lane each (lvl_warp,
+// beta_one_levels).  Nothing that a feature needs is more than one memory latency behind when its
+// level begins: the bounds of a level are loaded three levels ahead, the id and entry range of the
+// feature that a thread takes in it two ahead, its first entries' rows (and values), coefficient, draw
+// and squared norm one ahead.  The block's sum takes one barrier: every warp adds the warps' sums for
+// itself by a shuffle tree.
+//   Microseconds a link draw, with 1,024 threads, one feature ahead and a warp per short feature, then
+// as it is: 5,003 rows, 8,193 features, 250,000 entries, K = 32: 1,354 -> 996 (weighted 1,437 -> 996);
+// 20,000 rows, 32,768 features, 1M entries: 3,554 -> 2,324; 1,000 rows, 30,000 features, K = 8: 1,197
+// -> 393.  Entries held ahead: six made wide levels slower than two (1,718 at the last size before the
+// lanes, 1,500) and spilled 260 bytes with weights.
 constexpr int kZsMax = 26 * 1024;
 constexpr int kSmemThreads = 512;
-// entries held ahead per thread: with weights more than one leave no registers for the rings (six
-// spilled 260 bytes in the level chain: 1,506 us a link draw of 5,003 rows and 8,193 features at 32
-// components for 1,061; 1,436 us with the kernel of 1,024 threads and one feature ahead)
-constexpr int kNp = 6, kNpWeighted = 1;
+constexpr int kNp = 2;  // entries held ahead per thread
 constexpr int kSmemWarps = kSmemThreads / 32;
 // A chain whose other mode has a block-CG link (hyper_ordered.cu): each feature's sum as it was
 // recorded, a block's over 1,024 threads and its warps' sums added one after the other.
 constexpr int kOrderedThreads = 1024;
 
-// A level: features f0 .. f1 - 1 of the level order, a warp each or the block for each in turn.
+// A level: features f0 .. f1 - 1 of the level order, taken by (lvl_warp) the block each in turn, a
+// warp each or a lane each.
+enum { kByBlock = 0, kByWarp = 1, kByLane = 2 };
 struct LevelPre {
-  int f0, f1, warp;
+  int f0, f1, by;
 };
 // The id and entry range of the feature a thread takes (f < 0: none).  These and FeaturePre hold what
 // the loads return and nothing computed from it: an instruction that used a value here would
@@ -204,7 +207,7 @@ struct BetaOne {
 };
 
 __device__ __forceinline__ LevelPre fetch_level(const BetaOne& p, int L) {
-  if (L >= p.nlevels) return {0, 0, 1};
+  if (L >= p.nlevels) return {0, 0, kByWarp};
   return {p.lvl_ptr[L], p.lvl_ptr[L + 1], p.lvl_warp[L]};
 }
 __device__ __forceinline__ FeatureId fetch_id(const BetaOne& p, int q, int end) {
@@ -304,13 +307,16 @@ __global__ void __launch_bounds__(THREADS)
   for (int i = tid; i < N; i += THREADS)
     Zs[i] = (double)U[(size_t)i * ustride + d] - mu[d] - uhat[(size_t)i * hstride + d];
   // this thread's first feature of a level, and its share of the entries
-  auto first_id = [&](const LevelPre& l) { return fetch_id(p, l.warp ? l.f0 + warp : l.f0, l.f1); };
+  auto first_id = [&](const LevelPre& l) {
+    return fetch_id(p, l.f0 + (l.by == kByLane ? tid : l.by == kByWarp ? warp : 0), l.f1);
+  };
   auto share = [&](const LevelPre& l, const FeatureId& id) {
-    return fetch_feature<BINARY, NP>(p, id, l.warp ? lane : tid, l.warp ? 32 : THREADS);
+    return fetch_feature<BINARY, NP>(p, id, l.by == kByLane ? 0 : l.by == kByWarp ? lane : tid,
+                                     l.by == kByLane ? 1 : l.by == kByWarp ? 32 : THREADS);
   };
   // rings by level: bounds, ids and features; the loop runs four levels at a time so that every
   // ring index is a constant (a register that a load is still to fill is never moved)
-  LevelPre lev[4] = {fetch_level(p, 0), fetch_level(p, 1), fetch_level(p, 2), {0, 0, 1}};
+  LevelPre lev[4] = {fetch_level(p, 0), fetch_level(p, 1), fetch_level(p, 2), {0, 0, kByWarp}};
   FeatureId id[2] = {{-1, make_longlong2(0, 0)}, first_id(lev[1])};
   FeaturePre<BINARY, NP> pre[2];
   pre[0] = share(lev[0], first_id(lev[0]));
@@ -325,7 +331,16 @@ __global__ void __launch_bounds__(THREADS)
       id[u & 1] = first_id(lev[(u + 2) & 3]);
       pre[(u + 1) & 1] = share(lev[(u + 1) & 3], id[(u + 1) & 1]);
       FeaturePre<BINARY, NP> cur = pre[u & 1];
-      if (l.warp) {
+      if (l.by == kByLane) {
+        for (int q = l.f0 + tid; q < l.f1; q += THREADS) {
+          FeaturePre<BINARY, NP> next{};
+          if (q + THREADS < l.f1) next = share(l, fetch_id(p, q + THREADS, l.f1));
+          const double bn = new_coef(p, cur, feature_dot(p, cur, Zs, 0, 1));
+          beta[(size_t)cur.f * bstride + d] = bn;
+          feature_add(p, cur, Zs, 0, 1, cur.b - bn);
+          cur = next;
+        }
+      } else if (l.by == kByWarp) {
         // one feature per warp
         for (int q = l.f0 + warp; q < l.f1; q += WARPS) {
           FeaturePre<BINARY, NP> next{};
@@ -484,8 +499,7 @@ void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
       if (ordered)
         return Ft.val ? beta_smem<T, false, kOrderedThreads, 1>
                       : beta_smem<T, true, kOrderedThreads, 1>;
-      return Ft.val ? beta_smem<T, false, kSmemThreads, kNpWeighted>
-                    : beta_smem<T, true, kSmemThreads, kNp>;
+      return Ft.val ? beta_smem<T, false, kSmemThreads, kNp> : beta_smem<T, true, kSmemThreads, kNp>;
     };
     const auto run = f32 ? pick(0.f) : pick(0.0);
     run(Ft, colsq, lvl_ptr, lvl_feat, lvl_range, lvl_warp, nlevels, U, ustride, mu, uhat, hstride,
@@ -504,17 +518,18 @@ void launch_beta_one(const DevCsr& Ft, const double* colsq, const int* lvl_ptr,
   MG_CUDA(cudaGetLastError());
 }
 
-// Orders the features by level and splits each level into at most two: the long features, each taken by
-// the whole block in turn, and the others, a warp each.  The features of a level touch
-// disjoint rows, so their order does not matter; who takes a feature decides the order in which its
-// entries are added.  With Z in shared memory the split minimises the estimate: 700 cycles per
-// feature of the block (two shuffle trees and a barrier), 600 per 32 features of the warps plus 60
-// for every 32 entries of the longest one beyond the first 128.  k_beta_one, and every chain with a
-// block-CG link (`ordered`), gives a level to the warps unless it has few features and a long one.
+// Orders the features by level and splits each level into at most three: the long features, each taken
+// by the whole block in turn, the short ones, a lane each, and the others, a warp each.  The features
+// of a level touch disjoint rows, so their order does not matter; who takes a feature decides the
+// order in which its entries are added.  With Z in shared memory the block's share minimises the
+// estimate: 700 cycles per feature of the block (two shuffle trees and a barrier), 600 per 16
+// features of the warps plus 60 for every 32 entries of the longest one beyond the first 128.  Lanes
+// take the features that have no more entries than a thread holds ahead, where two rounds of the
+// warps or more are saved.  k_beta_one, and every chain with a block-CG link (`ordered`), gives a
+// level to the warps unless it has few features and a long one.
 void beta_one_levels(long long N, bool ordered, const std::vector<int>& level,
-                     const std::vector<long long>& ptr,
-                     std::vector<int>& lvl_ptr, std::vector<int>& order,
-                     std::vector<int>& lvl_warp) {
+                     const std::vector<long long>& ptr, std::vector<int>& lvl_ptr,
+                     std::vector<int>& order, std::vector<int>& lvl_warp) {
   const int nfeat = (int)level.size();
   auto len = [&](int f) { return ptr[f + 1] - ptr[f]; };
   order.resize(nfeat);
@@ -545,11 +560,20 @@ void beta_one_levels(long long N, bool ordered, const std::vector<int>& level,
     }
     if (cut > s) {
       lvl_ptr.push_back(cut);
-      lvl_warp.push_back(0);
+      lvl_warp.push_back(kByBlock);
     }
-    if (e > cut) {
+    // the shortest features of a wide level, whose entries a lane holds ahead
+    int lanes = e;
+    if (!ordered && N <= kZsMax)
+      while (lanes > cut && len(order[lanes - 1]) <= kNp) lanes--;
+    if (e - lanes < 2 * kSmemWarps) lanes = e;
+    if (lanes > cut) {
+      lvl_ptr.push_back(lanes);
+      lvl_warp.push_back(kByWarp);
+    }
+    if (e > lanes) {
       lvl_ptr.push_back(e);
-      lvl_warp.push_back(1);
+      lvl_warp.push_back(kByLane);
     }
     s = e;
   }

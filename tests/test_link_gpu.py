@@ -78,3 +78,23 @@ def test_univariate_levels_of_mixed_lengths(K, binary):
         assert relerr(s.uhat(0), m.uhat(0)) < 1e-9
         assert relerr(s.lambda_beta_univariate(0), m.lambda_beta_one(0)) < 1e-9
     s.close()
+
+
+@pytest.mark.parametrize("nshort", [31, 32, 33, 513, 1400])
+@pytest.mark.parametrize("binary", [True, False])
+def test_univariate_wide_levels(nshort, binary):
+    # features of 0 to 3 entries: a lane each up to two entries, where a level has 32 of them or more
+    rng = np.random.default_rng(nshort + binary)
+    w = small_uniform(seed=2, nrow=700, ncol=150, nobs=9000)
+    lengths = tuple(rng.permutation([0, 1, 2] * nshort)[:nshort]) + (3, 40, 0, 300, 2)
+    s, m = univariate_pair(w, 9, 55, 0, side_of_lengths(rng, 700, lengths, binary))
+    for it in (0, 1):
+        U = rng.normal(scale=0.5, size=(700, 9))
+        s.set_latents(0, U)
+        m.set("latents", 0, U)
+        s.update_prior(0, it)
+        assert m.update_prior(0, it) == 0
+        assert relerr(s.beta(0), m.beta(0)) < 1e-9
+        assert relerr(s.uhat(0), m.uhat(0)) < 1e-9
+        assert relerr(s.lambda_beta_univariate(0), m.lambda_beta_one(0)) < 1e-9
+    s.close()
