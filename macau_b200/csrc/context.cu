@@ -129,6 +129,7 @@ struct ModeData {
   int groups = 0;
   TuneChoice tune;
   int tune_state = 0;  // 0 not tuned, 1 timed here, 2 taken from the cache
+  std::string tune_key;  // that the record was timed or found under
 };
 
 // Work split of a CSR for the side-information SpMMs (k_spmm_split): rows longer than
@@ -490,6 +491,13 @@ class Context {
     t_sample_ = t_prior_ = t_eval_ = 0.0;
     drop_graphs();
     initialised_ = true;
+    for (int m = 0; m < 2; m++) {  // a record of another kernel: the priors have changed since
+      ModeData& md = md_[m];
+      if (md.tune_state == 0 || md.tune_key == tuning_key(m)) continue;
+      md.groups = md.tune_state = 0;
+      build_tasks(m, split_divisor_thr(m, 2));
+      MG_CUDA(cudaStreamSynchronize(s_));
+    }
     if (autotune_) autotune(autotune_ == 1);
   }
 
@@ -558,11 +566,13 @@ class Context {
     launch_sample(sp, KP_, mixed_, gram_, s_, num_sms_, md.groups);
   }
 
-  // Sampler kind of mode m in the autotuner's keys.
-  const char* tune_kind(int m) const {
-    if (uses_tc(m)) return "tc";
-    if (!mixed_) return "fp64";
-    return gram_ == 0 ? "bf16" : gram_ == 1 ? "fp16" : "tf32";
+  // Mode m's key in the autotuner's cache: the kernel that samples it under the chain's priors, and its
+  // rows.
+  std::string tuning_key(int m) const {
+    const bool one = prior_[m].one;
+    const std::string kind =
+        uses_tc(m) ? (one ? "tc-one" : "tc") : sample_kind(KP_, mixed_, gram_, link_chain(), one);
+    return tune_key(kind.c_str(), K_, num_sms_, md_[m].hptr);
   }
 
   // True when mode m's latents are drawn by the tensor-core sampler.
@@ -590,7 +600,7 @@ class Context {
       for (int m = 0; m < 2; m++) {
         ModeData& md = md_[m];
         const bool tc = uses_tc(m);
-        const std::string key = tune_key(tune_kind(m), K_, num_sms_, md.hptr);
+        const std::string key = md.tune_key = tuning_key(m);
         TuneChoice c;
         if (use_cache && TuneCache::get().find(key, &c)) {
           if (md.thr != c.thr || md.groups != c.groups) {
@@ -1361,7 +1371,7 @@ class Context {
     long long thr = split_divisor_thr(m, 2);
     if (autotune_ == 1) {  // a cached choice for this data: build its task lists right away
       TuneChoice c;
-      if (TuneCache::get().find(tune_key(tune_kind(m), K_, num_sms_, md.hptr), &c)) {
+      if (TuneCache::get().find(md.tune_key = tuning_key(m), &c)) {
         thr = c.thr;
         md.groups = c.groups;
         md.tune = c;

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <string>
 #include <vector>
 
 #include "common.cuh"
@@ -35,6 +36,8 @@ void launch_pad(const long long* ptr, const long long* pptr, long long nrows, co
 // default shape).
 void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStream_t s,
                    int num_sms, int groups = 0);
+// The kernel that launch_sample picks, as the autotuner's keys name it.
+std::string sample_kind(int KP, bool mixed, int gram, bool ordered, bool one);
 // Its FP64 form for KP <= 32, a warp per row with the Grams on the FP64 matrix instruction
 // (sample_mma.cu); groups = 2 or 4 (default) warps per CTA.
 void launch_sample_f64(const SampleParams& p, int KP, cudaStream_t s, int num_sms, int groups);

@@ -575,23 +575,37 @@ std::vector<int> sample_group_options(int KP, bool mixed, int gram) {
   return {1};
 }
 
+// Which kernel samples the rows.  K > 32: a group of warps per row and a panel factor; the univariate
+// prior and the FP16 and TF32 Grams, which need the whole Gram or other operands, keep k_sample.  K <=
+// 32 in FP64: a warp per row with the Grams on the FP64 matrix instruction.  FP64 rows of a chain with
+// a block-CG link keep k_sample for its order of summation (hyper_ordered.cu says why; the mixed group
+// sampler keeps that order by itself).
+enum class RowKernel { kSample, kGroup, kMma };
+static RowKernel row_kernel(int KP, bool mixed, int gram, bool ordered, bool one) {
+  if (KP > 32)
+    return !one && (mixed ? gram == kGeBf16 : !ordered) ? RowKernel::kGroup : RowKernel::kSample;
+  return !mixed && !ordered ? RowKernel::kMma : RowKernel::kSample;
+}
+
+std::string sample_kind(int KP, bool mixed, int gram, bool ordered, bool one) {
+  std::string kind = !mixed ? "fp64" : gram == kGeFp16 ? "fp16" : gram == kGeTf32 ? "tf32" : "bf16";
+  const RowKernel k = row_kernel(KP, mixed, gram, ordered, one);
+  if (k != RowKernel::kSample) kind += k == RowKernel::kGroup ? "-group" : "-mma";
+  return one ? kind + "-one" : kind;
+}
+
 void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStream_t s,
                    int num_sms, int groups) {
-  // K > 32: a group of warps per row and a panel factor.  The univariate prior and the FP16 and TF32
-  // Grams, which need the whole Gram or other operands, keep k_sample, and so do FP64 rows of a
-  // chain with a block-CG link, for their order of summation (hyper_ordered.cu says why; the mixed
-  // group sampler keeps that order by itself).
-  if (KP > 32 && !p.one && (mixed ? gram == kGeBf16 : !p.ordered))
+  const RowKernel k = row_kernel(KP, mixed, gram, p.ordered, p.one);
+  if (k == RowKernel::kGroup)
     return mixed ? launch_sample_wide_mixed(p, KP, s, num_sms, groups)
                  : launch_sample_wide(p, KP, s, num_sms, groups);
+  if (k == RowKernel::kMma) return launch_sample_f64(p, KP, s, num_sms, groups);
   if (mixed) {
     if (gram == kGeFp16) return launch_mixed<kGeFp16>(p, KP, groups, s, num_sms);
     if (gram == kGeTf32) return launch_mixed<kGeTf32>(p, KP, groups, s, num_sms);
     return launch_mixed<kGeBf16>(p, KP, groups, s, num_sms);
   } else {
-    // K <= 32: Grams on the FP64 matrix instruction, except in a chain with a block-CG link, whose rows
-    // keep the order of summation of k_sample (hyper_ordered.cu says why)
-    if (KP <= 32 && !p.ordered) return launch_sample_f64(p, KP, s, num_sms, groups);
     switch (KP) {
       case 8:
         if (groups == 2) return launch_t<8, 1, 2, false>(p, s, num_sms);

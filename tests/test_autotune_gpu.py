@@ -169,3 +169,42 @@ def test_batch_autotune_keeps_the_chains():
         assert cached[m]["finish_ctas_per_sm"] == info[m]["finish_ctas_per_sm"]
     for b in (tuned, plain, again):
         b.close()
+
+
+@pytest.mark.parametrize("K", [10, 64])
+def test_choices_belong_to_the_kernel_that_was_timed(K):
+    # FP64 rows: a plain chain, one with a block-CG link and one with the univariate prior take
+    # different kernels on the same ratings
+    rng = np.random.default_rng(K)
+    w = heavy_rows_workload(rng)
+    n = w["shape"][0]
+    side = (np.arange(n, dtype=np.int32), np.arange(n, dtype=np.int32) % 7, None, (n, 7))
+
+    def chain(kind, early=True):
+        s = _lib.Sampler(K, 1.5, seed=3)
+        if early:
+            s.set_option("autotune", 1)
+        s.set_relation_data(w["rows"], w["cols"], w["vals"], w["shape"])
+        if kind == "link":
+            s.set_side(0, *side, 5.0, 1e-6)
+        elif kind == "univariate":
+            s.set_side_univariate(0, *side, 5.0)
+        s.init()
+        return s
+
+    for kind in ("plain", "link", "univariate"):
+        first, again = chain(kind), chain(kind)
+        assert first.tuning()[0]["state"] == "timed", kind
+        assert again.tuning()[0]["state"] == "cached", kind
+        first.close()
+        again.close()
+    # a choice made before the priors were known does not outlive them
+    s = chain("plain", early=False)
+    default = s.tuning()
+    assert all(t["state"] == "cached" for t in s.autotune())
+    s.set_side(0, *side, 5.0, 1e-6)
+    s.init()
+    for t, d in zip(s.tuning(), default):
+        assert t["state"] == "default"
+        assert (t["split_threshold"], t["cta_groups"]) == (d["split_threshold"], d["cta_groups"])
+    s.close()
