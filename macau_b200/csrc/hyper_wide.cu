@@ -161,8 +161,6 @@ void stats_launch(const StatsArgs& a, int K, int stride, int uhat_stride, cudaSt
 struct NwArgs {
   const double* stats;  // `nparts` records of sums (K), then x x^T (K x K), added in order
   int nparts;
-  const double* bb;     // beta beta^T statistics of a Macau prior (one such record), or null
-  const double* lambda_beta;
   const double* mu0;    // null: zero
   const double* T0;     // null: the identity
   double kappa;
@@ -268,7 +266,6 @@ __device__ __forceinline__ void nw_tiles(const NwArgs& p, int K, Ctl* ctl, unsig
   __syncthreads();
   // M = J (T + N S + kappa mu0 mu0^T - kappa_c mu_c mu_c^T) J, a warp per tile; the identity in
   // the first `pad` rows and columns
-  const double lb = p.bb ? *p.lambda_beta : 0.0;
 #pragma unroll 5
   for (int q = warp; q < nb * (nb + 1) / 2; q += kNwThreads / 32) {
     const int a = 8 * (tri[q] >> 4) + g;
@@ -279,8 +276,7 @@ __device__ __forceinline__ void nw_tiles(const NwArgs& p, int K, Ctl* ctl, unsig
       v[e] = a == b ? 1.0 : 0.0;
       if (a >= pad && b >= pad) {
         const size_t at = j + (size_t)i * K;
-        double T = p.T0 ? p.T0[at] : (a == b ? 1.0 : 0.0);
-        if (p.bb) T += lb * p.bb[K + at];
+        const double T = p.T0 ? p.T0[at] : (a == b ? 1.0 : 0.0);
         v[e] = T + stat(K + at) + p.kappa * x[i] * x[j] - kappa_c * muc[i] * muc[j];
       }
     }
@@ -289,7 +285,7 @@ __device__ __forceinline__ void nw_tiles(const NwArgs& p, int K, Ctl* ctl, unsig
   }
   __syncthreads();
   if (warp < 8) {
-    wide_factor<KP, kNwHalf>(M, y, Di, nb, tid, 0, bad);
+    wide_factor<kNwHalf>(M, y, Di, nb, tid, 0, bad);
   } else {
     bartlett(Ct, z, K, n, nu_c, seed, sweep, (uint32_t)p.mode, tid - kNwHalf, kNwHalf);
   }
@@ -342,7 +338,7 @@ __device__ __forceinline__ void nw_tiles(const NwArgs& p, int K, Ctl* ctl, unsig
       y[tid] = z[tid] / sqrt(kappa_c);
     }
     group_sync<kNwHalf>(0);
-    wide_back<KP, kNwHalf>(M, y, Di, x, nb, tid, 0);
+    wide_back<kNwHalf>(M, y, Di, x, nb, tid, 0);
     if (tid < K) p.mu[tid] = x[tid] + muc[tid];
   } else {
     // Lambda = B B^T
@@ -419,12 +415,10 @@ void launch_stats_wide_pair(const PriorPair& pp, bool f32, int K, int stride, cu
 
 void launch_normal_wishart(const double* partials, int nparts, long long N, int K,
                            const double* mu0, double kappa, const double* T0, int nu,
-                           const double* bb, const double* lambda_beta, Ctl* ctl,
-                           unsigned long long seed, int mode, double* mu_out, double* Lambda_out,
-                           cudaStream_t s) {
+                           Ctl* ctl, unsigned long long seed, int mode, double* mu_out,
+                           double* Lambda_out, cudaStream_t s) {
   NwPair a{};
-  a.m[0] = NwArgs{partials, nparts, bb, lambda_beta, mu0, T0, kappa, N, nu, mode, mu_out,
-                  Lambda_out};
+  a.m[0] = NwArgs{partials, nparts, mu0, T0, kappa, N, nu, mode, mu_out, Lambda_out};
   nw_dispatch(a, 1, K, ctl, seed, s);
 }
 
@@ -433,8 +427,7 @@ void launch_normal_wishart_pair(const PriorPair& pp, int K, Ctl* ctl, unsigned l
   NwPair a{};
   for (int m = 0; m < 2; m++) {
     const bool few = few_parts(pp.nblocks[m], K);
-    a.m[m] = NwArgs{few ? pp.partials[m] : pp.final_[m], few ? pp.nblocks[m] : 1, nullptr, nullptr,
-                    pp.mu0[m], pp.T0[m], pp.kappa[m], pp.N[m], pp.nu[m], m, pp.mu[m],
+    a.m[m] = NwArgs{few ? pp.partials[m] : pp.final_[m], few ? pp.nblocks[m] : 1, pp.mu0[m], pp.T0[m], pp.kappa[m], pp.N[m], pp.nu[m], m, pp.mu[m],
                     pp.Lambda[m]};
   }
   nw_dispatch(a, 2, K, ctl, seed, s);

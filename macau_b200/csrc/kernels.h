@@ -89,15 +89,13 @@ void launch_reduce_parts(const double* parts, int nparts, int len, double* out, 
 bool few_parts(int nblocks, int K);
 void launch_stats(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
                   int uhat_stride, double* partials, int nblocks, cudaStream_t s);
-// One Normal-Wishart draw (hyper_wide.cu) from `nparts` statistics records, added in order; bb: one
-// record of beta beta^T (null without side information).
+// One Normal-Wishart draw (hyper_wide.cu) from `nparts` statistics records, added in order.
 void launch_normal_wishart(const double* partials, int nparts, long long N, int K,
                            const double* mu0, double kappa, const double* T0, int nu,
-                           const double* bb, const double* lambda_beta, Ctl* ctl,
-                           unsigned long long seed, int mode, double* mu_out, double* Lambda_out,
-                           cudaStream_t s);
+                           Ctl* ctl, unsigned long long seed, int mode, double* mu_out,
+                           double* Lambda_out, cudaStream_t s);
 // The same two for a chain with a block-CG link (hyper_ordered.cu; K <= 64), in a fixed order of
-// summation; `stats` is one record, `bb` one or null.
+// summation; `stats` is one record, `bb` one of beta beta^T (with lambda_beta) or null.
 void launch_link_stats(const void* U, bool f32, const double* Uhat, long long N, int K, int stride,
                        int uhat_stride, double* partials, int nblocks, cudaStream_t s);
 void launch_link_wishart(const double* stats, long long N, int K, const double* mu0, double kappa,

@@ -146,8 +146,8 @@ extern "C" int mg_normal_wishart_noalloc(const double* U, int64_t N, int K, int 
       launch_reduce_parts(partials, nb, len, stats, s);
       nb = 1;
     }
-    launch_normal_wishart(stats, nb, N, K, mu0, kappa, T, nu, nullptr, nullptr, ctl, seed, mode,
-                          mu_out, Lambda_out, s);
+    launch_normal_wishart(stats, nb, N, K, mu0, kappa, T, nu, ctl, seed, mode, mu_out, Lambda_out,
+                          s);
     int32_t status = 0;
     MG_CUDA(cudaMemcpyAsync(&status, &ctl->status, sizeof(status), cudaMemcpyDeviceToHost, s));
     MG_CUDA(cudaStreamSynchronize(s));

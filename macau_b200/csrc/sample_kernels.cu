@@ -559,7 +559,8 @@ void launch_mixed(const SampleParams& p, int KP, int groups, cudaStream_t s, int
       if constexpr (alt_ok)
         if (groups == 1) return launch_t<64, 4, 1, true, GE>(p, s, num_sms);
       return launch_t<64, 4, 2, true, GE>(p, s, num_sms);
-    case 128: return launch_t<128, 16, 1, true, GE>(p, s, num_sms);
+    case 128:  // BF16: the group sampler
+      if constexpr (GE != kGeBf16) return launch_t<128, 16, 1, true, GE>(p, s, num_sms);
   }
   throw MgError(MG_ERR_ARG, "unsupported latent dimension");
 }
@@ -619,7 +620,6 @@ void launch_sample(const SampleParams& p, int KP, bool mixed, int gram, cudaStre
       case 64:
         if (groups == 1) return launch_t<64, 4, 1, false>(p, s, num_sms);
         return launch_t<64, 4, 2, false>(p, s, num_sms);
-      case 128: return launch_t<128, 16, 1, false>(p, s, num_sms);
     }
   }
   throw MgError(MG_ERR_ARG, "unsupported latent dimension");

@@ -242,18 +242,7 @@ __global__ void __launch_bounds__(32 * G, 16 / G) k_sample_f64(const SampleParam
 #pragma unroll
           for (int b = 0; b < NB; b++) rhs_s[8 * b + g] = racc[b];
         __syncwarp();
-        double lm;
-        if (p.uhat) {  // Macau prior mean mu + Uhat[row]
-          const double mun = lane < K ? p.mu[lane] + p.uhat[(size_t)row * KP + lane] : 0.0;
-          lm = 0.0;
-          for (int j = 0; j < K; j++) {
-            const double mj = wshfl(mun, j);
-            if (lane < K) lm += p.Lambda[lane + j * K] * mj;
-          }
-        } else {
-          lm = lane < KP ? lmu_s[lane] : 0.0;
-        }
-        if (lane < KP) rhs_s[lane] += lm;
+        if (lane < KP) rhs_s[lane] += lmu_s[lane];  // no Uhat: link chains go through k_sample
         __syncwarp();
         if (warp_tiles_solve<NB>(Gs, Gs + C::TILES * 64, rhs_s, (K + 7) / 8, z, lane)) {
           __syncwarp();

@@ -204,10 +204,7 @@ __global__ void __launch_bounds__(Wide<KP>::T* G, (KP == 64 ? 4 : 2) / G)
       double* sp = p.scratch + (size_t)(tk.slot + tk.part) * kSlot;
 #pragma unroll
       for (int q = 0; q < NT; q++)
-#pragma unroll
-        for (int e = 0; e < 2; e += 2)
-          *reinterpret_cast<double2*>(sp + at + q * 64 + e) =
-              make_double2(acc[q][e], acc[q][e + 1]);
+        *reinterpret_cast<double2*>(sp + at + q * 64) = make_double2(acc[q][0], acc[q][1]);
       group_sync<T>(grp);
       if (tid < KP) sp[KP * KP + tid] = rhs_s[tid];
       __threadfence();
@@ -220,19 +217,17 @@ __global__ void __launch_bounds__(Wide<KP>::T* G, (KP == 64 ? 4 : 2) / G)
         __threadfence();
         const double* s0 = p.scratch + (size_t)tk.slot * kSlot;
 #pragma unroll
-        for (int q = 0; q < NT; q++)
-#pragma unroll
-          for (int e = 0; e < 2; e += 2) {
-            double a = 0.0, b = 0.0;
-            for (int part = 0; part < tk.nparts; part++) {
-              const double2 v = __ldcg(reinterpret_cast<const double2*>(
-                  s0 + (size_t)part * kSlot + at + q * 64 + e));
-              a += v.x;
-              b += v.y;
-            }
-            acc[q][e] = a;
-            acc[q][e + 1] = b;
+        for (int q = 0; q < NT; q++) {
+          double a = 0.0, b = 0.0;
+          for (int part = 0; part < tk.nparts; part++) {
+            const double2 v =
+                __ldcg(reinterpret_cast<const double2*>(s0 + (size_t)part * kSlot + at + q * 64));
+            a += v.x;
+            b += v.y;
           }
+          acc[q][0] = a;
+          acc[q][1] = b;
+        }
         if (tid < KP) {
           double r = 0.0;
           for (int part = 0; part < tk.nparts; part++)
@@ -245,7 +240,8 @@ __global__ void __launch_bounds__(Wide<KP>::T* G, (KP == 64 ? 4 : 2) / G)
 
     if (finish) {
       const int row = tk.row;
-      // the row's draws and the right-hand side Lambda (mu + Uhat[row]) + Gram rhs
+      // the row's draws and the right-hand side Lambda mu + Gram rhs (no Uhat: link chains go through
+      // k_sample)
       if (p.znoise) {
         if (tid < KP) z_s[tid] = tid < K ? p.znoise[(size_t)row * K + tid] : 0.0;
       } else if (tid < KP / 2) {
@@ -255,26 +251,17 @@ __global__ void __launch_bounds__(Wide<KP>::T* G, (KP == 64 ? 4 : 2) / G)
         z_s[2 * tid] = 2 * tid < K ? z0 : 0.0;
         z_s[2 * tid + 1] = 2 * tid + 1 < K ? z1 : 0.0;
       }
-      double lm = 0.0;
-      if (p.uhat) {
-        if (tid < K) x_s[tid] = p.mu[tid] + p.uhat[(size_t)row * KP + tid];
-        group_sync<T>(grp);
-        if (tid < K)
-          for (int j = 0; j < K; j++) lm += p.Lambda[tid + (size_t)j * K] * x_s[j];
-      } else {
-        group_sync<T>(grp);
-        if (tid < KP) lm = lmu_s[tid];
-      }
-      const double rr = tid < KP ? rhs_s[tid] + lm : 0.0;
+      group_sync<T>(grp);
+      const double rr = tid < KP ? rhs_s[tid] + lmu_s[tid] : 0.0;
       if (tid == 0) *bad = 0;
       if (part.diag) store64<KP, true>(M, p.Lambda, K, alpha, part.r0, part.c0, acc);
       else store64<KP, false>(M, p.Lambda, K, alpha, part.r0, part.c0, acc);
       if (tid < KP) rhs_s[tid] = rr;
       group_sync<T>(grp);
-      if (wide_factor<KP, T>(M, rhs_s, Di, nb, tid, grp, bad)) {
+      if (wide_factor<T>(M, rhs_s, Di, nb, tid, grp, bad)) {
         if (tid < 8 * nb) rhs_s[tid] += z_s[tid];
         group_sync<T>(grp);
-        wide_back<KP, T>(M, rhs_s, Di, x_s, nb, tid, grp);
+        wide_back<T>(M, rhs_s, Di, x_s, nb, tid, grp);
         if (tid < K) p.out_f64[(size_t)row * KP + tid] = x_s[tid];
       } else if (tid == 0) {
         atomicOr(&p.ctl->status, kStatCholFail);

@@ -302,7 +302,7 @@ __device__ __noinline__ bool redo_solve(double* M, double* y, const double* z, d
 
 template <int KP, int G>
 __global__ void __launch_bounds__(Mixed<KP>::T* G, (KP == 64 ? 6 : 2) / G)
-    k_sample_wide_mixed(const SampleParams p) {
+    k_sample_wide_mixed(const SampleParams p, int num_sms) {
   using C = Mixed<KP>;
   constexpr int T = C::T, TC = C::TC;
   extern __shared__ __align__(16) double smem_m[];
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(Mixed<KP>::T* G, (KP == 64 ? 6 : 2) / G)
   float* lam_s = reinterpret_cast<float*>(smem_m + KP);
   const int grp = threadIdx.x / T, tid = threadIdx.x % T;
   const int lane = tid & 31;
-  const int vt = (tid + 32 * (grp + 2 * (int)(blockIdx.x / 148))) % T;
+  const int vt = (tid + 32 * (grp + 2 * ((int)blockIdx.x / num_sms))) % T;
   double* M = smem_m + C::kCtaDoubles + (size_t)grp * C::kGroupDoubles;
   double* rhs_s = M + (size_t)C::TRI * 64;
   double* z_s = rhs_s + KP;
@@ -514,7 +514,7 @@ void launch_mixed(const SampleParams& p, cudaStream_t s, int num_sms) {
     per_sm = n < 1 ? 1 : n;
   }
   const int need = std::max(1, (p.ntasks + G - 1) / G);
-  kern<<<std::min(num_sms * per_sm, need), C::T * G, smem, s>>>(p);
+  kern<<<std::min(num_sms * per_sm, need), C::T * G, smem, s>>>(p, num_sms);
   MG_CUDA(cudaGetLastError());
 }
 

@@ -40,7 +40,7 @@ __device__ __forceinline__ double beta_coef(int lane, int dc, int d0, int f, dou
 
 // sample_beta (macauoneprior.cpp:216-257) for the dimensions d0 .. d0 + 3 of block blockIdx.x.
 // Z = U - mu - Uhat (N x zstride, this block's four columns) is formed first; then the features
-// are visited level by level.  lvl_feat lists the features sorted by (level, index), where a
+// are visited level by level.  lvl_feat lists the features sorted by level, where a
 // feature's level is one more than the highest level of an earlier feature sharing a row with
 // it, so the features of one level touch disjoint rows of Z and their updates commute: the
 // result equals the reference's feature-by-feature order.  A level marked in lvl_warp (many

@@ -1,6 +1,7 @@
-// Triangular matrices of 33 to 128 rows in shared memory as 8 x 8 tiles, for a group of
-// warps: the panel Cholesky factor with a right-hand side, the backward substitution, and the split
-// of a Gram's lower-triangle tiles over the warps (sample_wide.cu, hyper_wide.cu).
+// Triangular matrices in shared memory as 8 x 8 tiles: the panel Cholesky factor with a right-hand
+// side and the backward substitution, for a group of warps and up to 128 rows (sample_wide.cu,
+// hyper_wide.cu) and for one warp and up to 32 (sample_mma.cu); the tiles' layout and scalar updates
+// (sample_wide_mixed.cu); the split of a wide Gram's lower-triangle tiles over the warps.
 #pragma once
 #include "common.cuh"
 #include "mma_tiles.cuh"
@@ -181,7 +182,7 @@ __device__ __forceinline__ void solve_tile(double* T, const double* Di, int lane
 //   transposed inverse; barrier.  (Every row's owner factoring the diagonal tile for itself,
 //   without the second step, took 2,800 cycles a panel at K = 64 in FP64: 244 FP64 instructions
 //   a thread, in every warp.)
-template <int KP, int T>
+template <int T>
 __device__ __forceinline__ bool wide_factor(double* M, double* y, double* Di, int nb, int tid,
                                             int grp, volatile int* bad) {
   constexpr int W = T / 32;
@@ -242,7 +243,7 @@ __device__ __forceinline__ bool wide_factor(double* M, double* y, double* Di, in
 
 // x = L^{-T} b over the panels from the last, b in y (overwritten), Di the diagonal tiles'
 // transposed inverses; one barrier a panel.  Each warp forms the panel's eight x for itself.
-template <int KP, int T>
+template <int T>
 __device__ __forceinline__ void wide_back(const double* M, double* y, const double* Di, double* x,
                                           int nb, int tid, int grp) {
   const int warp = tid >> 5, r = tid & 7;
