@@ -83,9 +83,10 @@ __device__ __forceinline__ float fused_add(float x, float w, float a) { return f
 // added in CSR order; the indices come 32 at a time by one coalesced load, the next 32 ahead, and U
 // entries' gathers are in flight.  A part stores its FP64 partial row in A.parts; the last part of a row to
 // finish (arrival counter) adds the parts in part order and writes the row.  Whole rows give the
-// same sums as k_spmm.  A weighted entry enters by an explicit fused multiply-add: left to the
-// compiler, this loop's FP64 form rounded the product first, which moved the link matrices of chains
-// with weighted features by up to 1e-6 (hyper_ordered.cu).
+// same sums as k_spmm.  An entry enters by an explicit fused multiply-add, exact where the weight is 1:
+// left to the compiler, this loop's FP64 form rounded a weighted product first, which moved the
+// link matrices of chains with weighted features by up to 1e-6 (hyper_ordered.cu); choosing between
+// that and an addition cost 3 to 6 % of a link update.
 //   What bounds it: for short tasks the latency of index and gather, for the others the gathers
 //   from L2 (256 bytes per entry at 32 components).  U = 16: with 8 a link update of 5,003 x 4,099
 //   at 16 components takes 3.34 ms for 3.06, with 32 one of 20,000 x 32,768 at 32 19.9 ms for 16.7.
@@ -138,8 +139,7 @@ __global__ void __launch_bounds__(256)
             const V w = weighted ? __shfl_sync(0xffffffffu, w_cur, u + i) : (V)1;
             if (off + u + i < tk.len) {
 #pragma unroll
-              for (int c = 0; c < C; c++)
-                acc[c] = weighted ? fused_add(x[i][c], w, acc[c]) : acc[c] + x[i][c];
+              for (int c = 0; c < C; c++) acc[c] = fused_add(x[i][c], w, acc[c]);
             }
           }
         }
