@@ -311,30 +311,34 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---- the draw for 32 < K <= 64 ----
-// Left-looking lower Cholesky of the K x K column-major matrix A (shared memory) by the block,
-// thread i forming L(i, j); the strict upper triangle is zeroed.  False on a pivot that is not
+// Matrices in shared memory, column-major with an odd leading dimension, so that the threads of a warp
+// touch different banks along a row as along a column.
+__host__ __device__ __forceinline__ int odd_ld(int K) { return K | 1; }
+
+// Left-looking lower Cholesky of the K x K matrix A by the block, thread i forming L(i, j); the strict upper triangle is zeroed.  False on a pivot that is not
 // positive (the same value in every thread).
 __device__ bool block_chol(double* A, int K) {
+  const int ld = odd_ld(K);
   __syncthreads();
   for (int j = 0; j < K; j++) {
-    double d = A[j + j * K];
-    for (int p = 0; p < j; p++) d = fma(-A[j + p * K], A[j + p * K], d);
+    double d = A[j + j * ld];
+    for (int p = 0; p < j; p++) d = fma(-A[j + p * ld], A[j + p * ld], d);
     if (!(d > 0.0)) {
       __syncthreads();
       return false;
     }
     const double ljj = sqrt(d);
     for (int i = j + 1 + threadIdx.x; i < K; i += blockDim.x) {
-      double s = A[i + j * K];
-      for (int p = 0; p < j; p++) s = fma(-A[i + p * K], A[j + p * K], s);
-      A[i + j * K] = s / ljj;
+      double s = A[i + j * ld];
+      for (int p = 0; p < j; p++) s = fma(-A[i + p * ld], A[j + p * ld], s);
+      A[i + j * ld] = s / ljj;
     }
     __syncthreads();
-    if (threadIdx.x == 0) A[j + j * K] = ljj;
+    if (threadIdx.x == 0) A[j + j * ld] = ljj;
     __syncthreads();
   }
   for (int q = threadIdx.x; q < K * K; q += blockDim.x)
-    if (q % K < q / K) A[q] = 0.0;
+    if (q % K < q / K) A[q % K + q / K * ld] = 0.0;
   __syncthreads();
   return true;
 }
@@ -352,9 +356,9 @@ __global__ void __launch_bounds__(256)
                         int mode, double* __restrict__ mu_out, double* __restrict__ Lambda_out) {
   extern __shared__ __align__(16) double wsm[];
   __shared__ double muc[64], z[64];
-  const int KK = K * K;
+  const int KK = K * K, ld = odd_ld(K);
   const uint32_t sweep = ctl->sweep;
-  double *X = wsm, *Tc = X + KK, *c = Tc + KK, *W = c + KK;
+  double *X = wsm, *Tc = X + K * ld, *c = Tc + K * ld, *W = c + K * ld;
   const double lb = bb ? *lambda_beta : 0.0;
   const double kappa_c = kappa + (double)N;
   const int nu_c = nu + (int)N;
@@ -363,21 +367,21 @@ __global__ void __launch_bounds__(256)
   for (int e = threadIdx.x; e < KK; e += blockDim.x) {
     const int i = e % K, j = e / K;
     const double T = bb ? fma(lb, bb[K + e], T0[e]) : T0[e];  // latentprior.cpp:258-260
-    X[e] = fma(-(kappa_c * muc[i]), muc[j], fma(kappa * mu0[i], mu0[j], T + stats[K + e]));
+    X[i + j * ld] = fma(-(kappa_c * muc[i]), muc[j], fma(kappa * mu0[i], mu0[j], T + stats[K + e]));
   }
   bool ok = block_chol(X, K);
   if (ok) {
     for (int q = threadIdx.x; q < K; q += blockDim.x) {  // column q of X^{-1}
-      double* x = Tc + q * K;
+      double* x = Tc + q * ld;
       for (int i = 0; i < K; i++) {
         double s = i == q ? 1.0 : 0.0;
-        for (int p = 0; p < i; p++) s = fma(-X[i + p * K], x[p], s);
-        x[i] = s / X[i + i * K];
+        for (int p = 0; p < i; p++) s = fma(-X[i + p * ld], x[p], s);
+        x[i] = s / X[i + i * ld];
       }
       for (int i = K - 1; i >= 0; i--) {
         double s = x[i];
-        for (int p = i + 1; p < K; p++) s = fma(-X[p + i * K], x[p], s);
-        x[i] = s / X[i + i * K];
+        for (int p = i + 1; p < K; p++) s = fma(-X[p + i * ld], x[p], s);
+        x[i] = s / X[i + i * ld];
       }
     }
     ok = block_chol(Tc, K);
@@ -393,26 +397,29 @@ __global__ void __launch_bounds__(256)
       else if (j > i)
         v = normal_draw(seed, sweep, stream_id(kWishartOff, mode), (uint32_t)i,
                         (uint32_t)(j - i - 1));
-      c[e] = v;
+      c[i + j * ld] = v;
     }
     __syncthreads();
     for (int e = threadIdx.x; e < KK; e += blockDim.x) {  // W = c^T c
+      const int i = e % K, j = e / K;
       double s = 0.0;
-      for (int p = 0; p < K; p++) s = fma(c[p + e % K * K], c[p + e / K * K], s);
-      W[e] = s;
+      for (int p = 0; p < K; p++) s = fma(c[p + i * ld], c[p + j * ld], s);
+      W[i + j * ld] = s;
     }
     __syncthreads();
     for (int e = threadIdx.x; e < KK; e += blockDim.x) {  // X = L W
+      const int i = e % K, j = e / K;
       double s = 0.0;
-      for (int p = 0; p < K; p++) s = fma(Tc[e % K + p * K], W[p + e / K * K], s);
-      X[e] = s;
+      for (int p = 0; p < K; p++) s = fma(Tc[i + p * ld], W[p + j * ld], s);
+      X[i + j * ld] = s;
     }
     __syncthreads();
     for (int e = threadIdx.x; e < KK; e += blockDim.x) {  // Lambda = X L^T
+      const int i = e % K, j = e / K;
       double s = 0.0;
-      for (int p = 0; p < K; p++) s = fma(X[e % K + p * K], Tc[e / K + p * K], s);
+      for (int p = 0; p < K; p++) s = fma(X[i + p * ld], Tc[j + p * ld], s);
       Lambda_out[e] = s;
-      c[e] = s * kappa_c;
+      c[i + j * ld] = s * kappa_c;
     }
     ok = block_chol(c, K);
   }
@@ -427,8 +434,8 @@ __global__ void __launch_bounds__(256)
   if (threadIdx.x == 0)
     for (int i = K - 1; i >= 0; i--) {
       double s = z[i];
-      for (int p = i + 1; p < K; p++) s = fma(-c[p + i * K], z[p], s);
-      z[i] = s / c[i + i * K];
+      for (int p = i + 1; p < K; p++) s = fma(-c[p + i * ld], z[p], s);
+      z[i] = s / c[i + i * ld];
     }
   __syncthreads();
   for (int i = threadIdx.x; i < K; i += blockDim.x) mu_out[i] = z[i] + muc[i];
@@ -495,10 +502,10 @@ void launch_link_wishart(const double* stats, long long N, int K, const double* 
     MG_CUDA(cudaGetDevice(&dev));
     if (!configured[dev & 63]) {
       MG_CUDA(cudaFuncSetAttribute(k_link_wishart_wide, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(4 * 64 * 64 * sizeof(double))));
+                                   (int)(4 * 64 * 65 * sizeof(double))));
       configured[dev & 63] = true;
     }
-    k_link_wishart_wide<<<1, 256, 4 * sizeof(double) * K * K, s>>>(
+    k_link_wishart_wide<<<1, 256, 4 * sizeof(double) * K * odd_ld(K), s>>>(
         stats, N, K, mu0, kappa, T0, nu, bb, lambda_beta, ctl, seed, mode, mu_out, Lambda_out);
     MG_CUDA(cudaGetLastError());
     return;
