@@ -474,7 +474,8 @@ int launch_prior_pair(const PriorPair& pp, bool f32, int K, int stride, Ctl* ctl
 
 // Up to 16 partials are added by the Normal-Wishart block itself: one CTA reads them in less time
 // than the reduction's launch takes (2,000 + 1,500 rows, 28 partials in all: a sweep of 47 us lost
-// 3 us); with more, its reads of up to 2.5 MB would cost more than they save.
+// 3 us).  With more its reads cost what the launch does up to about 40 and more beyond (64 partials, a
+// call of mg_normal_wishart_noalloc: 50.8 us and 47.3 reduced first at K = 16, 63.5 and 55.3 at K = 32).
 bool few_parts(int nblocks, int K) { return K <= 32 && nblocks <= 16; }
 
 int stats_blocks(long long N) {  // at most two blocks per SM: fewer partials to reduce

@@ -133,15 +133,16 @@ extern "C" int mg_normal_wishart_noalloc(const double* U, int64_t N, int K, int 
     Ctl* ctl = reinterpret_cast<Ctl*>(base + kPartDoubles);
     int nb = stats_blocks(N);
     if (nb > kNoAllocMaxParts) nb = kNoAllocMaxParts;
-    // K > 32: the draw reads one reduced record, which takes the last partial's place
-    if (K > 32 && nb == kNoAllocMaxParts) nb--;
+    // more partials than the draw adds itself: one reduced record, which takes the last one's place
+    const bool few = few_parts(nb, K);
+    if (!few && nb == kNoAllocMaxParts) nb--;
     // the control block starts every call cleared (status = 0), then gets the sweep index
     MG_CUDA(cudaMemsetAsync(ctl, 0, sizeof(Ctl), s));
     launch_set_sweep(ctl, sweep, 0, s);
     launch_stats(U, false, nullptr, N, K, stride, 0, partials, nb, s);
     const int len = K + K * K;
     double* stats = partials;
-    if (K > 32) {
+    if (!few) {
       stats = partials + (size_t)(kNoAllocMaxParts - 1) * len;
       launch_reduce_parts(partials, nb, len, stats, s);
       nb = 1;
