@@ -696,10 +696,11 @@ __global__ void __launch_bounds__(256)
 
 // The same for NRP = 32 on the FP64 matrix instruction (a chain of fma over k in order, as above): a
 // warp takes 8 rows at a time, M's operands held in registers.
-//   What bounds it: the passes over X, R, P and KP from L2 (8.4 MB each at 32,768 rows).  Through
-//   shared memory, as k_cg_rows, they took 24 and 13 us there.
+//   What bounds it: the passes over X, R, P and KP from L2 (8.4 MB each at 32,768 rows), so two blocks
+// an SM: with one (134 registers) the update took 23.4 us there, 17.7 with two; P = R + Psi P 10.0.
+// Through shared memory, as k_cg_rows, 21.6 and 12.4.
 template <typename V, bool UPDATE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
     k_cg_rows32(long long nfeat, int n, const double* small, const V* __restrict__ P,
                 const V* __restrict__ KPm, V* __restrict__ R, double* __restrict__ X,
                 V* __restrict__ Pout, const uint32_t* __restrict__ done) {
