@@ -87,18 +87,21 @@ __device__ __forceinline__ float fused_add(float x, float w, float a) { return f
 // left to the compiler, this loop's FP64 form rounded a weighted product first, which moved the
 // link matrices of chains with weighted features by up to 1e-6 (hyper_ordered.cu); choosing between
 // that and an addition cost 3 to 6 % of a link update.
-//   What bounds it: for short tasks the latency of index and gather, for the others the gathers
-//   from L2 (256 bytes per entry at 32 components).  U = 16: with 8 a link update of 5,003 x 4,099
-//   at 16 components takes 3.34 ms for 3.06, with 32 one of 20,000 x 32,768 at 32 19.9 ms for 16.7.
+//   What bounds it: for few tasks the latency of index and gather, for many the instructions and the
+//   gathers from L2 (256 bytes per entry at 32 components).  16 gathers in flight, and 8 where there
+//   are 16,384 tasks or more, whose registers leave room for half as many warps again: link updates with
+//   16 and 8, in us: 5,003 x 4,099 at K = 16 2,025 and 2,138; 3,000 x 8,000 at K = 20 2,900 and 3,113;
+//   20,000 x 32,768 at K = 32 6,873 and 6,642; 100,000 x 300, weighted, 1,922 and 1,840 (1,899 with
+//   four gathers and no chunks).  32: 3.19 ms for 3.06 and 19.9 for 16.7 at the first and third.
 //   (Several lane groups per entry, each summing
 //   every second or fourth entry, are faster, but sum in another order: hyper_ordered.cu.)
-template <typename V, int NRP>
+template <typename V, int NRP, int GATHERS>
 __global__ void __launch_bounds__(256)
     k_spmm_split(const DevCsr A, const V* __restrict__ src, int sstride, V* __restrict__ dst,
                  int dstride, int ncomp, const V* __restrict__ add, int astride, double reg,
                  const double* __restrict__ reg_dev, const uint32_t* __restrict__ done) {
   if (done && *done) return;
-  constexpr int C = NRP / 32, U = 16 / C;
+  constexpr int C = NRP / 32, U = GATHERS / C;
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (blockDim.x >> 5);
   const bool weighted = sizeof(V) == 8 ? A.val != nullptr : A.valf != nullptr;
@@ -896,7 +899,8 @@ void spmm_t(const DevCsr& A, const V* src, int sstride, V* dst, int dstride, int
             const V* add, int astride, double reg, const double* reg_dev, cudaStream_t s,
             const uint32_t* done = nullptr) {
   if (A.tasks) {
-    k_spmm_split<V, NRP><<<grid_for(A.ntasks, 8), 256, 0, s>>>(
+    const auto kern = A.ntasks >= 16384 ? k_spmm_split<V, NRP, 8> : k_spmm_split<V, NRP, 16>;
+    kern<<<grid_for(A.ntasks, 8), 256, 0, s>>>(
         A, src, sstride, dst, dstride, ncomp, add, astride, reg, reg_dev, done);
     MG_CUDA(cudaGetLastError());
     return;

@@ -98,3 +98,22 @@ def test_univariate_wide_levels(nshort, binary):
         assert relerr(s.uhat(0), m.uhat(0)) < 1e-9
         assert relerr(s.lambda_beta_univariate(0), m.lambda_beta_one(0)) < 1e-9
     s.close()
+
+
+@pytest.mark.parametrize("K", [1, 16, 32, 33, 64])
+@pytest.mark.parametrize("binary", [True, False])
+def test_spmm_many_short_rows(K, binary):
+    # 16,384 tasks and more take 8 gathers at a time: rows of F at the edges of these; a row's sum of n
+    # <= 40 products is off by at most n n eps times the largest product
+    rng = np.random.default_rng(K + binary)
+    lengths = ((0, 1, 2, 3, 4, 7, 8, 9, 15, 16, 17, 31, 32, 33, 40) * 1134)[:17001]
+    F = side_of_lengths(rng, 700, lengths, binary).T.tocoo()
+    s = gpu_sampler(small_uniform(seed=1, nrow=17001, ncol=60, nobs=40000), K, 1.5, 5, init=False)
+    s.set_side(0, F.row, F.col, None if binary else F.data, F.shape, 50.0, 1e-6)
+    s.init()
+    s.set_latents(0, rng.normal(scale=0.5, size=(17001, K)))
+    s.update_prior(0, 2)
+    beta = s.beta(0)
+    bound = 40 * 40 * 2.3e-16 * np.abs(F.data).max() * np.abs(beta).max()
+    assert np.abs(s.uhat(0) - F @ beta).max() < bound
+    s.close()
