@@ -68,7 +68,7 @@ __device__ __forceinline__ double ordered_sums(const T* __restrict__ U,
 //   at K = 32, on one SM per block.  (4 x 4 tiles of fma over rows staged in shared memory: 126 us on
 //   average for 64 problems of up to 4,000 rows.)
 template <typename T>
-__device__ __forceinline__ void stats32_rows(const T* __restrict__ U,
+__device__ __forceinline__ void ordered_stats(const T* __restrict__ U,
                                              const double* __restrict__ Uhat, long long r0,
                                              long long r1, int K, int stride, int uhat_stride,
                                              double* __restrict__ out) {
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kStatThreads)
                  int stride, int uhat_stride, long long rows_per_block,
                  double* __restrict__ partials) {
   const long long r0 = (long long)blockIdx.x * rows_per_block;
-  stats32_rows(U, Uhat, r0, min(N, r0 + rows_per_block), K, stride, uhat_stride,
+  ordered_stats(U, Uhat, r0, min(N, r0 + rows_per_block), K, stride, uhat_stride,
                partials + (size_t)blockIdx.x * (K + K * K));
 }
 
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kStatThreads)
     k_stats_batch(const float* __restrict__ U, const int* __restrict__ row0,
                   const int* __restrict__ Kp, double* __restrict__ partials) {
   const int p = blockIdx.x;
-  stats32_rows<float>(U, nullptr, row0[p], row0[p + 1], Kp[p], 32, 0,
+  ordered_stats<float>(U, nullptr, row0[p], row0[p + 1], Kp[p], 32, 0,
                       partials + (size_t)p * (32 + 32 * 32));
 }
 

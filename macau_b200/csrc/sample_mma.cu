@@ -10,7 +10,7 @@
 // four entries at K = 32 where 4 x 8 register tiles on DFMA formed all 1,024 products per entry
 // from six 16-byte shared-memory loads a lane.
 //
-// What bounds it: the FP64 pipe (an m8n8k4 takes 16 cycles of a sub-partition, measured, 34
+// What bounds it: the FP64 pipe (an m8n8k4 takes 16 cycles of a sub-partition, measured, 36.9
 // TFLOP/s per GPU) for long rows, and the latency of the row finish for short ones; 16 warps per
 // SM at 128 registers keep four rows per sub-partition in flight, and the gathers run three
 // steps (12 entries) ahead of the products.  138,000 x 27,000 with 18M entries at K = 32: both
