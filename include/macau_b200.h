@@ -128,7 +128,8 @@ int mg_init(mg_ctx* ctx);
 
 /* One iteration `iter` of MacauX::run (macau.cpp:110-147): sample mode 0, sample mode 1,
  * update prior 0, update prior 1, evaluate the test set with n = iter < burnin ? 0 : iter-burnin
- * (when eval != 0).  Replays a captured CUDA graph when the sweep has no host-side decision. */
+ * (when eval != 0).  Replays a captured CUDA graph when the sweep has no host-side
+ * decision (built with the second sweep). */
 int mg_sweep(mg_ctx* ctx, int iter, int eval);
 
 /* `count` consecutive sweeps starting at `first_iter` without returning to the caller in

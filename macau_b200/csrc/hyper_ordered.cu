@@ -12,6 +12,9 @@
 //   * A batch runs many mixed-precision chains for many sweeps, each rounding Lambda to FP32 and its
 //     latents to BF16: of 64 problems over 40 sweeps about one met a Lambda whose last FP64 bit
 //     decided its FP32 rounding, and its latents were then 0.04 apart.
+//   * A single mixed chain without a link takes those kernels all the same: the same bit costs it its
+//     recorded course about once in 6,000 sweeps (6 of 28 chains at K = 8 to 64 within 1,500 sweeps),
+//     not in every call.  FP64 chains without a link differ by rounding alone.
 //   What bounds them: beside a solve nothing that matters (the draw takes 36 us on one SM at K <= 32);
 // in a batch the longest problem's statistics.
 #include "common.cuh"
@@ -347,7 +350,8 @@ __device__ bool block_chol(double* A, int K) {
 // 314-336) step by step, each matrix element one chain of fma over its index: T_c by the factor of X
 // and two substitutions per column, its factor L, Lambda = L (c^T c) L^T, the mean through the
 // factor of kappa_c Lambda.  The matrices are in shared memory.
-//   What bounds it: the substitutions, a thread per column.
+//   What bounds it: the substitutions, a thread per column: 364 us at K = 64 (0.81 ms with the matrices in
+// global memory), beside a solve of 3 ms and more.
 __global__ void __launch_bounds__(256)
     k_link_wishart_wide(const double* __restrict__ stats, long long N, int K,
                         const double* __restrict__ mu0, double kappa, const double* __restrict__ T0,

@@ -7,7 +7,7 @@
 // per CTA).  The best pair depends on the row-length histogram, K and the SM count, so the
 // context times every candidate on its own data and keeps the fastest.
 //
-// Choices are cached per process by (sampler kind, K, SM count, rows, entries, log2 histogram of
+// Choices are cached per process by (row kernel, K, SM count, rows, entries, log2 histogram of
 // the row lengths), and, when the environment variable MACAU_B200_TUNE_CACHE names a file, in
 // that file too (one "key value" line per choice), so later contexts on the same data skip the
 // timing.
